@@ -1,312 +1,620 @@
-// Edge-dominant gradient NCC (src/fvr/cone_beam_fvr.py:71-112), sm_100a.
+// Image-similarity kernels of the registration loss, sm_100a: the
+// edge-dominant gradient NCC (src/fvr/cone_beam_fvr.py:71-112) and the
+// zero-mean image NCC it is mixed with
+// (experiments/exp30_gpu_multistart_registration.py:120-134).
 //
 // For each image pair (pred a, target b) and channel: Sobel x / y responses
 // (zero padding) on the interior [crop, H-crop) x [crop, W-crop), their NCC
 // per direction, averaged; optionally the same on 3x3 box-blurred images
-// (zero padding, divisor 9) weighted by w.  Everything is expressed through
-// five moments per (direction, scale) -- S_u, S_v, S_uu, S_vv, S_uv -- so the
-// forward pass is one tiled stencil + reduction and the adjoint is one tiled
-// stencil that applies the transposed Sobel and box filters in shared memory.
+// (zero padding, divisor 9) weighted by w; optionally the NCC of the whole
+// images.  Everything is expressed through five moments per combination
+// -- S_u, S_v, S_uu, S_vv, S_uv -- so the forward pass is one stencil +
+// reduction pass over the images and the adjoint is one stencil pass that
+// applies the transposed Sobel and box filters to closed-form fields.
+//
+// Both passes march: a warp owns a strip of 64 columns (two per lane, the
+// outer lanes are halo) and walks down kEdgeRows rows, keeping the last rows'
+// horizontal sums in registers; horizontal neighbours come from the lane's
+// other column or one shuffle.  The pair (a, b) goes through the filters as
+// one packed f32x2 value.  No shared memory and no barriers.  Measured on 64
+// candidates x two views of 256 x 256 (kernel times): an earlier form with
+// 32 x 32 tiles in shared memory took 2 x 43 us (moments), 2 x 119 us
+// (finalize, one CTA for all pairs) and 2 x 91 us (adjoint), the image NCC
+// another 350 us as separate tensor operations; now 50, 9 and 72 us for both
+// views and both similarities.  The moments and adjoint passes are bound by
+// issued instructions (54 % issue active at 16 warps per SM; the images alone
+// take 5 and 10 us at the copy bandwidth).
 #include "fvr_common.cuh"
 
 namespace fvr {
 
-constexpr int kEdgeTile = 32;      // output tile edge
-constexpr int kEdgeThreads = 256;  // 8 rows of 32
-constexpr int kEdgeMom = 5;        // S_u, S_v, S_uu, S_vv, S_uv
-constexpr int kEdgeCombos = 4;     // fine x, fine y, coarse x, coarse y
+constexpr int kEdgeRows = 32;     // rows a warp produces
+constexpr int kEdgeWarps = 4;     // warps (independent strips) per CTA
+constexpr int kEdgeMom = 5;       // S_u, S_v, S_uu, S_vv, S_uv
+constexpr int kEdgeCombos = 4;    // fine x, fine y, coarse x, coarse y
+constexpr int kEdgeNM = (kEdgeCombos + 1) * kEdgeMom;  // and the whole images
+constexpr int kEdgeMaxViews = 4;
+constexpr int kMomCols = 60;      // columns a warp produces: 64 less two halo columns a side
+constexpr int kGradCols = 56;     // ... four halo columns a side
 
 struct EdgeArgs {
-  const float* a;  // [B][C][H][W]
-  const float* b;  // [Bt][C][H][W], Bt = 1 (broadcast) or B
-  int B, Bt, Cch, H, W, crop;
-  int coarse;       // 1: blurred scale enabled
-  int tiles_x, tiles_y;
+  const float* a[kEdgeMaxViews];  // per view [B][C][H][W]
+  const float* b[kEdgeMaxViews];  // [Bt][C][H][W], Bt = 1 (broadcast) or B
+  int Bt[kEdgeMaxViews];
+  float* grad[kEdgeMaxViews];     // adjoint: [B][C][H][W]
+  int views, B, Cch, H, W, crop;
+  int coarse;        // 1: blurred scale enabled
+  int vec;           // 1: every row starts on an 8-byte boundary
+  double base, ce, cn;  // out = base + sum over views (ce edge + cn ncc)
+  float w;           // weight of the blurred scale
 };
 
-// Sobel responses at smem position (i, j) of a tile `t` with row pitch p:
-// gx = sum kx * t, kx = [-1 0 1; -2 0 2; -1 0 1]; gy with ky = kx^T.
-__device__ __forceinline__ void sobel(const float* t, int p, int i, int j, float& gx, float& gy) {
-  const float* r0 = t + (i - 1) * p + j;
-  const float* r1 = t + i * p + j;
-  const float* r2 = t + (i + 1) * p + j;
-  gx = (r0[1] - r0[-1]) + 2.f * (r1[1] - r1[-1]) + (r2[1] - r2[-1]);
-  gy = (r2[-1] + 2.f * r2[0] + r2[1]) - (r0[-1] + 2.f * r0[0] + r0[1]);
+struct EdgeJob {
+  const float *a, *b;
+  int view, bi, ch;
+  int rb, re;        // rows [rb, re) of this warp
+  int strip;
+};
+
+// Pair p = (view, item, channel); job j of the pair = (row chunk, strip).
+__device__ __forceinline__ EdgeJob edge_job(const EdgeArgs& e, int64_t pair, int job, int strips) {
+  EdgeJob j;
+  j.view = static_cast<int>(pair / (e.B * e.Cch));
+  const int r = static_cast<int>(pair - static_cast<int64_t>(j.view) * e.B * e.Cch);
+  j.bi = r / e.Cch;
+  j.ch = r - j.bi * e.Cch;
+  const int64_t plane = static_cast<int64_t>(e.H) * e.W;
+  j.a = e.a[j.view] + (static_cast<int64_t>(j.bi) * e.Cch + j.ch) * plane;
+  j.b = e.b[j.view] + (static_cast<int64_t>(e.Bt[j.view] == 1 ? 0 : j.bi) * e.Cch + j.ch) * plane;
+  const int chunk = job / strips;
+  j.strip = job - chunk * strips;
+  j.rb = chunk * kEdgeRows;
+  j.re = min(e.H, j.rb + kEdgeRows);
+  return j;
 }
 
-// Zero-padded image window [r0, r0+n) x [c0, c0+n) into smem (pitch n).
-__device__ __forceinline__ void load_window(const float* img, int H, int W, int r0, int c0, int n, float* s) {
-  for (int k = threadIdx.x; k < n * n; k += blockDim.x) {
-    const int i = k / n, j = k - i * n;
-    const int r = r0 + i, c = c0 + j;
-    s[k] = (r >= 0 && r < H && c >= 0 && c < W) ? __ldg(img + static_cast<int64_t>(r) * W + c) : 0.f;
-  }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+__device__ __forceinline__ float2 twice_plus(float2 a, float2 b) { return __ffma2_rn(a, make_float2(2.f, 2.f), b); }
+__device__ __forceinline__ float2 shfl_up2(float2 v) {
+  return make_float2(__shfl_up_sync(0xffffffffu, v.x, 1), __shfl_up_sync(0xffffffffu, v.y, 1));
+}
+__device__ __forceinline__ float2 shfl_down2(float2 v) {
+  return make_float2(__shfl_down_sync(0xffffffffu, v.x, 1), __shfl_down_sync(0xffffffffu, v.y, 1));
 }
 
-// Box-blurred window (pitch n) from a zero-padded window (pitch n + 2) one
-// pixel wider on each side; blurred pixels outside the image are zero.
-__device__ __forceinline__ void blur_window(const float* src, int H, int W, int r0, int c0, int n, float* dst) {
-  const int p = n + 2;
-  for (int k = threadIdx.x; k < n * n; k += blockDim.x) {
-    const int i = k / n, j = k - i * n;
-    const int r = r0 + i, c = c0 + j;
-    float v = 0.f;
-    if (r >= 0 && r < H && c >= 0 && c < W) {
-      const float* q = src + i * p + j;
-      v = (q[0] + q[1] + q[2] + q[p] + q[p + 1] + q[p + 2] + q[2 * p] + q[2 * p + 1] + q[2 * p + 2]) * (1.f / 9.f);
+// Walks down the rows of both images at columns c, c + 1, as (a, b) pairs,
+// zero outside; two rows are in flight ahead of the one handed out.
+struct RowReader {
+  const float *a, *b;  // next row to load, at column c
+  int r, H, W, c;
+  bool vec, in0, in1;
+  float2 n0[2], n1[2];
+
+  __device__ __forceinline__ void load(float2 (&x)[2]) {
+    x[0] = x[1] = make_float2(0.f, 0.f);
+    if (r >= 0 && r < H) {
+      if (vec) {  // W and c even: both columns are inside or neither
+        if (in0) {
+          const float2 u = __ldg(reinterpret_cast<const float2*>(a));
+          const float2 v = __ldg(reinterpret_cast<const float2*>(b));
+          x[0] = make_float2(u.x, v.x);
+          x[1] = make_float2(u.y, v.y);
+        }
+      } else {
+        if (in0) x[0] = make_float2(__ldg(a), __ldg(b));
+        if (in1) x[1] = make_float2(__ldg(a + 1), __ldg(b + 1));
+      }
     }
-    dst[k] = v;
+    ++r;
+    a += W;
+    b += W;
   }
+  __device__ __forceinline__ void init(const EdgeArgs& e, const float* ia, const float* ib, int row, int col) {
+    r = row;
+    H = e.H;
+    W = e.W;
+    c = col;
+    vec = e.vec != 0;
+    in0 = c >= 0 && c < W;
+    in1 = c + 1 >= 0 && c + 1 < W;
+    const int64_t o = static_cast<int64_t>(row) * W + col;
+    a = ia + o;  // read only where the row and the column are inside
+    b = ib + o;
+    load(n0);
+    load(n1);
+  }
+  __device__ __forceinline__ void next(float2 (&x)[2]) {
+    x[0] = n0[0];
+    x[1] = n0[1];
+    n0[0] = n1[0];
+    n0[1] = n1[1];
+    load(n1);
+  }
+};
+
+// Horizontal parts of the filters at the lane's two columns: d = right - left
+// (Sobel x), s = left + 2 mid + right (Sobel y), h = left + mid + right (box).
+// The outermost column on each side of the warp comes out wrong (halo).
+__device__ __forceinline__ void row_parts(const float2 (&x)[2], float2 (&d)[2], float2 (&s)[2], float2 (&h)[2]) {
+  const float2 l = shfl_up2(x[1]), r = shfl_down2(x[0]);
+  d[0] = sub2(x[1], l);
+  d[1] = sub2(r, x[0]);
+  const float2 t0 = add2(x[1], l), t1 = add2(r, x[0]);
+  s[0] = twice_plus(x[0], t0);
+  s[1] = twice_plus(x[1], t1);
+  h[0] = add2(t0, x[0]);
+  h[1] = add2(t1, x[1]);
 }
 
-// Moments of one 32 x 32 tile of the interior -> partial[pair][tile][20] (fp64).
-__global__ void __launch_bounds__(kEdgeThreads) edge_moments_kernel(EdgeArgs a, double* __restrict__ partial) {
-  constexpr int T = kEdgeTile;
-  constexpr int NA = T + 4, NB = T + 2;
-  __shared__ float sa[NA * NA], sb[NA * NA], ba[NB * NB], bb[NB * NB];
-  __shared__ double red[kEdgeCombos * kEdgeMom * (kEdgeThreads / 32)];
-  const int pair = blockIdx.z;
-  const int bi = pair / a.Cch, ch = pair - bi * a.Cch;
-  const int bt = a.Bt == 1 ? 0 : bi;
-  const int64_t plane = static_cast<int64_t>(a.H) * a.W;
-  const float* img_a = a.a + (static_cast<int64_t>(bi) * a.Cch + ch) * plane;
-  const float* img_b = a.b + (static_cast<int64_t>(bt) * a.Cch + ch) * plane;
-  const int r0 = a.crop + blockIdx.y * T, c0 = a.crop + blockIdx.x * T;
-  const int r_end = a.H - a.crop, c_end = a.W - a.crop;
-  load_window(img_a, a.H, a.W, r0 - 2, c0 - 2, NA, sa);
-  load_window(img_b, a.H, a.W, r0 - 2, c0 - 2, NA, sb);
-  __syncthreads();
-  if (a.coarse) {
-    blur_window(sa, a.H, a.W, r0 - 1, c0 - 1, NB, ba);
-    blur_window(sb, a.H, a.W, r0 - 1, c0 - 1, NB, bb);
-    __syncthreads();
-  }
-  float acc[kEdgeCombos * kEdgeMom];
+// The last two rows' horizontal parts of the images and of the blurred
+// images.  step() takes row t and gives the Sobel responses g of row t - 1
+// and, with COARSE, those of the blurred images, gb, of row t - 2.
+template <bool COARSE>
+struct EdgeMarch {
+  float2 d0[2], d1[2], s0[2], s1[2], h0[2], h1[2];      // rows t - 2, t - 1
+  float2 bd0[2], bd1[2], bs0[2], bs1[2];                // blurred rows t - 3, t - 2
+
+  __device__ __forceinline__ void init() {
 #pragma unroll
-  for (int m = 0; m < kEdgeCombos * kEdgeMom; ++m) acc[m] = 0.f;
-  const int tj = threadIdx.x & 31;
-  for (int ti = threadIdx.x >> 5; ti < T; ti += kEdgeThreads / 32) {
-    const int r = r0 + ti, c = c0 + tj;
-    if (r >= r_end || c >= c_end) continue;
-    float u[4], v[4];
-    sobel(sa, NA, ti + 2, tj + 2, u[0], u[1]);
-    sobel(sb, NA, ti + 2, tj + 2, v[0], v[1]);
-    if (a.coarse) {
-      sobel(ba, NB, ti + 1, tj + 1, u[2], u[3]);
-      sobel(bb, NB, ti + 1, tj + 1, v[2], v[3]);
-    } else {
-      u[2] = u[3] = v[2] = v[3] = 0.f;
+    for (int j = 0; j < 2; ++j)
+      d0[j] = d1[j] = s0[j] = s1[j] = h0[j] = h1[j] = bd0[j] = bd1[j] = bs0[j] = bs1[j] = make_float2(0.f, 0.f);
+  }
+
+  // in_row: row t - 1 lies in the image; in_col[j]: column j does.
+  __device__ __forceinline__ void step(const float2 (&x)[2], bool in_row, const bool (&in_col)[2], float2 (&gx)[2],
+                                       float2 (&gy)[2], float2 (&gbx)[2], float2 (&gby)[2]) {
+    float2 d[2], s[2], h[2];
+    row_parts(x, d, s, h);
+    float2 bl[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      gx[j] = twice_plus(d1[j], add2(d0[j], d[j]));
+      gy[j] = sub2(s[j], s0[j]);
+      d0[j] = d1[j];
+      d1[j] = d[j];
+      s0[j] = s1[j];
+      s1[j] = s[j];
+      if (COARSE) {
+        const float2 v = __fmul2_rn(add2(add2(h0[j], h1[j]), h[j]), make_float2(1.f / 9.f, 1.f / 9.f));
+        bl[j] = in_row && in_col[j] ? v : make_float2(0.f, 0.f);
+        h0[j] = h1[j];
+        h1[j] = h[j];
+      }
     }
+    if (COARSE) {
+      float2 bd[2], bs[2], unused[2];
+      row_parts(bl, bd, bs, unused);
 #pragma unroll
-    for (int k = 0; k < kEdgeCombos; ++k) {
-      float* m = acc + k * kEdgeMom;
-      m[0] += u[k];
-      m[1] += v[k];
-      m[2] = fmaf(u[k], u[k], m[2]);
-      m[3] = fmaf(v[k], v[k], m[3]);
-      m[4] = fmaf(u[k], v[k], m[4]);
+      for (int j = 0; j < 2; ++j) {
+        gbx[j] = twice_plus(bd1[j], add2(bd0[j], bd[j]));
+        gby[j] = sub2(bs[j], bs0[j]);
+        bd0[j] = bd1[j];
+        bd1[j] = bd[j];
+        bs0[j] = bs1[j];
+        bs1[j] = bs[j];
+      }
     }
   }
-  // fp64 cross-lane / cross-warp sums
-  constexpr int NM = kEdgeCombos * kEdgeMom;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = kEdgeThreads / 32;
+};
+
+// Sums 32 per-lane values over the warp; lane l returns the total of v[l].
+// Each step halves the values a lane carries: 31 exchanges instead of 160.
+__device__ __forceinline__ double warp_sum_each(double (&v)[32]) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int m = 0; m < NM; ++m) {
-    const double s = warp_sum(static_cast<double>(acc[m]));
-    if (lane == 0) red[m * nw + wid] = s;
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const double send = up ? v[i] : v[i + o];
+      const double keep = up ? v[i + o] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
   }
-  __syncthreads();
-  if (threadIdx.x < NM) {
-    double s = 0.0;
-    for (int w = 0; w < nw; ++w) s += red[threadIdx.x * nw + w];
-    const int tile = blockIdx.y * a.tiles_x + blockIdx.x;
-    partial[(static_cast<int64_t>(pair) * a.tiles_x * a.tiles_y + tile) * NM + threadIdx.x] = s;
-  }
+  return v[0];
 }
 
-// Per pair: tile sums -> stats[pair][20]; per batch item: the loss value
-// (1 - w) * mean_c 0.5 (ncc_fx + ncc_fy) + w * (coarse), then the batch mean.
+// Moments of one strip of rows -> partial[pair][job][kEdgeNM] (fp64).  Products
+// are summed per lane in f32 (at most 2 x kEdgeRows terms), then in fp64.  The
+// whole images' mean may be large against their spread, so those moments are
+// taken about a value of the lane's own first row and moved to zero in fp64.
+template <bool COARSE, bool NCC>
+__global__ void __launch_bounds__(32 * kEdgeWarps, 4) edge_moments_kernel(EdgeArgs e, int strips, int jobs, int groups,
+                                                                       double* __restrict__ partial) {
+  const int64_t pair = blockIdx.x / groups;
+  const int job = static_cast<int>(blockIdx.x - pair * groups) * kEdgeWarps + (threadIdx.x >> 5);
+  if (job >= jobs) return;
+  const int lane = threadIdx.x & 31;
+  const EdgeJob jb = edge_job(e, pair, job, strips);
+  const int c = jb.strip * kMomCols - 2 + 2 * lane;
+  const bool own = lane >= 1 && lane <= 30;
+  bool in_img[2], in_edge[2], mine[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    in_img[j] = c + j >= 0 && c + j < e.W;
+    mine[j] = own && in_img[j];
+    in_edge[j] = own && c + j >= e.crop && c + j < e.W - e.crop;
+  }
+  float2 m1[kEdgeCombos], m2[kEdgeCombos];  // (S_u, S_v), (S_uu, S_vv)
+  float m3[kEdgeCombos];                    // S_uv
+#pragma unroll
+  for (int k = 0; k < kEdgeCombos; ++k) {
+    m1[k] = m2[k] = make_float2(0.f, 0.f);
+    m3[k] = 0.f;
+  }
+  auto add = [&](int k, float2 g) {
+    m1[k] = add2(m1[k], g);
+    m2[k] = __ffma2_rn(g, g, m2[k]);
+    m3[k] = fmaf(g.x, g.y, m3[k]);
+  };
+  float2 pivot = make_float2(0.f, 0.f), i1 = pivot, i2 = pivot;  // whole images: sums of (x - pivot), squares
+  float i3 = 0.f;
+  const int lo = max(jb.rb, e.crop), hi = min(jb.re, e.H - e.crop);  // interior rows of this job
+  EdgeMarch<COARSE> march;
+  march.init();
+  const int t_end = jb.re + (COARSE ? 2 : 1);
+  RowReader rows;
+  rows.init(e, jb.a, jb.b, jb.rb - 2, c);
+#pragma unroll 2
+  for (int t = jb.rb - 2; t < t_end; ++t) {
+    float2 x[2];
+    rows.next(x);
+    if (NCC && t >= jb.rb && t < jb.re) {
+      if (t == jb.rb) pivot = make_float2(0.5f * (x[0].x + x[1].x), 0.5f * (x[0].y + x[1].y));
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        if (mine[j]) {
+          const float2 u = sub2(x[j], pivot);
+          i1 = add2(i1, u);
+          i2 = __ffma2_rn(u, u, i2);
+          i3 = fmaf(u.x, u.y, i3);
+        }
+    }
+    float2 gx[2], gy[2], gbx[2], gby[2];
+    march.step(x, t - 1 >= 0 && t - 1 < e.H, in_img, gx, gy, gbx, gby);
+    if (t - 1 >= lo && t - 1 < hi) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        if (in_edge[j]) {
+          add(0, gx[j]);
+          add(1, gy[j]);
+        }
+    }
+    if (COARSE && t - 2 >= lo && t - 2 < hi) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        if (in_edge[j]) {
+          add(2, gbx[j]);
+          add(3, gby[j]);
+        }
+    }
+  }
+  double v[32];
+#pragma unroll
+  for (int k = 0; k < 32; ++k) v[k] = 0.0;
+#pragma unroll
+  for (int k = 0; k < kEdgeCombos; ++k) {
+    v[k * kEdgeMom] = m1[k].x;
+    v[k * kEdgeMom + 1] = m1[k].y;
+    v[k * kEdgeMom + 2] = m2[k].x;
+    v[k * kEdgeMom + 3] = m2[k].y;
+    v[k * kEdgeMom + 4] = m3[k];
+  }
+  if (NCC) {
+    const double n = static_cast<double>((mine[0] ? 1 : 0) + (mine[1] ? 1 : 0)) * (jb.re - jb.rb);
+    const double pu = pivot.x, pv = pivot.y, su = i1.x, sv = i1.y;
+    double* im = v + kEdgeCombos * kEdgeMom;
+    im[0] = su + n * pu;
+    im[1] = sv + n * pv;
+    im[2] = i2.x + pu * (2.0 * su + n * pu);
+    im[3] = i2.y + pv * (2.0 * sv + n * pv);
+    im[4] = i3 + pu * sv + pv * su + n * pu * pv;
+  }
+  const double s = warp_sum_each(v);
+  if (lane < kEdgeNM) partial[(pair * jobs + job) * kEdgeNM + lane] = s;
+}
+
+// NCC of one combination from its moments over n pixels, denominator
+// sqrt(max(S_uu S_vv, 1e-12)) of the centred sums.
 __device__ __forceinline__ double edge_ncc(const double* m, double n) {
   const double suu = m[2] - m[0] * m[0] / n, svv = m[3] - m[1] * m[1] / n, suv = m[4] - m[0] * m[1] / n;
   return suv / sqrt(fmax(suu * svv, 1e-12));
 }
 
-__global__ void edge_finalize_kernel(EdgeArgs a, const double* __restrict__ partial, float w,
-                                     double* __restrict__ stats, float* __restrict__ out, int reduction_mean) {
-  constexpr int NM = kEdgeCombos * kEdgeMom;
-  const int tiles = a.tiles_x * a.tiles_y;
-  const int npair = a.B * a.Cch;
-  for (int k = threadIdx.x; k < npair * NM; k += blockDim.x) {
-    const int pair = k / NM, m = k - pair * NM;
-    double s = 0.0;
-    for (int t = 0; t < tiles; ++t) s += partial[(static_cast<int64_t>(pair) * tiles + t) * NM + m];
-    stats[k] = s;
-  }
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  const double n = static_cast<double>(a.H - 2 * a.crop) * static_cast<double>(a.W - 2 * a.crop);
-  double total = 0.0;
-  for (int bi = 0; bi < a.B; ++bi) {
-    double fine = 0.0, coarse = 0.0;
-    for (int ch = 0; ch < a.Cch; ++ch) {
-      const double* st = stats + static_cast<int64_t>(bi * a.Cch + ch) * NM;
-      fine += 0.5 * (edge_ncc(st, n) + edge_ncc(st + kEdgeMom, n));
-      if (a.coarse) coarse += 0.5 * (edge_ncc(st + 2 * kEdgeMom, n) + edge_ncc(st + 3 * kEdgeMom, n));
+// One CTA per batch item: strip sums -> stats[pair][kEdgeNM] in job order,
+// then out = base + sum over views (ce edge + cn ncc), edge = the channel mean
+// of (1 - w) fine + w coarse.
+__global__ void __launch_bounds__(128) edge_finalize_kernel(EdgeArgs e, int jobs, const double* __restrict__ partial,
+                                                            double* __restrict__ stats, float* __restrict__ out,
+                                                            double* __restrict__ value) {
+  __shared__ double part[4][kEdgeNM];
+  const int bi = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const double n = static_cast<double>(e.H - 2 * e.crop) * static_cast<double>(e.W - 2 * e.crop);
+  const double n_img = static_cast<double>(e.H) * static_cast<double>(e.W);
+  double val = e.base;
+  for (int v = 0; v < e.views; ++v) {
+    double edge = 0.0, ncc = 0.0;
+    for (int ch = 0; ch < e.Cch; ++ch) {
+      const int64_t pair = (static_cast<int64_t>(v) * e.B + bi) * e.Cch + ch;
+      if (lane < kEdgeNM) {
+        double s = 0.0;
+        for (int t = wid; t < jobs; t += 4) s += partial[(pair * jobs + t) * kEdgeNM + lane];
+        part[wid][lane] = s;
+      }
+      __syncthreads();
+      if (threadIdx.x < kEdgeNM) {
+        const double s = ((part[0][lane] + part[1][lane]) + part[2][lane]) + part[3][lane];
+        part[0][lane] = s;
+        stats[pair * kEdgeNM + lane] = s;
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        const double* st = part[0];
+        const double fine = 0.5 * (edge_ncc(st, n) + edge_ncc(st + kEdgeMom, n));
+        edge += e.coarse ? (1.0 - e.w) * fine +
+                               e.w * 0.5 * (edge_ncc(st + 2 * kEdgeMom, n) + edge_ncc(st + 3 * kEdgeMom, n))
+                         : fine;
+        if (e.cn != 0.0) ncc += edge_ncc(st + kEdgeCombos * kEdgeMom, n_img);
+      }
+      __syncthreads();
     }
-    fine /= a.Cch;
-    coarse /= a.Cch;
-    const double val = a.coarse ? (1.0 - w) * fine + w * coarse : fine;
-    if (!reduction_mean) out[bi] = static_cast<float>(val);
-    total += val;
+    val += e.ce * edge / e.Cch + e.cn * ncc / e.Cch;
   }
-  if (reduction_mean) out[0] = static_cast<float>(total / a.B);
+  if (threadIdx.x == 0) {
+    if (out) out[bi] = static_cast<float>(val);
+    if (value) value[bi] = val;
+  }
 }
 
-// d value / d pred (or d target with wrt_b) for one 32 x 32 output tile of the
-// full image.  Interior gradient fields g_k(q) = alpha_k (v_k(q) - mean v_k)
-// + beta_k (u_k(q) - mean u_k) on the interior, transposed Sobel, and for the
-// blurred scale the transposed box filter.
-__global__ void __launch_bounds__(kEdgeThreads) edge_grad_kernel(EdgeArgs a, const double* __restrict__ stats,
-                                                                 float w, const float* __restrict__ g, int g_stride,
-                                                                 int reduction_mean, int wrt_b,
-                                                                 float* __restrict__ grad) {
-  constexpr int T = kEdgeTile;
-  constexpr int N4 = T + 8, N3 = T + 6, N2 = T + 4, N1 = T + 2;
-  extern __shared__ float smem[];
-  float* sa = smem;            // N4^2 : this image (differentiated), halo 4
-  float* sb = sa + N4 * N4;    // N4^2 : the other image
-  float* ba = sb + N4 * N4;    // N3^2 : blurred, halo 3
-  float* bb = ba + N3 * N3;    // N3^2
-  float* gfx = bb + N3 * N3;   // N1^2 : fine-scale fields, halo 1
-  float* gfy = gfx + N1 * N1;  // N1^2
-  float* gcx = gfy + N1 * N1;  // N2^2 : coarse-scale fields, halo 2
-  float* gcy = gcx + N2 * N2;  // N2^2
-  float* gbl = gcy + N2 * N2;  // N1^2 : gradient w.r.t. the blurred image, halo 1
-  __shared__ float coef[kEdgeCombos][4];  // alpha, beta, mean u, mean v
-  const int pair = blockIdx.z;
-  const int bi = pair / a.Cch, ch = pair - bi * a.Cch;
-  const int bt = a.Bt == 1 ? 0 : bi;
-  const int64_t plane = static_cast<int64_t>(a.H) * a.W;
-  const float* img_a = a.a + (static_cast<int64_t>(bi) * a.Cch + ch) * plane;
-  const float* img_b = a.b + (static_cast<int64_t>(bt) * a.Cch + ch) * plane;
-  if (wrt_b) {
-    const float* t = img_a;
-    img_a = img_b;
-    img_b = t;
-  }
-  const int r0 = blockIdx.y * T, c0 = blockIdx.x * T;
-  if (threadIdx.x < kEdgeCombos) {
+// out[0] = mean of value[B], in a fixed order.
+__global__ void edge_mean_kernel(const double* __restrict__ value, int B, float* __restrict__ out) {
+  double s = 0.0;
+  for (int i = threadIdx.x; i < B; i += 32) s += value[i];
+  s = warp_sum(s);
+  if (threadIdx.x == 0) out[0] = static_cast<float>(s / B);
+}
+
+// d out / d a (or d b with swap) of one strip of rows.  Interior gradient
+// fields g_k(q) = alpha_k (v_k(q) - mean v_k) + beta_k (u_k(q) - mean u_k) on
+// the interior, transposed Sobel, and for the blurred scale the transposed box
+// filter; the fine and the coarse fields go through the transposed Sobel
+// together as one f32x2 value.  Row t enters, row t - 4 leaves.
+template <bool COARSE, bool NCC>
+__global__ void __launch_bounds__(32 * kEdgeWarps, 4) edge_grad_kernel(EdgeArgs e, int strips, int jobs, int groups,
+                                                                    const double* __restrict__ stats,
+                                                                    const float* __restrict__ g, int64_t g_stride,
+                                                                    double g_scale, int swap) {
+  __shared__ float coef[kEdgeCombos + 1][3];  // alpha, beta, -(alpha mean v + beta mean u)
+  const int64_t pair = blockIdx.x / groups;
+  const int job = static_cast<int>(blockIdx.x - pair * groups) * kEdgeWarps + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  const EdgeJob jb = edge_job(e, pair, job < jobs ? job : 0, strips);
+  if (threadIdx.x < kEdgeCombos + 1) {
     const int k = threadIdx.x;
-    const double* m = stats + static_cast<int64_t>(pair) * kEdgeCombos * kEdgeMom + k * kEdgeMom;
+    const double* m = stats + pair * kEdgeNM + k * kEdgeMom;
     // u = the differentiated image's response, v = the other one's
-    const double su = wrt_b ? m[1] : m[0], sv = wrt_b ? m[0] : m[1];
-    const double suu_raw = wrt_b ? m[3] : m[2], svv_raw = wrt_b ? m[2] : m[3];
-    const double n = static_cast<double>(a.H - 2 * a.crop) * static_cast<double>(a.W - 2 * a.crop);
+    const double su = swap ? m[1] : m[0], sv = swap ? m[0] : m[1];
+    const double suu_raw = swap ? m[3] : m[2], svv_raw = swap ? m[2] : m[3];
+    const bool whole = k == kEdgeCombos;
+    const double n = whole ? static_cast<double>(e.H) * static_cast<double>(e.W)
+                           : static_cast<double>(e.H - 2 * e.crop) * static_cast<double>(e.W - 2 * e.crop);
     const double suu = suu_raw - su * su / n, svv = svv_raw - sv * sv / n, suv = m[4] - m[0] * m[1] / n;
-    const double prod = suu * svv;
-    const double den = sqrt(fmax(prod, 1e-12));
-    const double gv = static_cast<double>(g[g_stride * bi]) * (reduction_mean ? 1.0 / a.B : 1.0);
-    const double sw = k < 2 ? (a.coarse ? 1.0 - w : 1.0) : (a.coarse ? w : 0.0);
-    const double wk = gv * sw * 0.5 / a.Cch;
-    coef[k][0] = static_cast<float>(wk / den);
-    coef[k][1] = prod > 1e-12 ? static_cast<float>(-wk * suv * svv / (den * den * den)) : 0.f;
-    coef[k][2] = static_cast<float>(su / n);
-    coef[k][3] = static_cast<float>(sv / n);
-  }
-  load_window(img_a, a.H, a.W, r0 - 4, c0 - 4, N4, sa);
-  load_window(img_b, a.H, a.W, r0 - 4, c0 - 4, N4, sb);
-  __syncthreads();
-  if (a.coarse) {
-    blur_window(sa, a.H, a.W, r0 - 3, c0 - 3, N3, ba);
-    blur_window(sb, a.H, a.W, r0 - 3, c0 - 3, N3, bb);
-  }
-  const int ilo = a.crop, ihi = a.H - a.crop, jlo = a.crop, jhi = a.W - a.crop;
-  // fine fields at halo 1 (window origin r0 - 1)
-  for (int k = threadIdx.x; k < N1 * N1; k += blockDim.x) {
-    const int i = k / N1, j = k - i * N1;
-    const int r = r0 - 1 + i, c = c0 - 1 + j;
-    float fx = 0.f, fy = 0.f;
-    if (r >= ilo && r < ihi && c >= jlo && c < jhi) {
-      float ux, uy, vx, vy;
-      sobel(sa, N4, i + 3, j + 3, ux, uy);
-      sobel(sb, N4, i + 3, j + 3, vx, vy);
-      fx = coef[0][0] * (vx - coef[0][3]) + coef[0][1] * (ux - coef[0][2]);
-      fy = coef[1][0] * (vy - coef[1][3]) + coef[1][1] * (uy - coef[1][2]);
-    }
-    gfx[k] = fx;
-    gfy[k] = fy;
+    const double prod = suu * svv, den = sqrt(fmax(prod, 1e-12));
+    const double sw = k < 2 ? (e.coarse ? 1.0 - e.w : 1.0) : (e.coarse ? static_cast<double>(e.w) : 0.0);
+    const double wk = static_cast<double>(g[g_stride * jb.bi]) * g_scale * (whole ? e.cn : e.ce * sw * 0.5) / e.Cch;
+    const double al = wk / den, be = prod > 1e-12 ? -wk * suv * svv / (den * den * den) : 0.0;
+    coef[k][0] = static_cast<float>(al);
+    coef[k][1] = static_cast<float>(be);
+    coef[k][2] = static_cast<float>(-(al * sv + be * su) / n);
   }
   __syncthreads();
-  if (a.coarse) {
-    // coarse fields at halo 2 (window origin r0 - 2)
-    for (int k = threadIdx.x; k < N2 * N2; k += blockDim.x) {
-      const int i = k / N2, j = k - i * N2;
-      const int r = r0 - 2 + i, c = c0 - 2 + j;
-      float fx = 0.f, fy = 0.f;
-      if (r >= ilo && r < ihi && c >= jlo && c < jhi) {
-        float ux, uy, vx, vy;
-        sobel(ba, N3, i + 1, j + 1, ux, uy);
-        sobel(bb, N3, i + 1, j + 1, vx, vy);
-        fx = coef[2][0] * (vx - coef[2][3]) + coef[2][1] * (ux - coef[2][2]);
-        fy = coef[3][0] * (vy - coef[3][3]) + coef[3][1] * (uy - coef[3][2]);
-      }
-      gcx[k] = fx;
-      gcy[k] = fy;
-    }
-    __syncthreads();
-    // gradient w.r.t. the blurred image at halo 1: transposed Sobel, in-image only
-    for (int k = threadIdx.x; k < N1 * N1; k += blockDim.x) {
-      const int i = k / N1, j = k - i * N1;
-      const int r = r0 - 1 + i, c = c0 - 1 + j;
-      float s = 0.f;
-      if (r >= 0 && r < a.H && c >= 0 && c < a.W) {
-        const float* px = gcx + (i + 1) * N2 + (j + 1);
-        const float* py = gcy + (i + 1) * N2 + (j + 1);
-        // sum_d g(m - d) k[d]: kx[d] = dj (1 + (di == 0)), ky[d] = di (1 + (dj == 0))
-        s = (px[N2 - 1] - px[N2 + 1]) + 2.f * (px[-1] - px[1]) + (px[-N2 - 1] - px[-N2 + 1]);
-        s += (py[-N2 - 1] + 2.f * py[-N2] + py[-N2 + 1]) - (py[N2 - 1] + 2.f * py[N2] + py[N2 + 1]);
-      }
-      gbl[k] = s;
-    }
-    __syncthreads();
+  if (job >= jobs) return;
+  const int c = jb.strip * kGradCols - 4 + 2 * lane;
+  const bool own = lane >= 2 && lane <= 29;
+  bool in_img[2], in_edge[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    in_img[j] = c + j >= 0 && c + j < e.W;
+    in_edge[j] = c + j >= e.crop && c + j < e.W - e.crop;
   }
-  const int tj = threadIdx.x & 31;
-  const int64_t out_base = (static_cast<int64_t>(bi) * a.Cch + ch) * plane;
-  for (int ti = threadIdx.x >> 5; ti < T; ti += kEdgeThreads / 32) {
-    const int r = r0 + ti, c = c0 + tj;
-    if (r >= a.H || c >= a.W) continue;
-    const float* px = gfx + (ti + 1) * N1 + (tj + 1);
-    const float* py = gfy + (ti + 1) * N1 + (tj + 1);
-    float s = (px[N1 - 1] - px[N1 + 1]) + 2.f * (px[-1] - px[1]) + (px[-N1 - 1] - px[-N1 + 1]);
-    s += (py[-N1 - 1] + 2.f * py[-N1] + py[-N1 + 1]) - (py[N1 - 1] + 2.f * py[N1] + py[N1 + 1]);
-    if (a.coarse) {
-      const float* q = gbl + (ti + 1) * N1 + (tj + 1);
-      s += (q[-N1 - 1] + q[-N1] + q[-N1 + 1] + q[-1] + q[0] + q[1] + q[N1 - 1] + q[N1] + q[N1 + 1]) * (1.f / 9.f);
+  float al[kEdgeCombos + 1], be[kEdgeCombos + 1], k0[kEdgeCombos + 1];
+#pragma unroll
+  for (int k = 0; k < kEdgeCombos + 1; ++k) {
+    al[k] = coef[k][0];
+    be[k] = coef[k][1];
+    k0[k] = coef[k][2];
+  }
+  float* out = e.grad[jb.view] + (static_cast<int64_t>(jb.bi) * e.Cch + jb.ch) * static_cast<int64_t>(e.H) * e.W;
+  EdgeMarch<COARSE> march;
+  march.init();
+  const float2 zero = make_float2(0.f, 0.f);
+  float fx1[2] = {0.f, 0.f}, fy1[2] = {0.f, 0.f};             // fine fields of row t - 2
+  float2 e0[2] = {zero, zero}, e1[2] = {zero, zero};          // transposed Sobel x parts of rows t - 4, t - 3
+  float2 q0[2] = {zero, zero}, q1[2] = {zero, zero};          // transposed Sobel y parts
+  float h0[2] = {0.f, 0.f}, h1[2] = {0.f, 0.f};               // box parts of rows t - 5, t - 4
+  float of[2] = {0.f, 0.f};                                   // fine gradient of row t - 4
+  float im0[2] = {0.f, 0.f}, im1[2] = {0.f, 0.f}, im2[2] = {0.f, 0.f}, im3[2] = {0.f, 0.f};  // rows t - 4 .. t - 1
+  const int64_t W = e.W;
+  RowReader rows;
+  rows.init(e, swap ? jb.b : jb.a, swap ? jb.a : jb.b, jb.rb - 4, c);
+#pragma unroll 4
+  for (int t = jb.rb - 4; t < jb.re + 4; ++t) {
+    float2 x[2];
+    rows.next(x);
+    float2 gx[2], gy[2], gbx[2], gby[2];
+    march.step(x, t - 1 >= 0 && t - 1 < e.H, in_img, gx, gy, gbx, gby);
+    const bool rf = t - 1 >= e.crop && t - 1 < e.H - e.crop, rc = t - 2 >= e.crop && t - 2 < e.H - e.crop;
+    float2 Fx[2], Fy[2];  // (fine, coarse) fields of row t - 2
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      Fx[j] = make_float2(fx1[j], 0.f);
+      Fy[j] = make_float2(fy1[j], 0.f);
+      const bool f_in = rf && in_edge[j], c_in = rc && in_edge[j];
+      fx1[j] = f_in ? fmaf(al[0], gx[j].y, fmaf(be[0], gx[j].x, k0[0])) : 0.f;
+      fy1[j] = f_in ? fmaf(al[1], gy[j].y, fmaf(be[1], gy[j].x, k0[1])) : 0.f;
+      if (COARSE) {
+        Fx[j].y = c_in ? fmaf(al[2], gbx[j].y, fmaf(be[2], gbx[j].x, k0[2])) : 0.f;
+        Fy[j].y = c_in ? fmaf(al[3], gby[j].y, fmaf(be[3], gby[j].x, k0[3])) : 0.f;
+      }
     }
-    grad[out_base + static_cast<int64_t>(r) * a.W + c] = s;
+    float2 xl, xr, yl, yr;
+    if (COARSE) {
+      xl = shfl_up2(Fx[1]);
+      xr = shfl_down2(Fx[0]);
+      yl = shfl_up2(Fy[1]);
+      yr = shfl_down2(Fy[0]);
+    } else {
+      xl = make_float2(__shfl_up_sync(0xffffffffu, Fx[1].x, 1), 0.f);
+      xr = make_float2(__shfl_down_sync(0xffffffffu, Fx[0].x, 1), 0.f);
+      yl = make_float2(__shfl_up_sync(0xffffffffu, Fy[1].x, 1), 0.f);
+      yr = make_float2(__shfl_down_sync(0xffffffffu, Fy[0].x, 1), 0.f);
+    }
+    const float2 ev[2] = {sub2(xl, Fx[1]), sub2(Fx[0], xr)};
+    const float2 qv[2] = {twice_plus(Fy[0], add2(yl, Fy[1])), twice_plus(Fy[1], add2(Fy[0], yr))};
+    const bool r3 = t - 3 >= 0 && t - 3 < e.H;
+    float of_new[2], gb[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      // (fine gradient, gradient w.r.t. the blurred image) of row t - 3
+      const float2 o = add2(twice_plus(e1[j], add2(e0[j], ev[j])), sub2(q0[j], qv[j]));
+      e0[j] = e1[j];
+      e1[j] = ev[j];
+      q0[j] = q1[j];
+      q1[j] = qv[j];
+      of_new[j] = o.x;
+      gb[j] = r3 && in_img[j] ? o.y : 0.f;
+    }
+    float bt[2] = {0.f, 0.f};
+    if (COARSE) {
+      const float l = __shfl_up_sync(0xffffffffu, gb[1], 1), r = __shfl_down_sync(0xffffffffu, gb[0], 1);
+      const float m = gb[0] + gb[1];
+      const float h[2] = {l + m, m + r};
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        bt[j] = ((h0[j] + h1[j]) + h[j]) * (1.f / 9.f);
+        h0[j] = h1[j];
+        h1[j] = h[j];
+      }
+    }
+    float res[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      res[j] = of[j] + bt[j];
+      of[j] = of_new[j];
+      if (NCC) {
+        res[j] += im0[j];
+        im0[j] = im1[j];
+        im1[j] = im2[j];
+        im2[j] = im3[j];
+        im3[j] = fmaf(al[kEdgeCombos], x[j].y, fmaf(be[kEdgeCombos], x[j].x, k0[kEdgeCombos]));
+      }
+    }
+    const int r = t - 4;
+    if (r >= jb.rb && own) {
+      float* o = out + r * W + c;
+      if (e.vec) {
+        if (in_img[0]) *reinterpret_cast<float2*>(o) = make_float2(res[0], res[1]);
+      } else {
+        if (in_img[0]) o[0] = res[0];
+        if (in_img[1]) o[1] = res[1];
+      }
+    }
   }
 }
 
-constexpr int64_t kEdgeGradSmem =
-    (2 * (kEdgeTile + 8) * (kEdgeTile + 8) + 2 * (kEdgeTile + 6) * (kEdgeTile + 6) +
-     3 * (kEdgeTile + 2) * (kEdgeTile + 2) + 2 * (kEdgeTile + 4) * (kEdgeTile + 4)) *
-    static_cast<int64_t>(sizeof(float));
-
-static int edge_args(const float* a, const float* b, int64_t B, int64_t Bt, int64_t C, int64_t H, int64_t W,
-                     int64_t crop, float w, EdgeArgs* e) {
-  if (!a || !b || B < 1 || C < 1 || H < 3 || W < 3 || (Bt != 1 && Bt != B) || crop < 0) return FVR_ERR_ARG;
+static int edge_common(int64_t B, int64_t C, int64_t H, int64_t W, int64_t crop, float w, EdgeArgs* e) {
+  if (B < 1 || C < 1 || H < 3 || W < 3 || crop < 0) return FVR_ERR_ARG;
   if (H - 2 * crop < 1 || W - 2 * crop < 1 || B * C > 65535 || H > 32768 || W > 32768) return FVR_ERR_ARG;
-  e->a = a;
-  e->b = b;
   e->B = (int)B;
-  e->Bt = (int)Bt;
   e->Cch = (int)C;
   e->H = (int)H;
   e->W = (int)W;
   e->crop = (int)crop;
   e->coarse = (w > 0.f && W >= 96) ? 1 : 0;  // the reference tests the last dim (cone_beam_fvr.py:86, 107)
-  e->tiles_x = (int)cdiv64(W - 2 * crop, kEdgeTile);
-  e->tiles_y = (int)cdiv64(H - 2 * crop, kEdgeTile);
+  e->w = w;
+  e->vec = W % 2 == 0 ? 1 : 0;
+  return FVR_OK;
+}
+
+static int edge_view(EdgeArgs* e, int v, const float* a, const float* b, int64_t Bt, float* grad) {
+  if (!a || !b || (Bt != 1 && Bt != e->B)) return FVR_ERR_ARG;
+  e->a[v] = a;
+  e->b[v] = b;
+  e->Bt[v] = (int)Bt;
+  e->grad[v] = grad;
+  if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(grad)) & 7)
+    e->vec = 0;
+  return FVR_OK;
+}
+
+static int64_t edge_jobs(int64_t H, int64_t W, int cols) { return cdiv64(H, kEdgeRows) * cdiv64(W, cols); }
+
+// Strip records, then one fp64 value per item (for the batch mean).
+static int64_t edge_ws_bytes(int64_t views, int64_t B, int64_t C, int64_t H, int64_t W) {
+  return (views * B * C * edge_jobs(H, W, kMomCols) * kEdgeNM + B) * (int64_t)sizeof(double);
+}
+
+template <typename K>
+static int edge_grid(const EdgeArgs& e, int cols, K launch) {
+  const int64_t jobs = edge_jobs(e.H, e.W, cols), groups = cdiv64(jobs, kEdgeWarps);
+  const int64_t n = static_cast<int64_t>(e.views) * e.B * e.Cch * groups;
+  if (n > 2147483647) return FVR_ERR_ARG;
+  launch(static_cast<unsigned>(n), static_cast<int>(cdiv64(e.W, cols)), static_cast<int>(jobs),
+         static_cast<int>(groups));
+  FVR_LAUNCH_CHECK();
+  return FVR_OK;
+}
+
+static int edge_forward(const EdgeArgs& e, void* workspace, double* stats, float* out, bool mean, cudaStream_t s) {
+  double* part = static_cast<double*>(workspace);
+  const int rc = edge_grid(e, kMomCols, [&](unsigned n, int strips, int jobs, int groups) {
+    const dim3 block(32 * kEdgeWarps);
+    if (e.coarse && e.cn != 0.0) edge_moments_kernel<true, true><<<n, block, 0, s>>>(e, strips, jobs, groups, part);
+    else if (e.coarse) edge_moments_kernel<true, false><<<n, block, 0, s>>>(e, strips, jobs, groups, part);
+    else if (e.cn != 0.0) edge_moments_kernel<false, true><<<n, block, 0, s>>>(e, strips, jobs, groups, part);
+    else edge_moments_kernel<false, false><<<n, block, 0, s>>>(e, strips, jobs, groups, part);
+  });
+  if (rc) return rc;
+  const int jobs = (int)edge_jobs(e.H, e.W, kMomCols);
+  double* value = part + static_cast<int64_t>(e.views) * e.B * e.Cch * jobs * kEdgeNM;
+  edge_finalize_kernel<<<static_cast<unsigned>(e.B), 128, 0, s>>>(e, jobs, part, stats, mean ? nullptr : out,
+                                                                  mean ? value : nullptr);
+  FVR_LAUNCH_CHECK();
+  if (mean) {
+    edge_mean_kernel<<<1, 32, 0, s>>>(value, e.B, out);
+    FVR_LAUNCH_CHECK();
+  }
+  return FVR_OK;
+}
+
+static int edge_backward(const EdgeArgs& e, const double* stats, const float* g, int64_t g_stride, double g_scale,
+                         int swap, cudaStream_t s) {
+  return edge_grid(e, kGradCols, [&](unsigned n, int strips, int jobs, int groups) {
+    const dim3 block(32 * kEdgeWarps);
+    if (e.coarse && e.cn != 0.0)
+      edge_grad_kernel<true, true><<<n, block, 0, s>>>(e, strips, jobs, groups, stats, g, g_stride, g_scale, swap);
+    else if (e.coarse)
+      edge_grad_kernel<true, false><<<n, block, 0, s>>>(e, strips, jobs, groups, stats, g, g_stride, g_scale, swap);
+    else if (e.cn != 0.0)
+      edge_grad_kernel<false, true><<<n, block, 0, s>>>(e, strips, jobs, groups, stats, g, g_stride, g_scale, swap);
+    else
+      edge_grad_kernel<false, false><<<n, block, 0, s>>>(e, strips, jobs, groups, stats, g, g_stride, g_scale, swap);
+  });
+}
+
+static int reg_loss_args(const float* const* imgs, const float* const* refs, const int64_t* ref_batch, int views,
+                         float* const* grads, int64_t B, int64_t H, int64_t W, int64_t crop, float ms_weight,
+                         float edge_weight, EdgeArgs* e) {
+  if (!imgs || !refs || !ref_batch || views < 1 || views > kEdgeMaxViews) return FVR_ERR_ARG;
+  int rc = edge_common(B, 1, H, W, crop, ms_weight, e);
+  if (rc) return rc;
+  e->views = views;
+  e->base = 1.0;
+  e->ce = -static_cast<double>(edge_weight) / views;
+  e->cn = -(1.0 - static_cast<double>(edge_weight)) / views;
+  for (int v = 0; v < views; ++v)
+    if ((rc = edge_view(e, v, imgs[v], refs[v], ref_batch[v], grads ? grads[v] : nullptr))) return rc;
   return FVR_OK;
 }
 
@@ -318,47 +626,65 @@ extern "C" {
 
 int64_t fvr_edge_ncc_workspace(int64_t B, int64_t C, int64_t H, int64_t W, int64_t crop) {
   if (B < 1 || C < 1 || H - 2 * crop < 1 || W - 2 * crop < 1) return 0;
-  return B * C * cdiv64(H - 2 * crop, kEdgeTile) * cdiv64(W - 2 * crop, kEdgeTile) * kEdgeCombos * kEdgeMom *
-         (int64_t)sizeof(double);
+  return edge_ws_bytes(1, B, C, H, W);
 }
 
-int64_t fvr_edge_ncc_stats_count(void) { return kEdgeCombos * kEdgeMom; }
+int64_t fvr_edge_ncc_stats_count(void) { return kEdgeNM; }
 
 int fvr_edge_ncc_forward(const float* a, const float* b, int64_t B, int64_t Bt, int64_t C, int64_t H, int64_t W,
                          int64_t crop, float ms_weight, int reduction_mean, void* workspace, int64_t ws_bytes,
                          double* stats, float* out, void* stream) {
-  EdgeArgs e;
-  int rc = edge_args(a, b, B, Bt, C, H, W, crop, ms_weight, &e);
+  EdgeArgs e{};
+  int rc = edge_common(B, C, H, W, crop, ms_weight, &e);
   if (rc) return rc;
+  e.views = 1;
+  e.ce = 1.0;
+  if ((rc = edge_view(&e, 0, a, b, Bt, nullptr))) return rc;
   if (!workspace || !stats || !out) return FVR_ERR_ARG;
   if (ws_bytes < fvr_edge_ncc_workspace(B, C, H, W, crop)) return FVR_ERR_WORKSPACE;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  dim3 grid(e.tiles_x, e.tiles_y, static_cast<unsigned>(B * C));
-  edge_moments_kernel<<<grid, kEdgeThreads, 0, s>>>(e, static_cast<double*>(workspace));
-  FVR_LAUNCH_CHECK();
-  edge_finalize_kernel<<<1, 256, 0, s>>>(e, static_cast<const double*>(workspace), ms_weight, stats, out,
-                                         reduction_mean);
-  FVR_LAUNCH_CHECK();
-  return FVR_OK;
+  return edge_forward(e, workspace, stats, out, reduction_mean != 0, static_cast<cudaStream_t>(stream));
 }
 
 int fvr_edge_ncc_backward(const float* a, const float* b, int64_t B, int64_t Bt, int64_t C, int64_t H, int64_t W,
                           int64_t crop, float ms_weight, int reduction_mean, const double* stats, const float* g,
                           int64_t g_stride, int wrt_b, float* grad, void* stream) {
-  EdgeArgs e;
-  int rc = edge_args(a, b, B, Bt, C, H, W, crop, ms_weight, &e);
+  EdgeArgs e{};
+  int rc = edge_common(B, C, H, W, crop, ms_weight, &e);
   if (rc) return rc;
   if (!stats || !g || !grad) return FVR_ERR_ARG;
-  // the shared-memory opt-in is a per-device setting: made before every launch
-  if (cudaFuncSetAttribute(edge_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEdgeGradSmem) !=
-      cudaSuccess)
-    return FVR_ERR_CUDA;
-  dim3 grid(static_cast<unsigned>(cdiv64(W, kEdgeTile)), static_cast<unsigned>(cdiv64(H, kEdgeTile)),
-            static_cast<unsigned>(B * C));
-  edge_grad_kernel<<<grid, kEdgeThreads, kEdgeGradSmem, static_cast<cudaStream_t>(stream)>>>(
-      e, stats, ms_weight, g, (int)g_stride, reduction_mean, wrt_b, grad);
-  FVR_LAUNCH_CHECK();
-  return FVR_OK;
+  e.views = 1;
+  e.ce = 1.0;
+  if ((rc = edge_view(&e, 0, a, b, Bt, grad))) return rc;
+  return edge_backward(e, stats, g, g_stride, reduction_mean ? 1.0 / static_cast<double>(B) : 1.0, wrt_b != 0,
+                       static_cast<cudaStream_t>(stream));
+}
+
+int64_t fvr_reg_loss_workspace(int64_t views, int64_t B, int64_t H, int64_t W) {
+  if (views < 1 || B < 1 || H < 1 || W < 1) return 0;
+  return edge_ws_bytes(views, B, 1, H, W);
+}
+
+int fvr_reg_loss_forward(const float* const* imgs, const float* const* refs, const int64_t* ref_batch, int views,
+                         int64_t B, int64_t H, int64_t W, int64_t crop, float ms_weight, float edge_weight,
+                         void* workspace, int64_t ws_bytes, double* stats, float* out, void* stream) {
+  EdgeArgs e{};
+  const int rc = reg_loss_args(imgs, refs, ref_batch, views, nullptr, B, H, W, crop, ms_weight, edge_weight, &e);
+  if (rc) return rc;
+  if (!workspace || !stats || !out) return FVR_ERR_ARG;
+  if (ws_bytes < fvr_reg_loss_workspace(views, B, H, W)) return FVR_ERR_WORKSPACE;
+  return edge_forward(e, workspace, stats, out, false, static_cast<cudaStream_t>(stream));
+}
+
+int fvr_reg_loss_backward(const float* const* imgs, const float* const* refs, const int64_t* ref_batch, int views,
+                          int64_t B, int64_t H, int64_t W, int64_t crop, float ms_weight, float edge_weight,
+                          const double* stats, const float* g, int64_t g_stride, float* const* grads, void* stream) {
+  if (!stats || !g || !grads) return FVR_ERR_ARG;
+  for (int v = 0; v < views && v < kEdgeMaxViews; ++v)
+    if (!grads[v]) return FVR_ERR_ARG;
+  EdgeArgs e{};
+  const int rc = reg_loss_args(imgs, refs, ref_batch, views, grads, B, H, W, crop, ms_weight, edge_weight, &e);
+  if (rc) return rc;
+  return edge_backward(e, stats, g, g_stride, 1.0, 0, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

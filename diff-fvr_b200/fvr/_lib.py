@@ -64,6 +64,9 @@ SIGNATURES = {
     "fvr_edge_ncc_stats_count": (I64, []),
     "fvr_edge_ncc_forward": (I32, [P, P, I64, I64, I64, I64, I64, I64, F32, I32, P, I64, P, P, P]),
     "fvr_edge_ncc_backward": (I32, [P, P, I64, I64, I64, I64, I64, I64, F32, I32, P, P, I64, I32, P, P]),
+    "fvr_reg_loss_workspace": (I64, [I64, I64, I64, I64]),
+    "fvr_reg_loss_forward": (I32, [P, P, P, I32, I64, I64, I64, I64, F32, F32, P, I64, P, P, P]),
+    "fvr_reg_loss_backward": (I32, [P, P, P, I32, I64, I64, I64, I64, F32, F32, P, P, I64, P, P]),
     "fvr_tc_sncc_value_and_grad": (I32, [I32, P, P, I64, I64, I64, P, I64, I32, P, P, P, P, I64, F64, I32, P, I64, P,
                                          I64, P, P, P, I32, P]),
     "fvr_event_record": (I32, [P, P, I32]),
@@ -158,6 +161,7 @@ KERNELS_PER_CALL = {
     "fvr_np_ncc_moments": 2,
     "fvr_np_pair_moments": 2,
     "fvr_edge_ncc_forward": 2,
+    "fvr_reg_loss_forward": 2,
     "fvr_tc_sncc_value_and_grad": 2,
     "fvr_tc_sncc_value_and_grad_static": 2,
 }

@@ -14,6 +14,7 @@ replayed.
 """
 from __future__ import annotations
 
+import ctypes
 import math
 from typing import Callable, Tuple
 
@@ -63,11 +64,72 @@ def image_ncc(pred: torch.Tensor, target: torch.Tensor) -> torch.Tensor:
     return (num / den).squeeze(1)
 
 
+_EDGE_WEIGHT, _MS_WEIGHT = 0.75, 0.25  # edge against image NCC; blurred against fine scale of the edge NCC
+
+
+class _RegLossFn(torch.autograd.Function):
+    """biplanar_loss_per_candidate in three launches: one pass over both views'
+    images for every moment of the edge and image NCCs, a finalize, and in the
+    backward one pass that writes both views' image gradients."""
+
+    @staticmethod
+    def forward(ctx, imA, imB, refA, refB):
+        dev = L.require_cuda(imA, imB, refA, refB)
+        ims = [x.detach().contiguous() for x in (imA, imB)]
+        refs = [x.detach().contiguous() for x in (refA, refB)]
+        B, _, H, W = (int(x) for x in imA.shape)
+        ws_bytes = int(L.query("fvr_reg_loss_workspace", 2, B, H, W))
+        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
+        stats = torch.empty((2 * B, int(L.query("fvr_edge_ncc_stats_count"))), dtype=torch.float64, device=dev)
+        out = torch.empty(B, dtype=torch.float32, device=dev)
+        L.call("fvr_reg_loss_forward", *_RegLossFn._args(ims, refs), L.ptr(ws), ws_bytes, L.ptr(stats), L.ptr(out),
+               L.stream_ptr(dev))
+        ctx.save_for_backward(*ims, *refs, stats)
+        return out
+
+    @staticmethod
+    def _args(ims, refs):
+        B, _, H, W = (int(x) for x in ims[0].shape)
+        return ((ctypes.c_void_p * 2)(*[x.data_ptr() for x in ims]),
+                (ctypes.c_void_p * 2)(*[x.data_ptr() for x in refs]),
+                (ctypes.c_int64 * 2)(*[int(x.shape[0]) for x in refs]), 2, B, H, W, max(4, W // 8), _MS_WEIGHT,
+                _EDGE_WEIGHT)
+
+    @staticmethod
+    def backward(ctx, g):
+        *t, stats = ctx.saved_tensors
+        ims, refs = t[:2], t[2:]
+        g = g.detach().to(torch.float32).contiguous()
+        grads = [torch.empty_like(x) for x in ims]
+        L.call("fvr_reg_loss_backward", *_RegLossFn._args(ims, refs), L.ptr(stats), L.ptr(g), 1,
+               (ctypes.c_void_p * 2)(*[x.data_ptr() for x in grads]), L.stream_ptr(g.device))
+        return grads[0], grads[1], None, None
+
+
+def _reg_loss_fused(ims, refs) -> bool:
+    """The fused launch takes two views of one-channel CUDA images of one shape
+    against references of batch 1 or B that need no gradient; anything else
+    (CPU tensors, views of different sizes, more channels) is composed from
+    the separate losses."""
+    s = ims[0].shape
+    if len(s) != 4 or s[0] < 1 or s[1] != 1:
+        return False
+    grad = torch.is_grad_enabled()
+    return (all(x.is_cuda and x.device == ims[0].device and not x.is_complex() for x in (*ims, *refs))
+            and ims[1].shape == s
+            and all(r.dim() == 4 and r.shape[1:] == s[1:] and r.shape[0] in (1, s[0]) for r in refs)
+            and not (grad and any(r.requires_grad for r in refs)))
+
+
 def biplanar_loss_per_candidate(imA, imB, refA, refB) -> torch.Tensor:
     """1 - 0.5 (sim_A + sim_B), sim = 0.75 edge-dominant NCC + 0.25 image NCC
     (exp30:120-134); one value per candidate."""
+    if _reg_loss_fused((imA, imB), (refA, refB)):
+        return _RegLossFn.apply(imA.float(), imB.float(), refA.float(), refB.float())
+
     def pair(p, r):
-        return 0.75 * edge_dominant_ncc(p.float(), r.float(), reduction="none") + 0.25 * image_ncc(p, r)
+        return (_EDGE_WEIGHT * edge_dominant_ncc(p.float(), r.float(), multiscale_weight=_MS_WEIGHT, reduction="none")
+                + (1.0 - _EDGE_WEIGHT) * image_ncc(p, r))
 
     return 1.0 - 0.5 * (pair(imA, refA) + pair(imB, refB))
 
