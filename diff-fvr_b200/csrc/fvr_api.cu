@@ -25,6 +25,7 @@ __global__ void __launch_bounds__(256) copy_bytes_kernel(unsigned char* __restri
 namespace fvr {
 int check_word_tc(unsigned long long* out, int clear);
 int check_word_pou(unsigned long long* out, int clear);
+int check_word_pou_sep(unsigned long long* out, int clear);
 int check_word_slice3d(unsigned long long* out, int clear);
 int check_word_np(unsigned long long* out, int clear);
 }  // namespace fvr
@@ -40,6 +41,9 @@ int fvr_check_words(unsigned long long* out, int n, int clear) {
   if (!out || n < kUnits) return FVR_ERR_ARG;
   for (int i = 0; i < kUnits; ++i)
     if (readers[i](out + i, clear)) return FVR_ERR_CUDA;
+  unsigned long long sep = 0;  // the separable warp's word reports with the PoU family's
+  if (fvr::check_word_pou_sep(&sep, clear)) return FVR_ERR_CUDA;
+  if (out[1] == 0) out[1] = sep;
   return FVR_OK;
 #else
   (void)out;

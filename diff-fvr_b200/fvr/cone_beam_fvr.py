@@ -175,10 +175,26 @@ def _separable_rays(rx, ry):
     return rxc, ryr
 
 
+def _monotone(sep):
+    """Whether both separable ray tables run in one direction (the separable
+    warp adjoint marches along them)."""
+    if sep is None:
+        return False
+    steps = [np.diff(t.cpu().numpy()) for t in sep]
+    return all(bool((d >= 0).all()) or bool((d <= 0).all()) for d in steps)
+
+
+# The separable warp adjoint hands dL/dimgs to the block-image adjoint in a
+# [blocks, poses, P, P] buffer.  Beyond this size the one-launch adjoint runs
+# instead where it can: it keeps that gradient in shared memory (64 blocks x 64
+# poses x 128^2 is 268 MB: 1.0 against 1.4 ms).
+_GRAD_IMAGE_BYTES = 4 << 30
+
+
 def _prepared_lattice(lattice, device):
     """Device copies of an 11-tuple lattice's ray tables and its basis
-    (src0, u0, v0, n0) as 12 host doubles, and its separable ray tables when
-    it has them, cached per (storage, device): the lattice is a per-geometry
+    (src0, u0, v0, n0) as 12 host doubles, its separable ray tables when
+    it has them and whether those are monotone, cached per (storage, device): the lattice is a per-geometry
     constant, moved once.  The entry holds the lattice's own tensors, so their
     storage cannot be freed and reused by another lattice while the entry
     exists."""
@@ -190,7 +206,8 @@ def _prepared_lattice(lattice, device):
         basis = torch.cat([lattice[i].reshape(3) for i in (0, 2, 3, 4)]).detach().double().cpu()
         base = (_ct.c_double * 12)(*[float(x) for x in basis])
         rays = tuple(t.detach().to(device=device, dtype=torch.float32).contiguous() for t in lattice[5:8])
-        hit = (key, base, rays, tuple(lattice[:8]), _separable_rays(rays[0], rays[1]))
+        sep = _separable_rays(rays[0], rays[1])
+        hit = (key, base, rays, tuple(lattice[:8]), sep, _monotone(sep))
         _LATTICE_CACHE[key] = hit
     return hit
 
@@ -247,7 +264,7 @@ class _PinholeFn(torch.autograd.Function):
         m = mats.detach().to(device=dev, dtype=torch.float32).contiguous()
         N = int(m.shape[0])
         B, P = model.B, model.P
-        base = _LATTICE_CACHE[base_key][1]
+        _, base, _, _, sep, monotone = _LATTICE_CACHE[base_key]
         geo = torch.empty((N, int(L.query("fvr_pou_geo_stride"))), dtype=torch.float64, device=dev)
         offs = torch.empty((B, N, 3), dtype=torch.float64, device=dev)
         s = L.stream_ptr(dev)
@@ -258,25 +275,38 @@ class _PinholeFn(torch.autograd.Function):
         H, W = int(rx.shape[0]), int(rx.shape[1])
         out = torch.empty((N, 1, H, W), dtype=torch.float32, device=dev)
         with profiling.section("pou_warp"):
-            L.call("fvr_pou_warp", L.ptr(imgs), B, N, P, L.ptr(offs), _ct.c_void_p(offs.data_ptr() + 8),
-                   _ct.c_void_p(offs.data_ptr() + 16), 1, 3, L.ptr(rx), L.ptr(ry), L.ptr(ic), H * W, 0,
-                   1.0 / model.ds_block, float(P // 2), L.ptr(out), s)
+            if sep is not None and L.query("fvr_pou_warp_sep_supported", P, H, W):
+                L.call("fvr_pou_warp_sep", L.ptr(imgs), B, N, P, L.ptr(offs), L.ptr(sep[0]), L.ptr(sep[1]), L.ptr(ic),
+                       H, W, 1.0 / model.ds_block, float(P // 2), L.ptr(out), s)
+            else:
+                L.call("fvr_pou_warp", L.ptr(imgs), B, N, P, L.ptr(offs), _ct.c_void_p(offs.data_ptr() + 8),
+                       _ct.c_void_p(offs.data_ptr() + 16), 1, 3, L.ptr(rx), L.ptr(ry), L.ptr(ic), H * W, 0,
+                       1.0 / model.ds_block, float(P // 2), L.ptr(out), s)
         ctx.save_for_backward(geo, offs, imgs, rx, ry, ic)
-        ctx.meta = (model, base, mats.dtype, _LATTICE_CACHE[base_key][4])
+        ctx.meta = (model, base, mats.dtype, sep, monotone)
         return out
 
     @staticmethod
     def backward(ctx, g_out):
         geo, offs, imgs, rx, ry, ic = ctx.saved_tensors
-        model, base, mdt, sep = ctx.meta
+        model, base, mdt, sep, monotone = ctx.meta
         dev = geo.device
         B, N, P = model.B, int(geo.shape[0]), model.P
         H, W = int(rx.shape[0]), int(rx.shape[1])
         s = L.stream_ptr(dev)
         g = g_out.detach().to(device=dev, dtype=torch.float32).contiguous()
         goffs = torch.empty((3, B, N), dtype=torch.float64, device=dev)
-        if (sep is not None and model.fused_warp_adjoint and g.data_ptr() % 16 == 0 and ic.data_ptr() % 16 == 0
-                and L.query("fvr_pou_warp_image_adjoint_supported", P, H, W)):
+        if (monotone and model.fused_warp_adjoint and 4 * B * N * P * P <= _GRAD_IMAGE_BYTES
+                and L.query("fvr_pou_warp_sep_adjoint_supported", P, H, W)):
+            grad_imgs = torch.empty((B, N, P, P), dtype=torch.float32, device=dev)
+            with profiling.section("pou_warp_bwd"):
+                L.call("fvr_pou_warp_sep_adjoint", L.ptr(imgs), B, N, P, L.ptr(offs), L.ptr(sep[0]), L.ptr(sep[1]),
+                       L.ptr(ic), H, W, 1.0 / model.ds_block, float(P // 2), L.ptr(g), L.ptr(grad_imgs), L.ptr(goffs),
+                       s)
+            ws2, tiles = _block_images_adjoint(model, geo, N, grad_imgs, s)
+            del grad_imgs
+        elif (sep is not None and model.fused_warp_adjoint and g.data_ptr() % 16 == 0 and ic.data_ptr() % 16 == 0
+              and L.query("fvr_pou_warp_image_adjoint_supported", P, H, W)):
             # warp adjoint + block-image adjoint in one launch: dL/dimgs stays in shared memory
             st = model._stencil
             wsb = L.query("fvr_pou_slice_image_adjoint_workspace", B, N)
@@ -328,7 +358,7 @@ class PerspectiveSlabFVR(nn.Module):
                  dtype=torch.float32, use_triton=True, device=None):
         super().__init__()
         self.use_triton = bool(use_triton)
-        # pinhole adjoint: warp + block-image adjoint in one launch on separable lattices
+        # pinhole adjoint on separable lattices: by gathers (off: the general scatter)
         self.fused_warp_adjoint = True
         self._compiled_project_core = None
         self._compiled_project_invariant = None
@@ -520,7 +550,7 @@ class PerspectiveSlabFVR(nn.Module):
             H, W = int(lattice[1].shape[0]), int(lattice[1].shape[1])
             return torch.zeros((0, 1, H, W), dtype=torch.float32, device=home) + 0.0 * pose_mats.sum()
         if len(lattice) >= 11:
-            key, _, (rx, ry, ic), _, _ = _prepared_lattice(lattice, self._dev)
+            key, _, (rx, ry, ic), _, _, _ = _prepared_lattice(lattice, self._dev)
             mats = pose_mats if home == self._dev else pose_mats.to(self._dev)
             out = _PinholeFn.apply(mats, self, rx, ry, ic, key)
         else:

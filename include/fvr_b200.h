@@ -320,6 +320,21 @@ int64_t fvr_pou_slice_image_adjoint_workspace(int64_t B, int64_t N);
 int fvr_pou_slice_image_adjoint(int dtype, const void* stencil, const float* scales, int64_t B, int64_t P,
                                 const double* geo, int64_t N, const float* freqs, const float* grad_imgs,
                                 void* workspace, int64_t ws_bytes, void* stream);
+/* Pinhole warp + sum on a separable lattice: every pixel of detector column c
+ * has ray coordinate rxc[c] and every pixel of row r ryr[r] (f32); offs[B][N][3]
+ * = (d_b, cu, cv) fp64, ic[H*W].  out[N][H*W].
+ * The adjoint (rxc and ryr monotone) writes grad_imgs[B][N][P][P] (every
+ * element, nothing to clear) and goffs[3][B][N] = dL/d(d_b, cu, cv).
+ * Replaces pou_pinhole_warp_sum on the invariant lattice,
+ * triton_slice.py:341-496. */
+int fvr_pou_warp_sep_supported(int64_t P, int64_t H, int64_t W);
+int fvr_pou_warp_sep(const float* imgs, int64_t B, int64_t N, int64_t P, const double* offs, const float* rxc,
+                     const float* ryr, const float* ic, int64_t H, int64_t W, double inv_ds, double c_idx, float* out,
+                     void* stream);
+int fvr_pou_warp_sep_adjoint_supported(int64_t P, int64_t H, int64_t W);
+int fvr_pou_warp_sep_adjoint(const float* imgs, int64_t B, int64_t N, int64_t P, const double* offs, const float* rxc,
+                             const float* ryr, const float* ic, int64_t H, int64_t W, double inv_ds, double c_idx,
+                             const float* gout, float* grad_imgs, double* goffs, void* stream);
 /* Fused warp + block-image adjoint for a separable pinhole lattice (every
  * detector column shares one ray coordinate rxc[c], every row one ryr[r]):
  * from the detector gradient gout[N][H][W] (times ic[H][W]) and the forward
