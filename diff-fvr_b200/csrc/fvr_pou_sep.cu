@@ -39,10 +39,10 @@ __device__ __forceinline__ int sep_cell(double scale, double off, float ray, int
 // forward
 // ----------------------------------------------------------------------------
 
-constexpr int kSepThreads = 128;
+constexpr int kSepCols = 4;       // detector columns per thread
 constexpr int kSepBlocks = 32;    // blocks per round of the row table
-constexpr int kSepStages = 4;     // image-row slabs in flight
-constexpr int kSepSlabRows = 16;  // image rows a slab holds
+constexpr int kSepRingRows = 36;  // image rows of the slab ring
+constexpr int kSepStages = 4;     // slabs in the ring at most
 
 __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
   const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
@@ -54,38 +54,45 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+__device__ __forceinline__ float2 sub2(float2 x, float2 y) { return __ffma2_rn(y, make_float2(-1.f, -1.f), x); }
+__device__ __forceinline__ float2 bcast(float x) { return make_float2(x, x); }
+
 // out[n][r][c] = ic sum_b bilinear(imgs[b][n]).  A CTA owns RG detector rows x
-// 128 NC columns of one pose and runs over the blocks that touch its rows.
-// The image rows those detector rows sample are one contiguous piece of the
-// block image; it is copied to shared memory three blocks ahead (read on
-// demand, every image row cost one trip to memory: 567 us).  Per block a lane
-// interpolates each image row at its columns once and blends neighbouring
-// rows per detector row.
-// RG = 16 from two CTAs per SM on, 4 below, where the blocks' serial chain
-// counts more than the row reuse.  A kernel with one thread per pixel and the
-// row pairs blended in shared memory took 394 us for 64 blocks x 64 poses x
-// 256^2 pixels and 429 us for 8 blocks x 64 poses x 512^2 pixels.
-template <int RG, int NC>
-__global__ void __launch_bounds__(kSepThreads) pou_warp_sep_kernel(SepArgs a, int tiles, float* __restrict__ out) {
-  extern __shared__ __align__(16) float slab[];  // [kSepStages][kSepSlabRows * P]
+// 4 columns per thread of one pose and runs over the blocks that touch its
+// rows.  The image rows those detector rows sample are one contiguous piece of
+// the block image, copied to shared memory up to three blocks ahead (read on
+// demand, every image row cost a trip to memory: 567 us).  Per block a lane
+// interpolates each image row at its columns once, blends neighbouring rows
+// per detector row, and does both in f32x2 pairs.
+// More rows reuse an image row more often, fewer leave more CTAs (the rule is
+// at the launch).  Bound by dependent issue at 14 warps per SM.  64 blocks x 64
+// poses x 256^2 pixels: 207 us, and 394 us for a kernel with one thread per
+// pixel and the row pairs blended in shared memory; 8 blocks x 64 poses x
+// 512^2 pixels: 95 and 429 us.
+template <int RG>
+__global__ void __launch_bounds__(128) pou_warp_sep_kernel(SepArgs a, int tiles, float* __restrict__ out) {
+  constexpr int NC = kSepCols;
+  extern __shared__ __align__(16) float ring[];  // [kSepRingRows * P]
   __shared__ int2 rows[kSepBlocks][RG];          // (iy, ty) of the band's detector rows per block
-  __shared__ int list[kSepBlocks], first[kSepBlocks], count[kSepBlocks], n_live;  // live blocks and their image rows
-  const int n = blockIdx.y;
+  __shared__ int list[kSepBlocks], first[kSepBlocks], count[kSepBlocks];  // live blocks and their image rows
+  __shared__ double2 xmap[kSepBlocks];  // image column of a ray: xmap.x rx + xmap.y
+  __shared__ int n_live, slot_rows;
+  const int T = blockDim.x, n = blockIdx.y;
   const int band = blockIdx.x / tiles, tile = blockIdx.x - band * tiles;
-  const int P = a.P, r0 = band * RG, c0 = tile * kSepThreads * NC + threadIdx.x;
+  const int P = a.P, r0 = band * RG, c0 = tile * T * NC + threadIdx.x;
   const bool aligned = (P & 3) == 0 && (reinterpret_cast<uintptr_t>(a.imgs) & 15) == 0;
   float rx[NC];
 #pragma unroll
-  for (int j = 0; j < NC; ++j) rx[j] = c0 + kSepThreads * j < a.W ? __ldg(a.rxc + c0 + kSepThreads * j) : 0.f;
-  float acc[RG][NC];
+  for (int j = 0; j < NC; ++j) rx[j] = c0 + T * j < a.W ? __ldg(a.rxc + c0 + T * j) : 0.f;
+  float2 acc[RG][NC / 2];
 #pragma unroll
   for (int r = 0; r < RG; ++r)
 #pragma unroll
-    for (int j = 0; j < NC; ++j) acc[r][j] = 0.f;
+    for (int h = 0; h < NC / 2; ++h) acc[r][h] = bcast(0.f);
   for (int b0 = 0; b0 < a.B; b0 += kSepBlocks) {
     const int nb = min(kSepBlocks, a.B - b0);
     __syncthreads();  // the previous round's tables and slabs are no longer read
-    for (int e = threadIdx.x; e < nb * RG; e += kSepThreads) {
+    for (int e = threadIdx.x; e < nb * RG; e += T) {
       const int k = e / RG, r = e - k * RG;
       const double* o = a.offs + 3 * (static_cast<int64_t>(b0 + k) * a.N + n);
       float t = 0.f;
@@ -97,6 +104,10 @@ __global__ void __launch_bounds__(kSepThreads) pou_warp_sep_kernel(SepArgs a, in
     if (threadIdx.x < 32) {  // blocks in increasing order, with the image rows they need
       const int k = threadIdx.x;
       int lo = 0x7fffffff, hi = -1;
+      if (k < nb) {
+        const double* o = a.offs + 3 * (static_cast<int64_t>(b0 + k) * a.N + n);
+        xmap[k] = make_double2(o[0] * a.inv_ds, a.c_idx - o[1] * a.inv_ds);
+      }
       if (k < nb)
         for (int r = 0; r < RG; ++r) {
           const int iy = rows[k][r].x;
@@ -106,45 +117,58 @@ __global__ void __launch_bounds__(kSepThreads) pou_warp_sep_kernel(SepArgs a, in
           }
         }
       const unsigned m = __ballot_sync(0xffffffffu, hi >= 0);
+      const int need = hi >= 0 ? hi - lo + 1 : 0;
+      const bool fits = aligned && need <= kSepRingRows;
       if (hi >= 0) {
         const int i = __popc(m & ((1u << k) - 1u));
         list[i] = k;
         first[i] = lo;
-        count[i] = aligned && hi - lo < kSepSlabRows ? hi - lo + 1 : 0;  // 0: read from memory
+        count[i] = fits ? need : 0;  // 0: read from memory
       }
-      if (k == 0) n_live = __popc(m);
+      const int most = __reduce_max_sync(0xffffffffu, fits ? need : 0);
+      if (k == 0) {
+        n_live = __popc(m);
+        slot_rows = max(most, 1);
+      }
     }
     __syncthreads();
-    const int live = n_live;
+    const int live = n_live, slot = slot_rows * P, stages = min(kSepStages, kSepRingRows / slot_rows);
     auto fetch = [&](int i) {
       if (i < live) {
         const int q = count[i] * (P >> 2);
         const float* src = a.imgs + (static_cast<int64_t>(b0 + list[i]) * a.N + n) * P * P + first[i] * P;
-        float* dst = slab + (i % kSepStages) * kSepSlabRows * P;
-        for (int e = threadIdx.x; e < q; e += kSepThreads) cp_async16(dst + 4 * e, src + 4 * e);
+        float* dst = ring + (i % stages) * slot;
+        for (int e = threadIdx.x; e < q; e += T) cp_async16(dst + 4 * e, src + 4 * e);
       }
       cp_async_commit();
     };
-#pragma unroll
-    for (int i = 0; i < kSepStages - 1; ++i) fetch(i);
+    for (int i = 0; i < stages - 1; ++i) fetch(i);
     for (int i = 0; i < live; ++i) {
-      const int64_t bn = static_cast<int64_t>(b0 + list[i]) * a.N + n;
-      const double* o = a.offs + 3 * bn;
-      const double sx = __ldg(o) * a.inv_ds, ox = a.c_idx - __ldg(o + 1) * a.inv_ds;
+      const double2 xm = xmap[list[i]];
       int ix[NC];
-      float tx[NC];
+      float tj[NC];
       bool in0[NC], in1[NC];
 #pragma unroll
       for (int j = 0; j < NC; ++j) {
-        ix[j] = sep_cell(sx, ox, rx[j], P, tx[j]);
+        ix[j] = sep_cell(xm.x, xm.y, rx[j], P, tj[j]);
         in0[j] = ix[j] >= 0 && ix[j] < P;
         in1[j] = ix[j] >= -1 && ix[j] + 1 < P;
       }
-      cp_async_wait<kSepStages - 2>();
-      __syncthreads();  // slab i has landed for every thread; slab i - 1 is no longer read
-      fetch(i + kSepStages - 1);
-      int cur = -3;           // the march is in image cell `cur`
-      float lo[NC], hi[NC];   // x-interpolated rows cur and cur + 1
+      // slab i has landed for every thread, and slab i - 1 is no longer read
+      if (stages == 1) {
+        __syncthreads();
+        fetch(i);
+        cp_async_wait<0>();
+        __syncthreads();
+      } else {
+        if (stages == 2) cp_async_wait<0>();
+        else if (stages == 3) cp_async_wait<1>();
+        else cp_async_wait<2>();
+        __syncthreads();
+        fetch(i + stages - 1);
+      }
+      int cur = -3;                         // the march is in image cell `cur`
+      float2 lo[NC / 2], hi[NC / 2], dv[NC / 2];  // x-interpolated rows cur and cur + 1, their difference
       auto march = [&](auto row) {
 #pragma unroll
         for (int r = 0; r < RG; ++r) {
@@ -153,33 +177,51 @@ __global__ void __launch_bounds__(kSepThreads) pou_warp_sep_kernel(SepArgs a, in
           if (e.x != cur) {
             if (e.x == cur + 1) {
 #pragma unroll
-              for (int j = 0; j < NC; ++j) lo[j] = hi[j];
+              for (int h = 0; h < NC / 2; ++h) lo[h] = hi[h];
             } else {
               row(e.x, lo);
             }
             row(e.x + 1, hi);
+#pragma unroll
+            for (int h = 0; h < NC / 2; ++h) dv[h] = sub2(hi[h], lo[h]);
             cur = e.x;
           }
-          const float ty = __int_as_float(e.y);
+          const float2 ty = bcast(__int_as_float(e.y));
 #pragma unroll
-          for (int j = 0; j < NC; ++j) acc[r][j] += fmaf(ty, hi[j] - lo[j], lo[j]);
+          for (int h = 0; h < NC / 2; ++h) acc[r][h] = __ffma2_rn(ty, dv[h], __fadd2_rn(acc[r][h], lo[h]));
         }
       };
-      auto interpolate = [&](const float* q, bool in, float (&v)[NC]) {
+      float v0[NC], v1[NC];  // columns outside the image keep their zeros
+#pragma unroll
+      for (int j = 0; j < NC; ++j) v0[j] = v1[j] = 0.f;
+      auto interpolate = [&](const float* q, float2 (&v)[NC / 2]) {
 #pragma unroll
         for (int j = 0; j < NC; ++j) {
-          float v0 = 0.f, v1 = 0.f;
-          if (in && in0[j] && fvr_checked(ix[j], P, kSiteWarpTap)) v0 = q[ix[j]];
-          if (in && in1[j] && fvr_checked(ix[j] + 1, P, kSiteWarpTap)) v1 = q[ix[j] + 1];
-          v[j] = fmaf(tx[j], v1 - v0, v0);
+          if (in0[j] && fvr_checked(ix[j], P, kSiteWarpTap)) v0[j] = q[ix[j]];
+          if (in1[j] && fvr_checked(ix[j] + 1, P, kSiteWarpTap)) v1[j] = q[ix[j] + 1];
+        }
+#pragma unroll
+        for (int h = 0; h < NC / 2; ++h) {
+          const float2 u0 = make_float2(v0[2 * h], v0[2 * h + 1]), u1 = make_float2(v1[2 * h], v1[2 * h + 1]);
+          v[h] = __ffma2_rn(make_float2(tj[2 * h], tj[2 * h + 1]), sub2(u1, u0), u0);
         }
       };
+      auto clear = [&](float2 (&v)[NC / 2]) {
+#pragma unroll
+        for (int h = 0; h < NC / 2; ++h) v[h] = bcast(0.f);
+      };
       if (count[i] > 0) {
-        const float* base = slab + (i % kSepStages) * kSepSlabRows * P - first[i] * P;
-        march([&](int y, float (&v)[NC]) { interpolate(base + y * P, y >= 0 && y < P, v); });
+        const float* base = ring + (i % stages) * slot - first[i] * P;
+        march([&](int y, float2 (&v)[NC / 2]) {
+          if (y >= 0 && y < P) interpolate(base + y * P, v);
+          else clear(v);
+        });
       } else {
-        const float* img = a.imgs + bn * P * P;
-        march([&](int y, float (&v)[NC]) { interpolate(img + static_cast<int64_t>(y) * P, y >= 0 && y < P, v); });
+        const float* img = a.imgs + (static_cast<int64_t>(b0 + list[i]) * a.N + n) * P * P;
+        march([&](int y, float2 (&v)[NC / 2]) {
+          if (y >= 0 && y < P) interpolate(img + static_cast<int64_t>(y) * P, v);
+          else clear(v);
+        });
       }
     }
     cp_async_wait<0>();
@@ -188,12 +230,68 @@ __global__ void __launch_bounds__(kSepThreads) pou_warp_sep_kernel(SepArgs a, in
   for (int r = 0; r < RG; ++r) {
     if (r0 + r < a.Hd) {
       const int64_t q = static_cast<int64_t>(r0 + r) * a.W;
+      const float v[NC] = {acc[r][0].x, acc[r][0].y, acc[r][1].x, acc[r][1].y};
 #pragma unroll
       for (int j = 0; j < NC; ++j) {
-        const int c = c0 + kSepThreads * j;
-        if (c < a.W) out[static_cast<int64_t>(n) * a.Hd * a.W + q + c] = acc[r][j] * __ldg(a.ic + q + c);
+        const int c = c0 + T * j;
+        if (c < a.W) out[static_cast<int64_t>(n) * a.Hd * a.W + q + c] = v[j] * __ldg(a.ic + q + c);
       }
     }
+  }
+}
+
+// The same for few poses, where the marching kernel's serial chain over the
+// blocks shows (1 pose, 8 blocks, 256^2 pixels: 10.4 us): a CTA owns 4 rows x
+// 32 columns, its 8 warps take every eighth block each and their sums meet in
+// shared memory.  All taps of a block are independent loads.
+constexpr int kSepFewRows = 4, kSepFewWarps = 8;
+
+__global__ void __launch_bounds__(32 * kSepFewWarps) pou_warp_sep_few_kernel(SepArgs a, int tiles,
+                                                                             float* __restrict__ out) {
+  constexpr int RG = kSepFewRows;
+  __shared__ float part[kSepFewWarps][RG][32];
+  const int n = blockIdx.y, P = a.P, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int band = blockIdx.x / tiles, r0 = band * RG, c = (blockIdx.x - band * tiles) * 32 + lane;
+  const float rx = c < a.W ? __ldg(a.rxc + c) : 0.f;
+  const float ry = lane < RG && r0 + lane < a.Hd ? __ldg(a.ryr + r0 + lane) : 0.f;
+  float acc[RG];
+#pragma unroll
+  for (int r = 0; r < RG; ++r) acc[r] = 0.f;
+  for (int b = wid; b < a.B; b += kSepFewWarps) {
+    const int64_t bn = static_cast<int64_t>(b) * a.N + n;
+    const double* o = a.offs + 3 * bn;
+    const double sc = __ldg(o) * a.inv_ds;
+    float tx, ty;
+    const int ix = sep_cell(sc, a.c_idx - __ldg(o + 1) * a.inv_ds, rx, P, tx);
+    int iy = sep_cell(sc, a.c_idx - __ldg(o + 2) * a.inv_ds, ry, P, ty);  // lane r: detector row r
+    if (lane >= RG || r0 + lane >= a.Hd) iy = -2;
+    const float* img = a.imgs + bn * P * P;
+    const bool x0 = ix >= 0 && ix < P, x1 = ix >= -1 && ix + 1 < P;
+    float v[RG][4], t[RG];
+#pragma unroll
+    for (int r = 0; r < RG; ++r) {
+      const int y = __shfl_sync(0xffffffffu, iy, r);
+      t[r] = __shfl_sync(0xffffffffu, ty, r);
+      const bool y0 = y >= 0 && y < P, y1 = y >= -1 && y + 1 < P;
+      v[r][0] = x0 && y0 ? ldg_in(img, y * P + ix, P * P, kSiteWarpTap) : 0.f;
+      v[r][1] = x1 && y0 ? ldg_in(img, y * P + ix + 1, P * P, kSiteWarpTap) : 0.f;
+      v[r][2] = x0 && y1 ? ldg_in(img, (y + 1) * P + ix, P * P, kSiteWarpTap) : 0.f;
+      v[r][3] = x1 && y1 ? ldg_in(img, (y + 1) * P + ix + 1, P * P, kSiteWarpTap) : 0.f;
+    }
+#pragma unroll
+    for (int r = 0; r < RG; ++r) {
+      const float lo = fmaf(tx, v[r][1] - v[r][0], v[r][0]), hi = fmaf(tx, v[r][3] - v[r][2], v[r][2]);
+      acc[r] += fmaf(t[r], hi - lo, lo);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < RG; ++r) part[wid][r][lane] = acc[r];
+  __syncthreads();
+  if (wid < RG && r0 + wid < a.Hd && c < a.W) {
+    float s = 0.f;
+    for (int k = 0; k < kSepFewWarps; ++k) s += part[k][wid][lane];
+    const int64_t q = static_cast<int64_t>(r0 + wid) * a.W + c;
+    out[static_cast<int64_t>(n) * a.Hd * a.W + q] = s * __ldg(a.ic + q);
   }
 }
 
@@ -205,11 +303,12 @@ constexpr int kSepBand = 8;      // image rows of a unit at most
 constexpr int kSepPass = 128;    // detector columns of a march, four per lane
 constexpr int kSepWide = 256;    // detector columns of a warp's G buffer
 
-// Dynamic shared memory: column map (ix, tx) [W], row fractions [Hd], first
+// Dynamic shared memory: column map (ix, tx) [Wp] (W rounded up to four), row fractions [Hd], first
 // table position at or beyond each image index [P + 3] for columns and rows,
 // the warps' G buffers.
+__host__ __device__ constexpr int sep_padded(int W) { return (W + 3) / 4 * 4; }
 __host__ __device__ constexpr int64_t sep_adj_gbuf_at(int P, int Hd, int W) {
-  return (8LL * W + 4LL * Hd + 8LL * (P + 3) + 15) / 16 * 16;
+  return (8LL * sep_padded(W) + 4LL * Hd + 8LL * (P + 3) + 15) / 16 * 16;
 }
 __host__ __device__ constexpr int64_t sep_adj_smem(int P, int Hd, int W, int warps) {
   return sep_adj_gbuf_at(P, Hd, W) + 4LL * warps * kSepBand * kSepWide;
@@ -217,6 +316,7 @@ __host__ __device__ constexpr int64_t sep_adj_smem(int P, int Hd, int W, int war
 
 struct SepGrad {
   const float* gout;  // [N][Hd W]
+  const float4* gic;  // [N][Hd][Wp / 4]: gout ic, rows padded with zeros
   float* gimgs;       // [B][N][P][P]
   double* goffs;      // [3][B][N]: dL/d(d_b, cu, cv)
 };
@@ -232,25 +332,46 @@ __device__ __forceinline__ void sep_first(int* first, int count, int P, F cell) 
   }
 }
 
-__device__ __forceinline__ float2 sub2(float2 x, float2 y) { return __ffma2_rn(y, make_float2(-1.f, -1.f), x); }
-__device__ __forceinline__ float2 bcast(float x) { return make_float2(x, x); }
+// gic[n][r][c] = g[n][r][c] ic[r][c] with the rows padded by zeros to a
+// multiple of four columns: the adjoint reads every detector row once per
+// block, as aligned 16-byte words whatever the detector's width.
+__global__ void __launch_bounds__(256) pou_warp_sep_weigh_kernel(const float* __restrict__ g,
+                                                                 const float* __restrict__ ic, int Hd, int W, int Wp,
+                                                                 bool vec, float4* __restrict__ gic) {
+  const int quads = Hd * (Wp / 4), q = blockIdx.x * 256 + threadIdx.x;
+  if (q >= quads) return;
+  const int row = q / (Wp / 4), c = 4 * (q - row * (Wp / 4));
+  const float *gp = g + (static_cast<int64_t>(blockIdx.y) * Hd + row) * W + c, *ip = ic + static_cast<int64_t>(row) * W + c;
+  float4 v;
+  if (vec) {  // W a multiple of four, 16-byte aligned inputs
+    const float4 a = __ldg(reinterpret_cast<const float4*>(gp)), b = __ldg(reinterpret_cast<const float4*>(ip));
+    v = make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w);
+  } else {
+    v.x = __ldg(gp) * __ldg(ip);
+    v.y = c + 1 < W ? __ldg(gp + 1) * __ldg(ip + 1) : 0.f;
+    v.z = c + 2 < W ? __ldg(gp + 2) * __ldg(ip + 2) : 0.f;
+    v.w = c + 3 < W ? __ldg(gp + 3) * __ldg(ip + 3) : 0.f;
+  }
+  gic[static_cast<int64_t>(blockIdx.y) * quads + q] = v;
+}
 
 // One CTA per (pose, block).  Its units are bands of image rows (those the
 // detector reaches, split evenly over the warps) x groups of image columns
 // whose detector columns fit a G buffer; a warp takes a unit and writes
 // dL/dimgs there, every element once (nothing to clear, no atomics):
 //   march down the detector rows of cell y0 - 1, y0, .. for 128 detector
-//   columns at a time, four per lane in f32x2 pairs, keeping the cell's sums
+//   columns at a time, four neighbours per lane in f32x2 pairs, keeping the cell's sums
 //   A0 = sum g ic and A1 = sum ty g ic; leaving cell y gives G[y][c] =
 //   (A0 - A1)(y) + A1(y - 1) and, with the image row's value and slope at the
 //   column, the pose-offset sums;
 //   then lane x gathers G[y][c] over its detector columns, weight 1 - |px(c) - x|.
 // The sum of g ry dv/dpy comes from ry = (y + ty - oy) / scale: per cell
 // (y - oy) A0 + A1, so no third sum is kept while marching.
-// It replaced a gather along x for every detector row inside the slice-adjoint
-// kernel (that kernel took 1422 us for 64 blocks x 64 poses x 256^2 pixels)
-// and, for detectors that one could not take, a scatter with atomics (998 +
-// 106 us for 8 blocks x 64 poses x 512^2 pixels).
+// Bound by issue at 16 warps per SM (50 % issue active; three CTAs per SM
+// spill: 974 us).  64 blocks x 64 poses x 256^2 pixels: 495 us, with the
+// separate slice adjoint 1232 us against 1422 us for a gather along x of every
+// detector row inside the slice-adjoint kernel; 8 blocks x 64 poses x 512^2
+// pixels: 265 us against 1104 us for a scatter with atomics.
 template <int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(SepArgs a, SepGrad w) {
   constexpr int NW = THREADS / 32;
@@ -258,9 +379,9 @@ __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(Sep
   __shared__ double red[4][NW];
   // per thread: sums of g dv/dpx, g rx dv/dpx, g dv/dpy, g (y + ty - oy) dv/dpy (no registers held while marching)
   __shared__ double sums[4][THREADS];
-  const int P = a.P, Hd = a.Hd, W = a.W;
-  int2* cmap = reinterpret_cast<int2*>(smem);             // (ix, tx) per detector column
-  float* rty = reinterpret_cast<float*>(cmap + W);        // ty per detector row, in march order
+  const int P = a.P, Hd = a.Hd, W = a.W, Wp = sep_padded(W);
+  int2* cmap = reinterpret_cast<int2*>(smem);             // (ix, tx) per detector column, -2 in the padding
+  float* rty = reinterpret_cast<float*>(cmap + Wp);       // ty per detector row, in march order
   int* cfirst = reinterpret_cast<int*>(rty + Hd);
   int* rfirst = cfirst + (P + 3);
   const int n = blockIdx.x, b = blockIdx.y;
@@ -274,9 +395,9 @@ __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(Sep
   int* rcell = reinterpret_cast<int*>(smem + sep_adj_gbuf_at(P, Hd, W));  // in the G buffers until they are used
 #pragma unroll
   for (int k = 0; k < 4; ++k) sums[k][threadIdx.x] = 0.0;
-  for (int c = threadIdx.x; c < W; c += THREADS) {
-    float t;
-    const int i = sep_cell(sc, ox, __ldg(a.rxc + c), P, t);
+  for (int c = threadIdx.x; c < Wp; c += THREADS) {
+    float t = 0.f;
+    const int i = c < W ? sep_cell(sc, ox, __ldg(a.rxc + c), P, t) : -2;
     cmap[c] = make_int2(i, __float_as_int(t));
   }
   for (int k = threadIdx.x; k < Hd; k += THREADS) rcell[k] = sep_cell(sc, oy, __ldg(a.ryr + (rev_r ? Hd - 1 - k : k)), P, rty[k]);
@@ -321,7 +442,7 @@ __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(Sep
     for (int g = 0; g < groups; g += gs) {
       int c0, c1;
       columns(32 * g - 1, min(P, 32 * (g + gs)), c0, c1);
-      fits &= c1 - c0 <= kSepWide;
+      fits &= c1 - (c0 & ~3) <= kSepWide;
     }
     if (fits) break;
   }
@@ -337,28 +458,29 @@ __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(Sep
     const int kr0 = rfirst[y0], kr1 = rfirst[y1 + 1];  // cells y0 - 1 .. y1 - 1
     int ca, cb;
     columns(x0 - 1, x1, ca, cb);
-    float gsum[kSepBand];
+    float2 gsum[kSepBand / 2];  // rows 2 i, 2 i + 1
 #pragma unroll
-    for (int i = 0; i < kSepBand; ++i) gsum[i] = 0.f;
+    for (int i = 0; i < kSepBand / 2; ++i) gsum[i] = bcast(0.f);
     if (ca >= cb || kr0 >= kr1) {  // nothing reaches this unit
       for (int x = x0 + lane; x < x1; x += 32)
-        for (int y = y0; y < y1; ++y) gimg[static_cast<int64_t>(y) * P + x] = 0.f;
+        for (int y = y0; y < y1; ++y) gimg[y * P + x] = 0.f;
       continue;
     }
-    for (int kp = ca; kp < cb; kp += kSepWide) {  // several only for a single 32-column group
+    const int cs = ca & ~3;  // 16-byte words of a detector row
+    for (int kp = cs; kp < cb; kp += kSepWide) {  // several only for a single 32-column group
       const int ke = min(cb, kp + kSepWide);
       for (int sp = kp; sp < ke; sp += kSepPass) {
-        const int c = sp + lane;
+        const int c = sp + 4 * lane;
+        const bool on = c < Wp;
         float2 tx[2], A0[2], A1[2], p0[2], p1[2], Lp[2], sx[2], v0[2], v1[2], fy[2], f1[2];
         int ix[4];
-        bool on[4], in0[4], in1[4];  // column inside the detector; image values ix, ix + 1 belong to the sums
+        bool in0[4], in1[4];  // image values ix, ix + 1 belong to the sums
         float tj[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          on[j] = c + 32 * j < W;
-          const int2 e = on[j] ? cmap[c + 32 * j] : make_int2(-2, 0);
+          const int2 e = on ? cmap[c + j] : make_int2(-2, 0);
           // a column's sums belong to the unit that holds image column max(ix, 0)
-          const bool own = c + 32 * j < ke && max(e.x, 0) >= x0 && e.x < x1;
+          const bool own = c + j >= ca && c + j < ke && e.x >= -1 && max(e.x, 0) >= x0 && e.x < x1;
           ix[j] = e.x;
           tj[j] = __int_as_float(e.y);
           in0[j] = own && e.x >= 0;
@@ -380,28 +502,22 @@ __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(Sep
           if (in1[2]) v1[1].x = ldg_in(q, ix[2] + 1, P, kSiteWarpTap);
           if (in1[3]) v1[1].y = ldg_in(q, ix[3] + 1, P, kSiteWarpTap);
         };
-        const int64_t step = rev_r ? -static_cast<int64_t>(W) : W;
-        const float* gq = gout + static_cast<int64_t>(rev_r ? Hd - 1 - kr0 : kr0) * W + c;
-        const float* iq = a.ic + static_cast<int64_t>(rev_r ? Hd - 1 - kr0 : kr0) * W + c;
-        float2 gn[2], in[2];  // the next detector row's values
-        gn[0] = gn[1] = in[0] = in[1] = bcast(0.f);
-        auto load_row = [&]() {
-          if (on[0]) gn[0].x = __ldg(gq), in[0].x = __ldg(iq);
-          if (on[1]) gn[0].y = __ldg(gq + 32), in[0].y = __ldg(iq + 32);
-          if (on[2]) gn[1].x = __ldg(gq + 64), in[1].x = __ldg(iq + 64);
-          if (on[3]) gn[1].y = __ldg(gq + 96), in[1].y = __ldg(iq + 96);
-          gq += step;
-          iq += step;
-        };
+        const int step = rev_r ? -(Wp / 4) : Wp / 4;
+        const float4* gq = w.gic + (static_cast<int64_t>(n) * Hd + (rev_r ? Hd - 1 - kr0 : kr0)) * (Wp / 4) + c / 4;
+        float4 gn = make_float4(0.f, 0.f, 0.f, 0.f), gm = gn;  // the next two detector rows' values
         int kr = kr0;
-        load_row();
+        if (on) gn = __ldg(gq);
+        gq += step;
+        if (on && kr + 1 < kr1) gm = __ldg(gq);
         auto cell = [&](int kend) {
 #pragma unroll
           for (int h = 0; h < 2; ++h) A0[h] = A1[h] = bcast(0.f);
           for (; kr < kend; ++kr) {
             const float2 ty = bcast(rty[kr]);
-            const float2 g0 = __fmul2_rn(gn[0], in[0]), g1 = __fmul2_rn(gn[1], in[1]);
-            if (kr + 1 < kr1) load_row();
+            const float2 g0 = make_float2(gn.x, gn.y), g1 = make_float2(gn.z, gn.w);
+            gn = gm;
+            gq += step;
+            if (on && kr + 2 < kr1) gm = __ldg(gq);
             A0[0] = __fadd2_rn(A0[0], g0);
             A0[1] = __fadd2_rn(A0[1], g1);
             A1[0] = __ffma2_rn(ty, g0, A1[0]);
@@ -423,19 +539,18 @@ __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(Sep
           load_image(y);
           cell(rfirst[y + 2]);
           const float2 yo = bcast(static_cast<float>(static_cast<double>(y - 1) - oy));
-          float* Gy = G + (y - y0) * kSepWide + (sp - kp) + lane;
+          float2 g[2];
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            const float2 g = __fadd2_rn(sub2(A0[h], A1[h]), p1[h]);
-            Gy[64 * h] = g.x;
-            Gy[64 * h + 32] = g.y;
+            g[h] = __fadd2_rn(sub2(A0[h], A1[h]), p1[h]);
             const float2 d = sub2(v1[h], v0[h]);
             const float2 L = __ffma2_rn(tx[h], d, v0[h]), D = sub2(L, Lp[h]);
             Lp[h] = L;
-            sx[h] = __ffma2_rn(g, d, sx[h]);
+            sx[h] = __ffma2_rn(g[h], d, sx[h]);
             fy[h] = __ffma2_rn(p0[h], D, fy[h]);  // cell y - 1
             f1[h] = __ffma2_rn(__ffma2_rn(yo, p0[h], p1[h]), D, f1[h]);
           }
+          *reinterpret_cast<float4*>(G + (y - y0) * kSepWide + (c - kp)) = make_float4(g[0].x, g[0].y, g[1].x, g[1].y);
         }
         if (y1 == P) {  // the last cell's lower row lies outside the image
           const float2 yo = bcast(static_cast<float>(static_cast<double>(P - 1) - oy));
@@ -446,41 +561,44 @@ __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(Sep
             f1[h] = __ffma2_rn(__ffma2_rn(yo, A0[h], A1[h]), D, f1[h]);
           }
         }
-        double dx = 0.0, drx = 0.0;
         const float sj[4] = {sx[0].x, sx[0].y, sx[1].x, sx[1].y};
+        float dx = 0.f, drx = 0.f;
 #pragma unroll
         for (int j = 0; j < 4; ++j)
           if (in0[j] || in1[j]) {
-            dx += static_cast<double>(sj[j]);
-            drx += static_cast<double>(sj[j]) * static_cast<double>(__ldg(a.rxc + c + 32 * j));
+            dx += sj[j];
+            drx = fmaf(sj[j], __ldg(a.rxc + c + j), drx);
           }
-        sums[0][threadIdx.x] += dx;
-        sums[1][threadIdx.x] += drx;
+        sums[0][threadIdx.x] += static_cast<double>(dx);
+        sums[1][threadIdx.x] += static_cast<double>(drx);
         sums[2][threadIdx.x] += static_cast<double>((fy[0].x + fy[0].y) + (fy[1].x + fy[1].y));
         sums[3][threadIdx.x] += static_cast<double>((f1[0].x + f1[0].y) + (f1[1].x + f1[1].y));
       }
       __syncwarp();
       for (int xg = x0; xg < x1; xg += 32) {
         const int x = xg + lane;
-        if (kp == ca)
+        if (kp == cs)
 #pragma unroll
-          for (int i = 0; i < kSepBand; ++i) gsum[i] = 0.f;
+          for (int i = 0; i < kSepBand / 2; ++i) gsum[i] = bcast(0.f);
         int t0 = 0, t1 = 0;
         if (x < x1) columns(x - 1, x + 1, t0, t1);
         t1 = min(t1, ke);
         for (int k = max(t0, kp); k < t1; ++k) {
           const int2 e = cmap[k];
-          const float t = __int_as_float(e.y), wt = e.x == x ? 1.f - t : t;
+          const float t = __int_as_float(e.y);
+          const float2 wt = bcast(e.x == x ? 1.f - t : t);
           const float* q = G + (k - kp);
 #pragma unroll
-          for (int i = 0; i < kSepBand; ++i)
-            if (fvr_checked(i * kSepWide + k - kp, kSepBand * kSepWide, kSiteWarpFused))
-              gsum[i] = fmaf(wt, q[i * kSepWide], gsum[i]);
+          for (int i = 0; i < kSepBand / 2; ++i)
+            if (fvr_checked((2 * i + 1) * kSepWide + k - kp, kSepBand * kSepWide, kSiteWarpFused))
+              gsum[i] = __ffma2_rn(wt, make_float2(q[2 * i * kSepWide], q[(2 * i + 1) * kSepWide]), gsum[i]);
         }
         if (ke == cb && x < x1) {
 #pragma unroll
-          for (int i = 0; i < kSepBand; ++i)
-            if (y0 + i < y1) gimg[static_cast<int64_t>(y0 + i) * P + x] = gsum[i];
+          for (int i = 0; i < kSepBand / 2; ++i) {
+            if (y0 + 2 * i < y1) gimg[(y0 + 2 * i) * P + x] = gsum[i].x;
+            if (y0 + 2 * i + 1 < y1) gimg[(y0 + 2 * i + 1) * P + x] = gsum[i].y;
+          }
         }
       }
       __syncwarp();
@@ -542,27 +660,18 @@ static int sep_adjoint(const SepArgs& a, const SepGrad& w, cudaStream_t s) {
   return FVR_OK;
 }
 
-template <int RG, int NC>
+template <int RG>
 static int sep_forward(const SepArgs& a, float* out, cudaStream_t s) {
-  const int64_t smem = 4LL * kSepStages * kSepSlabRows * a.P;
+  const int64_t smem = 4LL * kSepRingRows * a.P;
   if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(pou_warp_sep_kernel<RG, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      cudaFuncSetAttribute(pou_warp_sep_kernel<RG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(smem)) != cudaSuccess)
     return FVR_ERR_CUDA;
-  const int tiles = static_cast<int>(cdiv64(a.W, kSepThreads * NC));
+  const int64_t warps = cdiv64(a.W, 32 * kSepCols), tiles = cdiv64(warps, 4), per = cdiv64(warps, tiles);
   const dim3 grid(static_cast<unsigned>(tiles * cdiv64(a.Hd, RG)), static_cast<unsigned>(a.N));
-  pou_warp_sep_kernel<RG, NC><<<grid, kSepThreads, smem, s>>>(a, tiles, out);
+  pou_warp_sep_kernel<RG><<<grid, static_cast<unsigned>(32 * per), smem, s>>>(a, static_cast<int>(tiles), out);
   FVR_LAUNCH_CHECK();
   return FVR_OK;
-}
-
-// Columns per thread: as many as a detector row has, up to four.
-template <int RG>
-static int sep_forward_cols(const SepArgs& a, float* out, cudaStream_t s) {
-  if (a.W <= kSepThreads) return sep_forward<RG, 1>(a, out, s);
-  if (a.W <= 2 * kSepThreads) return sep_forward<RG, 2>(a, out, s);
-  if (a.W <= 3 * kSepThreads) return sep_forward<RG, 3>(a, out, s);
-  return sep_forward<RG, 4>(a, out, s);
 }
 
 }  // namespace fvr
@@ -583,8 +692,16 @@ int fvr_pou_warp_sep(const float* imgs, int64_t B, int64_t N, int64_t P, const d
   if (rc) return rc;
   if (!out) return FVR_ERR_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (N * cdiv64(H, 16) * cdiv64(W, 4 * kSepThreads) >= 296) return sep_forward_cols<16>(a, out, s);
-  return sep_forward_cols<4>(a, out, s);
+  // rows per CTA by the CTAs that leaves (8 against 16 rows: 217 / 207 us at 1024 CTAs of 16 rows, 30 / 45 us at
+  // 336); below two CTAs per SM the blocks are split over warps
+  const int64_t tiles = N * cdiv64(W, 512);
+  if (tiles * cdiv64(H, 16) >= 888) return sep_forward<16>(a, out, s);
+  if (tiles * cdiv64(H, 8) >= 296) return sep_forward<8>(a, out, s);
+  const int xt = static_cast<int>(cdiv64(W, 32));
+  pou_warp_sep_few_kernel<<<dim3(static_cast<unsigned>(xt * cdiv64(H, kSepFewRows)), static_cast<unsigned>(N)),
+                            32 * kSepFewWarps, 0, s>>>(a, xt, out);
+  FVR_LAUNCH_CHECK();
+  return FVR_OK;
 }
 
 int fvr_pou_warp_sep_adjoint_supported(int64_t P, int64_t H, int64_t W) {
@@ -593,18 +710,81 @@ int fvr_pou_warp_sep_adjoint_supported(int64_t P, int64_t H, int64_t W) {
   return 4 * H <= 4LL * 8 * kSepBand * kSepWide && sep_adj_smem((int)P, (int)H, (int)W, 16) <= 200 * 1024 ? 1 : 0;
 }
 
+int64_t fvr_pou_warp_sep_adjoint_workspace(int64_t N, int64_t H, int64_t W) {
+  return N < 1 || H < 1 || W < 1 ? 0 : 4 * N * H * ((W + 3) / 4 * 4);
+}
+
 int fvr_pou_warp_sep_adjoint(const float* imgs, int64_t B, int64_t N, int64_t P, const double* offs, const float* rxc,
                              const float* ryr, const float* ic, int64_t H, int64_t W, double inv_ds, double c_idx,
-                             const float* gout, float* grad_imgs, double* goffs, void* stream) {
+                             const float* gout, void* workspace, int64_t ws_bytes, float* grad_imgs, double* goffs,
+                             void* stream) {
   SepArgs a;
   const int rc = sep_args(imgs, B, N, P, offs, rxc, ryr, ic, H, W, inv_ds, c_idx, &a);
   if (rc) return rc;
-  if (!gout || !grad_imgs || !goffs) return FVR_ERR_ARG;
+  if (!gout || !grad_imgs || !goffs || !workspace || (reinterpret_cast<uintptr_t>(workspace) & 15)) return FVR_ERR_ARG;
+  if (ws_bytes < fvr_pou_warp_sep_adjoint_workspace(N, H, W)) return FVR_ERR_WORKSPACE;
   if (!fvr_pou_warp_sep_adjoint_supported(P, H, W)) return FVR_ERR_UNSUPPORTED;
-  const SepGrad w{gout, grad_imgs, goffs};
+  float4* gic = static_cast<float4*>(workspace);
+  const SepGrad w{gout, gic, grad_imgs, goffs};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (B * N >= 296) return sep_adjoint<256, 2>(a, w, s);  // several CTAs per SM
+  const int Wp = sep_padded((int)W);
+  const bool vec = W % 4 == 0 && ((reinterpret_cast<uintptr_t>(gout) | reinterpret_cast<uintptr_t>(ic)) & 15) == 0;
+  pou_warp_sep_weigh_kernel<<<dim3((unsigned)cdiv64(H * (Wp / 4), 256), (unsigned)N), 256, 0, s>>>(
+      gout, ic, (int)H, (int)W, Wp, vec, gic);
+  FVR_LAUNCH_CHECK();
+  // 256 threads once two CTAs per SM can run, else all 16 warps on one (pose, block)
+  if (B * N >= 296) return sep_adjoint<256, 2>(a, w, s);
   return sep_adjoint<512, 1>(a, w, s);
+}
+
+int fvr_pou_pinhole_supported(int64_t P, int64_t H, int64_t W) {
+  return fvr_pou_image_supported(P) && fvr_pou_warp_sep_supported(P, H, W);
+}
+
+int fvr_pou_pinhole_forward(int dtype, const void* stencil, const float* scales, int64_t B, int64_t P,
+                            const float* mats, int64_t N, const double* base12, double vscale, const float* centers,
+                            const float* freqs, const float* rxc, const float* ryr, const float* ic, int64_t H,
+                            int64_t W, double inv_ds, double c_idx, double* geo, double* offs, float* imgs, float* out,
+                            void* stream) {
+  if (!mats || !out) return FVR_ERR_ARG;
+  if (!fvr_pou_pinhole_supported(P, H, W)) return FVR_ERR_UNSUPPORTED;
+  int rc = fvr_pou_pose(mats, nullptr, N, base12, vscale, centers, B, geo, offs, stream);
+  if (!rc) rc = fvr_pou_slice_image(dtype, stencil, scales, B, P, geo, N, freqs, imgs, stream);
+  if (!rc) rc = fvr_pou_warp_sep(imgs, B, N, P, offs, rxc, ryr, ic, H, W, inv_ds, c_idx, out, stream);
+  return rc;
+}
+
+// Workspace of the backward: weighed detector gradient | offset gradients |
+// slice-adjoint records, each on a 256-byte boundary.
+static int64_t pinhole_round(int64_t bytes) { return (bytes + 255) / 256 * 256; }
+
+int64_t fvr_pou_pinhole_backward_workspace(int64_t B, int64_t N, int64_t H, int64_t W) {
+  if (B < 1 || N < 1) return 0;
+  return pinhole_round(fvr_pou_warp_sep_adjoint_workspace(N, H, W)) + pinhole_round(24 * B * N) +
+         fvr_pou_slice_image_adjoint_workspace(B, N);
+}
+
+int fvr_pou_pinhole_backward(int dtype, const void* stencil, const float* scales, int64_t B, int64_t P,
+                             const double* geo, const double* offs, int64_t N, const double* base12, double vscale,
+                             const float* centers, const float* freqs, const float* imgs, const float* rxc,
+                             const float* ryr, const float* ic, int64_t H, int64_t W, double inv_ds, double c_idx,
+                             const float* gout, float* grad_imgs, void* workspace, int64_t ws_bytes, float* gmats,
+                             void* stream) {
+  if (!workspace || !grad_imgs || (reinterpret_cast<uintptr_t>(workspace) & 15) || !gmats || !offs) return FVR_ERR_ARG;
+  if (!fvr_pou_pinhole_supported(P, H, W) || !fvr_pou_warp_sep_adjoint_supported(P, H, W)) return FVR_ERR_UNSUPPORTED;
+  if (ws_bytes < fvr_pou_pinhole_backward_workspace(B, N, H, W)) return FVR_ERR_WORKSPACE;
+  const int64_t gic_bytes = fvr_pou_warp_sep_adjoint_workspace(N, H, W);
+  const int64_t part_bytes = fvr_pou_slice_image_adjoint_workspace(B, N);
+  char* w = static_cast<char*>(workspace);
+  double* goffs = reinterpret_cast<double*>(w + pinhole_round(gic_bytes));
+  double* part = reinterpret_cast<double*>(reinterpret_cast<char*>(goffs) + pinhole_round(24 * B * N));
+  int rc = fvr_pou_warp_sep_adjoint(imgs, B, N, P, offs, rxc, ryr, ic, H, W, inv_ds, c_idx, gout, workspace, gic_bytes,
+                                    grad_imgs, goffs, stream);
+  if (!rc)
+    rc = fvr_pou_slice_image_adjoint(dtype, stencil, scales, B, P, geo, N, freqs, grad_imgs, part, part_bytes, stream);
+  if (!rc)
+    rc = fvr_pou_pose_backward(part, 1, goffs, nullptr, 0, geo, centers, B, N, base12, vscale, gmats, nullptr, stream);
+  return rc;
 }
 
 }  // extern "C"

@@ -102,7 +102,14 @@ SIGNATURES = {
     "fvr_pou_warp_sep": (I32, [P, I64, I64, I64, P, P, P, P, I64, I64, F64, F64, P, P]),
     "fvr_pou_warp_sep_supported": (I32, [I64, I64, I64]),
     "fvr_pou_warp_sep_adjoint_supported": (I32, [I64, I64, I64]),
-    "fvr_pou_warp_sep_adjoint": (I32, [P, I64, I64, I64, P, P, P, P, I64, I64, F64, F64, P, P, P, P]),
+    "fvr_pou_warp_sep_adjoint_workspace": (I64, [I64, I64, I64]),
+    "fvr_pou_warp_sep_adjoint": (I32, [P, I64, I64, I64, P, P, P, P, I64, I64, F64, F64, P, P, I64, P, P, P]),
+    "fvr_pou_pinhole_supported": (I32, [I64, I64, I64]),
+    "fvr_pou_pinhole_forward": (I32, [I32, P, P, I64, I64, P, I64, P, F64, P, P, P, P, P, I64, I64, F64, F64, P, P, P,
+                                      P, P]),
+    "fvr_pou_pinhole_backward_workspace": (I64, [I64, I64, I64, I64]),
+    "fvr_pou_pinhole_backward": (I32, [I32, P, P, I64, I64, P, P, I64, P, F64, P, P, P, P, P, P, I64, I64, F64, F64, P,
+                                       P, P, I64, P, P]),
     "fvr_pou_warp": (I32, [P, I64, I64, I64, P, P, P, I32, I64, P, P, P, I64, I64, F64, F64, P, P]),
     "fvr_pou_warp_bwd_workspace": (I64, [I64, I64, I64]),
     "fvr_pou_warp_bwd": (I32, [P, I64, I64, I64, P, P, P, I32, I64, P, P, P, I64, I64, F64, F64, P, P, P, P, P, I64,
@@ -162,6 +169,9 @@ KERNELS_PER_CALL = {
     "fvr_tc_slice_adjoint": 2,
     "fvr_cncc_forward": 2,
     "fvr_pou_warp_bwd": 2,
+    "fvr_pou_warp_sep_adjoint": 2,
+    "fvr_pou_pinhole_forward": 3,
+    "fvr_pou_pinhole_backward": 4,
     "fvr_np_ncc_moments": 2,
     "fvr_np_pair_moments": 2,
     "fvr_edge_ncc_forward": 2,

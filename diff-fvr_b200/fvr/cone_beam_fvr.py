@@ -159,35 +159,36 @@ _LATTICE_CACHE: Dict[Tuple, Tuple] = {}
 _SEPARABLE_REL = 2.0 ** -20
 
 
-def _separable_rays(rx, ry):
-    """(rxc [W], ryr [H]) midpoints of the per-column rx and per-row ry ranges
-    of a lattice, or None when the rays do not separate (see _SEPARABLE_REL)."""
+def _separable_tables(rx, ry):
+    """``(sep, monotone)`` of a lattice's rays: sep = (rxc [W], ryr [H]), the
+    midpoints of the per-column rx and per-row ry ranges, or None when the rays
+    do not separate (see _SEPARABLE_REL); monotone says whether both tables run
+    in one direction (the separable warp adjoint marches along them)."""
     if rx.ndim != 2 or rx.shape != ry.shape:
-        return None
-    cmax, cmin = rx.amax(0), rx.amin(0)
-    rmax, rmin = ry.amax(1), ry.amin(1)
-    sx = float((cmax - cmin).max()) / max(float(rx.abs().max()), 1e-30)
-    sy = float((rmax - rmin).max()) / max(float(ry.abs().max()), 1e-30)
-    if not (sx <= _SEPARABLE_REL and sy <= _SEPARABLE_REL):
-        return None
-    rxc = (0.5 * (cmax.double() + cmin.double())).float().contiguous()
-    ryr = (0.5 * (rmax.double() + rmin.double())).float().contiguous()
-    return rxc, ryr
+        return None, False
+    # per column / row: the largest, the smallest and the largest magnitude, in one host transfer
+    cols, rows = torch.stack([rx.amax(0), rx.amin(0)]), torch.stack([ry.amax(1), ry.amin(1)])
+    host = torch.cat([cols, rows], dim=1).cpu().numpy().astype(np.float64)
+    tables = []
+    for hi, lo in (host[:, :rx.shape[1]], host[:, rx.shape[1]:]):
+        if not (hi - lo).max() <= _SEPARABLE_REL * max(np.abs(hi).max(), np.abs(lo).max(), 1e-30):
+            return None, False
+        tables.append((0.5 * (hi + lo)).astype(np.float32))
+    steps = [np.diff(t) for t in tables]
+    monotone = all(bool((d >= 0).all()) or bool((d <= 0).all()) for d in steps)
+    both = torch.from_numpy(np.concatenate(tables)).to(rx.device)
+    return (both[:rx.shape[1]].clone(), both[rx.shape[1]:].clone()), monotone
 
 
-def _monotone(sep):
-    """Whether both separable ray tables run in one direction (the separable
-    warp adjoint marches along them)."""
-    if sep is None:
-        return False
-    steps = [np.diff(t.cpu().numpy()) for t in sep]
-    return all(bool((d >= 0).all()) or bool((d <= 0).all()) for d in steps)
+def _separable_rays(rx, ry):
+    """The separable tables alone (None when the rays do not separate)."""
+    return _separable_tables(rx, ry)[0]
 
 
 # The separable warp adjoint hands dL/dimgs to the block-image adjoint in a
 # [blocks, poses, P, P] buffer.  Beyond this size the one-launch adjoint runs
 # instead where it can: it keeps that gradient in shared memory (64 blocks x 64
-# poses x 128^2 is 268 MB: 1.0 against 1.4 ms).
+# poses x 128^2 is 268 MB: 1.23 against 1.42 ms).
 _GRAD_IMAGE_BYTES = 4 << 30
 
 
@@ -206,8 +207,7 @@ def _prepared_lattice(lattice, device):
         basis = torch.cat([lattice[i].reshape(3) for i in (0, 2, 3, 4)]).detach().double().cpu()
         base = (_ct.c_double * 12)(*[float(x) for x in basis])
         rays = tuple(t.detach().to(device=device, dtype=torch.float32).contiguous() for t in lattice[5:8])
-        sep = _separable_rays(rays[0], rays[1])
-        hit = (key, base, rays, tuple(lattice[:8]), sep, _monotone(sep))
+        hit = (key, base, rays, tuple(lattice[:8]), *_separable_tables(rays[0], rays[1]))
         _LATTICE_CACHE[key] = hit
     return hit
 
@@ -269,11 +269,20 @@ class _PinholeFn(torch.autograd.Function):
         offs = torch.empty((B, N, 3), dtype=torch.float64, device=dev)
         s = L.stream_ptr(dev)
         vscale = float(P) * model.ds_block
+        H, W = int(rx.shape[0]), int(rx.shape[1])
+        out = torch.empty((N, 1, H, W), dtype=torch.float32, device=dev)
+        ctx.meta = (model, base, mats.dtype, sep, monotone)
+        if sep is not None and not profiling.active() and L.query("fvr_pou_pinhole_supported", P, H, W):
+            st = model._stencil
+            imgs = torch.empty((B, N, P, P), dtype=torch.float32, device=dev)
+            L.call("fvr_pou_pinhole_forward", st.code, L.ptr(st.data), L.ptr(st.scales), B, P, L.ptr(m), N, base,
+                   vscale, L.ptr(model.centers), L.ptr(model._freqs), L.ptr(sep[0]), L.ptr(sep[1]), L.ptr(ic), H, W,
+                   1.0 / model.ds_block, float(P // 2), L.ptr(geo), L.ptr(offs), L.ptr(imgs), L.ptr(out), s)
+            ctx.save_for_backward(geo, offs, imgs, rx, ry, ic)
+            return out
         L.call("fvr_pou_pose", L.ptr(m), None, N, base, vscale, L.ptr(model.centers), B, L.ptr(geo), L.ptr(offs), s)
         with profiling.section("pou_slice"):
             imgs = _block_images(model, geo, N, s)
-        H, W = int(rx.shape[0]), int(rx.shape[1])
-        out = torch.empty((N, 1, H, W), dtype=torch.float32, device=dev)
         with profiling.section("pou_warp"):
             if sep is not None and L.query("fvr_pou_warp_sep_supported", P, H, W):
                 L.call("fvr_pou_warp_sep", L.ptr(imgs), B, N, P, L.ptr(offs), L.ptr(sep[0]), L.ptr(sep[1]), L.ptr(ic),
@@ -283,7 +292,6 @@ class _PinholeFn(torch.autograd.Function):
                        _ct.c_void_p(offs.data_ptr() + 16), 1, 3, L.ptr(rx), L.ptr(ry), L.ptr(ic), H * W, 0,
                        1.0 / model.ds_block, float(P // 2), L.ptr(out), s)
         ctx.save_for_backward(geo, offs, imgs, rx, ry, ic)
-        ctx.meta = (model, base, mats.dtype, sep, monotone)
         return out
 
     @staticmethod
@@ -295,14 +303,28 @@ class _PinholeFn(torch.autograd.Function):
         H, W = int(rx.shape[0]), int(rx.shape[1])
         s = L.stream_ptr(dev)
         g = g_out.detach().to(device=dev, dtype=torch.float32).contiguous()
+        gather = (monotone and model.fused_warp_adjoint and 4 * B * N * P * P <= _GRAD_IMAGE_BYTES
+                  and L.query("fvr_pou_warp_sep_adjoint_supported", P, H, W))
+        if gather and not profiling.active() and L.query("fvr_pou_image_supported", P):
+            st = model._stencil
+            wsb = L.query("fvr_pou_pinhole_backward_workspace", B, N, H, W)
+            ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
+            grad_imgs = torch.empty_like(imgs)  # of the block images' size: the allocator reuses their blocks
+            gm = torch.empty((N, 4, 4), dtype=torch.float32, device=dev)
+            L.call("fvr_pou_pinhole_backward", st.code, L.ptr(st.data), L.ptr(st.scales), B, P, L.ptr(geo),
+                   L.ptr(offs), N, base, float(P) * model.ds_block, L.ptr(model.centers), L.ptr(model._freqs),
+                   L.ptr(imgs), L.ptr(sep[0]), L.ptr(sep[1]), L.ptr(ic), H, W, 1.0 / model.ds_block, float(P // 2),
+                   L.ptr(g), L.ptr(grad_imgs), L.ptr(ws), wsb, L.ptr(gm), s)
+            return gm.to(mdt), None, None, None, None, None
         goffs = torch.empty((3, B, N), dtype=torch.float64, device=dev)
-        if (monotone and model.fused_warp_adjoint and 4 * B * N * P * P <= _GRAD_IMAGE_BYTES
-                and L.query("fvr_pou_warp_sep_adjoint_supported", P, H, W)):
+        if gather:
             grad_imgs = torch.empty((B, N, P, P), dtype=torch.float32, device=dev)
+            wsb = L.query("fvr_pou_warp_sep_adjoint_workspace", N, H, W)
+            ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
             with profiling.section("pou_warp_bwd"):
                 L.call("fvr_pou_warp_sep_adjoint", L.ptr(imgs), B, N, P, L.ptr(offs), L.ptr(sep[0]), L.ptr(sep[1]),
-                       L.ptr(ic), H, W, 1.0 / model.ds_block, float(P // 2), L.ptr(g), L.ptr(grad_imgs), L.ptr(goffs),
-                       s)
+                       L.ptr(ic), H, W, 1.0 / model.ds_block, float(P // 2), L.ptr(g), L.ptr(ws), wsb,
+                       L.ptr(grad_imgs), L.ptr(goffs), s)
             ws2, tiles = _block_images_adjoint(model, geo, N, grad_imgs, s)
             del grad_imgs
         elif (sep is not None and model.fused_warp_adjoint and g.data_ptr() % 16 == 0 and ic.data_ptr() % 16 == 0

@@ -57,6 +57,11 @@ def _record(ev):
     L.call("fvr_event_record", ctypes.c_void_p(ev.cuda_event), L.stream_ptr(), ext)
 
 
+def active():
+    """True while any LaunchTimer is collecting."""
+    return _active is not None
+
+
 def timing(name):
     """True when a LaunchTimer is collecting ``name`` (a cheap check before
     entering :func:`section` on a hot path)."""

@@ -334,7 +334,29 @@ int fvr_pou_warp_sep(const float* imgs, int64_t B, int64_t N, int64_t P, const d
 int fvr_pou_warp_sep_adjoint_supported(int64_t P, int64_t H, int64_t W);
 int fvr_pou_warp_sep_adjoint(const float* imgs, int64_t B, int64_t N, int64_t P, const double* offs, const float* rxc,
                              const float* ryr, const float* ic, int64_t H, int64_t W, double inv_ds, double c_idx,
-                             const float* gout, float* grad_imgs, double* goffs, void* stream);
+                             const float* gout, void* workspace, int64_t ws_bytes, float* grad_imgs, double* goffs,
+                             void* stream);
+int64_t fvr_pou_warp_sep_adjoint_workspace(int64_t N, int64_t H, int64_t W);
+/* The whole pinhole step on a separable lattice, one call per direction
+ * (cone_beam_fvr.py:670-688): pose geometry, block images and warp; then the
+ * adjoint of all three from dL/dout to dL/dmats.  The arguments are those of
+ * the separate entry points; geo[N][geo_stride], offs[B][N][3] and
+ * imgs[B][N][P][P] are the caller's and pass from the forward to the backward,
+ * whose intermediates are grad_imgs[B][N][P][P] and the workspace (16-byte
+ * aligned). */
+int fvr_pou_pinhole_supported(int64_t P, int64_t H, int64_t W);
+int fvr_pou_pinhole_forward(int dtype, const void* stencil, const float* scales, int64_t B, int64_t P,
+                            const float* mats, int64_t N, const double* base12, double vscale, const float* centers,
+                            const float* freqs, const float* rxc, const float* ryr, const float* ic, int64_t H,
+                            int64_t W, double inv_ds, double c_idx, double* geo, double* offs, float* imgs, float* out,
+                            void* stream);
+int64_t fvr_pou_pinhole_backward_workspace(int64_t B, int64_t N, int64_t H, int64_t W);
+int fvr_pou_pinhole_backward(int dtype, const void* stencil, const float* scales, int64_t B, int64_t P,
+                             const double* geo, const double* offs, int64_t N, const double* base12, double vscale,
+                             const float* centers, const float* freqs, const float* imgs, const float* rxc,
+                             const float* ryr, const float* ic, int64_t H, int64_t W, double inv_ds, double c_idx,
+                             const float* gout, float* grad_imgs, void* workspace, int64_t ws_bytes, float* gmats,
+                             void* stream);
 /* Fused warp + block-image adjoint for a separable pinhole lattice (every
  * detector column shares one ray coordinate rxc[c], every row one ryr[r]):
  * from the detector gradient gout[N][H][W] (times ic[H][W]) and the forward

@@ -22,7 +22,8 @@ pytestmark = pytest.mark.gpu
     (1, 1, 16, 1, 1, 1.0, 0, 0.0), (2, 2, 30, 31, 33, 0.7, 0, 0.3), (3, 1, 64, 16, 32, 2.3, 0, 0.0),
     (2, 3, 64, 65, 64, 0.9, 1, 0.0), (17, 1, 40, 40, 300, 0.2, 0, 0.0), (2, 1, 64, 300, 47, 0.25, 2, 5.0),
     (2, 2, 96, 37, 129, 0.8, 3, -70.0), (1, 2, 33, 20, 270, 0.02, 0, 0.0), (2, 2, 160, 211, 247, 0.6, 0, 0.0),
-    (2, 300, 32, 33, 65, 0.6, 1, 0.0),
+    (2, 300, 32, 33, 65, 0.6, 1, 0.0), (34, 100, 20, 18, 70, 0.5, 0, 0.0), (2, 130, 32, 121, 130, 0.3, 2, 0.0),
+    (1, 60, 48, 130, 40, 0.28, 0, 0.0),
 ])
 def test_separable_warp_and_adjoint_vs_oracle(B, N, P, H, W, pitch, flip, shift):
     import fvr._lib as L
@@ -56,7 +57,9 @@ def test_separable_warp_and_adjoint_vs_oracle(B, N, P, H, W, pitch, flip, shift)
             1.0 / ds, c)
     L.call("fvr_pou_warp_sep", *head, L.ptr(out), L.stream_ptr(dev))
     assert L.query("fvr_pou_warp_sep_adjoint_supported", P, H, W) == 1
-    L.call("fvr_pou_warp_sep_adjoint", *head, L.ptr(t["g"]), L.ptr(gim), L.ptr(goffs), L.stream_ptr(dev))
+    ws = torch.empty(L.query("fvr_pou_warp_sep_adjoint_workspace", N, H, W), dtype=torch.uint8, device=dev)
+    L.call("fvr_pou_warp_sep_adjoint", *head, L.ptr(t["g"]), L.ptr(ws), ws.numel(), L.ptr(gim), L.ptr(goffs),
+           L.stream_ptr(dev))
     assert np.linalg.norm(ref) > 0
     assert rel_l2(out.cpu().numpy(), ref) < 2e-6
     assert rel_l2(gim.cpu().numpy(), gi) < 1e-5
