@@ -204,6 +204,144 @@ __global__ void pou_rays_prep_kernel(const float* __restrict__ trg, const double
   ic[o] = static_cast<float>(icv);
 }
 
+// Detector axes of an explicit lattice trg[N][H][W][3] (cone_beam_fvr.py:575-596):
+// u along its first row, v along its first column, n the unit v x u turned to
+// face away from the source, towards the lattice's centroid.  As tensor
+// operations this was 60 launches forward and backward around five renderer
+// kernels; the launches, not the kernels (243 of 1040 us), were the time.
+constexpr double kAxisEps = 1e-12;
+constexpr int kRaySumTiles = 32;
+
+// Coordinate sums over a tile of the lattice -> part[n][tile][3].
+__global__ void __launch_bounds__(256) pou_rays_sum_kernel(const float* __restrict__ trg, int K,
+                                                           double* __restrict__ part) {
+  __shared__ double red[3][8];
+  const int n = blockIdx.y, per = (K + gridDim.x - 1) / gridDim.x;
+  const int q0 = blockIdx.x * per, q1 = min(K, q0 + per);
+  double s[3] = {0.0, 0.0, 0.0};
+  for (int q = q0 + threadIdx.x; q < q1; q += blockDim.x) {
+    const float* t = trg + (static_cast<int64_t>(n) * K + q) * 3;
+    for (int k = 0; k < 3; ++k) s[k] += static_cast<double>(__ldg(t + k));
+  }
+  for (int k = 0; k < 3; ++k) {
+    const double v = warp_sum(s[k]);
+    if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    double v = 0.0;
+    for (int w = 0; w < 8; ++w) v += red[threadIdx.x][w];
+    part[(static_cast<int64_t>(n) * gridDim.x + blockIdx.x) * 3 + threadIdx.x] = v;
+  }
+}
+
+__device__ __forceinline__ void cross3(const double* a, const double* b, double* c) {
+  c[0] = a[1] * b[2] - a[2] * b[1];
+  c[1] = a[2] * b[0] - a[0] * b[2];
+  c[2] = a[0] * b[1] - a[1] * b[0];
+}
+__device__ __forceinline__ double dot3(const double* a, const double* b) {
+  return a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
+}
+
+// One CTA per pose: axes from the lattice corners, then the pose geometry and
+// block offsets of pou_pose_kernel.
+__global__ void __launch_bounds__(128) pou_rays_pose_kernel(const float* __restrict__ srcs,
+                                                            const float* __restrict__ trg, int N, int H, int W,
+                                                            int tiles, const double* __restrict__ part, double vscale,
+                                                            const float* __restrict__ centers, int B,
+                                                            double* __restrict__ geo, double* __restrict__ offs) {
+  __shared__ double g[kGeo];
+  const int n = blockIdx.x;
+  if (threadIdx.x == 0) {
+    const float* t0 = trg + static_cast<int64_t>(n) * H * W * 3;
+    const float *tu = t0 + 3 * static_cast<int64_t>(W - 1), *tv = t0 + 3 * static_cast<int64_t>(H - 1) * W;
+    double e[2][3], c[3], m[3] = {0.0, 0.0, 0.0};
+    for (int k = 0; k < 3; ++k) {
+      e[0][k] = static_cast<double>(tu[k]) - static_cast<double>(t0[k]);
+      e[1][k] = static_cast<double>(tv[k]) - static_cast<double>(t0[k]);
+    }
+    for (int a = 0; a < 2; ++a) {
+      const double inv = 1.0 / (sqrt(dot3(e[a], e[a])) + kAxisEps);
+      for (int k = 0; k < 3; ++k) e[a][k] *= inv;
+    }
+    cross3(e[1], e[0], c);
+    double inv = 1.0 / (sqrt(dot3(c, c)) + kAxisEps);
+    for (int t = 0; t < tiles; ++t)
+      for (int k = 0; k < 3; ++k) m[k] += part[(static_cast<int64_t>(n) * tiles + t) * 3 + k];
+    double facing = 0.0;
+    for (int k = 0; k < 3; ++k) {
+      g[k] = static_cast<double>(srcs[3 * n + k]);
+      facing += (m[k] / (static_cast<double>(H) * W) - g[k]) * c[k];
+    }
+    if (facing < 0.0) inv = -inv;
+    for (int k = 0; k < 3; ++k) {
+      g[3 + k] = e[0][k];
+      g[6 + k] = e[1][k];
+      g[9 + k] = c[k] * inv;
+    }
+    for (int k = 0; k < 3; ++k) {
+      g[12 + k] = g[3 + 2 - k] * vscale;
+      g[15 + k] = g[6 + 2 - k] * vscale;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < kGeo) geo[n * kGeo + threadIdx.x] = g[threadIdx.x];
+  for (int b = threadIdx.x; b < B; b += blockDim.x) {
+    const double d[3] = {centers[3 * b] - g[0], centers[3 * b + 1] - g[1], centers[3 * b + 2] - g[2]};
+    double* o = offs + 3 * (static_cast<int64_t>(b) * N + n);
+    o[0] = dot3(d, g + 9);
+    o[1] = dot3(d, g + 3);
+    o[2] = dot3(d, g + 6);
+  }
+}
+
+// y = e / (|e| + eps): dL/de from dL/dy.
+__device__ __forceinline__ void axis_backward(const double* e, const double* gy, double* ge) {
+  const double len = sqrt(dot3(e, e)), inv = 1.0 / (len + kAxisEps);
+  const double along = len > 0.0 ? dot3(e, gy) * inv * inv / len : 0.0;
+  for (int k = 0; k < 3; ++k) ge[k] = gy[k] * inv - e[k] * along;
+}
+
+// dL/d(src, u, v, n) (gvec) -> dL/dsrcs and the three corner points' share of
+// dL/dtrg (added to what the rays put there).  One thread per pose.
+__global__ void pou_rays_axes_bwd_kernel(const float* __restrict__ trg, const double* __restrict__ geo,
+                                         const float* __restrict__ gvec, int N, int H, int W,
+                                         float* __restrict__ gsrc, float* __restrict__ gtrg) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= N) return;
+  const double* g = geo + n * kGeo;
+  const int64_t o0 = static_cast<int64_t>(n) * H * W * 3, ou = o0 + 3 * static_cast<int64_t>(W - 1),
+                ov = o0 + 3 * static_cast<int64_t>(H - 1) * W;
+  double u[3], v[3], nn[3], gu[3], gv[3], gn[3], c[3], gc[3], a[3], e[3], ge[2][3];
+  for (int k = 0; k < 3; ++k) {
+    u[k] = g[3 + k];
+    v[k] = g[6 + k];
+    nn[k] = g[9 + k];
+    gsrc[3 * n + k] = gvec[12 * n + k];
+    gu[k] = gvec[12 * n + 3 + k];
+    gv[k] = gvec[12 * n + 6 + k];
+    gn[k] = gvec[12 * n + 9 + k];
+  }
+  cross3(v, u, c);
+  if (dot3(c, nn) < 0.0)
+    for (int k = 0; k < 3; ++k) gn[k] = -gn[k];
+  axis_backward(c, gn, gc);
+  cross3(u, gc, a);  // c = v x u
+  for (int k = 0; k < 3; ++k) gv[k] += a[k];
+  cross3(gc, v, a);
+  for (int k = 0; k < 3; ++k) gu[k] += a[k];
+  for (int k = 0; k < 3; ++k) e[k] = static_cast<double>(trg[ou + k]) - static_cast<double>(trg[o0 + k]);
+  axis_backward(e, gu, ge[0]);
+  for (int k = 0; k < 3; ++k) e[k] = static_cast<double>(trg[ov + k]) - static_cast<double>(trg[o0 + k]);
+  axis_backward(e, gv, ge[1]);
+  for (int k = 0; k < 3; ++k) {
+    gtrg[ou + k] = static_cast<float>(gtrg[ou + k] + ge[0][k]);
+    gtrg[ov + k] = static_cast<float>(gtrg[ov + k] + ge[1][k]);
+    gtrg[o0 + k] = static_cast<float>(gtrg[o0 + k] - ge[0][k] - ge[1][k]);
+  }
+}
+
 // ----------------------------------------------------------------------------
 // block slices  (cone_beam_fvr.py:480-505; triton_slice.py:46-143)
 // ----------------------------------------------------------------------------
@@ -2045,6 +2183,86 @@ int fvr_pou_rays_bwd(const float* trg, const double* geo, int64_t N, int64_t K, 
   if (ws_bytes < fvr_pou_rays_bwd_workspace(N, K)) return FVR_ERR_WORKSPACE;
   pou_rays_bwd_kernel<<<dim3((unsigned)cdiv64(K, 256), (unsigned)N), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       trg, geo, (int)N, (int)K, gray, gtrg, static_cast<double*>(workspace));
+  FVR_LAUNCH_CHECK();
+  return FVR_OK;
+}
+
+int fvr_pou_rays_forward(int dtype, const void* stencil, const float* scales, int64_t B, int64_t P, const float* srcs,
+                         const float* trg, int64_t N, int64_t H, int64_t W, double vscale, const float* centers,
+                         const float* freqs, double inv_ds, double c_idx, double* geo, double* offs, float* rays,
+                         float* imgs, float* out, void* stream) {
+  if (!srcs || !trg || !centers || !geo || !offs || !rays || !imgs || !out) return FVR_ERR_ARG;
+  if (B < 1 || N < 1 || N > 65535 || H < 1 || W < 1 || H * W > 2147483647) return FVR_ERR_ARG;
+  if (!fvr_pou_image_supported(P)) return FVR_ERR_UNSUPPORTED;
+  if (reinterpret_cast<uintptr_t>(imgs) & 15) return FVR_ERR_ARG;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int64_t K = H * W;
+  const int tiles = static_cast<int>(cdiv64(K, 2048) < kRaySumTiles ? cdiv64(K, 2048) : kRaySumTiles);
+  double* part = reinterpret_cast<double*>(imgs);  // at least 16 KB a pose, written by the images afterwards
+  pou_rays_sum_kernel<<<dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(N)), 256, 0, s>>>(trg, (int)K, part);
+  FVR_LAUNCH_CHECK();
+  pou_rays_pose_kernel<<<static_cast<unsigned>(N), 128, 0, s>>>(srcs, trg, (int)N, (int)H, (int)W, tiles, part, vscale,
+                                                               centers, (int)B, geo, offs);
+  FVR_LAUNCH_CHECK();
+  float *rx = rays, *ry = rays + N * K, *ic = rays + 2 * N * K;
+  int rc = fvr_pou_rays_prep(trg, geo, N, K, rx, ry, ic, stream);
+  if (!rc) rc = fvr_pou_slice_image(dtype, stencil, scales, B, P, geo, N, freqs, imgs, stream);
+  if (!rc)
+    rc = fvr_pou_warp(imgs, B, N, P, offs, offs + 1, offs + 2, 1, 3, rx, ry, ic, K, K, inv_ds, c_idx, out, stream);
+  return rc;
+}
+
+// Workspace of the backward, each part on a 256-byte boundary: dL/d(rx, ry, ic)
+// | dL/d(src, u, v, n) | offset gradients | warp, slice-adjoint and ray records.
+static int64_t rays_round(int64_t bytes) { return (bytes + 255) / 256 * 256; }
+
+int64_t fvr_pou_rays_backward_workspace(int64_t B, int64_t N, int64_t H, int64_t W) {
+  if (B < 1 || N < 1 || H < 1 || W < 1) return 0;
+  const int64_t K = H * W;
+  return rays_round(12 * N * K) + rays_round(48 * N) + rays_round(24 * B * N) +
+         rays_round(fvr_pou_warp_bwd_workspace(B, N, K)) + rays_round(fvr_pou_slice_image_adjoint_workspace(B, N)) +
+         fvr_pou_rays_bwd_workspace(N, K);
+}
+
+int fvr_pou_rays_backward(int dtype, const void* stencil, const float* scales, int64_t B, int64_t P, const float* trg,
+                          int64_t N, int64_t H, int64_t W, double vscale, const float* centers, const float* freqs,
+                          double inv_ds, double c_idx, const double* geo, const double* offs, const float* rays,
+                          const float* imgs, const float* gout, float* grad_imgs, void* workspace, int64_t ws_bytes,
+                          float* gsrc, float* gtrg, void* stream) {
+  if (!trg || !centers || !geo || !offs || !rays || !imgs || !gout || !grad_imgs || !workspace || !gsrc || !gtrg)
+    return FVR_ERR_ARG;
+  if (B < 1 || N < 1 || N > 65535 || H < 1 || W < 1 || H * W > 2147483647) return FVR_ERR_ARG;
+  if (!fvr_pou_image_supported(P)) return FVR_ERR_UNSUPPORTED;
+  if (ws_bytes < fvr_pou_rays_backward_workspace(B, N, H, W)) return FVR_ERR_WORKSPACE;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int64_t K = H * W;
+  const float *rx = rays, *ry = rays + N * K, *ic = rays + 2 * N * K;
+  char* w = static_cast<char*>(workspace);
+  auto take = [&](int64_t bytes) {
+    char* p = w;
+    w += rays_round(bytes);
+    return p;
+  };
+  float* gray = reinterpret_cast<float*>(take(12 * N * K));
+  float* gvec = reinterpret_cast<float*>(take(48 * N));
+  double* goffs = reinterpret_cast<double*>(take(24 * B * N));
+  const int64_t wb = fvr_pou_warp_bwd_workspace(B, N, K), sb = fvr_pou_slice_image_adjoint_workspace(B, N),
+                rb = fvr_pou_rays_bwd_workspace(N, K);
+  void* wpart = take(wb);
+  double* spart = reinterpret_cast<double*>(take(sb));
+  double* rpart = reinterpret_cast<double*>(take(rb));
+  if (cudaMemsetAsync(grad_imgs, 0, static_cast<size_t>(4 * B * N * P * P), s) != cudaSuccess) return FVR_ERR_CUDA;
+  int rc = fvr_pou_warp_bwd(imgs, B, N, P, offs, offs + 1, offs + 2, 1, 3, rx, ry, ic, K, K, inv_ds, c_idx, gout,
+                            grad_imgs, goffs, gray, wpart, wb, stream);
+  if (!rc)
+    rc = fvr_pou_slice_image_adjoint(dtype, stencil, scales, B, P, geo, N, freqs, grad_imgs, spart, sb, stream);
+  if (!rc) rc = fvr_pou_rays_bwd(trg, geo, N, K, gray, gtrg, rpart, rb, stream);
+  if (!rc)
+    rc = fvr_pou_pose_backward(spart, 1, goffs, rpart, cdiv64(K, 256), geo, centers, B, N, nullptr, vscale, nullptr,
+                               gvec, stream);
+  if (rc) return rc;
+  pou_rays_axes_bwd_kernel<<<static_cast<unsigned>(cdiv64(N, 32)), 32, 0, s>>>(trg, geo, gvec, (int)N, (int)H, (int)W,
+                                                                              gsrc, gtrg);
   FVR_LAUNCH_CHECK();
   return FVR_OK;
 }

@@ -604,10 +604,13 @@ class PerspectiveSlabFVR(nn.Module):
     def project_rays_batched(self, srcs, trg_pts, u_det=None, v_det=None, n_0=None):
         """Cone-beam line integrals for explicit sources ``(N, 3)`` and detector
         lattices ``(N, H, W, 3)`` (cone_beam_fvr.py:598-612)."""
-        from .cone_beam_rays import project_rays_batched
+        from .cone_beam_rays import lattice_rays_supported, project_lattice_rays, project_rays_batched
 
         home, dev = trg_pts.device, self._dev
         srcs, trg_pts = srcs.to(dev), trg_pts.to(dev)
+        if u_det is None and v_det is None and n_0 is None and lattice_rays_supported(self, srcs, trg_pts):
+            out = project_lattice_rays(self, srcs, trg_pts)
+            return out if out.device == home else out.to(home)
         u_det, v_det, n_0 = (None if a is None else a.to(dev) for a in (u_det, v_det, n_0))
         u_det, v_det, n_0 = self._extract_detector_basis(srcs, trg_pts, u_det, v_det, n_0)
         out = project_rays_batched(self, srcs, trg_pts, u_det, v_det, n_0)

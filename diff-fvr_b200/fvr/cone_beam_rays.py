@@ -77,6 +77,64 @@ class _RaysFn(torch.autograd.Function):
                 gvec[:, 9:12].to(sdt), None)
 
 
+class _LatticeRaysFn(torch.autograd.Function):
+    """The same for a lattice whose detector axes are its own (u, v, n from its
+    corners and centroid): axes, rays, images and warp, and their adjoint, in
+    one library call per direction."""
+
+    @staticmethod
+    def forward(ctx, srcs, trg, model):
+        dev = model._dev
+        f32 = dict(device=dev, dtype=torch.float32)
+        N, H, W, _ = (int(x) for x in trg.shape)
+        B, P = model.B, model.P
+        s0 = srcs.detach().to(**f32).reshape(N, 3).contiguous()
+        t = trg.detach().to(**f32).contiguous()
+        geo = torch.empty((N, int(L.query("fvr_pou_geo_stride"))), dtype=torch.float64, device=dev)
+        offs = torch.empty((B, N, 3), dtype=torch.float64, device=dev)
+        rays = torch.empty((3, N, H * W), **f32)
+        imgs = torch.empty((B, N, P, P), **f32)
+        out = torch.empty((N, H, W), **f32)
+        st = model._stencil
+        L.call("fvr_pou_rays_forward", st.code, L.ptr(st.data), L.ptr(st.scales), B, P, L.ptr(s0), L.ptr(t), N, H, W,
+               float(P) * model.ds_block, L.ptr(model.centers), L.ptr(model._freqs), 1.0 / model.ds_block,
+               float(P // 2), L.ptr(geo), L.ptr(offs), L.ptr(rays), L.ptr(imgs), L.ptr(out), L.stream_ptr(dev))
+        ctx.save_for_backward(t, geo, offs, rays, imgs)
+        ctx.meta = (model, srcs.dtype, trg.dtype, srcs.shape)
+        return out
+
+    @staticmethod
+    def backward(ctx, g_out):
+        t, geo, offs, rays, imgs = ctx.saved_tensors
+        model, sdt, tdt, sshape = ctx.meta
+        dev = geo.device
+        N, H, W = int(t.shape[0]), int(t.shape[1]), int(t.shape[2])
+        B, P = model.B, model.P
+        g = g_out.detach().to(device=dev, dtype=torch.float32).contiguous()
+        wsb = L.query("fvr_pou_rays_backward_workspace", B, N, H, W)
+        ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
+        grad_imgs = torch.empty_like(imgs)
+        gsrc = torch.empty((N, 3), dtype=torch.float32, device=dev)
+        gtrg = torch.empty_like(t)
+        st = model._stencil
+        L.call("fvr_pou_rays_backward", st.code, L.ptr(st.data), L.ptr(st.scales), B, P, L.ptr(t), N, H, W,
+               float(P) * model.ds_block, L.ptr(model.centers), L.ptr(model._freqs), 1.0 / model.ds_block,
+               float(P // 2), L.ptr(geo), L.ptr(offs), L.ptr(rays), L.ptr(imgs), L.ptr(g), L.ptr(grad_imgs),
+               L.ptr(ws), wsb, L.ptr(gsrc), L.ptr(gtrg), L.stream_ptr(dev))
+        return gsrc.reshape(sshape).to(sdt), gtrg.to(tdt), None
+
+
+def lattice_rays_supported(model, srcs, trg_pts):
+    """The one-call path: block images of a supported size, one (or more) poses."""
+    return (trg_pts.dim() == 4 and trg_pts.shape[-1] == 3 and 1 <= trg_pts.shape[0] <= 65535 and trg_pts.numel() > 0
+            and srcs.shape == (trg_pts.shape[0], 3) and bool(L.query("fvr_pou_image_supported", model.P)))
+
+
+def project_lattice_rays(model, srcs, trg_pts):
+    """(N, H, W) line integrals with the detector axes taken from ``trg_pts``."""
+    return _LatticeRaysFn.apply(srcs, trg_pts, model)
+
+
 def project_rays_batched(model, srcs, trg_pts, u_det, v_det, n_0):
     """(N, H, W) line integrals (cone_beam_fvr.py:423-478)."""
     dev = model._dev

@@ -337,6 +337,21 @@ int fvr_pou_warp_sep_adjoint(const float* imgs, int64_t B, int64_t N, int64_t P,
                              const float* gout, void* workspace, int64_t ws_bytes, float* grad_imgs, double* goffs,
                              void* stream);
 int64_t fvr_pou_warp_sep_adjoint_workspace(int64_t N, int64_t H, int64_t W);
+/* The explicit-ray step with the detector axes taken from the lattice
+ * (cone_beam_fvr.py:423-478, 575-596), one call per direction: srcs[N][3],
+ * trg[N][H][W][3] f32 -> out[N][H][W]; geo, offs, rays[3][N][H*W] and
+ * imgs[B][N][P][P] pass from the forward to the backward, which gives
+ * dL/dsrcs and dL/dtrg. */
+int fvr_pou_rays_forward(int dtype, const void* stencil, const float* scales, int64_t B, int64_t P, const float* srcs,
+                         const float* trg, int64_t N, int64_t H, int64_t W, double vscale, const float* centers,
+                         const float* freqs, double inv_ds, double c_idx, double* geo, double* offs, float* rays,
+                         float* imgs, float* out, void* stream);
+int64_t fvr_pou_rays_backward_workspace(int64_t B, int64_t N, int64_t H, int64_t W);
+int fvr_pou_rays_backward(int dtype, const void* stencil, const float* scales, int64_t B, int64_t P, const float* trg,
+                          int64_t N, int64_t H, int64_t W, double vscale, const float* centers, const float* freqs,
+                          double inv_ds, double c_idx, const double* geo, const double* offs, const float* rays,
+                          const float* imgs, const float* gout, float* grad_imgs, void* workspace, int64_t ws_bytes,
+                          float* gsrc, float* gtrg, void* stream);
 /* The whole pinhole step on a separable lattice, one call per direction
  * (cone_beam_fvr.py:670-688): pose geometry, block images and warp; then the
  * adjoint of all three from dL/dout to dL/dmats.  The arguments are those of
