@@ -1,5 +1,6 @@
 // Small fixed-radix DFTs on registers (radix 2, 3, 4, 5), shared by the
-// shared-memory line FFTs and the warp-level FFTs.
+// shared-memory line FFTs and the warp-level FFTs, with the mixed-radix plan
+// and the Stockham butterfly of the former.
 // Sign: forward e^{-2 pi i / r}, inverse e^{+2 pi i / r}; unnormalised.
 #pragma once
 
@@ -72,5 +73,62 @@ struct Dft<T, 5> {
     v[3] = csub(a2, ib2);
   }
 };
+
+constexpr int kMaxPass = 24;
+// Largest prime factor of a transform length (direct DFT pass, O(n * p) work).
+constexpr int kMaxPrime = 127;
+
+struct FftPlan {
+  int n;
+  int npass;
+  int radix[kMaxPass];
+};
+
+inline bool make_plan(int64_t n, FftPlan* plan) {
+  if (n < 1 || n > 16384) return false;
+  plan->n = static_cast<int>(n);
+  plan->npass = 0;
+  int64_t m = n;
+  const int order[] = {4, 2, 3, 5, 7, 11, 13};
+  for (int r : order) {
+    while (m % r == 0) {
+      if (plan->npass >= kMaxPass) return false;
+      plan->radix[plan->npass++] = r;
+      m /= r;
+    }
+  }
+  // remaining odd prime factors up to kMaxPrime run as direct DFT passes
+  for (int r = 17; r <= kMaxPrime && m > 1; r += 2) {
+    while (m % r == 0) {
+      if (plan->npass >= kMaxPass) return false;
+      plan->radix[plan->npass++] = r;
+      m /= r;
+    }
+  }
+  return m == 1;
+}
+
+template <typename T, int R>
+__device__ __forceinline__ void bfly(const Cx<T>* __restrict__ src, Cx<T>* __restrict__ dst, int j, int Ns, int n,
+                                     const Cx<T>* __restrict__ tw, bool inv) {
+  const int nb = n / R;
+  const int k = j % Ns;
+  Cx<T> v[R];
+#pragma unroll
+  for (int t = 0; t < R; ++t) v[t] = src[j + t * nb];
+  if (Ns > 1) {
+    const int step = n / (Ns * R);
+#pragma unroll
+    for (int t = 1; t < R; ++t) {
+      Cx<T> w = tw[k * t * step];
+      if (inv) w.y = -w.y;
+      v[t] = cmul(v[t], w);
+    }
+  }
+  Dft<T, R>::run(v, inv);
+  const int idx = (j / Ns) * Ns * R + k;
+#pragma unroll
+  for (int t = 0; t < R; ++t) dst[idx + t * Ns] = v[t];
+}
 
 }  // namespace fvr

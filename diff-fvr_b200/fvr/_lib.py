@@ -128,6 +128,11 @@ SIGNATURES = {
     "fvr_hu_to_attenuation": (I32, [P, I64, P, P]),
     "fvr_np_segment_slices": (I32, [P, I64, I64, I64, I64, P, I64, I64, P, P]),
     "fvr_np_pair_moments": (I32, [P, P, I64, I64, P, I64, P, P]),
+    "fvr_image_supported": (I32, [I64, I64]),
+    "fvr_tc_image": (I32, [I32, P, P, I64, I64, I64, P, I64, I32, P, I64, F64, P, P, P]),
+    "fvr_tc_image_backward": (I32, [I32, P, P, I64, I64, I64, P, I64, I32, P, I64, F64, P, P, P, P, P]),
+    "fvr_cncc_image_workspace": (I64, [I64]),
+    "fvr_cncc_image": (I32, [P, P, I64, I64, I64, I64, P, P, P, P, I64, P, P, P]),
     "fvr_cncc_workspace": (I64, [I64, I64]),
     "fvr_cncc_forward": (I32, [P, P, I64, I64, I64, P, P, I64, P, P, P]),
     "fvr_cncc_backward": (I32, [P, P, I64, I64, I64, P, P, P, P, P]),
@@ -172,6 +177,7 @@ KERNELS_PER_CALL = {
     "fvr_slice3d_bwd": 2,
     "fvr_tc_slice_adjoint": 2,
     "fvr_cncc_forward": 2,
+    "fvr_cncc_image": 2,
     "fvr_pou_warp_bwd": 2,
     "fvr_pou_warp_sep_adjoint": 2,
     "fvr_pou_pinhole_forward": 3,

@@ -305,8 +305,10 @@ def _slice_adjoint(eng, p, axes, view, R, kap, shift, G):
 
 
 class _ImageFn(torch.autograd.Function):
-    """relu(real(ifft2(ifftshift(S)))) (torch_engine.py:236-241); the ReLU and the
-    1/R^2 of ifft2 are fused into the last FFT pass."""
+    """relu(real(ifft2(ifftshift(S)))) (torch_engine.py:236-241).  Where an image
+    fits one CTA's shared memory each direction is one kernel; else slice, FFT
+    passes (the ReLU and the 1/R^2 of ifft2 fused into the last one) and slice
+    adjoint."""
 
     @staticmethod
     def forward(ctx, poses, eng, view, R):
@@ -315,25 +317,38 @@ class _ImageFn(torch.autograd.Function):
         C = int(p.shape[0])
         st = eng._stencil
         D, H, W = st.dims
-        axes = torch.empty((C, 8), dtype=torch.float64, device=dev)
         s = L.stream_ptr(dev)
+        kap = RT.kappa(R, eng.spacing[0])
+        img = torch.empty((C, 1, R, R), dtype=torch.float32, device=dev)
+        whole = bool(L.query("fvr_image_supported", R, R))
+        ctx.meta = (eng, view, R, kap, poses.dtype, whole)
+        if whole:
+            L.call("fvr_tc_image", *st.args(), L.ptr(p), C, view, L.ptr(RT.linspace(R, dev)), R, kap,
+                   L.ptr(RT.twiddles(R, L.F32_, dev)), L.ptr(img), s)
+            ctx.save_for_backward(p, img)
+            return img
+        axes = torch.empty((C, 8), dtype=torch.float64, device=dev)
         L.call("fvr_tc_axes", L.ptr(p), C, view, D, H, W, L.ptr(axes), s)
         buf = torch.empty((C, R, R), dtype=torch.complex64, device=dev)
-        kap = RT.kappa(R, eng.spacing[0])
         L.call("fvr_tc_slice", *st.args(), L.ptr(axes), C, L.ptr(RT.linspace(R, dev)), R, kap, 1, L.ptr(buf), s)
-        img = torch.empty((C, 1, R, R), dtype=torch.float32, device=dev)
         RT.fft2d(buf, inverse=True, scale=1.0 / (R * R), out_mode=RT.OUT_RELU, out=img, work=buf)
-        ctx.save_for_backward(p, axes, img)
-        ctx.meta = (eng, view, R, kap, poses.dtype)
+        ctx.save_for_backward(p, img, axes)
         return img
 
     @staticmethod
     def backward(ctx, g):
-        p, axes, img = ctx.saved_tensors
-        eng, view, R, kap, pdt = ctx.meta
+        eng, view, R, kap, pdt, whole = ctx.meta
+        p, img = ctx.saved_tensors[:2]
         dev = p.device
-        gm = torch.empty_like(img)
         gc = g.detach().to(device=dev, dtype=torch.float32).contiguous()
+        if whole:
+            grad = torch.empty((int(p.shape[0]), 6), dtype=torch.float32, device=dev)
+            L.call("fvr_tc_image_backward", *eng._stencil.args(), L.ptr(p), int(p.shape[0]), view,
+                   L.ptr(RT.linspace(R, dev)), R, kap, L.ptr(RT.twiddles(R, L.F32_, dev)), L.ptr(img), L.ptr(gc),
+                   L.ptr(grad), L.stream_ptr(dev))
+            return grad.to(pdt), None, None, None
+        axes = ctx.saved_tensors[2]
+        gm = torch.empty_like(img)
         L.call("fvr_relu_mask", L.ptr(img), L.ptr(gc), L.ptr(gm), img.numel(), L.stream_ptr(dev))
         # adjoint of S -> Re(ifft2(ifftshift(S))): fftshift(fft2(g)) / R^2, natural order
         G = RT.fft2d(gm.view(-1, R, R), inverse=False, out_shift=RT.SHIFT_FFT, scale=1.0 / (R * R))
@@ -343,7 +358,10 @@ class _ImageFn(torch.autograd.Function):
 
 class _ImageSpectralNCCFn(torch.autograd.Function):
     """spectral_ncc_loss (torch_engine.py:309-337): fftshift(fft2(.)) of both
-    images, high-pass, NCC; gradient to ``pred``."""
+    images, high-pass, NCC; gradient to ``pred``.  Where an image pair fits one
+    CTA's shared memory the loss and its image gradient are one kernel (the
+    loss is a scalar: backward scales the gradient); else FFT passes, moments
+    and the inverse transform of the spectral gradient."""
 
     @staticmethod
     def forward(ctx, pred, target, hp):
@@ -353,22 +371,35 @@ class _ImageSpectralNCCFn(torch.autograd.Function):
         Bt = target.numel() // (H * W)
         x = pred.detach().float().contiguous()
         t = target.detach().to(device=dev, dtype=torch.float32).contiguous()
+        loss = torch.empty((), dtype=torch.float32, device=dev)
+        whole = tuple(target.shape[-2:]) == (H, W) and bool(L.query("fvr_image_supported", H, W))
+        ctx.meta = (hp, B, Bt, H, W, pred.shape, pred.dtype, whole)
+        if whole:
+            grad = torch.empty(pred.shape, dtype=torch.float32, device=dev) if ctx.needs_input_grad[0] else None
+            wsb = L.query("fvr_cncc_image_workspace", B)
+            ws = torch.empty(max(wsb, 8), dtype=torch.uint8, device=dev)
+            L.call("fvr_cncc_image", L.ptr(x), L.ptr(t), B, Bt, H, W, L.ptr(hp), L.ptr(RT.twiddles(H, L.F32_, dev)),
+                   L.ptr(RT.twiddles(W, L.F32_, dev)), L.ptr(ws), wsb, L.ptr(loss), L.ptr(grad), L.stream_ptr(dev))
+            if grad is not None:
+                ctx.save_for_backward(grad)
+            return loss
         Fp = RT.fft2d(x, inverse=False, out_shift=RT.SHIFT_FFT)
         Ft = RT.fft2d(t, inverse=False, out_shift=RT.SHIFT_FFT)
         ws_bytes = L.query("fvr_cncc_workspace", B, H * W)
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
         mom = torch.empty((B, 3), dtype=torch.float64, device=dev)
-        loss = torch.empty((), dtype=torch.float32, device=dev)
         L.call("fvr_cncc_forward", L.ptr(Fp), L.ptr(Ft), B, Bt, H * W, L.ptr(hp), L.ptr(ws), ws_bytes, L.ptr(mom),
                L.ptr(loss), L.stream_ptr(dev))
         ctx.save_for_backward(Fp, Ft, mom)
-        ctx.meta = (hp, B, Bt, H, W, pred.shape, pred.dtype)
         return loss
 
     @staticmethod
     def backward(ctx, g):
+        hp, B, Bt, H, W, shape, dt, whole = ctx.meta
+        if whole:
+            (grad,) = ctx.saved_tensors
+            return (grad * g.detach().to(device=grad.device, dtype=grad.dtype)).to(dt), None, None
         Fp, Ft, mom = ctx.saved_tensors
-        hp, B, Bt, H, W, shape, dt = ctx.meta
         dev = Fp.device
         X = torch.empty_like(Fp)
         gg = g.detach().to(device=dev, dtype=torch.float32).contiguous()

@@ -527,6 +527,26 @@ int fvr_edge_ncc_backward(const float* a, const float* b, int64_t B, int64_t Bt,
                           int64_t crop, float ms_weight, int reduction_mean, const double* stats, const float* g,
                           int64_t g_stride, int wrt_b, float* grad, void* stream);
 
+/* ------------------------------------------- image path, one CTA per image -- */
+/* 1 when a [n0][n1] image and its transform fit one CTA's shared memory. */
+int fvr_image_supported(int64_t n0, int64_t n1);
+/* img[C][R][R] = relu(real(ifft2(ifftshift(S)))) of the modulated slices S
+ * (torch_engine.py:176-253), and its adjoint to the poses from dL/dimg (the
+ * ReLU mask is taken from img).  tw: fvr_fft_twiddles(R, FVR_F32). */
+int fvr_tc_image(int dtype, const void* stencil, const float* scales, int64_t D, int64_t H, int64_t W,
+                 const float* poses, int64_t C, int view, const float* lin, int64_t R, double kappa, const void* tw,
+                 float* img, void* stream);
+int fvr_tc_image_backward(int dtype, const void* stencil, const float* scales, int64_t D, int64_t H, int64_t W,
+                          const float* poses, int64_t C, int view, const float* lin, int64_t R, double kappa,
+                          const void* tw, const float* img, const float* gout, float* grad_poses, void* stream);
+/* Image-domain spectral NCC loss (torch_engine.py:309-337) of pred[B][n0][n1]
+ * against target[Bt][n0][n1] (Bt = 1 or B): loss[0], and with grad non-null
+ * dloss/dpred[B][n0][n1].  hp[n0][n1] or null; tw0, tw1: twiddles of n0, n1. */
+int64_t fvr_cncc_image_workspace(int64_t B);
+int fvr_cncc_image(const float* pred, const float* target, int64_t B, int64_t Bt, int64_t n0, int64_t n1,
+                   const float* hp, const void* tw0, const void* tw1, void* workspace, int64_t ws_bytes, float* loss,
+                   float* grad, void* stream);
+
 /* -------------------------------------------------- registration loss -- */
 /* Per-candidate loss over `views` (at most 4) views, imgs[v][B][H][W] against
  * refs[v][ref_batch[v]][H][W] (ref_batch 1 or B), f32:
