@@ -357,8 +357,32 @@ __global__ void __launch_bounds__(THREADS, 1) tc_image_adjoint_kernel(TcImageArg
 // image spectral NCC
 // ----------------------------------------------------------------------------
 
+// Largest magnitude of n values over the CTA, as float bits (non-negative
+// floats order as integers, infinity and NaN above them).
+template <int THREADS>
+__device__ __forceinline__ unsigned image_max(const float* p, int64_t n, unsigned* red) {
+  unsigned m = 0u;
+  for (int64_t i = threadIdx.x; i < n; i += THREADS) m = max(m, __float_as_uint(fabsf(__ldg(p + i))));
+  m = __reduce_max_sync(0xffffffffu, m);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+  __syncthreads();
+  m = 0u;
+  for (int w = 0; w < THREADS / 32; ++w) m = max(m, red[w]);
+  return m;
+}
+
+// Power of two that brings a largest magnitude (float bits) into [1, 2).
+__device__ __forceinline__ float unit_scale(unsigned bits) {
+  const int e = static_cast<int>(bits >> 23);
+  return e == 255 || bits == 0u ? 1.f : ldexpf(1.f, 127 - max(e, 1));
+}
+
 // ncc[b] of pred[b] and target[b or 0] (both multiplied by the high-pass table,
 // fftshift order, or unfiltered), and with grad the gradient of 1 - mean ncc.
+// The pair shares one transform, whose rounding follows the larger of the two,
+// so both are first scaled to one magnitude (exactly, by powers of two), and
+// the spectrum of an image of zeros is taken as zero.
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS, 1) cncc_image_kernel(ImgShape s, const float* __restrict__ pred,
                                                                     const float* __restrict__ target,
@@ -368,14 +392,17 @@ __global__ void __launch_bounds__(THREADS, 1) cncc_image_kernel(ImgShape s, cons
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double red[3][(THREADS / 32)];
   __shared__ float coef[2];
+  __shared__ unsigned wmax[THREADS / 32];
   const int b = blockIdx.x, n0 = s.n0, n1 = s.n1, pitch = n1 + 1;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t n = static_cast<int64_t>(n0) * n1;
   const ImgMem m = img_mem<THREADS>(smem, s);
   __syncthreads();
   const float *pp = pred + b * n, *tp = target + b * t_stride;
+  const unsigned pmax = image_max<THREADS>(pp, n, wmax), tmax = image_max<THREADS>(tp, n, wmax);
+  const float sp = unit_scale(pmax), st = unit_scale(tmax);
   for (int r = wid; r < n0; r += (THREADS / 32)) {
-    for (int k = lane; k < n1; k += 32) m.la[k] = Cx<float>{__ldg(pp + r * n1 + k), __ldg(tp + r * n1 + k)};
+    for (int k = lane; k < n1; k += 32) m.la[k] = Cx<float>{sp * __ldg(pp + r * n1 + k), st * __ldg(tp + r * n1 + k)};
     const Cx<float>* y = line_fft<false>(m.la, m.lb, s.p1, m.tw1, lane);
     for (int k = lane; k < n1; k += 32) m.buf[r * pitch + k] = y[k];
     __syncwarp();
@@ -395,6 +422,8 @@ __global__ void __launch_bounds__(THREADS, 1) cncc_image_kernel(ImgShape s, cons
     const Cx<float> z = m.buf[r * pitch + k], y = m.buf[rm * pitch + km];
     fp = Cx<float>{0.5f * (z.x + y.x), 0.5f * (z.y - y.y)};
     ft = Cx<float>{0.5f * (z.y + y.y), 0.5f * (y.x - z.x)};
+    if (pmax == 0u) fp = Cx<float>{0.f, 0.f};
+    if (tmax == 0u) ft = Cx<float>{0.f, 0.f};
     if (!hp) return 1.f;
     const int h0 = n0 / 2, h1 = n1 / 2;  // frequency k sits at (k + n/2) mod n of the table
     const float u = __ldg(hp + ((r + h0) % n0) * n1 + (k + h1) % n1);
@@ -421,12 +450,16 @@ __global__ void __launch_bounds__(THREADS, 1) cncc_image_kernel(ImgShape s, cons
     double t[3] = {0.0, 0.0, 0.0};
     for (int k = 0; k < 3; ++k)
       for (int w = 0; w < (THREADS / 32); ++w) t[k] += red[k][w];
+    const double up = 1.0 / sp, ut = 1.0 / st;  // back to the images' own scales
+    t[0] *= up * ut;
+    t[1] *= up * up;
+    t[2] *= ut * ut;
     const double e = sqrt(t[1] * t[2]);
     const double aa = 1.0 / (e + 1e-8);
     const double bb = e > 0.0 ? -t[0] * t[2] / (2.0 * e * (e + 1e-8) * (e + 1e-8)) : 0.0;
     ncc[b] = t[0] * aa;
-    coef[0] = static_cast<float>(-aa / B);
-    coef[1] = static_cast<float>(-2.0 * bb / B);
+    coef[0] = static_cast<float>(-aa / B * ut);
+    coef[1] = static_cast<float>(-2.0 * bb / B * up);
   }
   if (!grad) return;
   __syncthreads();

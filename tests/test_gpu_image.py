@@ -68,3 +68,24 @@ def test_image_spectral_ncc_vs_oracle(B, Bt, H, W, hp):
     ref = tc.spectral_ncc_loss_images_grad(p64, t64, hp, g=2.5)
     assert g.shape == t.shape
     assert rel_l2(g.cpu().numpy(), ref) < 2e-5
+
+
+def test_image_spectral_ncc_of_unlike_magnitudes():
+    """The pair shares one complex transform: an image of zeros (ncc 0, loss 1),
+    and images 1e-6 and 1e5 times the target keep their own accuracy (loss and
+    relative gradient as at equal magnitude)."""
+    import fvr
+
+    rng = np.random.default_rng(0)
+    base = (1.0 + rng.random((1, 1, 48, 40))).astype(np.float32)
+    targ = (base + 0.3 * rng.random(base.shape)).astype(np.float32)
+    pred = np.concatenate([0.0 * base, np.float32(1e-6) * base, np.float32(1e5) * base])
+    eng = fvr.TorchDiffFVREngine(torch.zeros((8, 8, 8)) + 1.0)
+    for i in range(3):
+        t = torch.from_numpy(pred[i:i + 1]).cuda().requires_grad_(True)
+        loss = eng.spectral_ncc_loss(t, torch.from_numpy(targ).cuda())
+        (g,) = torch.autograd.grad(loss, t)
+        p64, t64 = pred[i:i + 1].astype(np.float64), targ.astype(np.float64)
+        assert abs(float(loss) - tc.spectral_ncc_loss_images(p64, t64)) < 1e-6
+        if i:
+            assert rel_l2(g.cpu().numpy(), tc.spectral_ncc_loss_images_grad(p64, t64)) < 2e-5
