@@ -33,6 +33,9 @@ class _Item(ctypes.Structure):
                 ("sw", ctypes.c_int), ("pad", ctypes.c_int), ("off", ctypes.c_longlong)]
 
 
+_ITEM = np.dtype(_Item)  # the same record for arrays of items
+
+
 class DifferentiableFourierVolumeRenderer:
     """Differentiable & spectral Fourier volume rendering (diff_fvr.py:7-195)."""
 
@@ -73,19 +76,21 @@ class DifferentiableFourierVolumeRenderer:
             return self.pz, self.px
         return self.py, self.px
 
-    def _items(self, specs):
-        """specs: (yaw, pitch, roll, tx, ty, view) -> device item array, offsets, sizes."""
-        arr = (_Item * len(specs))()
-        off = 0
-        sizes = []
-        for i, (yaw, pitch, roll, tx, ty, view) in enumerate(specs):
+    def _specs_table(self, specs):
+        """specs: (yaw, pitch, roll, tx, ty, view) -> item records (host), each with its own slice offset; sizes
+        (rows, columns, offset) and the total element count."""
+        rows, sizes, off = [], [], 0
+        for yaw, pitch, roll, tx, ty, view in specs:
             sh, sw = self._dims(view)
-            arr[i] = _Item(float(yaw), float(pitch), float(roll), float(tx), float(ty), _view_code(view), sh, sw, 0,
-                           off)
+            rows.append((float(yaw), float(pitch), float(roll), float(tx), float(ty), _view_code(view), sh, sw, 0, off))
             sizes.append((sh, sw, off))
             off += sh * sw
-        dev_items = torch.frombuffer(bytearray(arr), dtype=torch.uint8).to(self._dev)
-        return dev_items, sizes, off
+        return np.array(rows, dtype=_ITEM), sizes, off
+
+    def _items(self, specs):
+        """Item records of the specs on the device, sizes and the total element count."""
+        table, sizes, total = self._specs_table(specs)
+        return torch.from_numpy(table.view(np.uint8)).to(self._dev), sizes, total
 
     def _euler_to_basis(self, yaw_deg, pitch_deg, roll_deg, view="lateral"):
         """Projection-plane basis (diff_fvr.py:56-104)."""
@@ -145,15 +150,46 @@ class DifferentiableFourierVolumeRenderer:
         return out
 
     def _ncc_moments(self, specs, targets):
-        """mom[item][5] for specs against device targets (list of complex128 [sh, sw])."""
-        items, sizes, total = self._items(specs)
-        tg = torch.empty(total, dtype=torch.complex128, device=self._dev)
-        for (sh, sw, o), t in zip(sizes, targets):
-            tg[o:o + sh * sw].copy_(t.reshape(-1))
+        """mom[item][5] for specs against their targets: complex128 [sh, sw], on
+        the device or on the host.  Items may share a target: a host target goes
+        to the device once, staged in page-locked memory beside the item records; a
+        device target is read in place."""
+        table, sizes, _ = self._specs_table(specs)
+        unique, index = [], []
+        for t in targets:
+            k = next((i for i, u in enumerate(unique) if u is t), len(unique))
+            if k == len(unique):
+                unique.append(t)
+            index.append(k)
+        flat = {}  # (target, elements) -> flat complex128 of that many values
+        for k, (sh, sw, _) in zip(index, sizes):
+            if (k, sh * sw) not in flat:
+                t = torch.as_tensor(unique[k], dtype=torch.complex128)
+                if t.is_cuda and (t.device != self._dev or t.data_ptr() % 16):
+                    t = t.to(self._dev, copy=True)
+                flat[k, sh * sw] = t.reshape(-1).expand(sh * sw).contiguous()
+        # one buffer: records, then the host targets, 256-byte boundaries
+        at, nbytes = {}, -(-table.nbytes // 256) * 256
+        for key, t in flat.items():
+            if not t.is_cuda:
+                at[key] = nbytes
+                nbytes += -(-t.numel() * 16 // 256) * 256
+        pinned = torch.empty(nbytes, dtype=torch.uint8, pin_memory=True)
+        buf = torch.empty(nbytes, dtype=torch.uint8, device=self._dev)
+        base = int(buf.data_ptr())
+        where = {key: base + at[key] if key in at else int(t.data_ptr()) for key, t in flat.items()}
+        # the records' offsets count elements from the buffer's start (16-byte elements, every target 16-byte aligned)
+        table["off"] = [(where[k, sh * sw] - base) // 16 for k, (sh, sw, _) in zip(index, sizes)]
+        parts = [(0, torch.from_numpy(table.view(np.uint8)))]
+        # byte views: the host copy is split over threads by element count
+        parts += [(at[key], torch.view_as_real(flat[key]).view(-1).view(torch.uint8)) for key in at]
+        for o, src in parts:  # each part's transfer runs while the next one is staged
+            pinned[o:o + src.numel()].copy_(src)
+            buf[o:o + src.numel()].copy_(pinned[o:o + src.numel()], non_blocking=True)
         ws_bytes = L.query("fvr_np_ncc_workspace", len(specs))
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=self._dev)
         mom = torch.empty((len(specs), 5), dtype=torch.float64, device=self._dev)
-        L.call("fvr_np_ncc_moments", L.ptr(self._f3d), self.pz, self.py, self.px, L.ptr(items), len(specs), L.ptr(tg),
+        L.call("fvr_np_ncc_moments", L.ptr(self._f3d), self.pz, self.py, self.px, L.ptr(buf), len(specs), L.ptr(buf),
                L.ptr(ws), ws_bytes, L.ptr(mom), L.stream_ptr(self._dev))
         return mom.cpu().numpy(), sizes
 

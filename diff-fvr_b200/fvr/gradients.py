@@ -8,6 +8,7 @@ same moments.  Only the 14 x 5 moments are copied back.
 """
 from __future__ import annotations
 
+import math
 from typing import Tuple
 
 import numpy as np
@@ -28,13 +29,13 @@ class SpectralGradientEngine:
     @staticmethod
     def _ncc_grad(m, sh, sw):
         """(ncc, d ncc/du, d ncc/dv) from the moments (gradients.py:45-74)."""
-        cross, es, et, iu, iv = m
-        ns, nt = np.sqrt(es), np.sqrt(et)
-        if ns * nt == 0:
+        cross, es, et, iu, iv = (float(x) for x in m)
+        # a sum of squares is negative only if it is not a number
+        norm = math.sqrt(es) * math.sqrt(et) if es >= 0.0 and et >= 0.0 else math.nan
+        if norm == 0:
             return 0.0, 0.0, 0.0
         # Re sum(-2 pi i (u/W) S conj(r_res)) with r_res = (T - ncc |T|/|S| S)/(|S||T|)
-        return float(cross / (ns * nt)), float(2.0 * np.pi / sw * iu / (ns * nt)), \
-            float(2.0 * np.pi / sh * iv / (ns * nt))
+        return cross / norm, 2.0 * math.pi / sw * iu / norm, 2.0 * math.pi / sh * iv / norm
 
     def compute_spectral_ncc_and_grad_translation(self, f_cand, f_target, view="lateral") -> Tuple[float, float, float]:
         """NCC of a candidate slice against a target and its exact in-plane
@@ -52,19 +53,16 @@ class SpectralGradientEngine:
         dL/droll, dL/dtx, dL/dty, dL/dtz] (gradients.py:76-135)."""
         r = self.renderer
         yaw, pitch, roll, tx, ty, tz = (float(x) for x in pose)
-        base = np.array([yaw, pitch, roll], dtype=np.float64)
+        base = (yaw, pitch, roll)
         specs = [(yaw, pitch, roll, tx, tz, "ap"), (yaw, pitch, roll, ty, tz, "lateral")]
         for i in range(3):
-            pp, pm = base.copy(), base.copy()
-            pp[i] += delta_rot_deg
-            pm[i] -= delta_rot_deg
+            pp = tuple(a + delta_rot_deg if j == i else a for j, a in enumerate(base))
+            pm = tuple(a - delta_rot_deg if j == i else a for j, a in enumerate(base))
             specs += [(*pp, tx, tz, "ap"), (*pm, tx, tz, "ap"), (*pp, ty, tz, "lateral"), (*pm, ty, tz, "lateral")]
-        dev = r._dev
-        t_ap = torch.as_tensor(np.asarray(f_target_ap), dtype=torch.complex128).to(dev)
-        t_lat = torch.as_tensor(np.asarray(f_target_lat), dtype=torch.complex128).to(dev)
+        t_ap, t_lat = np.asarray(f_target_ap), np.asarray(f_target_lat)
         targets = [t_ap if s[5] == "ap" else t_lat for s in specs]
         mom, sizes = r._ncc_moments(specs, targets)
-        res = [self._ncc_grad(mom[k], sizes[k][0], sizes[k][1]) for k in range(len(specs))]
+        res = [self._ncc_grad(m, sh, sw) for m, (sh, sw, _) in zip(mom.tolist(), sizes)]
         ncc_ap, d_ap_dtx, d_ap_dtz = res[0]
         ncc_lat, d_lat_dty, d_lat_dtz = res[1]
         loss = 0.5 * (1.0 - ncc_ap) + 0.5 * (1.0 - ncc_lat)
