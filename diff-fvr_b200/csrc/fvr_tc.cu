@@ -425,10 +425,14 @@ __global__ void __launch_bounds__(kSnccThreads, MINB) tc_sncc_moments_kernel(Snc
 }
 
 // Value-and-gradient epilogue, launched right after the moments kernel as its
-// programmatic dependent (one CTA of 512 threads).  The work goes in chunks
-// of candidates whose (view, candidate) items fit in shared memory:
-//  0. the slice-axes Jacobians of the first chunk's items, formed while the
-//     moments kernel still runs (later chunks: before their record sums);
+// programmatic dependent (CTAs of 512 threads).  The work goes in chunks
+// of candidates whose (view, candidate) items fit in shared memory, one CTA per
+// chunk (256 candidates x 2 views, 512^3 spectrum: the step takes 219 us, and
+// 227 us with one CTA serial over the chunks).
+// A single chunk also reduces the losses; several leave that to a small
+// dependent kernel that reads every candidate's ncc:
+//  0. the slice-axes Jacobians of the chunk's items, formed while the moments
+//     kernel still runs;
 //  1. after griddepcontrol.wait, one thread per (item, moment): the item's
 //     records summed in record order, every load of a thread issued in one
 //     round, kept in shared memory;
@@ -436,12 +440,35 @@ __global__ void __launch_bounds__(kSnccThreads, MINB) tc_sncc_moments_kernel(Snc
 //     (per axis gc (a A + 2 b B) through the Jacobian, translations from the
 //     phase moments);
 //  3. one thread per candidate: the views summed in order; the ncc sums for
-//     the losses accumulate per thread across chunks and are reduced in a
-//     fixed order at the end.
+//     the losses are reduced in a fixed order at the end.
 constexpr int kFinalThreads = 512;
 constexpr int kFinalChunkItems = 128;  // 128 items x 44 doubles = 44 KB of shared memory
 constexpr int kFinalPairs = (kFinalChunkItems * M_NGRAD + kFinalThreads - 1) / kFinalThreads;  // per thread
 constexpr int kFinalRecords = 4;  // records per (item, moment) per load round
+
+// loss[v] = 1 - mean_c ncc from per-thread ncc sums (fixed order: per thread,
+// per warp, across warps), loss[nv] their sum.
+__device__ __forceinline__ void sncc_losses(const double (&lsum)[kMaxViews], int nv, int C, float* loss,
+                                            double (*red)[kFinalThreads / 32]) {
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+#pragma unroll
+  for (int v = 0; v < kMaxViews; ++v) {
+    const double sv = warp_sum(lsum[v]);
+    if (lane == 0) red[v][w] = sv;
+  }
+  __syncthreads();
+  if (t == 0) {
+    double total = 0.0;
+    for (int v = 0; v < nv; ++v) {
+      double sv = 0.0;
+      for (int k = 0; k < kFinalThreads / 32; ++k) sv += red[v][k];
+      const double l = 1.0 - sv / C;
+      loss[v] = static_cast<float>(l);
+      total += l;
+    }
+    loss[nv] = static_cast<float>(total);
+  }
+}
 
 __global__ void __launch_bounds__(kFinalThreads) tc_sncc_final_kernel(SnccArgs a) {
   __shared__ double s_mom[kFinalChunkItems][M_NGRAD];
@@ -452,15 +479,15 @@ __global__ void __launch_bounds__(kFinalThreads) tc_sncc_final_kernel(SnccArgs a
   const double s3[3] = {a.sx, a.sy, a.sz};
   double lsum[kMaxViews] = {0.0, 0.0, 0.0, 0.0};
   const int cch = kFinalChunkItems / nv;  // candidates per chunk; chunk item li = v * cn + (c - c0)
-  for (int c0 = 0; c0 < C; c0 += cch) {
-    const int cn = min(cch, C - c0), ni = cn * nv;
-    if (c0 > 0) __syncthreads();  // the previous chunk is done with the shared arrays
+  {
+    const int c0 = blockIdx.x * cch, cn = min(cch, C - c0), ni = cn * nv;
     if (t < ni) {
       const int v = t / cn, c = c0 + (t - v * cn);
       double ax[8];
       slice_axes_jac(a.poses + 6 * c, view_lateral(a, v), a.sx, a.sy, a.sz, ax, s_jac[t]);
     }
-    if (c0 == 0) pdl_wait();  // the moments kernel has completed and its records are visible
+    if (gridDim.x > 1) pdl_launch_dependents();  // the loss kernel
+    pdl_wait();  // the moments kernel has completed and its records are visible
     // record sums: the thread's pairs p = t + k * 512, all their loads in one round
     const double* src[kFinalPairs];
 #pragma unroll
@@ -546,33 +573,30 @@ __global__ void __launch_bounds__(kFinalThreads) tc_sncc_final_kernel(SnccArgs a
       for (int k = 0; k < 6; ++k) g[k] = a.accumulate ? g[k] + rf[k] : rf[k];
     }
   }
-  // loss[v] = 1 - mean_c ncc (fixed order: per thread, per warp, across warps)
-  const int lane = t & 31, w = t >> 5;
-#pragma unroll
-  for (int v = 0; v < kMaxViews; ++v) {
-    const double sv = warp_sum(lsum[v]);
-    if (lane == 0) red[v][w] = sv;
-  }
-  __syncthreads();
-  if (t == 0) {
-    double total = 0.0;
-    for (int v = 0; v < nv; ++v) {
-      double sv = 0.0;
-      for (int k = 0; k < kFinalThreads / 32; ++k) sv += red[v][k];
-      const double l = 1.0 - sv / C;
-      a.loss[v] = static_cast<float>(l);
-      total += l;
-    }
-    a.loss[nv] = static_cast<float>(total);
-  }
+  if (gridDim.x == 1) sncc_losses(lsum, nv, C, a.loss, red);
 }
 
-// Launch the epilogue as a programmatic dependent of the kernel before it on
-// the stream (plain launch where the attribute is refused).
-static void launch_sncc_final(cudaStream_t s, const SnccArgs& a) {
+// The losses of a batch whose epilogue had several chunks.
+__global__ void __launch_bounds__(kFinalThreads) tc_sncc_loss_kernel(const double* __restrict__ mom, int C, int nv,
+                                                                     float* __restrict__ loss) {
+  __shared__ double red[kMaxViews][kFinalThreads / 32];
+  pdl_wait();  // the epilogue has completed (and the moments kernel before it)
+  double lsum[kMaxViews] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int v = 0; v < kMaxViews; ++v)
+    if (v < nv)
+      for (int c = threadIdx.x; c < C; c += kFinalThreads)
+        lsum[v] += __ldcg(mom + (static_cast<int64_t>(v) * C + c) * kMomStride + 17);
+  sncc_losses(lsum, nv, C, loss, red);
+}
+
+// Launch a kernel as a programmatic dependent of the kernel before it on the
+// stream (plain launch where the attribute is refused).
+template <typename... P, typename... A>
+static void launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(1);
-  cfg.blockDim = dim3(kFinalThreads);
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -580,10 +604,17 @@ static void launch_sncc_final(cudaStream_t s, const SnccArgs& a) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, tc_sncc_final_kernel, a) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...) != cudaSuccess) {
     (void)cudaGetLastError();
-    tc_sncc_final_kernel<<<1, kFinalThreads, 0, s>>>(a);
+    kernel<<<grid, block, 0, s>>>(static_cast<P>(args)...);
   }
+}
+
+static void launch_sncc_final(cudaStream_t s, const SnccArgs& a) {
+  const unsigned chunks = static_cast<unsigned>(cdiv64(a.C, kFinalChunkItems / a.nv));
+  launch_dependent(tc_sncc_final_kernel, chunks, kFinalThreads, s, a);
+  if (chunks > 1)
+    launch_dependent(tc_sncc_loss_kernel, 1, kFinalThreads, s, static_cast<const double*>(a.mom), a.C, a.nv, a.loss);
 }
 
 // Record sums (fp64, fixed order) -> mom[v][c][0..NM), ncc in mom[v][c][17];
@@ -594,6 +625,7 @@ __global__ void __launch_bounds__(1024) tc_sncc_finalize_kernel(const double* __
                                                                 float* __restrict__ ncc_out) {
   __shared__ double red[32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  pdl_wait();  // launched as a programmatic dependent of the moments kernel
   for (int item = w; item < nv * C; item += nw) {
     double s = 0.0;
     if (lane < NM) {
@@ -1016,8 +1048,9 @@ int fvr_tc_sncc_finalize(const void* workspace, int64_t C, int64_t R, int nviews
   if (!workspace || !mom || !loss || C < 1 || R < 1 || nviews < 1 || nviews > kMaxViews) return FVR_ERR_ARG;
   if (variant < 0 || variant >= kSnccVariants) return FVR_ERR_ARG;
   const SnccPlan plan = sncc_plan(C, R, nviews, variant);
-  tc_sncc_finalize_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const double*>(workspace), (int)C, nviews, plan.tiles, with_grad ? M_NGRAD : 3, mom, loss, ncc_out);
+  launch_dependent(tc_sncc_finalize_kernel, 1, 1024, static_cast<cudaStream_t>(stream),
+                   static_cast<const double*>(workspace), (int)C, nviews, plan.tiles, with_grad ? M_NGRAD : 3, mom, loss,
+                   ncc_out);
   FVR_LAUNCH_CHECK();
   return FVR_OK;
 }
