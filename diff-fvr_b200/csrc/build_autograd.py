@@ -4,7 +4,8 @@ the CUDA library through its C ABI and holds no kernels).
 
     python build_autograd.py [--force]
 
-Rebuilds only when the source or this script is newer than the library.
+Rebuilds only when the source, the C header or this script is newer than the
+library.
 """
 from __future__ import annotations
 
@@ -17,6 +18,7 @@ from pathlib import Path
 HERE = Path(__file__).resolve().parent
 SRC = HERE / "fvr_autograd.cpp"
 OUT = HERE.parent / "fvr" / "_fvr_autograd.so"
+INCLUDE = HERE.parent.parent / "include"  # fvr_b200.h
 
 
 def _command():
@@ -25,7 +27,7 @@ def _command():
     torch_dir = Path(torch.__file__).resolve().parent
     cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     incs = [torch_dir / "include", torch_dir / "include" / "torch" / "csrc" / "api" / "include",
-            Path(cuda_home) / "include", Path(sysconfig.get_paths()["include"])]
+            Path(cuda_home) / "include", Path(sysconfig.get_paths()["include"]), INCLUDE]
     abi = int(bool(torch._C._GLIBCXX_USE_CXX11_ABI))
     lib = torch_dir / "lib"
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
@@ -38,7 +40,7 @@ def _command():
 
 
 def build(force: bool = False) -> Path:
-    stamp = max(SRC.stat().st_mtime, Path(__file__).stat().st_mtime)
+    stamp = max(p.stat().st_mtime for p in (SRC, INCLUDE / "fvr_b200.h", Path(__file__)))
     if not force and OUT.exists() and OUT.stat().st_mtime >= stamp:
         return OUT
     subprocess.run(_command(), check=True)

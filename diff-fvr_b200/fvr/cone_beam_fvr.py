@@ -24,6 +24,7 @@ import torch
 import torch.nn as nn
 
 from . import _lib as L
+from . import _native as NA
 from . import _runtime as RT
 from . import profiling
 
@@ -195,7 +196,8 @@ _GRAD_IMAGE_BYTES = 4 << 30
 def _prepared_lattice(lattice, device):
     """Device copies of an 11-tuple lattice's ray tables and its basis
     (src0, u0, v0, n0) as 12 host doubles, its separable ray tables when
-    it has them and whether those are monotone, cached per (storage, device): the lattice is a per-geometry
+    it has them, whether those are monotone and the native binding's record of
+    them, cached per (storage, device): the lattice is a per-geometry
     constant, moved once.  The entry holds the lattice's own tensors, so their
     storage cannot be freed and reused by another lattice while the entry
     exists."""
@@ -207,7 +209,10 @@ def _prepared_lattice(lattice, device):
         basis = torch.cat([lattice[i].reshape(3) for i in (0, 2, 3, 4)]).detach().double().cpu()
         base = (_ct.c_double * 12)(*[float(x) for x in basis])
         rays = tuple(t.detach().to(device=device, dtype=torch.float32).contiguous() for t in lattice[5:8])
-        hit = (key, base, rays, tuple(lattice[:8]), *_separable_tables(rays[0], rays[1]))
+        sep, monotone = _separable_tables(rays[0], rays[1])
+        native = NA.module()
+        plan = native.PouLattice(list(base), sep[0], sep[1], rays[2]) if native is not None and sep is not None else None
+        hit = (key, base, rays, tuple(lattice[:8]), sep, monotone, plan)
         _LATTICE_CACHE[key] = hit
     return hit
 
@@ -254,6 +259,12 @@ def _block_images_adjoint(model, geo, N, grad_imgs, s):
     return ws, (P * P + 255) // 256
 
 
+def _gather_adjoint(model, monotone, N, H, W):
+    """Whether the backward of N poses takes the separable warp adjoint."""
+    return (monotone and model.fused_warp_adjoint and 4 * model.B * N * model.P * model.P <= _GRAD_IMAGE_BYTES
+            and bool(L.query("fvr_pou_warp_sep_adjoint_supported", model.P, H, W)))
+
+
 class _PinholeFn(torch.autograd.Function):
     """SE(3)-invariant pinhole path (cone_beam_fvr.py:547-573, 670-686):
     mats -> pose geometry -> block slices -> batched IFFT -> warp-sum."""
@@ -264,7 +275,7 @@ class _PinholeFn(torch.autograd.Function):
         m = mats.detach().to(device=dev, dtype=torch.float32).contiguous()
         N = int(m.shape[0])
         B, P = model.B, model.P
-        _, base, _, _, sep, monotone = _LATTICE_CACHE[base_key]
+        _, base, _, _, sep, monotone, _ = _LATTICE_CACHE[base_key]
         geo = torch.empty((N, int(L.query("fvr_pou_geo_stride"))), dtype=torch.float64, device=dev)
         offs = torch.empty((B, N, 3), dtype=torch.float64, device=dev)
         s = L.stream_ptr(dev)
@@ -303,8 +314,7 @@ class _PinholeFn(torch.autograd.Function):
         H, W = int(rx.shape[0]), int(rx.shape[1])
         s = L.stream_ptr(dev)
         g = g_out.detach().to(device=dev, dtype=torch.float32).contiguous()
-        gather = (monotone and model.fused_warp_adjoint and 4 * B * N * P * P <= _GRAD_IMAGE_BYTES
-                  and L.query("fvr_pou_warp_sep_adjoint_supported", P, H, W))
+        gather = _gather_adjoint(model, monotone, N, H, W)
         if gather and not profiling.active() and L.query("fvr_pou_image_supported", P):
             st = model._stencil
             wsb = L.query("fvr_pou_pinhole_backward_workspace", B, N, H, W)
@@ -572,12 +582,34 @@ class PerspectiveSlabFVR(nn.Module):
             H, W = int(lattice[1].shape[0]), int(lattice[1].shape[1])
             return torch.zeros((0, 1, H, W), dtype=torch.float32, device=home) + 0.0 * pose_mats.sum()
         if len(lattice) >= 11:
-            key, _, (rx, ry, ic), _, _, _ = _prepared_lattice(lattice, self._dev)
+            key, _, (rx, ry, ic), _, _, monotone, plan = _prepared_lattice(lattice, self._dev)
             mats = pose_mats if home == self._dev else pose_mats.to(self._dev)
-            out = _PinholeFn.apply(mats, self, rx, ry, ic, key)
+            H, W = int(rx.shape[0]), int(rx.shape[1])
+            native = NA.module()
+            grad = mats.requires_grad and torch.is_grad_enabled()
+            if (native is not None and plan is not None and tuple(mats.shape[1:]) == (4, 4)
+                    and L.query("fvr_pou_pinhole_supported", self.P, H, W)
+                    and (not grad or _gather_adjoint(self, monotone, int(mats.shape[0]), H, W))):
+                out = NA.call(native.pinhole, 7 if grad else 3, mats, self._native_plan(native), plan)
+            else:
+                out = _PinholeFn.apply(mats, self, rx, ry, ic, key)
         else:
             out = self._forward_explicit(pose_mats, lattice)
         return out if out.device == home else out.to(home)
+
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "_plan"}  # the native record is made again on first use
+
+    def _native_plan(self, native):
+        """The native binding's record of the block spectra and geometry constants (made again when one was replaced)."""
+        parts = (self._stencil, self.centers, self._freqs)
+        plan = getattr(self, "_plan", None)
+        if plan is None or any(a is not b for a, b in zip(plan[0], parts)):
+            st = self._stencil
+            plan = (parts, native.PouModel(st.code, st.data, st.scales, self.B, self.P, self.ds_block, self.centers,
+                                           self._freqs))
+            self._plan = plan
+        return plan[1]
 
     def _forward_explicit(self, pose_mats, lattice):
         from .cone_beam_rays import forward_explicit

@@ -9,6 +9,7 @@ import ctypes as _ct
 import torch
 
 from . import _lib as L
+from . import _native as NA
 
 
 class _RaysFn(torch.autograd.Function):
@@ -132,6 +133,10 @@ def lattice_rays_supported(model, srcs, trg_pts):
 
 def project_lattice_rays(model, srcs, trg_pts):
     """(N, H, W) line integrals with the detector axes taken from ``trg_pts``."""
+    native = NA.module()
+    if native is not None:
+        grad = torch.is_grad_enabled() and (srcs.requires_grad or trg_pts.requires_grad)
+        return NA.call(native.lattice_rays, 11 if grad else 5, srcs, trg_pts, model._native_plan(native))
     return _LatticeRaysFn.apply(srcs, trg_pts, model)
 
 

@@ -22,6 +22,7 @@ import numpy as np
 import torch
 
 from . import _lib as L
+from . import _native as NA
 from .cone_beam_fvr import edge_dominant_ncc
 from .graphs import no_gc_during_capture
 
@@ -125,6 +126,11 @@ def biplanar_loss_per_candidate(imA, imB, refA, refB) -> torch.Tensor:
     """1 - 0.5 (sim_A + sim_B), sim = 0.75 edge-dominant NCC + 0.25 image NCC
     (exp30:120-134); one value per candidate."""
     if _reg_loss_fused((imA, imB), (refA, refB)):
+        native = NA.module()
+        if native is not None:
+            grad = torch.is_grad_enabled() and (imA.requires_grad or imB.requires_grad)
+            return NA.call(native.reg_loss, 3 if grad else 2, imA.float(), imB.float(), refA, refB,
+                           max(4, int(imA.shape[-1]) // 8), _MS_WEIGHT, _EDGE_WEIGHT)
         return _RegLossFn.apply(imA.float(), imB.float(), refA.float(), refB.float())
 
     def pair(p, r):

@@ -31,13 +31,11 @@ import torch
 import torch.nn as nn
 
 from . import _lib as L
+from . import _native as NA
 from . import _runtime as RT
 from . import autotune, profiling
 
-try:  # native autograd binding (csrc/fvr_autograd.cpp, built next to the CUDA library)
-    from . import _fvr_autograd as _NATIVE
-except ImportError:
-    _NATIVE = None
+_NATIVE = NA._MOD  # native autograd binding (csrc/fvr_autograd.cpp, built next to the CUDA library), or None
 
 VIEW_AP, VIEW_LATERAL = 0, 1
 
@@ -466,6 +464,7 @@ class TorchDiffFVREngine(nn.Module):
         del planar
         self._fused_ws = {}  # (C, R, views, device) -> workspace of the fused value_and_grad
         self._fused_calls = {}  # prepared launches of the fused value_and_grad
+        self._image_plans = {}  # output size -> native record of the image path
 
     def _sncc_storage(self):
         """The spectrum copy the spectral-NCC moments kernels read: the x-pair
@@ -520,7 +519,28 @@ class TorchDiffFVREngine(nn.Module):
         if p.shape[0] == 0:  # an empty batch renders no image (still connected to the poses)
             R = int(out_res)
             return torch.zeros((0, 1, R, R), dtype=torch.float32, device=self._dev) + 0.0 * p.sum()
-        return _ImageFn.apply(p, self, _view_code(view), int(out_res))
+        R = int(out_res)
+        native = NA.module()
+        if native is not None and p.dim() == 2 and p.shape[1] == 6 and L.query("fvr_image_supported", R, R):
+            grad = p.requires_grad and torch.is_grad_enabled()
+            return NA.call(native.image, 2 if grad else 1, p, self._image_plan(native, R), _view_code(view))
+        return _ImageFn.apply(p, self, _view_code(view), R)
+
+    def __getstate__(self):
+        return {**self.__dict__, "_image_plans": {}}  # native records are made again on first use
+
+    def _image_plan(self, native, R):
+        """The native binding's record of the image path at one output size (made
+        again when the storage or the spacing was replaced)."""
+        st, kap = self._stencil, RT.kappa(R, self.spacing[0])
+        hit = self._image_plans.get(R)
+        if hit is None or hit[0] is not st or hit[1] != kap:
+            if len(self._image_plans) > 64:
+                self._image_plans.clear()
+            hit = (st, kap, native.ImagePlan(st.code, st.data, st.scales, *st.dims, R, kap, RT.linspace(R, self._dev),
+                                             RT.twiddles(R, L.F32_, self._dev)))
+            self._image_plans[R] = hit
+        return hit[2]
 
     def forward(self, poses: torch.Tensor, view: str = "ap", out_res: int = 128) -> torch.Tensor:
         """Batched differentiable forward pass returning ``(B, 1, out_res, out_res)``."""
@@ -581,4 +601,9 @@ class TorchDiffFVREngine(nn.Module):
         pred = pred_drr if pred_drr.is_cuda else pred_drr.to(self._dev)
         H, W = int(pred.shape[-2]), int(pred.shape[-1])
         hp = RT.hp_filter(H, W, cutoff_sigma, pred.device) if high_pass else None
+        native = NA.module()
+        if (native is not None and pred.numel() > 0 and tuple(target_drr.shape[-2:]) == (H, W)
+                and not pred.is_complex() and not target_drr.is_complex() and L.query("fvr_image_supported", H, W)):
+            return NA.call(native.image_ncc, 2, pred, target_drr, hp, RT.twiddles(H, L.F32_, pred.device),
+                           RT.twiddles(W, L.F32_, pred.device))
         return _ImageSpectralNCCFn.apply(pred, target_drr, hp)
