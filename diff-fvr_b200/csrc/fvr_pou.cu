@@ -430,8 +430,11 @@ constexpr int kPouImgThreads = 512;
 
 // Row / column split-position tables of one (pose, block) image: entry j < P
 // is the column part fx_j u, entry P + i the row part c + fy_i v (fp64, split
-// into integer cell and float fraction; .w = the frequency).
-__device__ __forceinline__ void pou_image_tables(const AxisTables& t, const PouSliceArgs& a, const double* g) {
+// into integer cell and float fraction; frac.w = the frequency, idx.w =
+// where(e), free for the caller).
+template <class Where>
+__device__ __forceinline__ void pou_image_tables(const AxisTables& t, const PouSliceArgs& a, const double* g,
+                                                 Where where) {
   for (int e = threadIdx.x; e < 2 * a.P; e += blockDim.x) {
     const bool col = e < a.P;
     const float kf = __ldg(a.freqs + (col ? e : e - a.P));
@@ -440,41 +443,53 @@ __device__ __forceinline__ void pou_image_tables(const AxisTables& t, const PouS
     const double py = col ? k * g[13] : fma(k, g[16], a.c);
     const double pz = col ? k * g[14] : fma(k, g[17], a.c);
     const double fx = floor(px), fy = floor(py), fz = floor(pz);
-    t.idx[e] = make_int4(static_cast<int>(fx), static_cast<int>(fy), static_cast<int>(fz), 0);
+    t.idx[e] = make_int4(static_cast<int>(fx), static_cast<int>(fy), static_cast<int>(fz), where(e));
     t.frac[e] = make_float4(static_cast<float>(px - fx), static_cast<float>(py - fy), static_cast<float>(pz - fz), kf);
   }
 }
 
 template <int DT, bool DERIV>
-__device__ __forceinline__ void pou_table_sample(const Stencil& st, const Raw<DT>& raw, const float4& fa,
-                                                 const float4& fb, Interp& o) {
+__device__ __forceinline__ void pou_table_sample(const Raw<DT>& raw, const float4& fa, const float4& fb, Interp2& o) {
   float tx = fa.x + fb.x, ty = fa.y + fb.y, tz = fa.z + fb.z;
   if (tx >= 1.f) tx -= 1.f;
   if (ty >= 1.f) ty -= 1.f;
   if (tz >= 1.f) tz -= 1.f;
-  Sample8 sm;
-  tab_decode<DT>(raw, sm);
-  trilerp<DERIV>(sm, tx, ty, tz, o);
-  const float sc = raw_scale(raw);
+  Sample8c sm;
+  tab_decode2<DT>(raw, sm);
+  trilerp2<DERIV>(sm, tx, ty, tz, o);
   if (DT == FVR_F16) {
-    o.sr *= sc;
-    o.si *= sc;
+    const float2 sc = f2(raw_scale(raw));
+    o.s = mul2(o.s, sc);
     if (DERIV) {
-      o.dxr *= sc;
-      o.dxi *= sc;
-      o.dyr *= sc;
-      o.dyi *= sc;
-      o.dzr *= sc;
-      o.dzi *= sc;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) o.d[k] = mul2(o.d[k], sc);
     }
   }
 }
 
-// Smem layout of the fused forward image kernel: the P x (P + 1) complex
-// image, then the 2P-entry tables.
-__host__ __device__ constexpr int64_t pou_image_smem(int P) {
-  return static_cast<int64_t>(P) * (P + 1) * 8 + 40 * 2 * static_cast<int64_t>(P) + 16;
-}
+// Shared-memory layout of a block image's half spectrum: rows of P / 2 pairs,
+// natural column k at col(k).  The warp transform leaves a lane's elements at a
+// stride of M between lanes (wfft_elem): for even M one slot of padding per 16
+// columns spreads a row store over the banks and keeps the natural-order reads
+// free of conflicts, and an odd pitch does so for the column accesses.
+template <int M>
+struct PouLayout {
+  static constexpr int P = 32 * M, H = P / 2;
+  static constexpr bool kPad = M % 2 == 0;
+  static constexpr int kCols = P + (kPad ? P / 16 : 0);
+  static constexpr int kPitch = kCols | 1;            // forward
+  static constexpr int kPitchAdj = (kCols + 2) | 1;   // adjoint: two more columns
+  __device__ static __forceinline__ int col(int k) { return kPad ? k + (k >> 4) : k; }
+  // column slot of a lane's transform result `slot`, base = col of its slot 0
+  __device__ static __forceinline__ int store_col(int lane, int base, int slot) {
+    constexpr int MH = M / 2;
+    if (M % 2) return wfft_elem<M>(lane, slot);
+    return base + (slot < MH ? slot : slot - MH + 17 * M);
+  }
+  static constexpr int64_t kTables = 64 * static_cast<int64_t>(P);  // idx + frac of 2 P entries
+  static constexpr int64_t kImage = (static_cast<int64_t>(H) * kPitch * 8 + 15) / 16 * 16;
+  static constexpr int64_t kAdjoint = (static_cast<int64_t>(H) * kPitchAdj * 8 + 15) / 16 * 16;
+};
 
 // Hermitian pairing of slice samples.  A block is real, so its centred
 // spectrum obeys F[c + m] = conj F[c - m] for |m| < P/2 in every axis (grid
@@ -517,9 +532,9 @@ __device__ __forceinline__ void pou_gather_row(const Stencil& st, const AxisTabl
   for (int m = 0; m < M; ++m) {
     const int c = lane + 32 * m;
     const int jj = c + H < P ? c + H : c - H;
-    Interp o;
-    pou_table_sample<DT, false>(st, raw[m], fa, tab.frac[jj], o);
-    x[m] = Cx<float>{o.sr, o.si};
+    Interp2 o;
+    pou_table_sample<DT, false>(raw[m], fa, tab.frac[jj], o);
+    x[m] = Cx<float>{o.s.x, o.s.y};
   }
 }
 
@@ -579,17 +594,17 @@ __device__ __forceinline__ void pou_gather_row_hermitian(const Stencil& st, cons
   for (int m = 0; m < M; ++m) {
     const int c = lane + 32 * m;
     const int jj = c + H < P ? c + H : c - H;
-    Interp o;
-    pou_table_sample<DT, false>(st, raw[m], fa, tab.frac[jj], o);
-    h[m] = Cx<float>{o.sr, o.si};
+    Interp2 o;
+    pou_table_sample<DT, false>(raw[m], fa, tab.frac[jj], o);
+    h[m] = Cx<float>{o.s.x, o.s.y};
   }
   for (;;) {
     if (pend) {
-      Interp o;
-      pou_table_sample<DT, false>(st, rawp, fap, tab.frac[jp], o);
+      Interp2 o;
+      pou_table_sample<DT, false>(rawp, fap, tab.frac[jp], o);
 #pragma unroll
       for (int m = 0; m < M; ++m)
-        if (m == mp) h[m] = Cx<float>{0.5f * (h[m].x + o.sr), 0.5f * (h[m].y - o.si)};
+        if (m == mp) h[m] = Cx<float>{0.5f * (h[m].x + o.s.x), 0.5f * (h[m].y - o.s.y)};
       pend &= pend - 1;
     }
     if (!__any_sync(0xffffffffu, pend != 0)) break;
@@ -612,20 +627,35 @@ __device__ __forceinline__ void pou_gather_row_hermitian(const Stencil& st, cons
 // and P/2 are real after the transform and share one FFT as real and
 // imaginary part), and the column pass transforms two real-output columns per
 // complex FFT.  That is P/2 + P/2 FFTs instead of 2P.
-template <int DT, int M>
-__global__ void __launch_bounds__(kPouImgThreads, 1) pou_slice_ifft_kernel(PouSliceArgs a, float* __restrict__ imgs) {
-  constexpr int P = 32 * M, PITCH = P + 1, H = P / 2, NW = kPouImgThreads / 32;
+//
+// Row 0 of the buffer holds rows 0 and P/2 as they come out of their shared
+// transform, and each column transform writes its P results over the two
+// columns of P/2 values it has read (position < P/2 to the first, the rest to
+// the second), so the buffer is P/2 rows high and two CTAs fit on an SM.
+//
+// Bound by instruction issue and by the latency of the random entry loads (f32
+// also by their bytes: the entries of one image are read about once, 537 MB
+// from HBM for 1024 images).  64 blocks x 64 poses, P = 128, f32: 700 us with a
+// full-height buffer, transforms that exchange both registers and an output
+// pass in transform order (8-way bank conflicts); 593 with the half buffer and
+// natural column order; 535 with the transform's one-register exchange; 489
+// with two CTAs an SM (4.4 TB/s).  bf16: 384.
+template <int DT, int M, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) pou_slice_ifft_kernel(PouSliceArgs a, float* __restrict__ imgs) {
+  using L = PouLayout<M>;
+  constexpr int P = 32 * M, PITCH = L::kPitch, H = P / 2, NW = NT / 32;
   extern __shared__ __align__(16) unsigned char smem[];
   Cx<float>* buf = reinterpret_cast<Cx<float>*>(smem);
-  const AxisTables tab = axis_tables(smem + ((static_cast<int64_t>(P) * PITCH * 8 + 15) / 16) * 16, 2 * P);
+  const AxisTables tab = axis_tables(smem + L::kImage, 2 * P);
   const int n = blockIdx.x, b = blockIdx.y;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const Stencil st = pou_block_stencil(a, b);
-  pou_image_tables(tab, a, a.geo + n * kGeo);
+  pou_image_tables(tab, a, a.geo + n * kGeo, [](int) { return 0; });
   WarpFft<M, true> fft;
   fft.init(lane);
   __syncthreads();
   // rows: unit 0 = natural rows 0 and H (table rows H and 0), unit u = row u
+  const int sc = L::col(wfft_elem<M>(lane, 0));
   for (int u = wid; u < H; u += NW) {
     Cx<float> h[M];
     if (u == 0) {
@@ -640,82 +670,104 @@ __global__ void __launch_bounds__(kPouImgThreads, 1) pou_slice_ifft_kernel(PouSl
       pou_gather_row_hermitian<DT, M>(st, tab, u, lane, h);
     }
     fft.run(h, lane);
-    if (u == 0) {
 #pragma unroll
-      for (int k = 0; k < M; ++k) {
-        buf[lane + 32 * k] = Cx<float>{h[k].x, 0.f};
-        buf[H * PITCH + lane + 32 * k] = Cx<float>{h[k].y, 0.f};
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < M; ++k) buf[u * PITCH + lane + 32 * k] = h[k];
-    }
+    for (int k = 0; k < M; ++k) buf[u * PITCH + L::store_col(lane, sc, k)] = h[k];
   }
   __syncthreads();
-  // columns: buffer columns 2t and 2t + 1 as real and imaginary part of one
-  // transform (rows r > H read as the conjugate of row P - r); the real
-  // results of both land in column 2t
+  // columns: t and t + H as real and imaginary part of one transform (rows
+  // r > H are the conjugate of row P - r)
   for (int t = wid; t < H; t += NW) {
-    const int c1 = 2 * t;
+    const int c0 = L::col(t), c1 = L::col(t + H);
     Cx<float> z[M];
 #pragma unroll
     for (int m = 0; m < M; ++m) {
       const int r = lane + 32 * m;
-      const int rr = r <= H ? r : P - r;
-      const float sg = r <= H ? 1.f : -1.f;
-      const Cx<float> p = buf[rr * PITCH + c1], q = buf[rr * PITCH + c1 + 1];
-      z[m] = Cx<float>{p.x - sg * q.y, sg * p.y + q.x};
+      const int rr = r < H ? r : r == H ? 0 : P - r;
+      const float sg = r == 0 || r == H ? 0.f : r < H ? 1.f : -1.f;
+      Cx<float> p = buf[rr * PITCH + c0], q = buf[rr * PITCH + c1];
+      if (r == H) {
+        p.x = p.y;
+        q.x = q.y;
+      }
+      z[m] = Cx<float>{fmaf(-sg, q.y, p.x), fmaf(sg, p.y, q.x)};
     }
+    __syncwarp();
     fft.run(z, lane);
 #pragma unroll
-    for (int k = 0; k < M; ++k) buf[(lane + 32 * k) * PITCH + c1] = z[k];
+    for (int k = 0; k < M; ++k) {
+      const int pos = lane + 32 * k;
+      buf[pos < H ? pos * PITCH + c0 : (pos - H) * PITCH + c1] = z[k];
+    }
   }
   __syncthreads();
-  // fftshift-ordered image, coalesced rows
+  // fftshift-ordered image: element (ky, t) holds columns t and t + H
   const float scale = 1.f / static_cast<float>(P * P);
   float* out = imgs + (static_cast<int64_t>(b) * a.N + n) * P * P;
-  for (int q = threadIdx.x; q < P * P; q += kPouImgThreads) {
-    const int y = q / P, xq = q - y * P;
-    const int ky = y + H < P ? y + H : y - H, kx = xq + H < P ? xq + H : xq - H;
-    const int px = wfft_pos<M>(kx);
-    const Cx<float> v = buf[wfft_pos<M>(ky) * PITCH + (px & ~1)];
-    out[q] = ((px & 1) ? v.y : v.x) * scale;
+  for (int q = threadIdx.x; q < P * H; q += NT) {
+    const int y = q / H, t = q - y * H;
+    const int pos = wfft_pos<M>(y + H < P ? y + H : y - H);
+    const Cx<float> v = buf[pos < H ? pos * PITCH + L::col(t) : (pos - H) * PITCH + L::col(t + H)];
+    out[y * P + t + H] = v.x * scale;
+    out[y * P + t] = v.y * scale;
   }
 }
 
-// Shared memory of the adjoint: the row-pair spectra [P/2][P + 1], the half
-// spectrum G [P][P/2 + 1], the axis tables, one partner queue per warp.
+// Shared memory of the adjoint: the half spectrum, the axis tables, one
+// partner queue per warp.
 constexpr int kPouQueue = 256;
 
-__host__ __device__ constexpr int64_t pou_adjoint_tables_at(int P) {
-  return ((static_cast<int64_t>(P / 2) * (P + 1) + static_cast<int64_t>(P) * (P / 2 + 1)) * 8 + 15) / 16 * 16;
-}
-
-__host__ __device__ constexpr int64_t pou_adjoint_smem(int P) {
-  return pou_adjoint_tables_at(P) + 40 * 2 * static_cast<int64_t>(P) + (kPouImgThreads / 32) * kPouQueue * 2;
-}
-
-// G at natural frequency indices (ki, kj) from the stored half kj <= P/2
-// (rows in transform order): G(-k) = conj G(k) for the transform of a real image.
 template <int M>
-__device__ __forceinline__ Cx<float> pou_half_spectrum(const Cx<float>* gb, int ki, int kj) {
-  constexpr int P = 32 * M, H = P / 2, GP = H + 1;
-  if (kj <= H) return gb[wfft_pos<M>(ki) * GP + kj];
-  const Cx<float> v = gb[wfft_pos<M>(ki == 0 ? 0 : P - ki) * GP + (P - kj)];
-  return Cx<float>{v.x, -v.y};
+__host__ __device__ constexpr int64_t pou_adjoint_smem(int threads) {
+  return PouLayout<M>::kAdjoint + PouLayout<M>::kTables + (threads / 32) * kPouQueue * 2;
 }
 
-// acc += w (fx, fy) x <G, dS/dp> for the sample at table position (i, j).
-template <int DT, int M>
-__device__ __forceinline__ void pou_adjoint_sample(const Stencil& st, const AxisTables& tab, const Cx<float>* gb,
-                                                   const Raw<DT>& raw, int i, int j, float w, float (&acc)[6]) {
-  constexpr int P = 32 * M, H = P / 2;
-  const float4 fa = tab.frac[P + i], fb = tab.frac[j];
-  Interp o;
-  pou_table_sample<DT, true>(st, raw, fa, fb, o);
-  const Cx<float> G = pou_half_spectrum<M>(gb, i + H < P ? i + H : i - H, j + H < P ? j + H : j - H);
+// Where G(ki, kj) is kept: columns kj <= P/2 only (G(-k) = conj G(k) for the
+// transform of a real image), transform position p < P/2 of column kj in
+// buffer column c0 row p, the others in column c1 row p - P/2, where c0 and c1
+// are the two buffer columns that the column's transform has read (kj and P -
+// kj; the self-paired columns 0 and P/2 have a second column of their own).
+// The axis tables carry this: idx.w of column entry j = c0 | c1 << 12 | conj
+// << 24, of row entry i two 16-bit halves, for ki and -ki: row offset | second
+// column << 15.
+template <int M>
+__device__ __forceinline__ int pou_where(int e) {
+  using L = PouLayout<M>;
+  constexpr int P = 32 * M, H = P / 2, GP = L::kPitchAdj;
+  static_assert(H * GP < 32768, "row offsets are 15-bit");
+  if (e < P) {
+    const int k = e + H < P ? e + H : e - H;
+    const int kj = k <= H ? k : P - k;
+    const int c1 = kj == 0 ? L::kCols : kj == H ? L::kCols + 1 : L::col(P - kj);
+    return L::col(kj) | c1 << 12 | (k > H ? 1 << 24 : 0);
+  }
+  const int ki = e - P + H < P ? e - P + H : e - P - H;
+  unsigned w[2];
+#pragma unroll
+  for (int v = 0; v < 2; ++v) {
+    const int pos = wfft_pos<M>(v == 0 || ki == 0 ? ki : P - ki);
+    w[v] = pos < H ? pos * GP : ((pos - H) * GP) | 0x8000;
+  }
+  return static_cast<int>(w[0] | w[1] << 16);
+}
+
+__device__ __forceinline__ float2 pou_spectrum(const Cx<float>* gb, int row, int col) {
+  const bool cj = (col >> 24) != 0;
+  const int r = cj ? static_cast<int>(static_cast<unsigned>(row) >> 16) : row & 0xffff;
+  const Cx<float> v = gb[(r & 0x7fff) + ((r & 0x8000) ? (col >> 12) & 0xfff : col & 0xfff)];
+  return make_float2(v.x, cj ? -v.y : v.y);
+}
+
+// acc += w (fx, fy) x <G, dS/dp> for the sample of row entry (fa, wa) and
+// column entry (fb, wb).
+template <int DT>
+__device__ __forceinline__ void pou_adjoint_sample(const Cx<float>* gb, const Raw<DT>& raw, const float4& fa,
+                                                   const float4& fb, int wa, int wb, float w, float (&acc)[6]) {
+  Interp2 o;
+  pou_table_sample<DT, true>(raw, fa, fb, o);
+  const float2 G = pou_spectrum(gb, wa, wb);
   const float gx = G.x * w, gy = G.y * w;
-  const float e0 = gx * o.dxr + gy * o.dxi, e1 = gx * o.dyr + gy * o.dyi, e2 = gx * o.dzr + gy * o.dzi;
+  const float e0 = gx * o.d[0].x + gy * o.d[0].y, e1 = gx * o.d[1].x + gy * o.d[1].y,
+              e2 = gx * o.d[2].x + gy * o.d[2].y;
   const float fx = fb.w, fy = fa.w;
   acc[0] = fmaf(fx, e0, acc[0]);
   acc[1] = fmaf(fx, e1, acc[1]);
@@ -745,7 +797,10 @@ __device__ __forceinline__ void pou_adjoint_queue(const Stencil& st, const AxisT
   }
 #pragma unroll
   for (int u = 0; u < GROUP; ++u)
-    if (qq[u] >= 0) pou_adjoint_sample<DT, M>(st, tab, gb, raw[u], qq[u] / P, qq[u] % P, wscale, acc);
+    if (qq[u] >= 0) {
+      const int i = P + qq[u] / P, j = qq[u] % P;
+      pou_adjoint_sample<DT>(gb, raw[u], tab.frac[i], tab.frac[j], tab.idx[i].w, tab.idx[j].w, wscale, acc);
+    }
   __syncwarp();
 }
 
@@ -780,8 +835,11 @@ __host__ __device__ constexpr int64_t pou_fused_extra(int P, int Hd, int W) {
   return 4LL * (kPouImgThreads / 32) * (W + 4) + 8LL * W + 8LL * Hd + 16LL * (P + 1) + 16;
 }
 
-__host__ __device__ constexpr int64_t pou_fused_smem(int P, int Hd, int W) {
-  return (pou_adjoint_smem(P) + 15) / 16 * 16 + pou_fused_extra(P, Hd, W);
+// The gradient image comes first in it (the partner queues take its place
+// after the row pass).
+template <int M>
+__host__ __device__ constexpr int64_t pou_fused_smem(int Hd, int W) {
+  return PouLayout<M>::kAdjoint + PouLayout<M>::kTables + 4LL * (32 * M) * (32 * M) + pou_fused_extra(32 * M, Hd, W);
 }
 
 // Detector-row pass of the fused adjoint for one layout: warp = (row band,
@@ -1038,37 +1096,47 @@ __device__ void pou_warp_gather_adjoint(const PouWarpSep& w, int n, int b, int N
 // with a mirror twice, and queues the partners of the others; the Nyquist row
 // has no partner and goes through the queue once.
 //
+// The column transforms work in place (pou_where tells where each ends up), so
+// one half spectrum of P/2 rows is all that is kept and two CTAs fit on an SM
+// up to P = 128.  Bounds as for the forward; 64 blocks x 64 poses, P = 128, f32:
+// 737 us with a buffer each for the row and the column transforms, 592 now
+// (bf16 513; 16 blocks x 24 poses, P = 160, bf16: 173 -> 102).  Walking the
+// samples one column strip a warp, to keep a column's table entry in registers,
+// was slower in f32 (676): neighbouring rows share cache lines.
+//
 // FUSED: dL/dimgs is not read from memory but formed in shared memory from
 // the detector gradient (pou_warp_gather_adjoint), which also gives this
 // (pose, block)'s pose-offset gradients; the warp adjoint kernel and the
 // block-image gradient buffer drop out.
-template <int DT, int M, bool FUSED>
-__global__ void __launch_bounds__(kPouImgThreads, 1) pou_fft_slice_adjoint_kernel(PouSliceArgs a,
-                                                                                  const float* __restrict__ gimg,
-                                                                                  PouWarpSep wsep,
-                                                                                  double* __restrict__ partial) {
-  constexpr int P = 32 * M, PITCH = P + 1, H = P / 2, GP = H + 1, NW = kPouImgThreads / 32, GROUP = 4;
+template <int DT, int M, int NT, int MINB, bool FUSED>
+__global__ void __launch_bounds__(NT, MINB) pou_fft_slice_adjoint_kernel(PouSliceArgs a,
+                                                                         const float* __restrict__ gimg,
+                                                                         PouWarpSep wsep,
+                                                                         double* __restrict__ partial) {
+  using L = PouLayout<M>;
+  constexpr int P = 32 * M, GP = L::kPitchAdj, H = P / 2, NW = NT / 32, GROUP = 4;
   constexpr int BATCH = 32 * GROUP, NQ = P / NW;
+  static_assert(NQ <= 32 && P % NW == 0 && (H * P) % NT == 0, "queue start and loop trip counts");
+  static_assert(!FUSED || NT == kPouImgThreads, "the detector side is written for that block");
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double red[6 * NW];
   Cx<float>* zr = reinterpret_cast<Cx<float>*>(smem);
-  Cx<float>* gb = zr + H * PITCH;
-  const AxisTables tab = axis_tables(smem + pou_adjoint_tables_at(P), 2 * P);
+  const AxisTables tab = axis_tables(smem + L::kAdjoint, 2 * P);
   const int n = blockIdx.x, b = blockIdx.y;
   const int64_t nblk = gridDim.y;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  unsigned short* queue =
-      reinterpret_cast<unsigned short*>(smem + pou_adjoint_tables_at(P) + 80 * P) + wid * kPouQueue;
+  unsigned char* after = smem + L::kAdjoint + L::kTables;
+  unsigned short* queue = reinterpret_cast<unsigned short*>(after) + wid * kPouQueue;
   const Stencil st = pou_block_stencil(a, b);
-  pou_image_tables(tab, a, a.geo + n * kGeo);
+  pou_image_tables(tab, a, a.geo + n * kGeo, [](int e) { return pou_where<M>(e); });
   WarpFft<M, false> fft;
   fft.init(lane);
-  const float* g = FUSED ? reinterpret_cast<const float*>(gb)
+  const float* g = FUSED ? reinterpret_cast<const float*>(after)
                          : gimg + (static_cast<int64_t>(b) * a.N + n) * P * P;
   if constexpr (FUSED) {
     double sums[4] = {0.0, 0.0, 0.0, 0.0};
-    pou_warp_gather_adjoint<M>(wsep, n, b, a.N, smem + (pou_adjoint_smem(P) + 15) / 16 * 16,
-                               reinterpret_cast<float*>(zr), reinterpret_cast<float*>(gb), sums);
+    pou_warp_gather_adjoint<M>(wsep, n, b, a.N, after + 4 * P * P, reinterpret_cast<float*>(zr),
+                               reinterpret_cast<float*>(after), sums);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const double v = warp_sum(sums[k]);
@@ -1086,6 +1154,7 @@ __global__ void __launch_bounds__(kPouImgThreads, 1) pou_fft_slice_adjoint_kerne
     }
   }
   // rows: transform input rows 2s, 2s + 1 (image rows y0, y0 + 1 after ifftshift) together
+  const int sc = L::col(wfft_elem<M>(lane, 0));
   for (int s = wid; s < H; s += NW) {
     const int y0 = 2 * s + H < P ? 2 * s + H : 2 * s - H;
     Cx<float> z[M];
@@ -1100,24 +1169,29 @@ __global__ void __launch_bounds__(kPouImgThreads, 1) pou_fft_slice_adjoint_kerne
     }
     fft.run(z, lane);
 #pragma unroll
-    for (int k = 0; k < M; ++k) zr[s * PITCH + lane + 32 * k] = z[k];
+    for (int k = 0; k < M; ++k) zr[s * GP + L::store_col(lane, sc, k)] = z[k];
   }
   __syncthreads();
   // columns kx = 0 .. P/2: split the pair spectra (Z(k) + conj Z(-k)) / 2 and
-  // (Z(k) - conj Z(-k)) / 2i, then transform over the rows
+  // (Z(k) - conj Z(-k)) / 2i, then transform over the rows, in place
   for (int kx = wid; kx <= H; kx += NW) {
-    const int p0 = wfft_pos<M>(kx), p1 = wfft_pos<M>(kx == 0 ? 0 : P - kx);
+    const int p0 = L::col(kx), p1 = L::col(kx == 0 ? 0 : P - kx);
+    const int p2 = kx == 0 ? L::kCols : kx == H ? L::kCols + 1 : p1;
     Cx<float> x[M];
 #pragma unroll
     for (int m = 0; m < M; ++m) {
-      const int y = lane + 32 * m, sr = (y >> 1) * PITCH;
+      const int y = lane + 32 * m, sr = (y >> 1) * GP;
       const Cx<float> A = zr[sr + p0], B = zr[sr + p1];
       x[m] = (y & 1) ? Cx<float>{0.5f * (A.y + B.y), 0.5f * (B.x - A.x)}
                      : Cx<float>{0.5f * (A.x + B.x), 0.5f * (A.y - B.y)};
     }
+    __syncwarp();
     fft.run(x, lane);
 #pragma unroll
-    for (int k = 0; k < M; ++k) gb[(lane + 32 * k) * GP + kx] = x[k];
+    for (int k = 0; k < M; ++k) {
+      const int pos = lane + 32 * k;
+      zr[pos < H ? pos * GP + p0 : (pos - H) * GP + p2] = x[k];
+    }
   }
   // the Nyquist row (table row 0) starts the queue
   if (lane < NQ) queue[lane] = static_cast<unsigned short>(wid * NQ + lane);
@@ -1129,13 +1203,13 @@ __global__ void __launch_bounds__(kPouImgThreads, 1) pou_fft_slice_adjoint_kerne
   // own samples t < H P: table rows H+1 .. P-1 (all columns), row H (columns
   // 0 and H .. P-1), rows 1 .. H-1 (column 0); H P is a multiple of the
   // thread count, so every warp runs the same iterations
-  for (int t0 = threadIdx.x; t0 < H * P; t0 += kPouImgThreads * GROUP) {
+  for (int t0 = threadIdx.x; t0 < H * P; t0 += NT * GROUP) {
     Raw<DT> raw[GROUP];
     int qi[GROUP], qj[GROUP];
     float wt[GROUP];
 #pragma unroll
     for (int u = 0; u < GROUP; ++u) {
-      const int t = t0 + u * kPouImgThreads;
+      const int t = t0 + u * NT;
       int i, j;
       if (t < (H - 1) * P) {
         i = H + 1 + t / P;
@@ -1172,16 +1246,18 @@ __global__ void __launch_bounds__(kPouImgThreads, 1) pou_fft_slice_adjoint_kerne
     }
 #pragma unroll
     for (int u = 0; u < GROUP; ++u)
-      if (wt[u] != 0.f) pou_adjoint_sample<DT, M>(st, tab, gb, raw[u], qi[u], qj[u], wt[u], acc);
+      if (wt[u] != 0.f)
+        pou_adjoint_sample<DT>(zr, raw[u], tab.frac[P + qi[u]], tab.frac[qj[u]], tab.idx[P + qi[u]].w,
+                               tab.idx[qj[u]].w, wt[u], acc);
     __syncwarp();
     if (tail - head >= BATCH) {
-      pou_adjoint_queue<DT, M, GROUP>(st, tab, gb, queue, head, BATCH, lane, scale, acc);
+      pou_adjoint_queue<DT, M, GROUP>(st, tab, zr, queue, head, BATCH, lane, scale, acc);
       head += BATCH;
     }
   }
   while (tail > head) {
     const int cnt = tail - head < BATCH ? tail - head : BATCH;
-    pou_adjoint_queue<DT, M, GROUP>(st, tab, gb, queue, head, cnt, lane, scale, acc);
+    pou_adjoint_queue<DT, M, GROUP>(st, tab, zr, queue, head, cnt, lane, scale, acc);
     head += cnt;
   }
 #pragma unroll
@@ -1842,25 +1918,46 @@ static PouBase make_base(const double* base12) {
 
 using namespace fvr;
 
-template <int DT, int M>
-static int pou_image_launch(bool adjoint, const PouSliceArgs& a, int B, const float* gimg, float* imgs,
-                            double* part, cudaStream_t s) {
-  const int64_t smem = adjoint ? pou_adjoint_smem(32 * M) : pou_image_smem(32 * M);
+template <int DT, int M, int NT, int MINB>
+static int pou_image_launch_nt(bool adjoint, const PouSliceArgs& a, int B, const float* gimg, float* imgs,
+                               double* part, cudaStream_t s) {
+  const int64_t smem = adjoint ? pou_adjoint_smem<M>(NT) : PouLayout<M>::kImage + PouLayout<M>::kTables;
   dim3 grid(static_cast<unsigned>(a.N), static_cast<unsigned>(B));
   // the shared-memory opt-in is a per-device setting: made before every launch
   if (adjoint) {
-    if (cudaFuncSetAttribute(pou_fft_slice_adjoint_kernel<DT, M, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem)) != cudaSuccess)
+    if (cudaFuncSetAttribute(pou_fft_slice_adjoint_kernel<DT, M, NT, MINB, false>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
       return FVR_ERR_CUDA;
-    pou_fft_slice_adjoint_kernel<DT, M, false><<<grid, kPouImgThreads, smem, s>>>(a, gimg, PouWarpSep{}, part);
+    pou_fft_slice_adjoint_kernel<DT, M, NT, MINB, false><<<grid, NT, smem, s>>>(a, gimg, PouWarpSep{}, part);
   } else {
-    if (cudaFuncSetAttribute(pou_slice_ifft_kernel<DT, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(pou_slice_ifft_kernel<DT, M, NT, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(smem)) != cudaSuccess)
       return FVR_ERR_CUDA;
-    pou_slice_ifft_kernel<DT, M><<<grid, kPouImgThreads, smem, s>>>(a, imgs);
+    pou_slice_ifft_kernel<DT, M, NT, MINB><<<grid, NT, smem, s>>>(a, imgs);
   }
   FVR_LAUNCH_CHECK();
   return FVR_OK;
+}
+
+template <int DT, int M>
+static int pou_image_launch(bool adjoint, const PouSliceArgs& a, int B, const float* gimg, float* imgs,
+                            double* part, cudaStream_t s) {
+  // Threads per image.  Two 256-thread CTAs on an SM overlap one's gathers with
+  // the other's transforms and finish a pair of images in 1.6 to 1.87 times
+  // what one 512-thread CTA takes for one (P = 64 .. 128, f32 and bf16), so
+  // they win by the count of waves; a grid that fits in one wave wants the 16
+  // warps.  P = 160: the adjoint's buffer leaves room for one CTA only, and
+  // the forward with two is slower by 1.7x (16 blocks x 64 poses, bf16).
+  if constexpr (M <= 4) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      return FVR_ERR_CUDA;
+    const int64_t images = static_cast<int64_t>(a.N) * B;
+    const int64_t one = (images + sms - 1) / sms, two = (images + 2 * sms - 1) / (2 * sms);
+    if (15 * two < 8 * one) return pou_image_launch_nt<DT, M, 256, 2>(adjoint, a, B, gimg, imgs, part, s);
+  }
+  return pou_image_launch_nt<DT, M, 512, 1>(adjoint, a, B, gimg, imgs, part, s);
 }
 
 template <int DT>
@@ -1877,11 +1974,11 @@ static int pou_image_dispatch(bool adjoint, const PouSliceArgs& a, int B, const 
 
 template <int DT, int M>
 static int pou_fused_launch(const PouSliceArgs& a, int B, const PouWarpSep& w, double* part, cudaStream_t s) {
-  const int64_t smem = pou_fused_smem(32 * M, w.Hd, w.W);
-  if (cudaFuncSetAttribute(pou_fft_slice_adjoint_kernel<DT, M, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  const int64_t smem = pou_fused_smem<M>(w.Hd, w.W);
+  if (cudaFuncSetAttribute(pou_fft_slice_adjoint_kernel<DT, M, kPouImgThreads, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(smem)) != cudaSuccess)  // per-device setting: before every launch
     return FVR_ERR_CUDA;
-  pou_fft_slice_adjoint_kernel<DT, M, true>
+  pou_fft_slice_adjoint_kernel<DT, M, kPouImgThreads, 1, true>
       <<<dim3(static_cast<unsigned>(a.N), static_cast<unsigned>(B)), kPouImgThreads, smem, s>>>(a, nullptr, w, part);
   FVR_LAUNCH_CHECK();
   return FVR_OK;
@@ -2057,7 +2154,9 @@ int fvr_pou_warp_image_adjoint_supported(int64_t P, int64_t H, int64_t W) {
       cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
     return 0;
   const int64_t static_bytes = 6 * (kPouImgThreads / 32) * static_cast<int64_t>(sizeof(double));
-  return pou_fused_smem(static_cast<int>(P), static_cast<int>(H), static_cast<int>(W)) + static_bytes <= optin ? 1 : 0;
+  const int h = static_cast<int>(H), w = static_cast<int>(W);
+  const int64_t bytes = P == 64 ? pou_fused_smem<2>(h, w) : P == 96 ? pou_fused_smem<3>(h, w) : pou_fused_smem<4>(h, w);
+  return bytes + static_bytes <= optin ? 1 : 0;
 }
 
 int fvr_pou_warp_image_adjoint(int dtype, const void* stencil, const float* scales, int64_t B, int64_t P,
