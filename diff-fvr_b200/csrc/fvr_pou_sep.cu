@@ -9,6 +9,8 @@
 // detector rows with the column's image position in registers, so the
 // position arithmetic (fp64), the column's two image loads and the x
 // interpolation are paid once per image row instead of once per pixel.
+#include <type_traits>
+
 #include "fvr_common.cuh"
 
 namespace fvr {
@@ -299,19 +301,22 @@ __global__ void __launch_bounds__(32 * kSepFewWarps) pou_warp_sep_few_kernel(Sep
 // adjoint
 // ----------------------------------------------------------------------------
 
-constexpr int kSepBand = 8;      // image rows of a unit at most
-constexpr int kSepPass = 128;    // detector columns of a march, four per lane
-constexpr int kSepWide = 256;    // detector columns of a warp's G buffer
+constexpr int kSepBand = 8;             // image rows of a gather unit
+constexpr int kSepPairs = 5;            // pairs of cell rows it reads (the last is half used)
+constexpr int kSepPass = 128;           // detector columns of a march, four per lane
+constexpr int kSepStepCols = 512;        // detector columns of a step: 18 cell rows of 512 or 34 of 256
+constexpr int kSepBufBytes = 8 * (2 * kSepBand + 2) * kSepStepCols;  // cell-row sums of a CTA, 72 KB
+static_assert(8 * (4 * kSepBand + 2) * (kSepStepCols / 2) <= kSepBufBytes, "four bands of half rows");
 
 // Dynamic shared memory: column map (ix, tx) [Wp] (W rounded up to four), row fractions [Hd], first
 // table position at or beyond each image index [P + 3] for columns and rows,
-// the warps' G buffers.
+// the buffer of cell-row sums.
 __host__ __device__ constexpr int sep_padded(int W) { return (W + 3) / 4 * 4; }
 __host__ __device__ constexpr int64_t sep_adj_gbuf_at(int P, int Hd, int W) {
   return (8LL * sep_padded(W) + 4LL * Hd + 8LL * (P + 3) + 15) / 16 * 16;
 }
-__host__ __device__ constexpr int64_t sep_adj_smem(int P, int Hd, int W, int warps) {
-  return sep_adj_gbuf_at(P, Hd, W) + 4LL * warps * kSepBand * kSepWide;
+__host__ __device__ constexpr int64_t sep_adj_smem(int P, int Hd, int W) {
+  return sep_adj_gbuf_at(P, Hd, W) + kSepBufBytes;
 }
 
 struct SepGrad {
@@ -355,29 +360,34 @@ __global__ void __launch_bounds__(256) pou_warp_sep_weigh_kernel(const float* __
   gic[static_cast<int64_t>(blockIdx.y) * quads + q] = v;
 }
 
-// One CTA per (pose, block).  Its units are bands of image rows (those the
-// detector reaches, split evenly over the warps) x groups of image columns
-// whose detector columns fit a G buffer; a warp takes a unit and writes
-// dL/dimgs there, every element once (nothing to clear, no atomics):
-//   march down the detector rows of cell y0 - 1, y0, .. for 128 detector
-//   columns at a time, four neighbours per lane in f32x2 pairs, keeping the cell's sums
-//   A0 = sum g ic and A1 = sum ty g ic; leaving cell y gives G[y][c] =
-//   (A0 - A1)(y) + A1(y - 1) and, with the image row's value and slope at the
-//   column, the pose-offset sums;
-//   then lane x gathers G[y][c] over its detector columns, weight 1 - |px(c) - x|.
-// The sum of g ry dv/dpy comes from ry = (y + ty - oy) / scale: per cell
-// (y - oy) A0 + A1, so no third sum is kept while marching.
-// Bound by issue at 16 warps per SM (50 % issue active; three CTAs per SM
-// spill: 974 us).  64 blocks x 64 poses x 256^2 pixels: 495 us, with the
-// separate slice adjoint 1232 us against 1422 us for a gather along x of every
-// detector row inside the slice-adjoint kernel; 8 blocks x 64 poses x 512^2
-// pixels: 265 us against 1104 us for a scatter with atomics.
+// One CTA per (pose, block).  A detector pixel lies in one cell of the block
+// image, [x, x + 1) x [y, y + 1), at fractions (tx, ty); everything the adjoint
+// needs of the pixels is their four moments per cell, sums of g ic times 1, tx,
+// ty, tx ty.  The CTA walks down the image rows that the detector reaches in
+// steps of a few 8-row bands, over as many 32-column groups as its buffer holds
+// the detector columns of:
+//   its warps march down the detector rows of the step's cells, 128 detector
+//   columns at a time, four neighbours per lane in f32x2 pairs: per cell row
+//   and column A0 = sum g ic and A1 = sum ty g ic, to the buffer;
+//   then a warp takes a band of a group: lane x sums its cell's columns, S0, S1
+//   = sum A0, A1 and T0, T1 = sum tx A0, tx A1, and with S = S0 - S1 + S1(y - 1)
+//   and T alike, dL/dimg[y][x] = S - T + T(x - 1); the pose-offset sums take
+//   the image's differences over the cell.
+// Every element of dL/dimgs is written once (nothing to clear, no atomics).
+// The sums of g rx dv/dpx and g ry dv/dpy come from rx = (x + tx - ox) / scale
+// and ry alike, in f32 relative to the integer next to ox, oy.
+// Bound by issue.  64 blocks x 64 poses x 256^2 pixels: 437 us, against 495
+// with bands marched by one warp each and the image's values and differences
+// interpolated at every detector column (two loads and nine operations per
+// image row and detector column); 8 blocks x 64 poses x 512^2 pixels: 138
+// against 265.
 template <int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(SepArgs a, SepGrad w) {
   constexpr int NW = THREADS / 32;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double red[4][NW];
-  // per thread: sums of g dv/dpx, g rx dv/dpx, g dv/dpy, g (y + ty - oy) dv/dpy (no registers held while marching)
+  // per thread: sums of g dv/dpx, g (x + tx - ox) dv/dpx, g dv/dpy, g (y + ty - oy) dv/dpy (no registers held
+  // while marching)
   __shared__ double sums[4][THREADS];
   const int P = a.P, Hd = a.Hd, W = a.W, Wp = sep_padded(W);
   int2* cmap = reinterpret_cast<int2*>(smem);             // (ix, tx) per detector column, -2 in the padding
@@ -392,7 +402,7 @@ __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(Sep
   // march order: increasing image position
   const bool rev_c = sc * (static_cast<double>(__ldg(a.rxc + W - 1)) - static_cast<double>(__ldg(a.rxc))) < 0.0;
   const bool rev_r = sc * (static_cast<double>(__ldg(a.ryr + Hd - 1)) - static_cast<double>(__ldg(a.ryr))) < 0.0;
-  int* rcell = reinterpret_cast<int*>(smem + sep_adj_gbuf_at(P, Hd, W));  // in the G buffers until they are used
+  int* rcell = reinterpret_cast<int*>(smem + sep_adj_gbuf_at(P, Hd, W));  // in the sum buffer until it is used
 #pragma unroll
   for (int k = 0; k < 4; ++k) sums[k][threadIdx.x] = 0.0;
   for (int c = threadIdx.x; c < Wp; c += THREADS) {
@@ -434,194 +444,245 @@ __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(Sep
   }
   for (int q = threadIdx.x; q < ya * P; q += THREADS) gimg[q] = 0.f;
   for (int q = yb * P + threadIdx.x; q < P * P; q += THREADS) gimg[q] = 0.f;
-  // as many 32-column groups per unit as the G buffer takes
+  // as many 32-column groups per step as have their detector columns in the buffer (one group: in column passes if
+  // they are more); rows of half the length leave room for up to four bands, of which those that keep the warps
+  // busiest are taken
   const int groups = (P + 31) / 32;
-  int gs = groups;
-  for (; gs > 1; --gs) {
-    bool fits = true;
+  int gs = groups, cols = 0;
+  for (;; --gs) {
+    cols = 0;
     for (int g = 0; g < groups; g += gs) {
       int c0, c1;
       columns(32 * g - 1, min(P, 32 * (g + gs)), c0, c1);
-      fits &= c1 - (c0 & ~3) <= kSepWide;
+      cols = max(cols, c1 - (c0 & ~3));
     }
-    if (fits) break;
+    if (gs == 1 || cols <= kSepStepCols) break;
   }
-  const int supers = (groups + gs - 1) / gs;
-  const int nbands = yb > ya ? ((yb - ya + kSepBand - 1) / kSepBand + NW - 1) / NW * NW : 0;
-  float* G = reinterpret_cast<float*>(smem + sep_adj_gbuf_at(P, Hd, W)) + wid * kSepBand * kSepWide;
-  for (int u = wid; u < nbands * supers; u += NW) {
-    const int sg = u / nbands, band = u - sg * nbands;
-    const int y0 = ya + static_cast<int>(static_cast<int64_t>(band) * (yb - ya) / nbands);
-    const int y1 = ya + static_cast<int>(static_cast<int64_t>(band + 1) * (yb - ya) / nbands);
-    if (y0 >= y1) continue;
-    const int x0 = 32 * gs * sg, x1 = min(P, x0 + 32 * gs);
-    const int kr0 = rfirst[y0], kr1 = rfirst[y1 + 1];  // cells y0 - 1 .. y1 - 1
-    int ca, cb;
-    columns(x0 - 1, x1, ca, cb);
-    float2 gsum[kSepBand / 2];  // rows 2 i, 2 i + 1
+  const bool narrow = cols <= kSepStepCols / 2;
+  int bands = 1;
+  for (int v = 2; v <= (narrow ? 4 : 2); ++v) {
+    const int r0 = (bands * gs + NW - 1) / NW, r1 = (v * gs + NW - 1) / NW;
+    if (r1 * bands <= r0 * v) bands = v;
+  }
+  float* buf = reinterpret_cast<float*>(smem + sep_adj_gbuf_at(P, Hd, W));
+  const int step = rev_r ? -(Wp / 4) : Wp / 4;
+  // x0 - ox, y0 - 1 - oy relative to the nearest integer of ox, oy; what is left of them is applied at the end, in f64
+  const double rox = rint(ox), roy = rint(oy);
+  float dx = 0.f, drx = 0.f, fy = 0.f, f1 = 0.f;
+  auto steps = [&](auto row_length) {
+    constexpr int pitch = decltype(row_length)::value;
+    for (int xc = 0; xc < P; xc += 32 * gs) {
+      const int xe = min(P, xc + 32 * gs);
+      int ca, cb;
+      columns(xc - 1, xe, ca, cb);
+      const int cs = ca & ~3;  // 16-byte words of a detector row
+      for (int ys = ya; ys < yb; ys += bands * kSepBand) {
+        const int rows = min(bands * kSepBand, yb - ys);  // cells ys - 1 .. ys + rows - 1
+        // lane's cell (two rows a pair) and, lane = cell row, the cell left of the group: sums over columns
+        float2 S0[kSepPairs], T0[kSepPairs], S1[kSepPairs], T1[kSepPairs];
+        float L0, LT0, L1, LT1;
+        for (int kp = cs; kp < max(cb, cs + 1); kp += pitch) {
+          const int ke = min(cb, kp + pitch);
+          const int passes = (ke - kp + kSepPass - 1) / kSepPass, parts = passes % 2 ? NW : passes % 4 ? NW / 2 : NW / 4;
+          __syncthreads();
+          for (int u = wid; u < passes * parts; u += NW) {
+            const int pass = u / parts, part = u - pass * parts;
+            int cell = (rows + 1) * part / parts;
+            const int cell1 = (rows + 1) * (part + 1) / parts;
+            if (cell >= cell1) continue;
+            const int c = kp + kSepPass * pass + 4 * lane;
+            const bool on = c < Wp, keep = c < kp + pitch;
+            const int kr1 = rfirst[ys + cell1];
+            int kr = rfirst[ys + cell], kend = rfirst[ys + cell + 1];
+            const float4* gq =
+                w.gic + (static_cast<int64_t>(n) * Hd + (rev_r ? Hd - 1 - kr : kr)) * (Wp / 4) + c / 4;
+            float4* q = reinterpret_cast<float4*>(buf + 2 * cell * pitch + (c - kp));
+            float4 nxt[4];
 #pragma unroll
-    for (int i = 0; i < kSepBand / 2; ++i) gsum[i] = bcast(0.f);
-    if (ca >= cb || kr0 >= kr1) {  // nothing reaches this unit
-      for (int x = x0 + lane; x < x1; x += 32)
-        for (int y = y0; y < y1; ++y) gimg[y * P + x] = 0.f;
-      continue;
-    }
-    const int cs = ca & ~3;  // 16-byte words of a detector row
-    for (int kp = cs; kp < cb; kp += kSepWide) {  // several only for a single 32-column group
-      const int ke = min(cb, kp + kSepWide);
-      for (int sp = kp; sp < ke; sp += kSepPass) {
-        const int c = sp + 4 * lane;
-        const bool on = c < Wp;
-        float2 tx[2], A0[2], A1[2], p0[2], p1[2], Lp[2], sx[2], v0[2], v1[2], fy[2], f1[2];
-        int ix[4];
-        bool in0[4], in1[4];  // image values ix, ix + 1 belong to the sums
-        float tj[4];
+            for (int j = 0; j < 4; ++j) {
+              nxt[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (on && kr + j < kr1) nxt[j] = __ldg(gq + j * step);
+            }
+            float2 A0[2], A1[2];
+            A0[0] = A0[1] = A1[0] = A1[1] = bcast(0.f);
+            auto flush = [&] {
+              if (keep) {
+                q[0] = make_float4(A0[0].x, A0[0].y, A0[1].x, A0[1].y);
+                q[pitch / 4] = make_float4(A1[0].x, A1[0].y, A1[1].x, A1[1].y);
+              }
+              q += pitch / 2;
+              A0[0] = A0[1] = A1[0] = A1[1] = bcast(0.f);
+              ++cell;
+              kend = rfirst[ys + cell + 1];
+            };
+            for (; kr < kr1; kr += 4) {
+              float4 cur[4];
+              gq += 4 * step;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int2 e = on ? cmap[c + j] : make_int2(-2, 0);
-          // a column's sums belong to the unit that holds image column max(ix, 0)
-          const bool own = c + j >= ca && c + j < ke && e.x >= -1 && max(e.x, 0) >= x0 && e.x < x1;
-          ix[j] = e.x;
-          tj[j] = __int_as_float(e.y);
-          in0[j] = own && e.x >= 0;
-          in1[j] = own && e.x + 1 < P;
-        }
+              for (int j = 0; j < 4; ++j) {
+                cur[j] = nxt[j];
+                if (on && kr + 4 + j < kr1) nxt[j] = __ldg(gq + j * step);
+              }
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          tx[h] = make_float2(tj[2 * h], tj[2 * h + 1]);
-          A0[h] = A1[h] = p0[h] = p1[h] = Lp[h] = sx[h] = v0[h] = v1[h] = fy[h] = f1[h] = bcast(0.f);
-        }
-        auto load_image = [&](int y) {  // lanes outside keep their zeros
-          const float* q = img + y * P;
-          if (in0[0]) v0[0].x = ldg_in(q, ix[0], P, kSiteWarpTap);
-          if (in0[1]) v0[0].y = ldg_in(q, ix[1], P, kSiteWarpTap);
-          if (in0[2]) v0[1].x = ldg_in(q, ix[2], P, kSiteWarpTap);
-          if (in0[3]) v0[1].y = ldg_in(q, ix[3], P, kSiteWarpTap);
-          if (in1[0]) v1[0].x = ldg_in(q, ix[0] + 1, P, kSiteWarpTap);
-          if (in1[1]) v1[0].y = ldg_in(q, ix[1] + 1, P, kSiteWarpTap);
-          if (in1[2]) v1[1].x = ldg_in(q, ix[2] + 1, P, kSiteWarpTap);
-          if (in1[3]) v1[1].y = ldg_in(q, ix[3] + 1, P, kSiteWarpTap);
-        };
-        const int step = rev_r ? -(Wp / 4) : Wp / 4;
-        const float4* gq = w.gic + (static_cast<int64_t>(n) * Hd + (rev_r ? Hd - 1 - kr0 : kr0)) * (Wp / 4) + c / 4;
-        float4 gn = make_float4(0.f, 0.f, 0.f, 0.f), gm = gn;  // the next two detector rows' values
-        int kr = kr0;
-        if (on) gn = __ldg(gq);
-        gq += step;
-        if (on && kr + 1 < kr1) gm = __ldg(gq);
-        auto cell = [&](int kend) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) A0[h] = A1[h] = bcast(0.f);
-          for (; kr < kend; ++kr) {
-            const float2 ty = bcast(rty[kr]);
-            const float2 g0 = make_float2(gn.x, gn.y), g1 = make_float2(gn.z, gn.w);
-            gn = gm;
-            gq += step;
-            if (on && kr + 2 < kr1) gm = __ldg(gq);
-            A0[0] = __fadd2_rn(A0[0], g0);
-            A0[1] = __fadd2_rn(A0[1], g1);
-            A1[0] = __ffma2_rn(ty, g0, A1[0]);
-            A1[1] = __ffma2_rn(ty, g1, A1[1]);
+              for (int j = 0; j < 4; ++j) {
+                if (kr + j < kr1) {
+                  while (kr + j >= kend) flush();
+                  const float2 ty = bcast(rty[kr + j]);
+                  const float2 g0 = make_float2(cur[j].x, cur[j].y), g1 = make_float2(cur[j].z, cur[j].w);
+                  A0[0] = __fadd2_rn(A0[0], g0);
+                  A0[1] = __fadd2_rn(A0[1], g1);
+                  A1[0] = __ffma2_rn(ty, g0, A1[0]);
+                  A1[1] = __ffma2_rn(ty, g1, A1[1]);
+                }
+              }
+            }
+            while (cell < cell1) flush();
           }
-        };
-        if (y0 > 0) {
-          load_image(y0 - 1);
+          __syncthreads();
+          for (int u = wid; u < gs * bands; u += NW) {
+            const int band = u / gs, xg = xc + 32 * (u - band * gs), y0 = ys + band * kSepBand;
+            const int nr = min(kSepBand, ys + rows - y0);
+            if (nr <= 0 || xg >= P) continue;
+            const int x = xg + lane;
+            const bool in = x < P, right = x + 1 < P;
+            if (kp == cs) {
 #pragma unroll
-          for (int h = 0; h < 2; ++h) Lp[h] = __ffma2_rn(tx[h], sub2(v1[h], v0[h]), v0[h]);
+              for (int i = 0; i < kSepPairs; ++i) S0[i] = T0[i] = S1[i] = T1[i] = bcast(0.f);
+              L0 = LT0 = L1 = LT1 = 0.f;
+            }
+            float vi[kSepBand + 1], ri[kSepBand + 1];  // image rows y0 - 1 .. y0 + nr - 1 at x, x + 1
+            {
+              const float* q = img + (y0 - 1) * P + x;
+              const bool last = ke == cb;
+#pragma unroll
+              for (int i = 0; i <= kSepBand; ++i) {
+                const bool row = last && in && i <= nr && y0 + i > 0;
+                vi[i] = row ? __ldg(q + i * P) : 0.f;
+                ri[i] = row && right ? __ldg(q + i * P + 1) : 0.f;
+              }
+            }
+            const float* bq = buf + 2 * band * kSepBand * pitch - kp;
+            int t0 = 0, t1 = 0, l0, l1;
+            if (in) columns(x, x + 1, t0, t1);
+            t1 = min(t1, ke);
+            for (int k = max(t0, kp); k < t1; ++k) {
+              if (!fvr_checked(k - kp, pitch, kSiteWarpFused)) continue;
+              const float2 t = bcast(__int_as_float(cmap[k].y));
+              const float* q = bq + k;
+#pragma unroll
+              for (int i = 0; i < kSepPairs; ++i) {
+                const float2 v0 = make_float2(q[4 * i * pitch], q[(4 * i + 2) * pitch]);
+                const float2 v1 = make_float2(q[(4 * i + 1) * pitch], q[(4 * i + 3) * pitch]);
+                S0[i] = __fadd2_rn(S0[i], v0);
+                T0[i] = __ffma2_rn(t, v0, T0[i]);
+                S1[i] = __fadd2_rn(S1[i], v1);
+                T1[i] = __ffma2_rn(t, v1, T1[i]);
+              }
+            }
+            columns(xg - 1, xg, l0, l1);
+            if (lane <= nr)
+              for (int k = max(l0, kp); k < min(l1, ke); ++k) {
+                const float t = __int_as_float(cmap[k].y), v0 = bq[2 * lane * pitch + k],
+                            v1 = bq[(2 * lane + 1) * pitch + k];
+                L0 += v0;
+                L1 += v1;
+                LT0 = fmaf(t, v0, LT0);
+                LT1 = fmaf(t, v1, LT1);
+              }
+            if (ke < cb) continue;
+            // this unit's sums: with x and y relative to the lane's cell and to cell row y0 - 1
+            float ux = 0.f, urx = 0.f, uy = 0.f, ury = 0.f;
+            // the left cell's S and T of image row y0 + lane - 1 (lane >= 1)
+            const float up = __shfl_up_sync(0xffffffffu, L1, 1), upt = __shfl_up_sync(0xffffffffu, LT1, 1);
+            const float LS = (L0 - L1) + up, LT = (LT0 - LT1) + upt;
+            if (xg == 0 && l0 < l1) {  // column -1 is no image column: its sums are taken here, image values 0 there
+              const int y = y0 + lane - 1;  // row y of the cell
+              const float v = lane <= nr && y >= 0 ? img[y * P] : 0.f;
+              const float below = lane <= nr && y + 1 < P ? img[(y + 1) * P] : 0.f;
+              if (lane >= 1 && lane <= nr) {
+                dx = fmaf(LS, v, dx);
+                drx = fmaf(fmaf(static_cast<float>(-1 - rox), LS, LT), v, drx);
+              }
+              if (lane < nr || (lane == nr && y0 + nr == P)) {
+                const float D = below - v, p = LT0 * D;
+                uy = p;
+                ury = fmaf(static_cast<float>(lane), p, LT1 * D);
+              }
+            }
+            float* gq = gimg + y0 * P + x;
+            float vp = vi[0], dp = ri[0] - vi[0];
+            auto at = [](const float2(&a)[kSepPairs], int i) { return i & 1 ? a[i / 2].y : a[i / 2].x; };
+            auto row = [&](int i) {
+              const float v = vi[i + 1], d = ri[i + 1] - v;
+              const float SG = (at(S0, i + 1) - at(S1, i + 1)) + at(S1, i);
+              const float TG = (at(T0, i + 1) - at(T1, i + 1)) + at(T1, i);
+              const float tl = __shfl_up_sync(0xffffffffu, TG, 1), t0l = __shfl_sync(0xffffffffu, LT, i + 1);
+              if (in) gq[i * P] = (SG - TG) + (lane == 0 ? t0l : tl);
+              ux = fmaf(SG, d, ux);
+              urx = fmaf(TG, d, urx);
+              const float Dv = v - vp, Dd = d - dp;  // cell y - 1
+              const float p = fmaf(at(T0, i), Dd, at(S0, i) * Dv);
+              uy += p;
+              ury = fmaf(at(S1, i), Dv, fmaf(static_cast<float>(i), p, ury));
+              ury = fmaf(at(T1, i), Dd, ury);
+              vp = v;
+              dp = d;
+            };
+            if (nr == kSepBand && y0 + nr < P) {
+#pragma unroll
+              for (int i = 0; i < kSepBand; ++i) row(i);
+            } else {
+#pragma unroll
+              for (int i = 0; i < kSepBand; ++i)
+                if (i < nr) {
+                  row(i);
+                  if (i + 1 == nr && y0 + nr == P) {  // the last cell's lower row lies outside the image
+                    const float p = fmaf(at(T0, i + 1), -dp, at(S0, i + 1) * -vp);
+                    uy += p;
+                    ury = fmaf(at(S1, i + 1), -vp, fmaf(static_cast<float>(i + 1), p, ury));
+                    ury = fmaf(at(T1, i + 1), -dp, ury);
+                  }
+                }
+            }
+            dx += ux;
+            drx += fmaf(static_cast<float>(x - rox), ux, urx);
+            fy += uy;
+            f1 += fmaf(static_cast<float>(y0 - 1 - roy), uy, ury);
+          }
         }
-        cell(rfirst[y0 + 1]);
-        for (int y = y0; y < y1; ++y) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            p0[h] = A0[h];
-            p1[h] = A1[h];
-          }
-          load_image(y);
-          cell(rfirst[y + 2]);
-          const float2 yo = bcast(static_cast<float>(static_cast<double>(y - 1) - oy));
-          float2 g[2];
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            g[h] = __fadd2_rn(sub2(A0[h], A1[h]), p1[h]);
-            const float2 d = sub2(v1[h], v0[h]);
-            const float2 L = __ffma2_rn(tx[h], d, v0[h]), D = sub2(L, Lp[h]);
-            Lp[h] = L;
-            sx[h] = __ffma2_rn(g[h], d, sx[h]);
-            fy[h] = __ffma2_rn(p0[h], D, fy[h]);  // cell y - 1
-            f1[h] = __ffma2_rn(__ffma2_rn(yo, p0[h], p1[h]), D, f1[h]);
-          }
-          *reinterpret_cast<float4*>(G + (y - y0) * kSepWide + (c - kp)) = make_float4(g[0].x, g[0].y, g[1].x, g[1].y);
-        }
-        if (y1 == P) {  // the last cell's lower row lies outside the image
-          const float2 yo = bcast(static_cast<float>(static_cast<double>(P - 1) - oy));
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const float2 D = sub2(bcast(0.f), Lp[h]);
-            fy[h] = __ffma2_rn(A0[h], D, fy[h]);
-            f1[h] = __ffma2_rn(__ffma2_rn(yo, A0[h], A1[h]), D, f1[h]);
-          }
-        }
-        const float sj[4] = {sx[0].x, sx[0].y, sx[1].x, sx[1].y};
-        float dx = 0.f, drx = 0.f;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (in0[j] || in1[j]) {
-            dx += sj[j];
-            drx = fmaf(sj[j], __ldg(a.rxc + c + j), drx);
-          }
         sums[0][threadIdx.x] += static_cast<double>(dx);
         sums[1][threadIdx.x] += static_cast<double>(drx);
-        sums[2][threadIdx.x] += static_cast<double>((fy[0].x + fy[0].y) + (fy[1].x + fy[1].y));
-        sums[3][threadIdx.x] += static_cast<double>((f1[0].x + f1[0].y) + (f1[1].x + f1[1].y));
+        sums[2][threadIdx.x] += static_cast<double>(fy);
+        sums[3][threadIdx.x] += static_cast<double>(f1);
+        dx = drx = fy = f1 = 0.f;
       }
-      __syncwarp();
-      for (int xg = x0; xg < x1; xg += 32) {
-        const int x = xg + lane;
-        if (kp == cs)
-#pragma unroll
-          for (int i = 0; i < kSepBand / 2; ++i) gsum[i] = bcast(0.f);
-        int t0 = 0, t1 = 0;
-        if (x < x1) columns(x - 1, x + 1, t0, t1);
-        t1 = min(t1, ke);
-        for (int k = max(t0, kp); k < t1; ++k) {
-          const int2 e = cmap[k];
-          const float t = __int_as_float(e.y);
-          const float2 wt = bcast(e.x == x ? 1.f - t : t);
-          const float* q = G + (k - kp);
-#pragma unroll
-          for (int i = 0; i < kSepBand / 2; ++i)
-            if (fvr_checked((2 * i + 1) * kSepWide + k - kp, kSepBand * kSepWide, kSiteWarpFused))
-              gsum[i] = __ffma2_rn(wt, make_float2(q[2 * i * kSepWide], q[(2 * i + 1) * kSepWide]), gsum[i]);
-        }
-        if (ke == cb && x < x1) {
-#pragma unroll
-          for (int i = 0; i < kSepBand / 2; ++i) {
-            if (y0 + 2 * i < y1) gimg[(y0 + 2 * i) * P + x] = gsum[i].x;
-            if (y0 + 2 * i + 1 < y1) gimg[(y0 + 2 * i + 1) * P + x] = gsum[i].y;
-          }
-        }
-      }
-      __syncwarp();
     }
-  }
-  // a block in the source plane (scale near 0) does not determine ry from the image row: sum g ry dv/dpy directly
+  };
+  if (narrow) steps(std::integral_constant<int, kSepStepCols / 2>{});
+  else steps(std::integral_constant<int, kSepStepCols>{});
+  sums[1][threadIdx.x] += (rox - ox) * sums[0][threadIdx.x];
+  sums[3][threadIdx.x] += (roy - oy) * sums[2][threadIdx.x];
+  // a block in the source plane (scale near 0) does not determine rx and ry from the image position: the sums of
+  // g rx dv/dpx and g ry dv/dpy directly
   const bool direct = fabs(sc) < 1.0;
-  double s_ry = sums[3][threadIdx.x];
+  double s_rx = sums[1][threadIdx.x], s_ry = sums[3][threadIdx.x];
   if (direct) {
-    s_ry = 0.0;
+    s_rx = s_ry = 0.0;
     for (int64_t q = threadIdx.x; q < static_cast<int64_t>(Hd) * W; q += THREADS) {
       const int r = static_cast<int>(q / W), c = static_cast<int>(q - static_cast<int64_t>(r) * W);
-      const float ry = __ldg(a.ryr + r);
+      const float rx = __ldg(a.rxc + c), ry = __ldg(a.ryr + r);
       float ty;
       const int iy = sep_cell(sc, oy, ry, P, ty), ix = cmap[c].x;
       if (iy < -1 || iy >= P || ix < -1 || ix >= P) continue;
       const float tx = __int_as_float(cmap[c].y);
       auto at = [&](int y, int x) { return y >= 0 && y < P && x >= 0 && x < P ? __ldg(img + y * P + x) : 0.f; };
-      const float D = (1.f - tx) * (at(iy + 1, ix) - at(iy, ix)) + tx * (at(iy + 1, ix + 1) - at(iy, ix + 1));
-      s_ry += static_cast<double>(__ldg(gout + q) * __ldg(a.ic + q)) * static_cast<double>(ry) * static_cast<double>(D);
+      const float v00 = at(iy, ix), v01 = at(iy, ix + 1), v10 = at(iy + 1, ix), v11 = at(iy + 1, ix + 1);
+      const double g = static_cast<double>(__ldg(gout + q) * __ldg(a.ic + q));
+      s_rx += g * static_cast<double>(rx) * static_cast<double>((1.f - ty) * (v01 - v00) + ty * (v11 - v10));
+      s_ry += g * static_cast<double>(ry) * static_cast<double>((1.f - tx) * (v10 - v00) + tx * (v11 - v01));
     }
   }
-  const double mine[4] = {sums[0][threadIdx.x], sums[1][threadIdx.x], sums[2][threadIdx.x], s_ry};
+  const double mine[4] = {sums[0][threadIdx.x], s_rx, sums[2][threadIdx.x], s_ry};
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const double t = warp_sum(mine[k]);
@@ -633,7 +694,7 @@ __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(Sep
     for (int k = 0; k < 4; ++k)
       for (int v = 0; v < NW; ++v) t[k] += red[k][v];
     const int64_t BN = static_cast<int64_t>(a.B) * a.N;
-    w.goffs[bn] = a.inv_ds * (t[1] + (direct ? t[3] : t[3] / sc));
+    w.goffs[bn] = a.inv_ds * (direct ? t[1] + t[3] : (t[1] + t[3]) / sc);
     w.goffs[BN + bn] = -a.inv_ds * t[0];
     w.goffs[2 * BN + bn] = -a.inv_ds * t[2];
   }
@@ -649,7 +710,7 @@ static int sep_args(const float* imgs, int64_t B, int64_t N, int64_t P, const do
 
 template <int THREADS, int MINB>
 static int sep_adjoint(const SepArgs& a, const SepGrad& w, cudaStream_t s) {
-  const int64_t smem = sep_adj_smem(a.P, a.Hd, a.W, THREADS / 32);
+  const int64_t smem = sep_adj_smem(a.P, a.Hd, a.W);
   // the shared-memory opt-in is a per-device setting: made before every launch
   if (cudaFuncSetAttribute(pou_warp_sep_adjoint_kernel<THREADS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(smem)) != cudaSuccess)
@@ -706,8 +767,8 @@ int fvr_pou_warp_sep(const float* imgs, int64_t B, int64_t N, int64_t P, const d
 
 int fvr_pou_warp_sep_adjoint_supported(int64_t P, int64_t H, int64_t W) {
   if (!fvr_pou_warp_sep_supported(P, H, W)) return 0;
-  // the row cells are staged in the G buffers; two 256-thread CTAs and one of 512 threads fit an SM
-  return 4 * H <= 4LL * 8 * kSepBand * kSepWide && sep_adj_smem((int)P, (int)H, (int)W, 16) <= 200 * 1024 ? 1 : 0;
+  // the row cells are staged in the buffer of cell-row sums, beside which the tables have 72 KB
+  return H <= 16384 && sep_adj_gbuf_at((int)P, (int)H, (int)W) <= 72 * 1024 ? 1 : 0;
 }
 
 int64_t fvr_pou_warp_sep_adjoint_workspace(int64_t N, int64_t H, int64_t W) {

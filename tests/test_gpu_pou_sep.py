@@ -67,6 +67,48 @@ def test_separable_warp_and_adjoint_vs_oracle(B, N, P, H, W, pitch, flip, shift)
         assert rel_l2(got, want) < 1e-5
 
 
+@pytest.mark.parametrize("db0,H,W,P,pitch", [
+    (0.0, 33, 70, 40, 1.0), (0.9, 40, 65, 64, 1.0), (2.5, 31, 130, 64, 1.0), (-650.0, 70, 300, 96, 0.5),
+    (-2.0, 20, 33, 33, 1.0), (650.0, 9, 140, 129, 0.7), (700.0, 140, 600, 64, 0.25),
+])
+def test_separable_adjoint_moments_vs_oracle(db0, H, W, P, pitch):
+    """The adjoint's cell moments where their reference points matter: blocks in
+    and next to the source plane (every pixel in one cell; rx and ry taken from
+    the lattice), behind it (reversed columns and rows), images whose last
+    column group is one column wide, units of several column groups, and more
+    than 128 detector columns in one.  Same tolerances as above; the offset
+    gradients of the blocks at depth 2 to 2.5 multiply a ray coordinate of at
+    most 0.1 that is recovered from a position next to an integer, hence 1e-4
+    there."""
+    import fvr._lib as L
+
+    rng = np.random.default_rng(P + H + W)
+    B, N, ds, c = 2, 2, 1.5, float(P // 2)
+    db = db0 + rng.uniform(-0.05, 0.05, (B, N))
+    cu, cv = rng.uniform(-4, 4, (B, N)), rng.uniform(-4, 4, (B, N))
+    rxc = ((np.arange(W) - 0.5 * W + 0.37) * pitch * ds / 700.0).astype(np.float32)
+    ryr = ((np.arange(H) - 0.5 * H + 0.41) * pitch * ds / 700.0).astype(np.float32)
+    imgs = rng.standard_normal((B, N, P, P)).astype(np.float32)
+    ic = (1.0 + 0.1 * rng.random((H, W))).astype(np.float32)
+    g = rng.standard_normal((N, H, W)).astype(np.float32)
+    rx, ry = np.broadcast_to(rxc[None, :], (H, W)), np.broadcast_to(ryr[:, None], (H, W))
+    gi, gd, gu, gv = opou.warp_sum_adjoint(imgs.astype(np.float64), db, cu, cv, rx.astype(np.float64),
+                                           ry.astype(np.float64), ic.astype(np.float64), 1.0 / ds, c,
+                                           g.astype(np.float64))
+    dev = torch.device("cuda", 0)
+    t = {k: torch.from_numpy(np.ascontiguousarray(v)).to(dev) for k, v in
+         dict(imgs=imgs, offs=np.stack([db, cu, cv], -1), rxc=rxc, ryr=ryr, ic=ic, g=g).items()}
+    gim = torch.full((B, N, P, P), float("nan"), device=dev)
+    goffs = torch.full((3, B, N), float("nan"), dtype=torch.float64, device=dev)
+    ws = torch.empty(L.query("fvr_pou_warp_sep_adjoint_workspace", N, H, W), dtype=torch.uint8, device=dev)
+    L.call("fvr_pou_warp_sep_adjoint", L.ptr(t["imgs"]), B, N, P, L.ptr(t["offs"]), L.ptr(t["rxc"]), L.ptr(t["ryr"]),
+           L.ptr(t["ic"]), H, W, 1.0 / ds, c, L.ptr(t["g"]), L.ptr(ws), ws.numel(), L.ptr(gim), L.ptr(goffs),
+           L.stream_ptr(dev))
+    assert rel_l2(gim.cpu().numpy(), gi) < 1e-5
+    for got, want, tol in zip(goffs.cpu().numpy(), (gd, gu, gv), (1e-4 if abs(db0) < 3 else 1e-5, 1e-5, 1e-5)):
+        assert rel_l2(got, want) < tol
+
+
 def test_large_gradient_buffers_take_the_one_launch_adjoint(monkeypatch):
     """Above _GRAD_IMAGE_BYTES the adjoint that keeps dL/dimgs in shared memory
     runs (fvr_pou_warp_image_adjoint); same pose gradient."""
