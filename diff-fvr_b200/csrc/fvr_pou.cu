@@ -184,6 +184,17 @@ __global__ void pou_pose_kernel(const float* __restrict__ mats, const float* __r
   }
 }
 
+// Ray coordinates (rx, ry) and the reciprocal obliquity of point t in the frame g.
+__device__ __forceinline__ void explicit_ray(const float* __restrict__ t, const double* __restrict__ g, double& rx,
+                                             double& ry, double& ic) {
+  const double r0 = t[0] - g[0], r1 = t[1] - g[1], r2 = t[2] - g[2];
+  const double inv = 1.0 / sqrt(fmax(r0 * r0 + r1 * r1 + r2 * r2, 1e-12));
+  const double h0 = r0 * inv, h1 = r1 * inv, h2 = r2 * inv;
+  ic = 1.0 / fmax(h0 * g[9] + h1 * g[10] + h2 * g[11], 0.1);
+  rx = (h0 * g[3] + h1 * g[4] + h2 * g[5]) * ic;
+  ry = (h0 * g[6] + h1 * g[7] + h2 * g[8]) * ic;
+}
+
 // Explicit rays (cone_beam_fvr.py:451-457): per pose and pixel
 // rx = (r.u)/cos, ry = (r.v)/cos, ic = 1/cos with r the unit ray, cos = max(r.n, 0.1).
 __global__ void pou_rays_prep_kernel(const float* __restrict__ trg, const double* __restrict__ geo, int N, int K,
@@ -191,17 +202,12 @@ __global__ void pou_rays_prep_kernel(const float* __restrict__ trg, const double
   const int n = blockIdx.y;
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= K) return;
-  const double* g = geo + n * kGeo;
-  const float* t = trg + (static_cast<int64_t>(n) * K + q) * 3;
-  const double r0 = t[0] - g[0], r1 = t[1] - g[1], r2 = t[2] - g[2];
-  const double inv = 1.0 / sqrt(fmax(r0 * r0 + r1 * r1 + r2 * r2, 1e-12));
-  const double h0 = r0 * inv, h1 = r1 * inv, h2 = r2 * inv;
-  const double c = fmax(h0 * g[9] + h1 * g[10] + h2 * g[11], 0.1);
-  const double icv = 1.0 / c;
   const int64_t o = static_cast<int64_t>(n) * K + q;
-  rx[o] = static_cast<float>((h0 * g[3] + h1 * g[4] + h2 * g[5]) * icv);
-  ry[o] = static_cast<float>((h0 * g[6] + h1 * g[7] + h2 * g[8]) * icv);
-  ic[o] = static_cast<float>(icv);
+  double x, y, c;
+  explicit_ray(trg + 3 * o, geo + n * kGeo, x, y, c);
+  rx[o] = static_cast<float>(x);
+  ry[o] = static_cast<float>(y);
+  ic[o] = static_cast<float>(c);
 }
 
 // Detector axes of an explicit lattice trg[N][H][W][3] (cone_beam_fvr.py:575-596):
@@ -306,7 +312,7 @@ __device__ __forceinline__ void axis_backward(const double* e, const double* gy,
 // dL/d(src, u, v, n) (gvec) -> dL/dsrcs and the three corner points' share of
 // dL/dtrg (added to what the rays put there).  One thread per pose.
 __global__ void pou_rays_axes_bwd_kernel(const float* __restrict__ trg, const double* __restrict__ geo,
-                                         const float* __restrict__ gvec, int N, int H, int W,
+                                         const double* __restrict__ gvec, int N, int H, int W,
                                          float* __restrict__ gsrc, float* __restrict__ gtrg) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= N) return;
@@ -318,7 +324,7 @@ __global__ void pou_rays_axes_bwd_kernel(const float* __restrict__ trg, const do
     u[k] = g[3 + k];
     v[k] = g[6 + k];
     nn[k] = g[9 + k];
-    gsrc[3 * n + k] = gvec[12 * n + k];
+    gsrc[3 * n + k] = static_cast<float>(gvec[12 * n + k]);
     gu[k] = gvec[12 * n + 3 + k];
     gv[k] = gvec[12 * n + 6 + k];
     gn[k] = gvec[12 * n + 9 + k];
@@ -1290,7 +1296,23 @@ struct WarpArgs {
   int B, N, P, K;
   int64_t ray_stride;
   int chunk;  // blocks per row-strip round (0: every CTA takes the per-pixel path)
+  // explicit rays: the points and poses that rx, ry were rounded from, or null
+  const float* trg = nullptr;
+  const double* geo = nullptr;
 };
+
+// Ray coordinates of pixel rq of pose n: as given, or unrounded from the points
+// (an image position of some hundred pixels keeps 1e-5 pixels in float32).
+template <typename OT>
+__device__ __forceinline__ void warp_ray(const WarpArgs<OT>& a, int n, int64_t rq, double& rx, double& ry) {
+  if (a.trg) {
+    double c;
+    explicit_ray(a.trg + 3 * rq, a.geo + n * kGeo, rx, ry, c);
+  } else {
+    rx = __ldg(a.rx + rq);
+    ry = __ldg(a.ry + rq);
+  }
+}
 
 // Row strips.  The pinhole lattice's detector rows share one ray coordinate
 // ry up to the float rounding of the lattice (about 1e-7 relative), so for a
@@ -1604,7 +1626,8 @@ __global__ void __launch_bounds__(256) pou_warp_kernel(WarpArgs<OT> a, float* __
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = q < a.K;
   const int64_t rq = n * a.ray_stride + q;
-  const double rx = live ? __ldg(a.rx + rq) : 0.0, ry = live ? __ldg(a.ry + rq) : 0.0;
+  double rx = 0.0, ry = 0.0;
+  if (live) warp_ray(a, n, rq, rx, ry);
   const WarpCull wc = warp_cull(a, n, live, rx, ry, touch, tl);
   float acc = 0.f;
   if (wc.rows) {
@@ -1652,7 +1675,8 @@ __global__ void __launch_bounds__(256) pou_warp_bwd_kernel(WarpArgs<OT> a, const
   for (int i = threadIdx.x; i < 3 * a.B; i += blockDim.x) sacc[i] = 0.0;
   const bool live = q < a.K;
   const int64_t rq = n * a.ray_stride + q;
-  const double rx = live ? __ldg(a.rx + rq) : 0.0, ry = live ? __ldg(a.ry + rq) : 0.0;
+  double rx = 0.0, ry = 0.0;
+  if (live) warp_ray(a, n, rq, rx, ry);
   const WarpCull wc = warp_cull(a, n, live, rx, ry, touch, tl);
   const float g = live ? __ldg(gout + static_cast<int64_t>(n) * a.K + q) * __ldg(a.ic + rq) : 0.f;
   // the row-strip path's fixed-point scale: the CTA's largest weight (float
@@ -1671,12 +1695,12 @@ __global__ void __launch_bounds__(256) pou_warp_bwd_kernel(WarpArgs<OT> a, const
     warp_rows_adjoint(a, n, live, rx, g, scale_exp, wc, tl, strip, grad_imgs, sacc);
   } else {
     const int P = a.P;
-    const float inv_ds = static_cast<float>(a.inv_ds);
-    float grx = 0.f, gry = 0.f, ssum = 0.f;  // explicit rays: dL/drx, dL/dry, sum_b sample
+    double grx = 0.0, gry = 0.0;  // explicit rays: dL/drx, dL/dry, sum_b sample
+    float ssum = 0.f;
     for (int i = 0; i < wc.nt; ++i) {
       const int b = tl[i];
       const int64_t bn = static_cast<int64_t>(b) * a.N + n;
-      float gdb = 0.f, gcu = 0.f, gcv = 0.f;
+      double gdb = 0.0, gcu = 0.0, gcv = 0.0;
       bool hit = false;
       if (live) {
         const double db = static_cast<double>(a.db[bn * a.ostride]);
@@ -1700,22 +1724,22 @@ __global__ void __launch_bounds__(256) pou_warp_bwd_kernel(WarpArgs<OT> a, const
             if (x0 && y1) atomic_add_in(gi, (iy + 1) * P + ix, P * P, kSiteWarpGrad, g * (1.f - tx) * ty);
             if (x1 && y1) atomic_add_in(gi, (iy + 1) * P + ix + 1, P * P, kSiteWarpGrad, g * tx * ty);
           }
-          const float dpx = ((v01 - v00) * (1.f - ty) + (v11 - v10) * ty) * inv_ds;
-          const float dpy = ((v10 - v00) * (1.f - tx) + (v11 - v01) * tx) * inv_ds;
-          gdb = g * (dpx * static_cast<float>(rx) + dpy * static_cast<float>(ry));
+          // f64: the offsets' and the rays' shares of a turn of the detector nearly cancel
+          const double sx = px - fx, sy = py - fy, d00 = v00, d01 = v01, d10 = v10, d11 = v11;
+          const double dpx = ((d01 - d00) * (1.0 - sy) + (d11 - d10) * sy) * a.inv_ds;
+          const double dpy = ((d10 - d00) * (1.0 - sx) + (d11 - d01) * sx) * a.inv_ds;
+          gdb = g * (dpx * rx + dpy * ry);
           gcu = -g * dpx;
           gcv = -g * dpy;
           if (gray) {
-            const float dbf = static_cast<float>(db);
-            grx += g * dpx * dbf;
-            gry += g * dpy * dbf;
+            grx += g * dpx * db;
+            gry += g * dpy * db;
             ssum += (v00 * (1.f - tx) + v01 * tx) * (1.f - ty) + (v10 * (1.f - tx) + v11 * tx) * ty;
           }
         }
       }
       if (!__any_sync(0xffffffffu, hit)) continue;  // nothing to add from this warp
-      const double s0 = warp_sum(static_cast<double>(gdb)), s1 = warp_sum(static_cast<double>(gcu)),
-                   s2 = warp_sum(static_cast<double>(gcv));
+      const double s0 = warp_sum(gdb), s1 = warp_sum(gcu), s2 = warp_sum(gcv);
       if ((threadIdx.x & 31) == 0) {
         atomicAdd(sacc + 3 * b, s0);
         atomicAdd(sacc + 3 * b + 1, s1);
@@ -1724,8 +1748,8 @@ __global__ void __launch_bounds__(256) pou_warp_bwd_kernel(WarpArgs<OT> a, const
     }
     if (gray && live) {
       float* o = gray + (static_cast<int64_t>(n) * a.K + q) * 3;
-      o[0] = grx;
-      o[1] = gry;
+      o[0] = static_cast<float>(grx);
+      o[1] = static_cast<float>(gry);
       o[2] = __ldg(gout + static_cast<int64_t>(n) * a.K + q) * ssum;  // direct dL/dic
     }
   }
@@ -1814,7 +1838,7 @@ __global__ void __launch_bounds__(256) pou_pose_bwd_kernel(const double* __restr
                                                            const double* __restrict__ geo,
                                                            const float* __restrict__ centers, int B, int N,
                                                            PouBase base, double vscale, float* __restrict__ gmats,
-                                                           float* __restrict__ gvec) {
+                                                           float* __restrict__ gvec, double* __restrict__ gvec64) {
   constexpr int NA = 18;  // gux[3], gvx[3], gs[3], gu[3], gv[3], gn[3]
   __shared__ double red[NA * 8];
   const int n = blockIdx.x;
@@ -1880,6 +1904,15 @@ __global__ void __launch_bounds__(256) pou_pose_bwd_kernel(const double* __restr
       o[3 + k] = static_cast<float>(gu[k]);
       o[6 + k] = static_cast<float>(gv[k]);
       o[9 + k] = static_cast<float>(gn[k]);
+    }
+  }
+  if (gvec64) {
+    double* o = gvec64 + 12 * n;
+    for (int k = 0; k < 3; ++k) {
+      o[k] = gs[k];
+      o[3 + k] = gu[k];
+      o[6 + k] = gv[k];
+      o[9 + k] = gn[k];
     }
   }
   if (gmats) {
@@ -2186,9 +2219,10 @@ int fvr_pou_warp_image_adjoint(int dtype, const void* stencil, const float* scal
   return FVR_ERR_DTYPE;
 }
 
-int fvr_pou_warp(const float* imgs, int64_t B, int64_t N, int64_t P, const void* db, const void* cu, const void* cv,
-                 int offs_f64, int64_t ostride, const float* rx, const float* ry, const float* ic, int64_t K,
-                 int64_t ray_stride, double inv_ds, double c_idx, float* out, void* stream) {
+static int pou_warp(const float* imgs, int64_t B, int64_t N, int64_t P, const void* db, const void* cu,
+                    const void* cv, int offs_f64, int64_t ostride, const float* rx, const float* ry, const float* ic,
+                    int64_t K, int64_t ray_stride, double inv_ds, double c_idx, float* out, void* stream,
+                    const float* trg = nullptr, const double* geo = nullptr) {
   if (!imgs || !db || !cu || !cv || !rx || !ry || !ic || !out || B < 1 || N < 1 || P < 2 || K < 1 || N > 65535 ||
       B > 4096)
     return FVR_ERR_ARG;
@@ -2199,7 +2233,7 @@ int fvr_pou_warp(const float* imgs, int64_t B, int64_t N, int64_t P, const void*
   if (offs_f64) {
     WarpArgs<double> a{imgs, static_cast<const double*>(db), static_cast<const double*>(cu),
                        static_cast<const double*>(cv), (int)ostride, rx, ry, ic, inv_ds, c_idx, (int)B, (int)N,
-                       (int)P, (int)K, ray_stride, chunk};
+                       (int)P, (int)K, ray_stride, chunk, trg, geo};
     if (!warp_smem_ok(pou_warp_kernel<double>, sm)) return FVR_ERR_CUDA;
     pou_warp_kernel<double><<<grid, 256, sm, s>>>(a, out);
   } else {
@@ -2213,14 +2247,21 @@ int fvr_pou_warp(const float* imgs, int64_t B, int64_t N, int64_t P, const void*
   return FVR_OK;
 }
 
+int fvr_pou_warp(const float* imgs, int64_t B, int64_t N, int64_t P, const void* db, const void* cu, const void* cv,
+                 int offs_f64, int64_t ostride, const float* rx, const float* ry, const float* ic, int64_t K,
+                 int64_t ray_stride, double inv_ds, double c_idx, float* out, void* stream) {
+  return pou_warp(imgs, B, N, P, db, cu, cv, offs_f64, ostride, rx, ry, ic, K, ray_stride, inv_ds, c_idx, out, stream);
+}
+
 int64_t fvr_pou_warp_bwd_workspace(int64_t B, int64_t N, int64_t K) {
   return N * cdiv64(K, 256) * 3 * B * (int64_t)sizeof(double);
 }
 
-int fvr_pou_warp_bwd(const float* imgs, int64_t B, int64_t N, int64_t P, const void* db, const void* cu,
-                     const void* cv, int offs_f64, int64_t ostride, const float* rx, const float* ry, const float* ic,
-                     int64_t K, int64_t ray_stride, double inv_ds, double c_idx, const float* gout, float* grad_imgs,
-                     double* goffs, float* gray, void* workspace, int64_t ws_bytes, void* stream) {
+static int pou_warp_bwd(const float* imgs, int64_t B, int64_t N, int64_t P, const void* db, const void* cu,
+                        const void* cv, int offs_f64, int64_t ostride, const float* rx, const float* ry,
+                        const float* ic, int64_t K, int64_t ray_stride, double inv_ds, double c_idx, const float* gout,
+                        float* grad_imgs, double* goffs, float* gray, void* workspace, int64_t ws_bytes, void* stream,
+                        const float* trg = nullptr, const double* geo = nullptr) {
   if (!imgs || !db || !cu || !cv || !rx || !ry || !ic || !gout || !goffs || !workspace || B < 1 || N < 1 || P < 2 ||
       K < 1 || N > 65535 || B > 4096)
     return FVR_ERR_ARG;
@@ -2234,7 +2275,7 @@ int fvr_pou_warp_bwd(const float* imgs, int64_t B, int64_t N, int64_t P, const v
   if (offs_f64) {
     WarpArgs<double> a{imgs, static_cast<const double*>(db), static_cast<const double*>(cu),
                        static_cast<const double*>(cv), (int)ostride, rx, ry, ic, inv_ds, c_idx, (int)B, (int)N,
-                       (int)P, (int)K, ray_stride, chunk};
+                       (int)P, (int)K, ray_stride, chunk, trg, geo};
     if (!warp_smem_ok(pou_warp_bwd_kernel<double>, sm)) return FVR_ERR_CUDA;
     pou_warp_bwd_kernel<double><<<grid, 256, sm, s>>>(a, gout, grad_imgs, part, gray);
   } else {
@@ -2251,6 +2292,14 @@ int fvr_pou_warp_bwd(const float* imgs, int64_t B, int64_t N, int64_t P, const v
   return FVR_OK;
 }
 
+int fvr_pou_warp_bwd(const float* imgs, int64_t B, int64_t N, int64_t P, const void* db, const void* cu,
+                     const void* cv, int offs_f64, int64_t ostride, const float* rx, const float* ry, const float* ic,
+                     int64_t K, int64_t ray_stride, double inv_ds, double c_idx, const float* gout, float* grad_imgs,
+                     double* goffs, float* gray, void* workspace, int64_t ws_bytes, void* stream) {
+  return pou_warp_bwd(imgs, B, N, P, db, cu, cv, offs_f64, ostride, rx, ry, ic, K, ray_stride, inv_ds, c_idx, gout,
+                      grad_imgs, goffs, gray, workspace, ws_bytes, stream);
+}
+
 int fvr_pou_pose_backward(const double* sl_part, int64_t tiles, const double* goffs, const double* ray_part,
                           int64_t rtiles, const double* geo, const float* centers, int64_t B, int64_t N,
                           const double* base12, double vscale, float* gmats, float* gvec, void* stream) {
@@ -2260,7 +2309,7 @@ int fvr_pou_pose_backward(const double* sl_part, int64_t tiles, const double* go
   if (N > 2147483647) return FVR_ERR_ARG;
   pou_pose_bwd_kernel<<<static_cast<unsigned>(N), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       sl_part, (int)tiles, goffs, ray_part, (int)rtiles, geo, centers, (int)B, (int)N,
-      make_base(base12 ? base12 : zero12), vscale, gmats, gvec);
+      make_base(base12 ? base12 : zero12), vscale, gmats, gvec, nullptr);
   FVR_LAUNCH_CHECK();
   return FVR_OK;
 }
@@ -2307,7 +2356,8 @@ int fvr_pou_rays_forward(int dtype, const void* stencil, const float* scales, in
   int rc = fvr_pou_rays_prep(trg, geo, N, K, rx, ry, ic, stream);
   if (!rc) rc = fvr_pou_slice_image(dtype, stencil, scales, B, P, geo, N, freqs, imgs, stream);
   if (!rc)
-    rc = fvr_pou_warp(imgs, B, N, P, offs, offs + 1, offs + 2, 1, 3, rx, ry, ic, K, K, inv_ds, c_idx, out, stream);
+    rc = pou_warp(imgs, B, N, P, offs, offs + 1, offs + 2, 1, 3, rx, ry, ic, K, K, inv_ds, c_idx, out, stream, trg,
+                  geo);
   return rc;
 }
 
@@ -2318,7 +2368,7 @@ static int64_t rays_round(int64_t bytes) { return (bytes + 255) / 256 * 256; }
 int64_t fvr_pou_rays_backward_workspace(int64_t B, int64_t N, int64_t H, int64_t W) {
   if (B < 1 || N < 1 || H < 1 || W < 1) return 0;
   const int64_t K = H * W;
-  return rays_round(12 * N * K) + rays_round(48 * N) + rays_round(24 * B * N) +
+  return rays_round(12 * N * K) + rays_round(96 * N) + rays_round(24 * B * N) +
          rays_round(fvr_pou_warp_bwd_workspace(B, N, K)) + rays_round(fvr_pou_slice_image_adjoint_workspace(B, N)) +
          fvr_pou_rays_bwd_workspace(N, K);
 }
@@ -2343,7 +2393,7 @@ int fvr_pou_rays_backward(int dtype, const void* stencil, const float* scales, i
     return p;
   };
   float* gray = reinterpret_cast<float*>(take(12 * N * K));
-  float* gvec = reinterpret_cast<float*>(take(48 * N));
+  double* gvec = reinterpret_cast<double*>(take(96 * N));
   double* goffs = reinterpret_cast<double*>(take(24 * B * N));
   const int64_t wb = fvr_pou_warp_bwd_workspace(B, N, K), sb = fvr_pou_slice_image_adjoint_workspace(B, N),
                 rb = fvr_pou_rays_bwd_workspace(N, K);
@@ -2351,15 +2401,17 @@ int fvr_pou_rays_backward(int dtype, const void* stencil, const float* scales, i
   double* spart = reinterpret_cast<double*>(take(sb));
   double* rpart = reinterpret_cast<double*>(take(rb));
   if (cudaMemsetAsync(grad_imgs, 0, static_cast<size_t>(4 * B * N * P * P), s) != cudaSuccess) return FVR_ERR_CUDA;
-  int rc = fvr_pou_warp_bwd(imgs, B, N, P, offs, offs + 1, offs + 2, 1, 3, rx, ry, ic, K, K, inv_ds, c_idx, gout,
-                            grad_imgs, goffs, gray, wpart, wb, stream);
+  int rc = pou_warp_bwd(imgs, B, N, P, offs, offs + 1, offs + 2, 1, 3, rx, ry, ic, K, K, inv_ds, c_idx, gout,
+                        grad_imgs, goffs, gray, wpart, wb, stream, trg, geo);
   if (!rc)
     rc = fvr_pou_slice_image_adjoint(dtype, stencil, scales, B, P, geo, N, freqs, grad_imgs, spart, sb, stream);
   if (!rc) rc = fvr_pou_rays_bwd(trg, geo, N, K, gray, gtrg, rpart, rb, stream);
-  if (!rc)
-    rc = fvr_pou_pose_backward(spart, 1, goffs, rpart, cdiv64(K, 256), geo, centers, B, N, nullptr, vscale, nullptr,
-                               gvec, stream);
   if (rc) return rc;
+  const double zero12[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+  pou_pose_bwd_kernel<<<static_cast<unsigned>(N), 256, 0, s>>>(spart, 1, goffs, rpart, (int)cdiv64(K, 256), geo, centers,
+                                                              (int)B, (int)N, make_base(zero12), vscale, nullptr,
+                                                              nullptr, gvec);
+  FVR_LAUNCH_CHECK();
   pou_rays_axes_bwd_kernel<<<static_cast<unsigned>(cdiv64(N, 32)), 32, 0, s>>>(trg, geo, gvec, (int)N, (int)H, (int)W,
                                                                               gsrc, gtrg);
   FVR_LAUNCH_CHECK();
