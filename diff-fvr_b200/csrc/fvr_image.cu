@@ -1,5 +1,5 @@
 // Parallel-beam image path on whole images in shared memory, sm_100a
-// (src/fvr/torch_engine.py:236-253, 309-337): one CTA per image.
+// (src/fvr/torch_engine.py:236-253, 309-337): one CTA or two per image.
 //
 //  * tc_image_kernel: modulated slice -> inverse 2D FFT -> real part -> ReLU;
 //  * tc_image_adjoint_kernel: ReLU mask -> 2D FFT of the image gradient ->
@@ -12,13 +12,18 @@
 // rows 0 .. n0/2 of a Hermitian spectrum (or over pairs of real rows), the
 // column pass over pairs of real columns (or over the columns 0 .. n1/2), so a
 // transform is n0/2 + n1/2 lines.  A warp transforms a line on its own: copy to
-// its scratch, Stockham passes, copy back.
+// its scratch, Stockham passes, copy back.  While SMs are left over, a cluster
+// of two CTAs shares an image: each takes half the lines of a pass and writes
+// the results to the CTA that reads them next.
 //
 // As separate passes over memory an image step (render, image NCC, pose
 // gradient) was 19 launches, ten of them line-FFT passes of 22 us for 64 images
-// of 96 x 96; here it is five.  Kernels at that size: render 28 us, NCC with its
-// image gradient 36 us, adjoint 33 us (288 us before); bound by issue in the 64
-// CTAs, 32 warps each (16 warps: 35, 59 and 44 us).
+// of 96 x 96; here it is five.  Kernels at that size: render 19 us, NCC with its
+// image gradient 31 us, adjoint 24 us (288 us before; with one CTA an image 28,
+// 39 and 33); bound by issue in the 128 CTAs, 32 warps each, and by the
+// latency of a line's passes.
+#include <cooperative_groups.h>
+
 #include "fvr_dft.cuh"
 #include "fvr_slice.cuh"
 
@@ -170,38 +175,82 @@ __device__ __forceinline__ ImgMem img_mem(unsigned char* smem, const ImgShape& s
   return m;
 }
 
-// Inverse transform (unnormalised) of a Hermitian spectrum to a real image.
-// row(r, k) gives the spectrum's value at row r <= n0/2; it may read buffer
-// row r and row (n0 - r) mod n0.  On return (after a barrier) the image's
-// columns 2t and 2t + 1 are the real and imaginary part of buffer column 2t.
-template <int THREADS, typename F>
-__device__ __forceinline__ void hermitian_to_real(const ImgShape& s, const ImgMem& m, F row) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, pitch = s.n1 + 1, half = s.n0 / 2;
-  for (int r = wid; r <= half; r += (THREADS / 32)) {
-    for (int k = lane; k < s.n1; k += 32) m.la[k] = row(r, k);
-    const Cx<float>* y = line_fft<true>(m.la, m.lb, s.p1, m.tw1, lane);
-    for (int k = lane; k < s.n1; k += 32) m.buf[r * pitch + k] = y[k];
-    __syncwarp();
-  }
-  __syncthreads();
-  for (int c = 2 * wid; c < s.n1; c += 2 * (THREADS / 32)) {
-    const bool two = c + 1 < s.n1;
-    for (int r = lane; r < s.n0; r += 32) {
-      const int rr = r <= half ? r : s.n0 - r;
-      const float sg = r <= half ? 1.f : -1.f;  // rows above n0/2 are conjugates
-      const Cx<float> p = m.buf[rr * pitch + c], q = two ? m.buf[rr * pitch + c + 1] : Cx<float>{0.f, 0.f};
-      m.la[r] = Cx<float>{p.x - sg * q.y, sg * p.y + q.x};
-    }
-    const Cx<float>* y = line_fft<true>(m.la, m.lb, s.p0, m.tw0, lane);
-    for (int r = lane; r < s.n0; r += 32) m.buf[r * pitch + c] = y[r];
-    __syncwarp();
-  }
-  __syncthreads();
-}
+// The CTAs of a cluster share an image (one CTA: all of it).  Of the columns of
+// the half spectrum, kx = 0 .. n1/2, rank r takes [c0, c1) together with their
+// mirrors n1 - kx, of the row pairs [p0, p1).  A pass writes a line's results
+// into the buffer of the rank that reads them next, which holds nothing else
+// there; a cluster barrier stands between passes.
+struct ImgPart {
+  int nr, rank, h, c0, c1, p0, p1, pc;  // pc: first row pair of rank 1
+  int n_up;                             // own columns above n1 / 2
 
-__device__ __forceinline__ float real_pixel(const ImgShape& s, const ImgMem& m, int y, int x) {
-  const Cx<float> v = m.buf[y * (s.n1 + 1) + (x & ~1)];
-  return (x & 1) ? v.y : v.x;
+  __device__ __forceinline__ void init(int n0, int n1) {
+    const auto cl = cooperative_groups::this_cluster();
+    nr = static_cast<int>(cl.num_blocks());
+    rank = static_cast<int>(cl.block_rank());
+    h = n1 / 2;
+    const int pairs = (n0 + 1) / 2;
+    c0 = (h + 1) * rank / nr;
+    c1 = (h + 1) * (rank + 1) / nr;
+    p0 = pairs * rank / nr;
+    p1 = pairs * (rank + 1) / nr;
+    pc = nr > 1 ? pairs / nr : pairs;
+    n_up = max(0, min(c1, (n1 + 1) / 2) - max(c0, 1));
+  }
+  __device__ __forceinline__ int cols() const { return c1 - c0 + n_up; }
+  // natural index of own column e < cols()
+  __device__ __forceinline__ int col(int e, int n1) const {
+    return e < c1 - c0 ? c0 + e : n1 - max(c0, 1) - (e - (c1 - c0));
+  }
+  __device__ __forceinline__ int col_rank(int k, int n1) const {
+    return nr > 1 && min(k, n1 - k) >= (h + 1) / nr ? 1 : 0;
+  }
+  __device__ __forceinline__ int row_rank(int y) const { return (y >> 1) >= pc ? 1 : 0; }
+  // every rank's copy of a shared-memory array
+  template <typename T>
+  __device__ __forceinline__ void map(T* p, T* (&out)[2]) const {
+    out[0] = out[1] = p;
+    if (nr > 1) out[1 - rank] = cooperative_groups::this_cluster().map_shared_rank(p, 1 - rank);
+  }
+  __device__ __forceinline__ void sync() const {
+    if (nr > 1) cooperative_groups::this_cluster().sync();
+    else __syncthreads();
+  }
+};
+
+// Inverse transform (unnormalised) of a Hermitian spectrum to a real image:
+// the columns kx <= n1/2, then the rows two at a time as real and imaginary
+// part of one line.  col(r, kx) gives the spectrum in an own column; it may
+// read buffer columns kx and (n1 - kx) mod n1.  out(y, x, v) takes the image
+// of the own row pairs.
+template <int THREADS, typename F, typename O>
+__device__ __forceinline__ void hermitian_to_real(const ImgShape& s, const ImgMem& m, const ImgPart& part, F col, O out) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, pitch = s.n1 + 1;
+  Cx<float>* bufs[2];
+  part.map(m.buf, bufs);
+  for (int kx = part.c0 + wid; kx < part.c1; kx += (THREADS / 32)) {
+    for (int r = lane; r < s.n0; r += 32) m.la[r] = col(r, kx);
+    const Cx<float>* y = line_fft<true>(m.la, m.lb, s.p0, m.tw0, lane);
+    for (int r = lane; r < s.n0; r += 32) bufs[part.row_rank(r)][r * pitch + kx] = y[r];
+    __syncwarp();
+  }
+  part.sync();
+  for (int t = part.p0 + wid; t < part.p1; t += (THREADS / 32)) {
+    const bool two = 2 * t + 1 < s.n0;
+    const Cx<float>* src = m.buf + 2 * t * pitch;
+    for (int k = lane; k < s.n1; k += 32) {
+      const int kk = k <= part.h ? k : s.n1 - k;
+      const float sg = kk == 0 || 2 * kk == s.n1 ? 0.f : k <= part.h ? 1.f : -1.f;  // those are real
+      const Cx<float> p = src[kk], q = two ? src[pitch + kk] : Cx<float>{0.f, 0.f};
+      m.la[k] = Cx<float>{p.x - sg * q.y, sg * p.y + q.x};
+    }
+    const Cx<float>* z = line_fft<true>(m.la, m.lb, s.p1, m.tw1, lane);
+    for (int x = lane; x < s.n1; x += 32) {
+      out(2 * t, x, z[x].x);
+      if (two) out(2 * t + 1, x, z[x].y);
+    }
+    __syncwarp();
+  }
 }
 
 // ----------------------------------------------------------------------------
@@ -220,31 +269,35 @@ template <int DT, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1) tc_image_kernel(TcImageArgs a, float* __restrict__ img) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double ax[8];
-  const int c = blockIdx.x, R = a.sl.R, pitch = R + 1, h = R / 2;
+  const int R = a.sl.R, pitch = R + 1, h = R / 2;
   const ImgMem m = img_mem<THREADS>(smem, a.sh);
+  ImgPart part;
+  part.init(R, R);
+  const int c = blockIdx.x / part.nr, cols = part.cols();
   if (threadIdx.x == 0) slice_axes(a.poses + 6 * c, a.lateral, a.sl.sx, a.sl.sy, a.sl.sz, ax);
   __syncthreads();
-  for (int q = threadIdx.x; q < R * R; q += THREADS) {
-    const int i = q / R, j = q - i * R;
+  for (int q = threadIdx.x; q < R * cols; q += THREADS) {
+    const int i = q / cols, jj = part.col(q - i * cols, R), j = jj + h < R ? jj + h : jj + h - R;
     Interp o;
     float sn, cs;
     slice_sample<DT, false>(a.sl, ax, __ldg(a.sl.lin + i), __ldg(a.sl.lin + j), o, sn, cs);
-    const int ii = i < h ? i - h + R : i - h, jj = j < h ? j - h + R : j - h;  // ifftshift position
+    const int ii = i < h ? i - h + R : i - h;  // ifftshift position
     m.buf[ii * pitch + jj] = Cx<float>{o.sr * cs - o.si * sn, o.sr * sn + o.si * cs};
   }
-  __syncthreads();
+  part.sync();
   // Re ifft2(S) = ifft2 of S's Hermitian part
-  hermitian_to_real<THREADS>(a.sh, m, [&](int r, int k) {
-    const Cx<float> p = m.buf[r * pitch + k], q = m.buf[(r == 0 ? 0 : R - r) * pitch + (k == 0 ? 0 : R - k)];
-    return Cx<float>{0.5f * (p.x + q.x), 0.5f * (p.y - q.y)};
-  });
   const float scale = 1.f / (static_cast<float>(R) * static_cast<float>(R));
   float* out = img + static_cast<int64_t>(c) * R * R;
-  for (int q = threadIdx.x; q < R * R; q += THREADS) {
-    const int y = q / R;
-    const float v = real_pixel(a.sh, m, y, q - y * R) * scale;
-    out[q] = v > 0.f ? v : 0.f;
-  }
+  hermitian_to_real<THREADS>(
+      a.sh, m, part,
+      [&](int r, int k) {
+        const Cx<float> p = m.buf[r * pitch + k], q = m.buf[(r == 0 ? 0 : R - r) * pitch + (k == 0 ? 0 : R - k)];
+        return Cx<float>{0.5f * (p.x + q.x), 0.5f * (p.y - q.y)};
+      },
+      [&](int y, int x, float z) {
+        const float v = z * scale;
+        out[y * R + x] = v > 0.f ? v : 0.f;
+      });
 }
 
 // ----------------------------------------------------------------------------
@@ -262,8 +315,11 @@ __global__ void __launch_bounds__(THREADS, 1) tc_image_adjoint_kernel(TcImageArg
                                                                           const float* __restrict__ gout,
                                                                           float* __restrict__ grad) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ double ax[8], red[8][(THREADS / 32)];
-  const int c = blockIdx.x, R = a.sl.R, half = R / 2, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  __shared__ double ax[8], red[8][(THREADS / 32)], sums[2][8];
+  const int R = a.sl.R, half = R / 2, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  ImgPart part;
+  part.init(R, R);
+  const int c = blockIdx.x / part.nr, cols = part.cols();
   const int zp = R + 1, gp = half + 1;
   Cx<float>* zr = reinterpret_cast<Cx<float>*>(smem);
   Cx<float>* gb = zr + (R + 1) / 2 * zp;
@@ -272,10 +328,12 @@ __global__ void __launch_bounds__(THREADS, 1) tc_image_adjoint_kernel(TcImageArg
   for (int i = threadIdx.x; i < R; i += THREADS)
     tw[i] = Cx<float>{__ldg(&a.sh.tw1[i].x), __ldg(&a.sh.tw1[i].y)};
   if (threadIdx.x == 0) slice_axes(a.poses + 6 * c, a.lateral, a.sl.sx, a.sl.sy, a.sl.sz, ax);
-  __syncthreads();
+  Cx<float>* zrs[2];
+  part.map(zr, zrs);
+  part.sync();
   const float *im = img + static_cast<int64_t>(c) * R * R, *go = gout + static_cast<int64_t>(c) * R * R;
   // rows 2s and 2s + 1 of the masked gradient as real and imaginary part of one line
-  for (int s = wid; s < (R + 1) / 2; s += (THREADS / 32)) {
+  for (int s = part.p0 + wid; s < part.p1; s += (THREADS / 32)) {
     const int y = 2 * s;
     for (int k = lane; k < R; k += 32) {
       const float u = __ldg(im + y * R + k) > 0.f ? __ldg(go + y * R + k) : 0.f;
@@ -283,12 +341,12 @@ __global__ void __launch_bounds__(THREADS, 1) tc_image_adjoint_kernel(TcImageArg
       la[k] = Cx<float>{u, v};
     }
     const Cx<float>* z = line_fft<false>(la, lb, a.sh.p1, tw, lane);
-    for (int k = lane; k < R; k += 32) zr[s * zp + k] = z[k];
+    for (int k = lane; k < R; k += 32) zrs[part.col_rank(k, R)][s * zp + k] = z[k];
     __syncwarp();
   }
-  __syncthreads();
+  part.sync();
   const float scale = 1.f / (static_cast<float>(R) * static_cast<float>(R));
-  for (int kx = wid; kx <= half; kx += (THREADS / 32)) {
+  for (int kx = part.c0 + wid; kx < part.c1; kx += (THREADS / 32)) {
     const int km = kx == 0 ? 0 : R - kx;
     for (int y = lane; y < R; y += 32) {
       const Cx<float> A = zr[(y >> 1) * zp + kx], B = zr[(y >> 1) * zp + km];
@@ -302,13 +360,13 @@ __global__ void __launch_bounds__(THREADS, 1) tc_image_adjoint_kernel(TcImageArg
   __syncthreads();
   // dL/dS = e^{-i phi} G and dL/dphi = Re(conj(G) i S) per sample
   double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int q = threadIdx.x; q < R * R; q += THREADS) {
-    const int i = q / R, j = q - i * R;
+  for (int q = threadIdx.x; q < R * cols; q += THREADS) {
+    const int i = q / cols, kj = part.col(q - i * cols, R), j = kj + half < R ? kj + half : kj + half - R;
     const float ku = __ldg(a.sl.lin + i), kv = __ldg(a.sl.lin + j);
     Interp o;
     float sn, cs;
     slice_sample<DT, true>(a.sl, ax, ku, kv, o, sn, cs);
-    const int ki = i < half ? i - half + R : i - half, kj = j < half ? j - half + R : j - half;
+    const int ki = i < half ? i - half + R : i - half;
     Cx<float> g;  // G at frequency (ki, kj); G(-k) = conj G(k)
     if (kj <= half) {
       g = gb[ki * gp + kj];
@@ -338,17 +396,21 @@ __global__ void __launch_bounds__(THREADS, 1) tc_image_adjoint_kernel(TcImageArg
   if (threadIdx.x < 8) {
     double t = 0.0;
     for (int w = 0; w < (THREADS / 32); ++w) t += red[threadIdx.x][w];
-    red[threadIdx.x][0] = t;
+    double* p[2];
+    part.map(&sums[part.rank][threadIdx.x], p);
+    *p[0] = t;  // to rank 0
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const double du[3] = {red[0][0], red[1][0], red[2][0]}, dv[3] = {red[3][0], red[4][0], red[5][0]};
+  part.sync();
+  if (part.rank == 0 && threadIdx.x == 0) {
+    double r[8];
+    for (int k = 0; k < 8; ++k) r[k] = part.nr > 1 ? sums[0][k] + sums[1][k] : sums[0][k];
+    const double du[3] = {r[0], r[1], r[2]}, dv[3] = {r[3], r[4], r[5]};
     double ga[3];
     axes_vjp(a.poses + 6 * c, a.lateral, a.sl.sx, a.sl.sy, a.sl.sz, du, dv, ga);
     float* o = grad + 6 * c;
     for (int k = 0; k < 3; ++k) o[k] = static_cast<float>(ga[k]);
-    o[3] = static_cast<float>(a.kappa * red[6][0]);
-    o[4] = static_cast<float>(a.kappa * red[7][0]);
+    o[3] = static_cast<float>(a.kappa * r[6]);
+    o[4] = static_cast<float>(a.kappa * r[7]);
     o[5] = 0.f;
   }
 }
@@ -393,22 +455,29 @@ __global__ void __launch_bounds__(THREADS, 1) cncc_image_kernel(ImgShape s, cons
   __shared__ double red[3][(THREADS / 32)];
   __shared__ float coef[2];
   __shared__ unsigned wmax[THREADS / 32];
-  const int b = blockIdx.x, n0 = s.n0, n1 = s.n1, pitch = n1 + 1;
+  __shared__ double sums[2][3];
+  const int n0 = s.n0, n1 = s.n1, pitch = n1 + 1;
+  ImgPart part;
+  part.init(n0, n1);
+  const int b = blockIdx.x / part.nr, cols = part.cols();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t n = static_cast<int64_t>(n0) * n1;
   const ImgMem m = img_mem<THREADS>(smem, s);
-  __syncthreads();
+  Cx<float>* bufs[2];
+  part.map(m.buf, bufs);
+  part.sync();
   const float *pp = pred + b * n, *tp = target + b * t_stride;
   const unsigned pmax = image_max<THREADS>(pp, n, wmax), tmax = image_max<THREADS>(tp, n, wmax);
   const float sp = unit_scale(pmax), st = unit_scale(tmax);
-  for (int r = wid; r < n0; r += (THREADS / 32)) {
+  for (int r = n0 * part.rank / part.nr + wid; r < n0 * (part.rank + 1) / part.nr; r += (THREADS / 32)) {
     for (int k = lane; k < n1; k += 32) m.la[k] = Cx<float>{sp * __ldg(pp + r * n1 + k), st * __ldg(tp + r * n1 + k)};
     const Cx<float>* y = line_fft<false>(m.la, m.lb, s.p1, m.tw1, lane);
-    for (int k = lane; k < n1; k += 32) m.buf[r * pitch + k] = y[k];
+    for (int k = lane; k < n1; k += 32) bufs[part.col_rank(k, n1)][r * pitch + k] = y[k];
     __syncwarp();
   }
-  __syncthreads();
-  for (int c = wid; c < n1; c += (THREADS / 32)) {
+  part.sync();
+  for (int e = wid; e < cols; e += (THREADS / 32)) {
+    const int c = part.col(e, n1);
     for (int r = lane; r < n0; r += 32) m.la[r] = m.buf[r * pitch + c];
     const Cx<float>* y = line_fft<false>(m.la, m.lb, s.p0, m.tw0, lane);
     for (int r = lane; r < n0; r += 32) m.buf[r * pitch + c] = y[r];
@@ -432,8 +501,8 @@ __global__ void __launch_bounds__(THREADS, 1) cncc_image_kernel(ImgShape s, cons
   };
   float acc[3] = {0.f, 0.f, 0.f};
   const int rows = n0 / 2 + 1;
-  for (int q = threadIdx.x; q < rows * n1; q += THREADS) {
-    const int r = q / n1, k = q - r * n1;
+  for (int q = threadIdx.x; q < rows * cols; q += THREADS) {
+    const int r = q / cols, k = part.col(q - r * cols, n1);
     Cx<float> fp, ft;
     const float w = spectra(r, k, fp, ft) * (r == 0 || 2 * r == n0 ? 1.f : 2.f);
     acc[0] = fmaf(w, fmaf(fp.x, ft.x, fp.y * ft.y), acc[0]);
@@ -446,10 +515,17 @@ __global__ void __launch_bounds__(THREADS, 1) cncc_image_kernel(ImgShape s, cons
     if (lane == 0) red[k][wid] = v;
   }
   __syncthreads();
+  if (threadIdx.x < 3) {
+    double t = 0.0;
+    for (int w = 0; w < (THREADS / 32); ++w) t += red[threadIdx.x][w];
+    double* p[2];
+    part.map(&sums[part.rank][threadIdx.x], p);
+    for (int r = 0; r < part.nr; ++r) *p[r] = t;
+  }
+  part.sync();
   if (threadIdx.x == 0) {
-    double t[3] = {0.0, 0.0, 0.0};
-    for (int k = 0; k < 3; ++k)
-      for (int w = 0; w < (THREADS / 32); ++w) t[k] += red[k][w];
+    double t[3];
+    for (int k = 0; k < 3; ++k) t[k] = part.nr > 1 ? sums[0][k] + sums[1][k] : sums[0][k];
     const double up = 1.0 / sp, ut = 1.0 / st;  // back to the images' own scales
     t[0] *= up * ut;
     t[1] *= up * up;
@@ -457,23 +533,22 @@ __global__ void __launch_bounds__(THREADS, 1) cncc_image_kernel(ImgShape s, cons
     const double e = sqrt(t[1] * t[2]);
     const double aa = 1.0 / (e + 1e-8);
     const double bb = e > 0.0 ? -t[0] * t[2] / (2.0 * e * (e + 1e-8) * (e + 1e-8)) : 0.0;
-    ncc[b] = t[0] * aa;
+    if (part.rank == 0) ncc[b] = t[0] * aa;
     coef[0] = static_cast<float>(-aa / B * ut);
     coef[1] = static_cast<float>(-2.0 * bb / B * up);
   }
   if (!grad) return;
   __syncthreads();
   const float ca = coef[0], cb = coef[1];
-  hermitian_to_real<THREADS>(s, m, [&](int r, int k) {
-    Cx<float> fp, ft;
-    const float w = spectra(r, k, fp, ft);
-    return Cx<float>{w * (ca * ft.x + cb * fp.x), w * (ca * ft.y + cb * fp.y)};
-  });
   float* out = grad + b * n;
-  for (int q = threadIdx.x; q < n0 * n1; q += THREADS) {
-    const int y = q / n1;
-    out[q] = real_pixel(s, m, y, q - y * n1);
-  }
+  hermitian_to_real<THREADS>(
+      s, m, part,
+      [&](int r, int k) {
+        Cx<float> fp, ft;
+        const float w = spectra(r, k, fp, ft);
+        return Cx<float>{w * (ca * ft.x + cb * fp.x), w * (ca * ft.y + cb * fp.y)};
+      },
+      [&](int y, int x, float v) { out[y * n1 + x] = v; });
 }
 
 // loss = 1 - mean ncc, in a fixed order.
@@ -512,20 +587,36 @@ static int image_args(int dtype, const void* stencil, const float* scales, int64
   return FVR_OK;
 }
 
-// Launches kernel<1024> where its line buffers fit, else kernel<512>.  The
-// shared-memory opt-in is a per-device setting: made before every launch.
-template <typename K1, typename K2, typename... A>
-static int img_launch(K1 wide, int64_t wide_smem, K2 narrow, int64_t narrow_smem, int64_t images, cudaStream_t s,
+// Launches kernel<1024> where its line buffers fit, else kernel<512>, two CTAs
+// to an image where that pays: a pair takes 0.67 (render) to 0.79 (NCC) of one
+// CTA's time for 96 x 96 images, so it does while all pairs fit in one wave,
+// and not at 150 images (three waves of pairs 213 us, two of single CTAs 210).
+// The shared-memory opt-in is a per-device setting: made before every launch.
+template <typename K, typename... A>
+static int img_launch(K wide, int64_t wide_smem, K narrow, int64_t narrow_smem, int64_t images, cudaStream_t s,
                       A... args) {
   const bool w = wide_smem <= kImgSmemMax;
   const int64_t smem = w ? wide_smem : narrow_smem;
-  const cudaError_t e = w ? cudaFuncSetAttribute(wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                          : cudaFuncSetAttribute(narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return FVR_ERR_CUDA;
-  if (w) wide<<<static_cast<unsigned>(images), 1024, smem, s>>>(args...);
-  else narrow<<<static_cast<unsigned>(images), 512, smem, s>>>(args...);
-  FVR_LAUNCH_CHECK();
-  return FVR_OK;
+  const K k = w ? wide : narrow;
+  int dev = 0, sms = 0;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return FVR_ERR_CUDA;
+  const int64_t one = (images + sms - 1) / sms, two = (2 * images + sms - 1) / sms;
+  const unsigned pair = 3 * two < 4 * one ? 2 : 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(images) * pair);
+  cfg.blockDim = dim3(w ? 1024 : 512);
+  cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = pair;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, args...) == cudaSuccess ? FVR_OK : FVR_ERR_CUDA;
 }
 
 }  // namespace fvr

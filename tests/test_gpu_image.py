@@ -89,3 +89,30 @@ def test_image_spectral_ncc_of_unlike_magnitudes():
         assert abs(float(loss) - tc.spectral_ncc_loss_images(p64, t64)) < 1e-6
         if i:
             assert rel_l2(g.cpu().numpy(), tc.spectral_ncc_loss_images_grad(p64, t64)) < 2e-5
+
+
+@pytest.mark.parametrize("R", [6, 29, 64, 99, 128])
+def test_two_ctas_an_image_equal_one(R):
+    """Few images take two CTAs each, more than half the SMs' number one: the
+    line transforms are the same arithmetic either way, so images agree bit for
+    bit; the sums of the NCC and of the pose gradient are float64 sums of the
+    same float32 products in another order, 1e-6."""
+    import fvr
+
+    n = torch.cuda.get_device_properties(0).multi_processor_count // 2 + 3
+    eng = fvr.TorchDiffFVREngine(torch.from_numpy(tc.make_ellipsoid_volume(24, 3)), spacing=(0.8, 0.8, 1.2))
+    poses = torch.from_numpy(tc.make_poses(n, 4)).cuda()
+    targ = eng(poses[:1] + 0.01, view="ap", out_res=R).detach()
+
+    def run(p):
+        p = p.clone().requires_grad_(True)
+        img = eng(p, view="ap", out_res=R)
+        loss = eng.spectral_ncc_loss(img, targ)
+        (g,) = torch.autograd.grad(loss * p.shape[0], p)
+        return img.detach(), g
+
+    img, g = run(poses)
+    for lo, hi in ((0, 1), (n // 2, n // 2 + 3)):
+        few, gf = run(poses[lo:hi])
+        assert torch.equal(few, img[lo:hi])
+        assert rel_l2(g[lo:hi].cpu().numpy(), gf.cpu().numpy()) < 1e-5
