@@ -453,20 +453,27 @@ __device__ __forceinline__ void sncc_losses(const double (&lsum)[kMaxViews], int
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
 #pragma unroll
   for (int v = 0; v < kMaxViews; ++v) {
+    if (v >= nv) break;
     const double sv = warp_sum(lsum[v]);
     if (lane == 0) red[v][w] = sv;
   }
   __syncthreads();
-  if (t == 0) {
-    double total = 0.0;
-    for (int v = 0; v < nv; ++v) {
+  if (w == 0) {  // a lane per view
+    double l = 0.0;
+    if (lane < nv) {
       double sv = 0.0;
-      for (int k = 0; k < kFinalThreads / 32; ++k) sv += red[v][k];
-      const double l = 1.0 - sv / C;
-      loss[v] = static_cast<float>(l);
-      total += l;
+#pragma unroll
+      for (int k = 0; k < kFinalThreads / 32; ++k) sv += red[lane][k];
+      l = 1.0 - sv / C;
+      loss[lane] = static_cast<float>(l);
     }
-    loss[nv] = static_cast<float>(total);
+    double total = 0.0;
+#pragma unroll
+    for (int v = 0; v < kMaxViews; ++v) {
+      const double lv = __shfl_sync(0xffffffffu, l, v);
+      if (v < nv) total += lv;
+    }
+    if (lane == 0) loss[nv] = static_cast<float>(total);
   }
 }
 
