@@ -753,11 +753,14 @@ int fvr_pou_warp_sep(const float* imgs, int64_t B, int64_t N, int64_t P, const d
   if (rc) return rc;
   if (!out) return FVR_ERR_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // rows per CTA by the CTAs that leaves (8 against 16 rows: 217 / 207 us at 1024 CTAs of 16 rows, 30 / 45 us at
-  // 336); below two CTAs per SM the blocks are split over warps
-  const int64_t tiles = N * cdiv64(W, 512);
-  if (tiles * cdiv64(H, 16) >= 888) return sep_forward<16>(a, out, s);
-  if (tiles * cdiv64(H, 8) >= 296) return sep_forward<8>(a, out, s);
+  // The most rows per CTA that leave 8 warps an SM, four rows down to 5 warps an SM, below that the blocks split over
+  // warps.  16 / 8 / 4 rows / split, us (warps at 16 rows): 64 blocks x 256^2 pixels, 64 poses (2048) 202 / 207 / 254 /
+  // 743, 32 poses 158 / 115 / 162 / 376, 16 poses 148 / 92 / 83 / 190, 8 poses 146 / 85 / 67 / 96, 4 poses 147 / 86 /
+  // 63 / 49; 8 blocks x 512^2, 16 poses (2048) 28 / 32 / 37 / 134, 4 poses 20 / 14 / 13 / 36.
+  const int64_t row_warps = N * cdiv64(W, 32 * kSepCols);
+  if (row_warps * cdiv64(H, 16) >= 8 * 148) return sep_forward<16>(a, out, s);
+  if (row_warps * cdiv64(H, 8) >= 8 * 148) return sep_forward<8>(a, out, s);
+  if (row_warps * cdiv64(H, 4) >= 5 * 148) return sep_forward<4>(a, out, s);
   const int xt = static_cast<int>(cdiv64(W, 32));
   pou_warp_sep_few_kernel<<<dim3(static_cast<unsigned>(xt * cdiv64(H, kSepFewRows)), static_cast<unsigned>(N)),
                             32 * kSepFewWarps, 0, s>>>(a, xt, out);

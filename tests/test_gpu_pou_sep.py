@@ -67,6 +67,32 @@ def test_separable_warp_and_adjoint_vs_oracle(B, N, P, H, W, pitch, flip, shift)
         assert rel_l2(got, want) < 1e-5
 
 
+@pytest.mark.parametrize("B,N,P,H,W", [(3, 40, 40, 45, 140), (1, 75, 33, 37, 60), (9, 21, 64, 67, 300),
+                                       (2, 186, 32, 13, 33)])
+def test_separable_warp_of_four_rows_vs_oracle(B, N, P, H, W):
+    """Detectors and pose counts that leave 5 to 8 warps an SM: four rows per
+    CTA, row counts that are no multiple of four.  Tolerance as above."""
+    import fvr._lib as L
+
+    rng = np.random.default_rng(P + H + W)
+    ds, c = 1.5, float(P // 2)
+    db, cu, cv = (m + rng.uniform(-s, s, (B, N)) for m, s in ((700.0, 60), (0.0, 4), (0.0, 4)))
+    rxc = ((np.arange(W) - 0.5 * W + 0.37) * 0.6 * ds / 700.0).astype(np.float32)
+    ryr = ((np.arange(H) - 0.5 * H + 0.41) * 0.6 * ds / 700.0).astype(np.float32)
+    imgs = rng.standard_normal((B, N, P, P)).astype(np.float32)
+    ic = (1.0 + 0.1 * rng.random((H, W))).astype(np.float32)
+    rx, ry = np.broadcast_to(rxc[None, :], (H, W)), np.broadcast_to(ryr[:, None], (H, W))
+    ref = opou.warp_sum(imgs.astype(np.float64), db, cu, cv, rx.astype(np.float64), ry.astype(np.float64),
+                        ic.astype(np.float64), 1.0 / ds, c)
+    dev = torch.device("cuda", 0)
+    t = {k: torch.from_numpy(np.ascontiguousarray(v)).to(dev) for k, v in
+         dict(imgs=imgs, offs=np.stack([db, cu, cv], -1), rxc=rxc, ryr=ryr, ic=ic).items()}
+    out = torch.full((N, H, W), float("nan"), device=dev)
+    L.call("fvr_pou_warp_sep", L.ptr(t["imgs"]), B, N, P, L.ptr(t["offs"]), L.ptr(t["rxc"]), L.ptr(t["ryr"]),
+           L.ptr(t["ic"]), H, W, 1.0 / ds, c, L.ptr(out), L.stream_ptr(dev))
+    assert rel_l2(out.cpu().numpy(), ref) < 2e-6
+
+
 @pytest.mark.parametrize("db0,H,W,P,pitch", [
     (0.0, 33, 70, 40, 1.0), (0.9, 40, 65, 64, 1.0), (2.5, 31, 130, 64, 1.0), (-650.0, 70, 300, 96, 0.5),
     (-2.0, 20, 33, 33, 1.0), (650.0, 9, 140, 129, 0.7), (700.0, 140, 600, 64, 0.25),
