@@ -2,10 +2,10 @@
 //
 // A Python autograd node costs about 45 us of host time per call forward and
 // needs the interpreter lock on the autograd engine's thread backward; the
-// calls below are one library launch sequence per direction (kernels of 80 to
+// calls below are one library launch sequence per direction (kernels of 70 to
 // 135 us at ordinary sizes), so the host was the bound: one pose of the
-// pinhole renderer 155 us, now 106; the explicit rays 201 -> 137; the image step
-// 190 -> 130; the registration loss 181 -> 145.
+// pinhole renderer 155 us from the Python node, 97 from here; the explicit rays
+// 201 and 130; the image step 190 and 112; the registration loss 181 and 149.
 //
 // Each node calls the C ABI through addresses the Python side hands over once
 // (bind); this file holds no kernels.  What a model, lattice or engine keeps

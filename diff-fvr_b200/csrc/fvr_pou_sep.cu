@@ -68,9 +68,9 @@ __device__ __forceinline__ float2 bcast(float x) { return make_float2(x, x); }
 // per detector row, and does both in f32x2 pairs.
 // More rows reuse an image row more often, fewer leave more CTAs (the rule is
 // at the launch).  Bound by dependent issue at 14 warps per SM.  64 blocks x 64
-// poses x 256^2 pixels: 207 us, and 394 us for a kernel with one thread per
+// poses x 256^2 pixels: 203 us, and 394 us for a kernel with one thread per
 // pixel and the row pairs blended in shared memory; 8 blocks x 64 poses x
-// 512^2 pixels: 95 and 429 us.
+// 512^2 pixels: 94 and 429 us.
 template <int RG>
 __global__ void __launch_bounds__(128) pou_warp_sep_kernel(SepArgs a, int tiles, float* __restrict__ out) {
   constexpr int NC = kSepCols;

@@ -527,7 +527,7 @@ int fvr_edge_ncc_backward(const float* a, const float* b, int64_t B, int64_t Bt,
                           int64_t crop, float ms_weight, int reduction_mean, const double* stats, const float* g,
                           int64_t g_stride, int wrt_b, float* grad, void* stream);
 
-/* ------------------------------------------- image path, one CTA per image -- */
+/* ------------------------------------------- image path, whole images ------ */
 /* 1 when a [n0][n1] image and its transform fit one CTA's shared memory. */
 int fvr_image_supported(int64_t n0, int64_t n1);
 /* img[C][R][R] = relu(real(ifft2(ifftshift(S)))) of the modulated slices S

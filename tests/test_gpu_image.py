@@ -1,4 +1,4 @@
-"""The one-CTA-per-image kernels (image forward and adjoint, image spectral
+"""The whole-image kernels (image forward and adjoint, image spectral
 NCC) against the float64 oracle at the sizes where they can go wrong: odd and
 even lengths (self-conjugate rows and columns), lengths below a warp, with
 prime factors above the register butterflies (7, 29, 47) and a single prime,
