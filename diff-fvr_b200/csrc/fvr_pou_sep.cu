@@ -5,10 +5,11 @@
 // column (d_b rx[c] - cu) / ds + c0 by every pixel of detector column c and at
 // image row (d_b ry[r] - cv) / ds + c0 by every pixel of row r: the bilinear
 // warp is a 1-D interpolation along x followed by one along y, and its adjoint
-// the two transposed ones in the other order.  Both kernels march down the
-// detector rows with the column's image position in registers, so the
-// position arithmetic (fp64), the column's two image loads and the x
-// interpolation are paid once per image row instead of once per pixel.
+// the two transposed ones in the other order.  The kernels march down the
+// detector rows: forward, the position arithmetic (fp64), a column's two image
+// loads and its x interpolation are paid once per image row instead of once per
+// pixel; the adjoint reduces the pixels to four moments per image cell, which is
+// all that the image gradient and the pose offsets need of them.
 #include <type_traits>
 
 #include "fvr_common.cuh"
