@@ -263,6 +263,9 @@ class Image : public torch::autograd::Function<Image> {
 };
 
 // Image spectral NCC: the forward keeps dloss/dpred, the backward scales it.
+// That gradient's own dependence on pred is not recorded, so neither is its
+// product with the upstream gradient: a second derivative is refused instead of
+// losing that term.
 class ImageNcc : public torch::autograd::Function<ImageNcc> {
  public:
   static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& pred, const at::Tensor& target,
@@ -290,7 +293,7 @@ class ImageNcc : public torch::autograd::Function<ImageNcc> {
     torch::autograd::variable_list out(6);
     if (!go[0].defined()) return out;
     const at::Tensor grad = ctx->get_saved_variables()[0];
-    out[0] = to_type(grad * go[0].to(grad.device(), grad.scalar_type()), ctx->saved_data["type"].toInt());
+    out[0] = to_type(grad * go[0].detach().to(grad.device(), grad.scalar_type()), ctx->saved_data["type"].toInt());
     return out;
   }
 };
@@ -379,6 +382,19 @@ T as_ptr(int64_t v) {
   return reinterpret_cast<T>(static_cast<intptr_t>(v));
 }
 
+// dL/dposes as the forward kept it, tied to the poses it was formed at: its own
+// derivative is not computed, so asking for it is an error (the derivative by
+// the upstream gradient, which only scales it, is there).
+class FirstOrder : public torch::autograd::Function<FirstOrder> {
+ public:
+  static at::Tensor forward(torch::autograd::AutogradContext*, const at::Tensor& grad, const at::Tensor&) {
+    return grad.view(grad.sizes());
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext*, torch::autograd::variable_list) {
+    TORCH_CHECK(false, "the spectral NCC loss has no second derivative in the poses");
+  }
+};
+
 class SnccLoss : public torch::autograd::Function<SnccLoss> {
  public:
   // Returns sum_v loss_v as a 0-dim tensor; keeps dL/dposes for backward.
@@ -400,6 +416,7 @@ class SnccLoss : public torch::autograd::Function<SnccLoss> {
     TORCH_CHECK(rc == 0, "fvr_tc_sncc_value_and_grad failed with status ", rc, ": ",
                 k.status ? k.status(rc) : "");
     ctx->save_for_backward({grad});
+    ctx->saved_data["poses"] = poses;  // for the graph only: later writes to them are no matter
     ctx->saved_data["pdt"] = static_cast<int64_t>(poses.scalar_type());
     return loss.select(0, nv);
   }
@@ -408,6 +425,7 @@ class SnccLoss : public torch::autograd::Function<SnccLoss> {
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
                                                  torch::autograd::variable_list go) {
     at::Tensor grad = ctx->get_saved_variables()[0];
+    if (at::GradMode::is_enabled()) grad = FirstOrder::apply(grad, ctx->saved_data["poses"].toTensor());
     at::Tensor r = go[0].defined() ? grad * go[0].to(grad.scalar_type()) : at::zeros_like(grad);
     const auto pdt = static_cast<at::ScalarType>(ctx->saved_data["pdt"].toInt());
     if (r.scalar_type() != pdt) r = r.to(pdt);

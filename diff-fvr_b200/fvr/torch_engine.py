@@ -230,6 +230,19 @@ def _sncc_loss(eng, p, views, hp, R, ftargs):
     return _SpectralNCCFn.apply(p, eng, views, hp, R, *ftargs)
 
 
+class _FirstOrder(torch.autograd.Function):
+    """A pose gradient tied to the poses it was formed at: its own derivative is
+    not computed, so asking for it is an error."""
+
+    @staticmethod
+    def forward(ctx, grad, poses):
+        return grad.view(grad.shape)
+
+    @staticmethod
+    def backward(ctx, g):
+        raise RuntimeError("the spectral NCC loss has no second derivative in the poses")
+
+
 class _SpectralNCCFn(torch.autograd.Function):
     """Zero-IFFT spectral NCC (torch_engine.py:269-307), summed over the given
     views.  When the poses need a gradient, the forward pass already runs the
@@ -248,6 +261,7 @@ class _SpectralNCCFn(torch.autograd.Function):
             loss = torch.empty(nv + 1, dtype=torch.float32, device=eng._dev)
             _sncc_fused(eng, p, views, ftargs, hp, R, out=grad, loss_out=loss)
             ctx.save_for_backward(grad)
+            ctx.poses = poses  # for the graph only: later writes to them are no matter
             return loss[nv]
         _, loss = _sncc_forward(eng, p, views, ftargs, hp, R, False)
         return loss[nv]
@@ -256,6 +270,8 @@ class _SpectralNCCFn(torch.autograd.Function):
     def backward(ctx, g):
         (grad,) = ctx.saved_tensors
         views, pdt = ctx.meta
+        if torch.is_grad_enabled():  # recorded: differentiable by the upstream gradient alone
+            grad = _FirstOrder.apply(grad, ctx.poses)
         return ((grad * g.to(grad.dtype)).to(pdt), None, None, None, None) + (None,) * len(views)
 
 
