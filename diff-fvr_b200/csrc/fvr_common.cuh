@@ -23,6 +23,11 @@ namespace fvr {
 
 constexpr int kWarp = 32;
 
+// Dynamic shared memory a launch may ask for without the opt-in: the 48 KB
+// that a CTA has are the kernel's static arrays' as well, and those take 8 KB
+// at most in the kernels that are launched by this rule.
+constexpr int64_t kSmemPlain = 40 * 1024;
+
 // ---- bounds-checked debug build --------------------------------------------
 // Built with -DFVR_CHECK (libfvr_b200_check.so), every global or shared
 // access guarded by fvr_checked(index, extent, site) whose index falls

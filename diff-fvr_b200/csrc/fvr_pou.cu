@@ -2021,11 +2021,10 @@ static int warp_strip_chunk(int64_t P, int planes) {
   return static_cast<int>(c < kWarpStripMax ? c : kWarpStripMax);
 }
 
-// Opt a warp kernel in to `sm` bytes of dynamic shared memory when that is
-// above the default 48 KB.
+// Opt a warp kernel in to `sm` bytes of dynamic shared memory when it needs to.
 template <typename K>
 static bool warp_smem_ok(K kernel, size_t sm) {
-  return sm <= 48 * 1024 ||
+  return sm <= static_cast<size_t>(kSmemPlain) ||
          cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm)) == cudaSuccess;
 }
 

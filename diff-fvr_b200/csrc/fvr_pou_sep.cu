@@ -725,7 +725,7 @@ static int sep_adjoint(const SepArgs& a, const SepGrad& w, cudaStream_t s) {
 template <int RG>
 static int sep_forward(const SepArgs& a, float* out, cudaStream_t s) {
   const int64_t smem = 4LL * kSepRingRows * a.P;
-  if (smem > 48 * 1024 &&
+  if (smem > kSmemPlain &&  // a per-device setting: before every such launch
       cudaFuncSetAttribute(pou_warp_sep_kernel<RG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(smem)) != cudaSuccess)
     return FVR_ERR_CUDA;

@@ -800,7 +800,7 @@ template <int DT, bool GRAD, int VI>
 static void launch_sncc_v(dim3 grid, int smem, cudaStream_t st, const SnccArgs& a, bool pdl) {
   constexpr SnccVariant v = sncc_variant(VI);
   auto k = tc_sncc_moments_kernel<DT, GRAD, v.group, v.min_blocks>;
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (smem > kSmemPlain) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (pdl) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
