@@ -21,6 +21,13 @@ OUT = HERE.parent / "fvr" / "_fvr_autograd.so"
 INCLUDE = HERE.parent.parent / "include"  # fvr_b200.h
 
 
+# The libstdc++ that torch runs on, named as a file: where the compiler finds no
+# libstdc++.so of its own, -lstdc++ takes the static archive, and a second copy
+# of the library in the process crashes at the first number written to a stream
+# (any error message of torch's or of ours).
+_STDCXX = ("-l:libstdc++.so.6",)
+
+
 def _command():
     import torch
 
@@ -34,7 +41,7 @@ def _command():
            f"-D_GLIBCXX_USE_CXX11_ABI={abi}", "-DTORCH_API_INCLUDE_EXTENSION_H",
            "-DTORCH_EXTENSION_NAME=_fvr_autograd"]
     cmd += [f"-I{p}" for p in incs]
-    cmd += [str(SRC), "-o", str(OUT), f"-L{lib}", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu",
+    cmd += [str(SRC), "-o", str(OUT), f"-L{lib}", *_STDCXX, "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu",
             "-ltorch_python", f"-Wl,-rpath,{lib}"]
     return cmd
 
