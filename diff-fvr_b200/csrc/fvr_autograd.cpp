@@ -63,8 +63,20 @@ struct Api {
 };
 Api api;
 
-void check(int rc, const char* name) {
-  TORCH_CHECK(rc == 0, name, " failed with status ", rc, ": ", api.status ? api.status(rc) : "");
+// The package's FvrError, in a forward as in a backward (the autograd engine
+// hands its Python type on).  Everything else, an allocation that fails among
+// it, keeps the type it has in torch.
+PyObject* error_type = nullptr;
+struct LibraryError : torch::PyTorchError {
+  using PyTorchError::PyTorchError;
+  PyObject* python_type() override { return error_type ? error_type : PyExc_RuntimeError; }
+};
+
+void check(int rc, const char* name, const char* (*status)(int) = nullptr) {
+  if (rc == 0) return;
+  if (!status) status = api.status;
+  throw LibraryError(std::string(name) + " failed with status " + std::to_string(rc) + ": " +
+                     (status ? status(rc) : ""));
 }
 
 void* current_stream(c10::DeviceIndex device) { return c10::cuda::getCurrentCUDAStream(device).stream(); }
@@ -404,17 +416,17 @@ class SnccLoss : public torch::autograd::Function<SnccLoss> {
     if (!p.is_cuda() || p.get_device() != k.device || p.scalar_type() != at::kFloat)
       p = p.to(at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(k.device)), at::kFloat);
     p = p.contiguous();
-    TORCH_CHECK(p.dim() == 2 && p.size(0) == k.C && p.size(1) == 6, "poses must have shape (", k.C, ", 6)");
+    if (p.dim() != 2 || p.size(0) != k.C || p.size(1) != 6)
+      throw LibraryError("poses must have shape (" + std::to_string(k.C) + ", 6)");
     const auto opts = at::TensorOptions().dtype(at::kFloat).device(at::kCUDA, k.device);
     const int nv = static_cast<int>(k.views.size());
     at::Tensor grad = at::empty({k.C, 6}, opts);
     at::Tensor loss = at::empty({nv + 1}, opts);
     cudaStream_t s = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(k.device)).stream();
-    const int rc = k.fn(k.dtype, k.stencil, k.scales, k.D, k.H, k.W, p.data_ptr<float>(), k.C, nv, k.views.data(),
-                        k.ftargs.data(), k.hp, k.lin, k.R, k.kappa, k.variant, nullptr, 0, k.ws, k.ws_bytes,
-                        loss.data_ptr<float>(), nullptr, grad.data_ptr<float>(), 0, s);
-    TORCH_CHECK(rc == 0, "fvr_tc_sncc_value_and_grad failed with status ", rc, ": ",
-                k.status ? k.status(rc) : "");
+    check(k.fn(k.dtype, k.stencil, k.scales, k.D, k.H, k.W, p.data_ptr<float>(), k.C, nv, k.views.data(),
+               k.ftargs.data(), k.hp, k.lin, k.R, k.kappa, k.variant, nullptr, 0, k.ws, k.ws_bytes,
+               loss.data_ptr<float>(), nullptr, grad.data_ptr<float>(), 0, s),
+          "fvr_tc_sncc_value_and_grad", k.status);
     ctx->save_for_backward({grad});
     ctx->saved_data["poses"] = poses;  // for the graph only: later writes to them are no matter
     ctx->saved_data["pdt"] = static_cast<int64_t>(poses.scalar_type());
@@ -510,20 +522,28 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         k->tw = std::move(tw);
         return k;
       }));
-  m.def("pinhole", [](const at::Tensor& mats, ModelPtr k, LatticePtr l) { return Pinhole::apply(mats, k, l); });
-  m.def("lattice_rays", [](const at::Tensor& srcs, const at::Tensor& trg, ModelPtr k) {
-    return LatticeRays::apply(srcs, trg, k);
-  });
-  m.def("image", [](const at::Tensor& poses, ImagePtr k, int64_t view) { return Image::apply(poses, k, view); });
-  m.def("image_ncc", [](const at::Tensor& pred, const at::Tensor& target, c10::optional<at::Tensor> hp,
-                        const at::Tensor& tw0, const at::Tensor& tw1) {
-    const bool need = at::GradMode::is_enabled() && pred.requires_grad();
-    return ImageNcc::apply(pred, target.detach(), hp, tw0, tw1, need);
-  });
-  m.def("reg_loss", [](const at::Tensor& a, const at::Tensor& b, const at::Tensor& ra, const at::Tensor& rb,
-                       int64_t crop, double ms, double edge) {
-    return RegLoss::apply(a, b, ra.detach(), rb.detach(), crop, ms, edge);
-  });
+  m.def("set_error_type", [](py::object type) { error_type = type.release().ptr(); },
+        "the exception raised for a library status");
+  // wrapped: torch's own exceptions (out of memory among them) and ours arrive as their Python types
+  m.def("pinhole", torch::wrap_pybind_function(
+                       [](const at::Tensor& mats, ModelPtr k, LatticePtr l) { return Pinhole::apply(mats, k, l); }));
+  m.def("lattice_rays", torch::wrap_pybind_function([](const at::Tensor& srcs, const at::Tensor& trg, ModelPtr k) {
+          return LatticeRays::apply(srcs, trg, k);
+        }));
+  m.def("image", torch::wrap_pybind_function([](const at::Tensor& poses, ImagePtr k, int64_t view) {
+          return Image::apply(poses, k, view);
+        }));
+  m.def("image_ncc",
+        torch::wrap_pybind_function([](const at::Tensor& pred, const at::Tensor& target, c10::optional<at::Tensor> hp,
+                                       const at::Tensor& tw0, const at::Tensor& tw1) {
+          const bool need = at::GradMode::is_enabled() && pred.requires_grad();
+          return ImageNcc::apply(pred, target.detach(), hp, tw0, tw1, need);
+        }));
+  m.def("reg_loss",
+        torch::wrap_pybind_function([](const at::Tensor& a, const at::Tensor& b, const at::Tensor& ra,
+                                       const at::Tensor& rb, int64_t crop, double ms, double edge) {
+          return RegLoss::apply(a, b, ra.detach(), rb.detach(), crop, ms, edge);
+        }));
   pybind11::class_<SnccCall>(m, "SnccCall")
       .def(pybind11::init([](int64_t fn, int64_t status, int dtype, int64_t stencil, int64_t scales, int64_t D,
                              int64_t H, int64_t W, int64_t C, std::vector<int> views, std::vector<int64_t> ftargs,
@@ -559,6 +579,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
            pybind11::arg("views"), pybind11::arg("ftargs"), pybind11::arg("hp"), pybind11::arg("lin"),
            pybind11::arg("R"), pybind11::arg("kappa"), pybind11::arg("variant"), pybind11::arg("ws"),
            pybind11::arg("ws_bytes"), pybind11::arg("device"), pybind11::arg("keep"));
-  m.def("sncc_loss", &sncc_loss, "sum_v spectral-NCC loss of the prepared call; differentiable in poses",
+  m.def("sncc_loss", torch::wrap_pybind_function(sncc_loss), "sum_v spectral-NCC loss of the prepared call; differentiable in poses",
         pybind11::arg("poses"), pybind11::arg("call"));
 }

@@ -19,6 +19,8 @@ try:
     from . import _fvr_autograd as _MOD
 except ImportError:
     _MOD = None
+if hasattr(_MOD, "set_error_type"):
+    _MOD.set_error_type(L.FvrError)
 
 _ENTRIES = ("fvr_status_string", "fvr_pou_pinhole_forward", "fvr_pou_pinhole_backward",
             "fvr_pou_pinhole_backward_workspace", "fvr_pou_rays_forward", "fvr_pou_rays_backward",
@@ -43,9 +45,7 @@ def module():
 
 
 def call(fn, launches, *args):
-    """``fn(*args)`` with the library's errors as FvrError; ``launches``: kernels of the call."""
+    """``fn(*args)``; ``launches``: kernels of the call.  A library status is an
+    FvrError, in the backward too; torch's errors keep their types."""
     L.launch_count[0] += launches
-    try:
-        return fn(*args)
-    except RuntimeError as e:
-        raise L.FvrError(str(e)) from None
+    return fn(*args)

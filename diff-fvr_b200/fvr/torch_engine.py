@@ -222,11 +222,7 @@ def _sncc_loss(eng, p, views, hp, R, ftargs):
     if (_NATIVE is not None and p.requires_grad and torch.is_grad_enabled()
             and not profiling.timing("tc_sncc_moments")):
         call = _fused_call(eng, int(p.shape[0]), R, views, ftargs, hp, p)
-        L.launch_count[0] += 2
-        try:
-            return _NATIVE.sncc_loss(p, call.native)
-        except RuntimeError as e:
-            raise L.FvrError(str(e)) from None
+        return NA.call(_NATIVE.sncc_loss, 2, p, call.native)
     return _SpectralNCCFn.apply(p, eng, views, hp, R, *ftargs)
 
 
