@@ -59,7 +59,7 @@ struct Api {
   decltype(&fvr_reg_loss_forward) reg_loss_forward = nullptr;
   decltype(&fvr_reg_loss_backward) reg_loss_backward = nullptr;
   decltype(&fvr_reg_loss_workspace) reg_loss_workspace = nullptr;
-  int64_t geo_stride = 0, edge_stats = 0;
+  int64_t geo_stride = 0, reg_stats = 0;
 };
 Api api;
 
@@ -322,7 +322,7 @@ class RegLoss : public torch::autograd::Function<RegLoss> {
     const std::array<at::Tensor, 4> t{as(a, d, at::kFloat), as(b, d, at::kFloat), as(ra, d, at::kFloat),
                                       as(rb, d, at::kFloat)};
     const int64_t B = a.size(0), H = a.size(2), W = a.size(3), ws_bytes = api.reg_loss_workspace(2, B, H, W);
-    at::Tensor ws = at::empty({ws_bytes}, on(d, at::kByte)), stats = at::empty({2 * B, api.edge_stats}, on(d, at::kDouble));
+    at::Tensor ws = at::empty({ws_bytes}, on(d, at::kByte)), stats = at::empty({2 * B, api.reg_stats}, on(d, at::kDouble));
     at::Tensor out = at::empty({B}, on(d, at::kFloat));
     const float* imgs[2] = {fptr(t[0]), fptr(t[1])};
     const float* refs[2] = {fptr(t[2]), fptr(t[3])};
@@ -451,7 +451,7 @@ at::Tensor sncc_loss(const at::Tensor& poses, const SnccCall& call) {
 
 }  // namespace
 
-void bind(const std::map<std::string, int64_t>& a, int64_t geo_stride, int64_t edge_stats) {
+void bind(const std::map<std::string, int64_t>& a, int64_t geo_stride, int64_t reg_stats) {
   auto set = [&](auto& f, const char* name) {
     const auto it = a.find(name);
     TORCH_CHECK(it != a.end() && it->second != 0, "no address for ", name);
@@ -472,14 +472,14 @@ void bind(const std::map<std::string, int64_t>& a, int64_t geo_stride, int64_t e
   set(api.reg_loss_backward, "fvr_reg_loss_backward");
   set(api.reg_loss_workspace, "fvr_reg_loss_workspace");
   api.geo_stride = geo_stride;
-  api.edge_stats = edge_stats;
+  api.reg_stats = reg_stats;
 }
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   namespace py = pybind11;
   m.doc() = "Native autograd binding of libfvr_b200.so";
   m.def("bind", &bind, "addresses of the C entry points and two record sizes", py::arg("addresses"),
-        py::arg("geo_stride"), py::arg("edge_stats"));
+        py::arg("geo_stride"), py::arg("reg_stats"));
   py::class_<PouModel, ModelPtr>(m, "PouModel")
       .def(py::init([](int dtype, at::Tensor stencil, c10::optional<at::Tensor> scales, int64_t B, int64_t P, double ds,
                        at::Tensor centers, at::Tensor freqs) {

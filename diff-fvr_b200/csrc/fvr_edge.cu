@@ -32,7 +32,8 @@ constexpr int kEdgeRows = 32;     // rows a warp produces
 constexpr int kEdgeWarps = 4;     // warps (independent strips) per CTA
 constexpr int kEdgeMom = 5;       // S_u, S_v, S_uu, S_vv, S_uv
 constexpr int kEdgeCombos = 4;    // fine x, fine y, coarse x, coarse y
-constexpr int kEdgeNM = (kEdgeCombos + 1) * kEdgeMom;  // and the whole images
+constexpr int kEdgeStats = kEdgeCombos * kEdgeMom;     // moments kept for the backward of the edge NCC
+constexpr int kEdgeNM = kEdgeStats + kEdgeMom;         // ... and of the registration loss: the whole images'
 constexpr int kEdgeMaxViews = 4;
 constexpr int kMomCols = 60;      // columns a warp produces: 64 less two halo columns a side
 constexpr int kGradCols = 56;     // ... four halo columns a side
@@ -44,6 +45,7 @@ struct EdgeArgs {
   float* grad[kEdgeMaxViews];     // adjoint: [B][C][H][W]
   int views, B, Cch, H, W, crop;
   int coarse;        // 1: blurred scale enabled
+  int nm;            // moments per pair in stats: kEdgeStats or kEdgeNM
   int vec;           // 1: every row starts on an 8-byte boundary
   double base, ce, cn;  // out = base + sum over views (ce edge + cn ncc)
   float w;           // weight of the blurred scale
@@ -322,7 +324,7 @@ __device__ __forceinline__ double edge_ncc(const double* m, double n) {
   return suv / sqrt(fmax(suu * svv, 1e-12));
 }
 
-// One CTA per batch item: strip sums -> stats[pair][kEdgeNM] in job order,
+// One CTA per batch item: strip sums -> stats[pair][nm] in job order,
 // then out = base + sum over views (ce edge + cn ncc), edge = the channel mean
 // of (1 - w) fine + w coarse.
 __global__ void __launch_bounds__(128) edge_finalize_kernel(EdgeArgs e, int jobs, const double* __restrict__ partial,
@@ -346,7 +348,7 @@ __global__ void __launch_bounds__(128) edge_finalize_kernel(EdgeArgs e, int jobs
       if (threadIdx.x < kEdgeNM) {
         const double s = ((part[0][lane] + part[1][lane]) + part[2][lane]) + part[3][lane];
         part[0][lane] = s;
-        stats[pair * kEdgeNM + lane] = s;
+        if (lane < e.nm) stats[pair * e.nm + lane] = s;
       }
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -392,7 +394,9 @@ __global__ void __launch_bounds__(32 * kEdgeWarps, 4) edge_grad_kernel(EdgeArgs 
   const EdgeJob jb = edge_job(e, pair, job < jobs ? job : 0, strips);
   if (threadIdx.x < kEdgeCombos + 1) {
     const int k = threadIdx.x;
-    const double* m = stats + pair * kEdgeNM + k * kEdgeMom;
+    const bool kept = (k + 1) * kEdgeMom <= e.nm;
+    const double none[kEdgeMom] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    const double* m = kept ? stats + pair * e.nm + k * kEdgeMom : none;
     // u = the differentiated image's response, v = the other one's
     const double su = swap ? m[1] : m[0], sv = swap ? m[0] : m[1];
     const double suu_raw = swap ? m[3] : m[2], svv_raw = swap ? m[2] : m[3];
@@ -531,6 +535,7 @@ static int edge_common(int64_t B, int64_t C, int64_t H, int64_t W, int64_t crop,
   e->H = (int)H;
   e->W = (int)W;
   e->crop = (int)crop;
+  e->nm = kEdgeStats;
   e->coarse = (w > 0.f && W >= 96) ? 1 : 0;  // the reference tests the last dim (cone_beam_fvr.py:86, 107)
   e->w = w;
   e->vec = W % 2 == 0 ? 1 : 0;
@@ -610,6 +615,7 @@ static int reg_loss_args(const float* const* imgs, const float* const* refs, con
   int rc = edge_common(B, 1, H, W, crop, ms_weight, e);
   if (rc) return rc;
   e->views = views;
+  e->nm = kEdgeNM;
   e->base = 1.0;
   e->ce = -static_cast<double>(edge_weight) / views;
   e->cn = -(1.0 - static_cast<double>(edge_weight)) / views;
@@ -629,7 +635,7 @@ int64_t fvr_edge_ncc_workspace(int64_t B, int64_t C, int64_t H, int64_t W, int64
   return edge_ws_bytes(1, B, C, H, W);
 }
 
-int64_t fvr_edge_ncc_stats_count(void) { return kEdgeNM; }
+int64_t fvr_edge_ncc_stats_count(void) { return kEdgeStats; }
 
 int fvr_edge_ncc_forward(const float* a, const float* b, int64_t B, int64_t Bt, int64_t C, int64_t H, int64_t W,
                          int64_t crop, float ms_weight, int reduction_mean, void* workspace, int64_t ws_bytes,
@@ -663,6 +669,8 @@ int64_t fvr_reg_loss_workspace(int64_t views, int64_t B, int64_t H, int64_t W) {
   if (views < 1 || B < 1 || H < 1 || W < 1) return 0;
   return edge_ws_bytes(views, B, 1, H, W);
 }
+
+int64_t fvr_reg_loss_stats_count(void) { return kEdgeNM; }
 
 int fvr_reg_loss_forward(const float* const* imgs, const float* const* refs, const int64_t* ref_batch, int views,
                          int64_t B, int64_t H, int64_t W, int64_t crop, float ms_weight, float edge_weight,

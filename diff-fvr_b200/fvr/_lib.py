@@ -64,6 +64,7 @@ SIGNATURES = {
     "fvr_edge_ncc_stats_count": (I64, []),
     "fvr_edge_ncc_forward": (I32, [P, P, I64, I64, I64, I64, I64, I64, F32, I32, P, I64, P, P, P]),
     "fvr_edge_ncc_backward": (I32, [P, P, I64, I64, I64, I64, I64, I64, F32, I32, P, P, I64, I32, P, P]),
+    "fvr_reg_loss_stats_count": (I64, []),
     "fvr_reg_loss_workspace": (I64, [I64, I64, I64, I64]),
     "fvr_reg_loss_forward": (I32, [P, P, P, I32, I64, I64, I64, I64, F32, F32, P, I64, P, P, P]),
     "fvr_reg_loss_backward": (I32, [P, P, P, I32, I64, I64, I64, I64, F32, F32, P, P, I64, P, P]),

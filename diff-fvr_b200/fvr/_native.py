@@ -39,7 +39,7 @@ def module():
         if not hasattr(_MOD, "bind"):  # built before these nodes existed
             return None
         _MOD.bind({n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in _ENTRIES},
-                  int(lib.fvr_pou_geo_stride()), int(lib.fvr_edge_ncc_stats_count()))
+                  int(lib.fvr_pou_geo_stride()), int(lib.fvr_reg_loss_stats_count()))
         _bound = lib
     return _MOD
 

@@ -81,7 +81,7 @@ class _RegLossFn(torch.autograd.Function):
         B, _, H, W = (int(x) for x in imA.shape)
         ws_bytes = int(L.query("fvr_reg_loss_workspace", 2, B, H, W))
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-        stats = torch.empty((2 * B, int(L.query("fvr_edge_ncc_stats_count"))), dtype=torch.float64, device=dev)
+        stats = torch.empty((2 * B, int(L.query("fvr_reg_loss_stats_count"))), dtype=torch.float64, device=dev)
         out = torch.empty(B, dtype=torch.float32, device=dev)
         L.call("fvr_reg_loss_forward", *_RegLossFn._args(ims, refs), L.ptr(ws), ws_bytes, L.ptr(stats), L.ptr(out),
                L.stream_ptr(dev))

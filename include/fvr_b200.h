@@ -512,8 +512,8 @@ int fvr_se3_exp_backward(const float* theta, const float* grad_mats, int64_t N, 
  * [crop, W-crop), NCC per direction (denominator sqrt(max(Suu Svv, 1e-12))),
  * 0.5 (x + y) averaged over channels; when ms_weight > 0 and W >= 96 mixed
  * (1 - w) fine + w (same on 3x3 box-blurred images, zero padding, divisor 9).
- * out[0] = batch mean (reduction_mean) or out[B].  stats[B*C][n] (fp64
- * moments, n = fvr_edge_ncc_stats_count()) is kept for the backward.
+ * out[0] = batch mean (reduction_mean) or out[B].  stats[B*C][20] (fp64
+ * moments, fvr_edge_ncc_stats_count()) is kept for the backward.
  * Replaces edge_dominant_ncc, src/fvr/cone_beam_fvr.py:71-112. */
 int64_t fvr_edge_ncc_workspace(int64_t B, int64_t C, int64_t H, int64_t W, int64_t crop);
 int64_t fvr_edge_ncc_stats_count(void);
@@ -552,11 +552,12 @@ int fvr_cncc_image(const float* pred, const float* target, int64_t B, int64_t Bt
  * refs[v][ref_batch[v]][H][W] (ref_batch 1 or B), f32:
  *   out[b] = 1 - mean over v of (edge_weight edge + (1 - edge_weight) ncc),
  * edge as fvr_edge_ncc_forward with one channel, ncc the zero-mean NCC of the
- * whole images (denominator sqrt(max(Saa Sbb, 1e-12))).  stats[views*B][n]
- * (n = fvr_edge_ncc_stats_count()) is kept for the backward, which writes
+ * whole images (denominator sqrt(max(Saa Sbb, 1e-12))).  stats[views*B][25]
+ * (fvr_reg_loss_stats_count()) is kept for the backward, which writes
  * d out / d imgs scaled by the upstream g[b * g_stride] into grads[v][B][H][W].
  * The pointer arrays are host memory.  Replaces the loss of
  * experiments/exp30_gpu_multistart_registration.py:120-134. */
+int64_t fvr_reg_loss_stats_count(void);
 int64_t fvr_reg_loss_workspace(int64_t views, int64_t B, int64_t H, int64_t W);
 int fvr_reg_loss_forward(const float* const* imgs, const float* const* refs, const int64_t* ref_batch, int views,
                          int64_t B, int64_t H, int64_t W, int64_t crop, float ms_weight, float edge_weight,

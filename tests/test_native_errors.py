@@ -29,7 +29,7 @@ def failing_entry():
     def bind(name):
         addr = {n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in NA._ENTRIES}
         addr[name] = ctypes.cast(fake, ctypes.c_void_p).value
-        NA._MOD.bind(addr, int(lib.fvr_pou_geo_stride()), int(lib.fvr_edge_ncc_stats_count()))
+        NA._MOD.bind(addr, int(lib.fvr_pou_geo_stride()), int(lib.fvr_reg_loss_stats_count()))
 
     assert NA.module() is not None
     yield bind
