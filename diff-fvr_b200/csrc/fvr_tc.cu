@@ -411,8 +411,9 @@ __global__ void __launch_bounds__(kSnccThreads, MINB) tc_sncc_moments_kernel(Snc
   const int row_begin = tile * a.tile_rows;
   const int row_end = min(row_begin + a.tile_rows, R);
   const SnccTab tab = sncc_tab(tab_smem, R + a.tile_rows);
-  pdl_launch_dependents();
   pdl_wait();  // launched as a programmatic dependent: the kernel before it has completed (else a no-op)
+  // only now: the epilogue reads the poses, which that kernel may have written, before it waits for this one
+  pdl_launch_dependents();
   if (threadIdx.x == 0) sncc_item_axes(a, v, c, ax_s);
   __syncthreads();
   build_sncc_tables(tab, R, row_begin, row_end - row_begin, a.lin, ax_s, a.sx, a.sy, a.sz, a.kpi);
@@ -432,7 +433,8 @@ __global__ void __launch_bounds__(kSnccThreads, MINB) tc_sncc_moments_kernel(Snc
 // A single chunk also reduces the losses; several leave that to a small
 // dependent kernel that reads every candidate's ncc:
 //  0. the slice-axes Jacobians of the chunk's items, formed while the moments
-//     kernel still runs;
+//     kernel still runs (its CTAs release this launch once whatever wrote the
+//     poses has completed; read at L2, where that is visible);
 //  1. after griddepcontrol.wait, one thread per (item, moment): the item's
 //     records summed in record order, every load of a thread issued in one
 //     round, kept in shared memory;
@@ -491,7 +493,10 @@ __global__ void __launch_bounds__(kFinalThreads) tc_sncc_final_kernel(SnccArgs a
     if (t < ni) {
       const int v = t / cn, c = c0 + (t - v * cn);
       double ax[8];
-      slice_axes_jac(a.poses + 6 * c, view_lateral(a, v), a.sx, a.sy, a.sz, ax, s_jac[t]);
+      float p[6];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) p[k] = __ldcg(a.poses + 6 * c + k);
+      slice_axes_jac(p, view_lateral(a, v), a.sx, a.sy, a.sz, ax, s_jac[t]);
     }
     if (gridDim.x > 1) pdl_launch_dependents();  // the loss kernel
     pdl_wait();  // the moments kernel has completed and its records are visible
