@@ -150,6 +150,7 @@ def edge_dominant_ncc(pred, target, border_crop=None, multiscale_weight=0.25, re
 
 
 _LATTICE_CACHE: Dict[Tuple, Tuple] = {}
+_LATTICE_USED = (0, 2, 3, 4, 5, 6, 7)  # src0, u0, v0, n0, rx, ry, ic of the lattice tuple
 
 
 # A lattice is taken as separable (one ray coordinate per detector column and
@@ -197,13 +198,20 @@ def _prepared_lattice(lattice, device):
     """Device copies of an 11-tuple lattice's ray tables and its basis
     (src0, u0, v0, n0) as 12 host doubles, its separable ray tables when
     it has them, whether those are monotone and the native binding's record of
-    them, cached per (storage, device): the lattice is a per-geometry
-    constant, moved once.  The entry holds the lattice's own tensors, so their
-    storage cannot be freed and reused by another lattice while the entry
-    exists."""
-    key = tuple(int(t.data_ptr()) for t in lattice[:8]) + (str(device),)
+    them, cached per device and view of storage (address, shape, strides, type:
+    a crop or every second pixel starts at the same address): the lattice is a
+    per-geometry constant, moved once, and prepared again after a write to it
+    (the tensors' versions; inference tensors have none).  The entry holds the
+    lattice's own tensors, so their storage cannot be freed and reused by
+    another lattice while the entry exists."""
+    key, versions = [device], []
+    for i in _LATTICE_USED:
+        t = lattice[i]
+        key += (t.data_ptr(), t.shape, t.stride(), t.dtype)
+        versions.append(0 if t.is_inference() else t._version)
+    key = tuple(key)
     hit = _LATTICE_CACHE.get(key)
-    if hit is None:
+    if hit is None or hit[0] != versions:
         if len(_LATTICE_CACHE) > 64:
             _LATTICE_CACHE.clear()
         basis = torch.cat([lattice[i].reshape(3) for i in (0, 2, 3, 4)]).detach().double().cpu()
@@ -212,7 +220,7 @@ def _prepared_lattice(lattice, device):
         sep, monotone = _separable_tables(rays[0], rays[1])
         native = NA.module()
         plan = native.PouLattice(list(base), sep[0], sep[1], rays[2]) if native is not None and sep is not None else None
-        hit = (key, base, rays, tuple(lattice[:8]), sep, monotone, plan)
+        hit = (versions, base, rays, tuple(lattice[:8]), sep, monotone, plan)
         _LATTICE_CACHE[key] = hit
     return hit
 
@@ -270,12 +278,12 @@ class _PinholeFn(torch.autograd.Function):
     mats -> pose geometry -> block slices -> batched IFFT -> warp-sum."""
 
     @staticmethod
-    def forward(ctx, mats, model, rx, ry, ic, base_key):
+    def forward(ctx, mats, model, lattice):
         dev = model._dev
         m = mats.detach().to(device=dev, dtype=torch.float32).contiguous()
         N = int(m.shape[0])
         B, P = model.B, model.P
-        _, base, _, _, sep, monotone, _ = _LATTICE_CACHE[base_key]
+        _, base, (rx, ry, ic), _, sep, monotone, _ = lattice
         geo = torch.empty((N, int(L.query("fvr_pou_geo_stride"))), dtype=torch.float64, device=dev)
         offs = torch.empty((B, N, 3), dtype=torch.float64, device=dev)
         s = L.stream_ptr(dev)
@@ -325,7 +333,7 @@ class _PinholeFn(torch.autograd.Function):
                    L.ptr(offs), N, base, float(P) * model.ds_block, L.ptr(model.centers), L.ptr(model._freqs),
                    L.ptr(imgs), L.ptr(sep[0]), L.ptr(sep[1]), L.ptr(ic), H, W, 1.0 / model.ds_block, float(P // 2),
                    L.ptr(g), L.ptr(grad_imgs), L.ptr(ws), wsb, L.ptr(gm), s)
-            return gm.to(mdt), None, None, None, None, None
+            return gm.to(mdt), None, None
         goffs = torch.empty((3, B, N), dtype=torch.float64, device=dev)
         if gather:
             grad_imgs = torch.empty((B, N, P, P), dtype=torch.float32, device=dev)
@@ -362,7 +370,7 @@ class _PinholeFn(torch.autograd.Function):
         gm = torch.empty((N, 4, 4), dtype=torch.float32, device=dev)
         L.call("fvr_pou_pose_backward", L.ptr(ws2), tiles, L.ptr(goffs), None, 0, L.ptr(geo), L.ptr(model.centers), B,
                N, base, float(P) * model.ds_block, L.ptr(gm), None, s)
-        return gm.to(mdt), None, None, None, None, None
+        return gm.to(mdt), None, None
 
 
 class PerspectiveSlabFVR(nn.Module):
@@ -582,7 +590,8 @@ class PerspectiveSlabFVR(nn.Module):
             H, W = int(lattice[1].shape[0]), int(lattice[1].shape[1])
             return torch.zeros((0, 1, H, W), dtype=torch.float32, device=home) + 0.0 * pose_mats.sum()
         if len(lattice) >= 11:
-            key, _, (rx, ry, ic), _, _, monotone, plan = _prepared_lattice(lattice, self._dev)
+            entry = _prepared_lattice(lattice, self._dev)
+            _, _, (rx, _, _), _, _, monotone, plan = entry
             mats = pose_mats if home == self._dev else pose_mats.to(self._dev)
             H, W = int(rx.shape[0]), int(rx.shape[1])
             native = NA.module()
@@ -592,7 +601,7 @@ class PerspectiveSlabFVR(nn.Module):
                     and (not grad or _gather_adjoint(self, monotone, int(mats.shape[0]), H, W))):
                 out = NA.call(native.pinhole, 7 if grad else 3, mats, self._native_plan(native), plan)
             else:
-                out = _PinholeFn.apply(mats, self, rx, ry, ic, key)
+                out = _PinholeFn.apply(mats, self, entry)
         else:
             out = self._forward_explicit(pose_mats, lattice)
         return out if out.device == home else out.to(home)
