@@ -197,8 +197,8 @@ _GRAD_IMAGE_BYTES = 4 << 30
 def _prepared_lattice(lattice, device):
     """Device copies of an 11-tuple lattice's ray tables and its basis
     (src0, u0, v0, n0) as 12 host doubles, its separable ray tables when
-    it has them, whether those are monotone and the native binding's record of
-    them, cached per device and view of storage (address, shape, strides, type:
+    it has them, whether those are monotone and a place for the native
+    binding's record of them, cached per device and view of storage (address, shape, strides, type:
     a crop or every second pixel starts at the same address): the lattice is a
     per-geometry constant, moved once, and prepared again after a write to it
     (the tensors' versions; inference tensors have none).  The entry holds the
@@ -218,11 +218,19 @@ def _prepared_lattice(lattice, device):
         base = (_ct.c_double * 12)(*[float(x) for x in basis])
         rays = tuple(t.detach().to(device=device, dtype=torch.float32).contiguous() for t in lattice[5:8])
         sep, monotone = _separable_tables(rays[0], rays[1])
-        native = NA.module()
-        plan = native.PouLattice(list(base), sep[0], sep[1], rays[2]) if native is not None and sep is not None else None
-        hit = (versions, base, rays, tuple(lattice[:8]), sep, monotone, plan)
+        hit = (versions, base, rays, tuple(lattice[:8]), sep, monotone, [None])
         _LATTICE_CACHE[key] = hit
     return hit
+
+
+def _lattice_plan(native, entry):
+    """The native binding's record of a prepared separable lattice, made when the
+    binding first takes a call on it (the lattice may have been prepared where
+    only the Python nodes run)."""
+    _, base, rays, _, sep, _, plan = entry
+    if plan[0] is None:
+        plan[0] = native.PouLattice(list(base), sep[0], sep[1], rays[2])
+    return plan[0]
 
 
 def _block_images(model, geo, N, s):
@@ -591,15 +599,16 @@ class PerspectiveSlabFVR(nn.Module):
             return torch.zeros((0, 1, H, W), dtype=torch.float32, device=home) + 0.0 * pose_mats.sum()
         if len(lattice) >= 11:
             entry = _prepared_lattice(lattice, self._dev)
-            _, _, (rx, _, _), _, _, monotone, plan = entry
+            _, _, (rx, _, _), _, sep, monotone, _ = entry
             mats = pose_mats if home == self._dev else pose_mats.to(self._dev)
             H, W = int(rx.shape[0]), int(rx.shape[1])
             native = NA.module()
             grad = mats.requires_grad and torch.is_grad_enabled()
-            if (native is not None and plan is not None and tuple(mats.shape[1:]) == (4, 4)
+            if (native is not None and sep is not None and tuple(mats.shape[1:]) == (4, 4)
                     and L.query("fvr_pou_pinhole_supported", self.P, H, W)
                     and (not grad or _gather_adjoint(self, monotone, int(mats.shape[0]), H, W))):
-                out = NA.call(native.pinhole, 7 if grad else 3, mats, self._native_plan(native), plan)
+                out = NA.call(native.pinhole, 7 if grad else 3, mats, self._native_plan(native),
+                              _lattice_plan(native, entry))
             else:
                 out = _PinholeFn.apply(mats, self, entry)
         else:

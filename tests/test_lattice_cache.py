@@ -54,6 +54,20 @@ def test_a_written_lattice_is_prepared_again():
 
 
 @pytest.mark.gpu
+def test_a_lattice_first_used_under_a_launch_timer_takes_the_native_node():
+    from fvr import profiling, synthetic
+    from fvr.cone_beam_fvr import PerspectiveSlabFVR
+
+    m = PerspectiveSlabFVR.from_volume(synthetic.make_ellipsoid_volume(40, 2), vox_mm=2.0, grid_blocks=(2, 2, 2),
+                                       block_res=32, overlap=0.5)
+    mats = synthetic.make_pinhole_mats(2, 5, device="cuda").requires_grad_(True)
+    lat = _lattice(24, 40, "cuda")
+    with profiling.LaunchTimer(["pou_warp"]):
+        assert "_PinholeFn" in m.forward_pinhole(mats, lat).grad_fn.name()
+    assert "_PinholeFn" not in m.forward_pinhole(mats, lat).grad_fn.name()
+
+
+@pytest.mark.gpu
 def test_rendering_on_views_and_after_a_write():
     from fvr import synthetic
     from fvr.cone_beam_fvr import PerspectiveSlabFVR
