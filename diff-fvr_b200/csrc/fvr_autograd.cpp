@@ -146,7 +146,9 @@ class Pinhole : public torch::autograd::Function<Pinhole> {
                               offs.data_ptr<double>(), imgs.data_ptr<float>(), out.data_ptr<float>(),
                               current_stream(d.index())),
           "fvr_pou_pinhole_forward");
-    ctx->save_for_backward({geo, offs, imgs});
+    // the obliquity table may be the caller's own tensor: kept as one, so that a write to it before the backward is seen
+    // (an inference tensor has no version and cannot be kept by a node)
+    ctx->save_for_backward({geo, offs, imgs, l->ic.is_inference() ? at::Tensor() : l->ic});
     ctx->saved_data["model"] = keep(m);
     ctx->saved_data["lattice"] = keep(l);
     ctx->saved_data["type"] = static_cast<int64_t>(mats.scalar_type());
@@ -160,6 +162,7 @@ class Pinhole : public torch::autograd::Function<Pinhole> {
     const at::Tensor &geo = saved[0], &offs = saved[1], &imgs = saved[2];
     const ModelPtr m = kept<PouModel>(ctx->saved_data["model"]);
     const LatticePtr l = kept<PouLattice>(ctx->saved_data["lattice"]);
+    const at::Tensor& ic = saved[3].defined() ? saved[3] : l->ic;
     const at::Device d = m->device();
     c10::cuda::CUDAGuard guard(d);
     const int64_t N = geo.size(0), ws_bytes = api.pinhole_backward_workspace(m->B, N, l->H, l->W);
@@ -168,7 +171,7 @@ class Pinhole : public torch::autograd::Function<Pinhole> {
     at::Tensor grad = at::empty({N, 4, 4}, on(d, at::kFloat));
     check(api.pinhole_backward(m->dtype, m->stencil.data_ptr(), fptr(m->scales), m->B, m->P, geo.data_ptr<double>(),
                                offs.data_ptr<double>(), N, l->base.data(), m->vscale(), fptr(m->centers),
-                               fptr(m->freqs), fptr(imgs), fptr(l->rxc), fptr(l->ryr), fptr(l->ic), l->H, l->W,
+                               fptr(m->freqs), fptr(imgs), fptr(l->rxc), fptr(l->ryr), fptr(ic), l->H, l->W,
                                1.0 / m->ds, m->c(), fptr(g), gimgs.data_ptr<float>(), ws.data_ptr(), ws_bytes,
                                grad.data_ptr<float>(), current_stream(d.index())),
           "fvr_pou_pinhole_backward");

@@ -82,3 +82,40 @@ def test_rendering_on_views_and_after_a_write():
     assert torch.allclose(coarse, full[:, :, ::2, ::2], rtol=1e-5, atol=1e-5 * float(full.max()))
     lat[7].mul_(2.0)
     assert torch.allclose(m.forward_pinhole(mats, lat), 2.0 * full, rtol=1e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("native", [True, False])
+def test_a_write_between_forward_and_backward_is_an_error(native, monkeypatch):
+    """autograd's rule for what a node keeps, on the native node as on the Python node."""
+    import fvr._native as NA
+    from fvr import synthetic
+    from fvr.cone_beam_fvr import PerspectiveSlabFVR
+
+    if not native:
+        monkeypatch.setattr(NA, "_MOD", None)
+    m = PerspectiveSlabFVR.from_volume(synthetic.make_ellipsoid_volume(40, 2), vox_mm=2.0, grid_blocks=(2, 2, 2),
+                                       block_res=32, overlap=0.5)
+    mats = synthetic.make_pinhole_mats(2, 5, device="cuda").requires_grad_(True)
+    lat = _lattice(24, 40, "cuda")
+    out = m.forward_pinhole(mats, lat).sum()
+    lat[7].mul_(2.0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        out.backward()
+
+
+@pytest.mark.gpu
+def test_a_lattice_of_inference_tensors_still_gives_gradients():
+    from fvr import synthetic
+    from fvr.cone_beam_fvr import PerspectiveSlabFVR
+
+    m = PerspectiveSlabFVR.from_volume(synthetic.make_ellipsoid_volume(40, 2), vox_mm=2.0, grid_blocks=(2, 2, 2),
+                                       block_res=32, overlap=0.5)
+    with torch.inference_mode():
+        inf = _lattice(24, 40, "cuda")
+    grads = []
+    for lat in (inf, _lattice(24, 40, "cuda")):
+        mats = synthetic.make_pinhole_mats(2, 5, device="cuda").requires_grad_(True)
+        m.forward_pinhole(mats, lat).sum().backward()
+        grads.append(mats.grad)
+    assert torch.equal(*grads)
