@@ -545,13 +545,14 @@ class TorchDiffFVREngine(nn.Module):
         """The native binding's record of the image path at one output size (made
         again when the storage or the spacing was replaced)."""
         st, kap = self._stencil, RT.kappa(R, self.spacing[0])
-        hit = self._image_plans.get(R)
+        plans = self.__dict__.setdefault("_image_plans", {})  # engines saved before there were records have none
+        hit = plans.get(R)
         if hit is None or hit[0] is not st or hit[1] != kap:
-            if len(self._image_plans) > 64:
-                self._image_plans.clear()
+            if len(plans) > 64:
+                plans.clear()
             hit = (st, kap, native.ImagePlan(st.code, st.data, st.scales, *st.dims, R, kap, RT.linspace(R, self._dev),
                                              RT.twiddles(R, L.F32_, self._dev)))
-            self._image_plans[R] = hit
+            plans[R] = hit
         return hit[2]
 
     def forward(self, poses: torch.Tensor, view: str = "ap", out_res: int = 128) -> torch.Tensor:
