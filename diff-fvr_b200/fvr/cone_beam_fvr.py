@@ -620,14 +620,13 @@ class PerspectiveSlabFVR(nn.Module):
 
     def _native_plan(self, native):
         """The native binding's record of the block spectra and geometry constants (made again when one was replaced)."""
-        parts = (self._stencil, self.centers, self._freqs)
+        st, numbers = self._stencil, (self.B, self.P, self.ds_block)
+        parts = (st, self.centers, self._freqs)
         plan = getattr(self, "_plan", None)
-        if plan is None or any(a is not b for a, b in zip(plan[0], parts)):
-            st = self._stencil
-            plan = (parts, native.PouModel(st.code, st.data, st.scales, self.B, self.P, self.ds_block, self.centers,
-                                           self._freqs))
+        if plan is None or plan[1] != numbers or any(a is not b for a, b in zip(plan[0], parts)):
+            plan = (parts, numbers, native.PouModel(st.code, st.data, st.scales, *numbers, self.centers, self._freqs))
             self._plan = plan
-        return plan[1]
+        return plan[2]
 
     def _forward_explicit(self, pose_mats, lattice):
         from .cone_beam_rays import forward_explicit

@@ -124,7 +124,7 @@ def _fused_call(eng, C, R, views, ftargs, hp, p):
     nv = len(views)
     direct = all(f.is_cuda and f.device == dev and f.dtype == torch.complex64 and f.is_contiguous() for f in ftargs)
     key = (C, R, tuple(views), tuple(int(f.data_ptr()) for f in ftargs), 0 if hp is None else int(hp.data_ptr()),
-           id(st))
+           id(st), eng.spacing[0])
     hit = eng._fused_calls.get(key) if direct else None
     if hit is not None:
         return hit
