@@ -126,8 +126,11 @@ class _LatticeRaysFn(torch.autograd.Function):
 
 
 def lattice_rays_supported(model, srcs, trg_pts):
-    """The one-call path: block images of a supported size, one (or more) poses."""
-    return (trg_pts.dim() == 4 and trg_pts.shape[-1] == 3 and 1 <= trg_pts.shape[0] <= 65535 and trg_pts.numel() > 0
+    """The one-call path: block images of a supported size, one (or more) poses,
+    points of at most 32 bits (it forms the detector axes from the points as
+    float32; of float64 points they are formed in float64)."""
+    return (trg_pts.dtype in (torch.float32, torch.float16, torch.bfloat16) and trg_pts.dim() == 4
+            and trg_pts.shape[-1] == 3 and 1 <= trg_pts.shape[0] <= 65535 and trg_pts.numel() > 0
             and srcs.shape == (trg_pts.shape[0], 3) and bool(L.query("fvr_pou_image_supported", model.P)))
 
 
