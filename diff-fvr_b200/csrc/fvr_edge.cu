@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(32 * kEdgeWarps, 4) edge_moments_kernel(EdgeAr
     float2 x[2];
     rows.next(x);
     if (NCC && t >= jb.rb && t < jb.re) {
-      if (t == jb.rb) pivot = make_float2(0.5f * (x[0].x + x[1].x), 0.5f * (x[0].y + x[1].y));
+      if (t == jb.rb) pivot = x[0];  // the lane's first column: the second may lie outside
 #pragma unroll
       for (int j = 0; j < 2; ++j)
         if (mine[j]) {

@@ -1,0 +1,29 @@
+"""The image-NCC share of the registration loss on images whose mean is large
+against their spread, odd widths among them: sums about a value of the image
+itself, so 1e-6 relative against float64 whatever the mean."""
+import pytest
+import torch
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,W", [(40, 41), (70, 128)])
+@pytest.mark.parametrize("mean", [0.0, 10.0, 100.0, 1000.0])
+def test_image_ncc_of_images_with_a_mean(mean, H, W, monkeypatch):
+    import fvr.registration as reg
+
+    monkeypatch.setattr(reg, "_EDGE_WEIGHT", 0.0)
+    g = torch.Generator(device="cuda").manual_seed(int(mean) + H)
+    a, b, ra, rb = (mean * s + torch.randn((n, 1, H, W), generator=g, device="cuda")
+                    for s, n in ((1.0, 3), (0.5, 3), (1.0, 3), (2.0, 1)))
+    ra = (ra + a) / 2  # correlated with a
+    loss = reg.biplanar_loss_per_candidate(a, b, ra, rb)
+
+    def ncc(p, r):
+        p, r = (t - t.mean(dim=(-2, -1), keepdim=True) for t in (p, r))
+        return ((p * r).sum(dim=(-2, -1)) / (p.square().sum(dim=(-2, -1)) * r.square().sum(dim=(-2, -1))).sqrt())[:, 0]
+
+    want = 1.0 - 0.5 * (ncc(a.double(), ra.double()) + ncc(b.double(), rb.double()))
+    assert rel_l2(loss.cpu().numpy(), want.cpu().numpy()) < 1e-6
