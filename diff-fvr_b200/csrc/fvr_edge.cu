@@ -381,13 +381,17 @@ __global__ void edge_mean_kernel(const double* __restrict__ value, int B, float*
 // fields g_k(q) = alpha_k (v_k(q) - mean v_k) + beta_k (u_k(q) - mean u_k) on
 // the interior, transposed Sobel, and for the blurred scale the transposed box
 // filter; the fine and the coarse fields go through the transposed Sobel
-// together as one f32x2 value.  Row t enters, row t - 4 leaves.
+// together as one f32x2 value.  Row t enters, row t - 4 leaves.  Three CTAs an
+// SM (168 registers): 71 us with the coefficients and means in registers, 84 with
+// four CTAs, which spill (72 before the fields were centred).
 template <bool COARSE, bool NCC>
-__global__ void __launch_bounds__(32 * kEdgeWarps, 4) edge_grad_kernel(EdgeArgs e, int strips, int jobs, int groups,
+__global__ void __launch_bounds__(32 * kEdgeWarps, 3) edge_grad_kernel(EdgeArgs e, int strips, int jobs, int groups,
                                                                     const double* __restrict__ stats,
                                                                     const float* __restrict__ g, int64_t g_stride,
                                                                     double g_scale, int swap) {
-  __shared__ float coef[kEdgeCombos + 1][3];  // alpha, beta, -(alpha mean v + beta mean u)
+  // alpha, beta, -mean u, -mean v, and what the means' rounding to float leaves of alpha mean v + beta mean u
+  __shared__ float4 coef[kEdgeCombos + 1];
+  __shared__ float rest[kEdgeCombos + 1];
   const int64_t pair = blockIdx.x / groups;
   const int job = static_cast<int>(blockIdx.x - pair * groups) * kEdgeWarps + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -408,9 +412,10 @@ __global__ void __launch_bounds__(32 * kEdgeWarps, 4) edge_grad_kernel(EdgeArgs 
     const double sw = k < 2 ? (e.coarse ? 1.0 - e.w : 1.0) : (e.coarse ? static_cast<double>(e.w) : 0.0);
     const double wk = static_cast<double>(g[g_stride * jb.bi]) * g_scale * (whole ? e.cn : e.ce * sw * 0.5) / e.Cch;
     const double al = wk / den, be = prod > 1e-12 ? -wk * suv * svv / (den * den * den) : 0.0;
-    coef[k][0] = static_cast<float>(al);
-    coef[k][1] = static_cast<float>(be);
-    coef[k][2] = static_cast<float>(-(al * sv + be * su) / n);
+    const double mu = su / n, mv = sv / n;
+    const float fu = static_cast<float>(mu), fv = static_cast<float>(mv);
+    coef[k] = make_float4(static_cast<float>(al), static_cast<float>(be), -fu, -fv);
+    rest[k] = static_cast<float>(al * (fv - mv) + be * (fu - mu));
   }
   __syncthreads();
   if (job >= jobs) return;
@@ -422,13 +427,23 @@ __global__ void __launch_bounds__(32 * kEdgeWarps, 4) edge_grad_kernel(EdgeArgs 
     in_img[j] = c + j >= 0 && c + j < e.W;
     in_edge[j] = c + j >= e.crop && c + j < e.W - e.crop;
   }
-  float al[kEdgeCombos + 1], be[kEdgeCombos + 1], k0[kEdgeCombos + 1];
+  // alpha (v - mean v) + beta (u - mean u): centred first, since a mean may be large against the spread
+  float4 cc[kEdgeCombos + 1];
+  float kk[kEdgeCombos + 1];
 #pragma unroll
-  for (int k = 0; k < kEdgeCombos + 1; ++k) {
-    al[k] = coef[k][0];
-    be[k] = coef[k][1];
-    k0[k] = coef[k][2];
+  for (int k = 0; k <= kEdgeCombos; ++k) {
+    cc[k] = coef[k];
+    kk[k] = rest[k];
   }
+  auto fields = [&](int k, const float2 (&x)[2], float (&f)[2]) {
+    const float4 c = cc[k];
+    const float k0 = kk[k];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float2 d = add2(x[j], make_float2(c.z, c.w));
+      f[j] = fmaf(c.x, d.y, fmaf(c.y, d.x, k0));
+    }
+  };
   float* out = e.grad[jb.view] + (static_cast<int64_t>(jb.bi) * e.Cch + jb.ch) * static_cast<int64_t>(e.H) * e.W;
   EdgeMarch<COARSE> march;
   march.init();
@@ -450,16 +465,25 @@ __global__ void __launch_bounds__(32 * kEdgeWarps, 4) edge_grad_kernel(EdgeArgs 
     march.step(x, t - 1 >= 0 && t - 1 < e.H, in_img, gx, gy, gbx, gby);
     const bool rf = t - 1 >= e.crop && t - 1 < e.H - e.crop, rc = t - 2 >= e.crop && t - 2 < e.H - e.crop;
     float2 Fx[2], Fy[2];  // (fine, coarse) fields of row t - 2
+    float vx[2], vy[2];
+    fields(0, gx, vx);
+    fields(1, gy, vy);
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       Fx[j] = make_float2(fx1[j], 0.f);
       Fy[j] = make_float2(fy1[j], 0.f);
-      const bool f_in = rf && in_edge[j], c_in = rc && in_edge[j];
-      fx1[j] = f_in ? fmaf(al[0], gx[j].y, fmaf(be[0], gx[j].x, k0[0])) : 0.f;
-      fy1[j] = f_in ? fmaf(al[1], gy[j].y, fmaf(be[1], gy[j].x, k0[1])) : 0.f;
-      if (COARSE) {
-        Fx[j].y = c_in ? fmaf(al[2], gbx[j].y, fmaf(be[2], gbx[j].x, k0[2])) : 0.f;
-        Fy[j].y = c_in ? fmaf(al[3], gby[j].y, fmaf(be[3], gby[j].x, k0[3])) : 0.f;
+      const bool f_in = rf && in_edge[j];
+      fx1[j] = f_in ? vx[j] : 0.f;
+      fy1[j] = f_in ? vy[j] : 0.f;
+    }
+    if (COARSE) {
+      fields(2, gbx, vx);
+      fields(3, gby, vy);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const bool c_in = rc && in_edge[j];
+        Fx[j].y = c_in ? vx[j] : 0.f;
+        Fy[j].y = c_in ? vy[j] : 0.f;
       }
     }
     float2 xl, xr, yl, yr;
@@ -501,7 +525,8 @@ __global__ void __launch_bounds__(32 * kEdgeWarps, 4) edge_grad_kernel(EdgeArgs 
         h1[j] = h[j];
       }
     }
-    float res[2];
+    float res[2], vn[2];
+    if (NCC) fields(kEdgeCombos, x, vn);
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       res[j] = of[j] + bt[j];
@@ -511,7 +536,7 @@ __global__ void __launch_bounds__(32 * kEdgeWarps, 4) edge_grad_kernel(EdgeArgs 
         im0[j] = im1[j];
         im1[j] = im2[j];
         im2[j] = im3[j];
-        im3[j] = fmaf(al[kEdgeCombos], x[j].y, fmaf(be[kEdgeCombos], x[j].x, k0[kEdgeCombos]));
+        im3[j] = vn[j];
       }
     }
     const int r = t - 4;

@@ -1,6 +1,7 @@
 """The image-NCC share of the registration loss on images whose mean is large
 against their spread, odd widths among them: sums about a value of the image
-itself, so 1e-6 relative against float64 whatever the mean."""
+itself, so 1e-6 relative against float64 whatever the mean; the gradient is two
+products of centred values per pixel, a few roundings, the same 1e-6."""
 import pytest
 import torch
 
@@ -19,11 +20,18 @@ def test_image_ncc_of_images_with_a_mean(mean, H, W, monkeypatch):
     a, b, ra, rb = (mean * s + torch.randn((n, 1, H, W), generator=g, device="cuda")
                     for s, n in ((1.0, 3), (0.5, 3), (1.0, 3), (2.0, 1)))
     ra = (ra + a) / 2  # correlated with a
-    loss = reg.biplanar_loss_per_candidate(a, b, ra, rb)
+    x, y = a.clone().requires_grad_(True), b.clone().requires_grad_(True)
+    loss = reg.biplanar_loss_per_candidate(x, y, ra, rb)
+    up = torch.tensor([1.0, -0.5, 2.0], device="cuda")
+    got = torch.autograd.grad(loss, (x, y), up)
 
     def ncc(p, r):
         p, r = (t - t.mean(dim=(-2, -1), keepdim=True) for t in (p, r))
         return ((p * r).sum(dim=(-2, -1)) / (p.square().sum(dim=(-2, -1)) * r.square().sum(dim=(-2, -1))).sqrt())[:, 0]
 
-    want = 1.0 - 0.5 * (ncc(a.double(), ra.double()) + ncc(b.double(), rb.double()))
-    assert rel_l2(loss.cpu().numpy(), want.cpu().numpy()) < 1e-6
+    x64, y64 = a.double().requires_grad_(True), b.double().requires_grad_(True)
+    want = 1.0 - 0.5 * (ncc(x64, ra.double()) + ncc(y64, rb.double()))
+    want_g = torch.autograd.grad(want, (x64, y64), up.double())
+    assert rel_l2(loss.detach().cpu().numpy(), want.detach().cpu().numpy()) < 1e-6
+    for p, q in zip(got, want_g):
+        assert rel_l2(p.cpu().numpy(), q.cpu().numpy()) < 1e-6
