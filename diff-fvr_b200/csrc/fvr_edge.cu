@@ -20,22 +20,22 @@
 // candidates x two views of 256 x 256 (kernel times): an earlier form with
 // 32 x 32 tiles in shared memory took 2 x 43 us (moments), 2 x 119 us
 // (finalize, one CTA for all pairs) and 2 x 91 us (adjoint), the image NCC
-// another 350 us as separate tensor operations; now 50, 9 and 72 us for both
+// another 350 us as separate tensor operations; now 57, 9 and 66 us for both
 // views and both similarities.  The moments and adjoint passes are bound by
-// issued instructions (54 % issue active at 16 warps per SM; the images alone
-// take 5 and 10 us at the copy bandwidth).
+// issued instructions (the images alone take 5 and 10 us at the copy
+// bandwidth).  A CTA is one warp, so that an SM starts the next strip whenever
+// one of its warps is done.
 #include "fvr_common.cuh"
 
 namespace fvr {
 
-constexpr int kEdgeRows = 32;     // rows a warp produces
-constexpr int kEdgeWarps = 4;     // warps (independent strips) per CTA
+constexpr int kEdgeRows = 32;     // rows a CTA (one warp) produces
 constexpr int kEdgeMom = 5;       // S_u, S_v, S_uu, S_vv, S_uv
 constexpr int kEdgeCombos = 4;    // fine x, fine y, coarse x, coarse y
 constexpr int kEdgeStats = kEdgeCombos * kEdgeMom;     // moments kept for the backward of the edge NCC
 constexpr int kEdgeNM = kEdgeStats + kEdgeMom;         // ... and of the registration loss: the whole images'
 constexpr int kEdgeMaxViews = 4;
-constexpr int kMomCols = 60;      // columns a warp produces: 64 less two halo columns a side
+constexpr int kMomCols = 60;      // columns it produces: 64 less two halo columns a side
 constexpr int kGradCols = 56;     // ... four halo columns a side
 
 struct EdgeArgs {
@@ -218,16 +218,17 @@ __device__ __forceinline__ double warp_sum_each(double (&v)[32]) {
 }
 
 // Moments of one strip of rows -> partial[pair][job][kEdgeNM] (fp64).  Products
-// are summed per lane in f32 (at most 2 x kEdgeRows terms), then in fp64.  The
+// are summed per lane in f32 over two rows (four terms), then in fp64: 57 us for
+// 64 candidates x two views of 256 x 256, and 54 with all 64 terms of a lane in
+// f32, 64 with four warps to a CTA.  The
 // whole images' mean may be large against their spread, so those moments are
 // taken about a value of the lane's own first row and moved to zero in fp64.
 template <bool COARSE, bool NCC>
-__global__ void __launch_bounds__(32 * kEdgeWarps, 4) edge_moments_kernel(EdgeArgs e, int strips, int jobs, int groups,
-                                                                       double* __restrict__ partial) {
-  const int64_t pair = blockIdx.x / groups;
-  const int job = static_cast<int>(blockIdx.x - pair * groups) * kEdgeWarps + (threadIdx.x >> 5);
-  if (job >= jobs) return;
-  const int lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(32, 12) edge_moments_kernel(EdgeArgs e, int strips, int jobs,
+                                                              double* __restrict__ partial) {
+  const int64_t pair = blockIdx.x / jobs;
+  const int job = static_cast<int>(blockIdx.x - pair * jobs);
+  const int lane = threadIdx.x;
   const EdgeJob jb = edge_job(e, pair, job, strips);
   const int c = jb.strip * kMomCols - 2 + 2 * lane;
   const bool own = lane >= 1 && lane <= 30;
@@ -238,28 +239,52 @@ __global__ void __launch_bounds__(32 * kEdgeWarps, 4) edge_moments_kernel(EdgeAr
     mine[j] = own && in_img[j];
     in_edge[j] = own && c + j >= e.crop && c + j < e.W - e.crop;
   }
-  float2 m1[kEdgeCombos], m2[kEdgeCombos];  // (S_u, S_v), (S_uu, S_vv)
-  float m3[kEdgeCombos];                    // S_uv
-#pragma unroll
-  for (int k = 0; k < kEdgeCombos; ++k) {
-    m1[k] = m2[k] = make_float2(0.f, 0.f);
-    m3[k] = 0.f;
-  }
+  float2 m1[kEdgeCombos] = {}, m2[kEdgeCombos] = {};  // (S_u, S_v), (S_uu, S_vv) of at most two rows
+  float m3[kEdgeCombos] = {};                         // S_uv
+  double sum[kEdgeNM] = {};                           // ... of all rows
   auto add = [&](int k, float2 g) {
     m1[k] = add2(m1[k], g);
     m2[k] = __ffma2_rn(g, g, m2[k]);
     m3[k] = fmaf(g.x, g.y, m3[k]);
   };
-  float2 pivot = make_float2(0.f, 0.f), i1 = pivot, i2 = pivot;  // whole images: sums of (x - pivot), squares
-  float i3 = 0.f;
+  float2 pivot = make_float2(0.f, 0.f), i1, i2;  // whole images: sums of (x - pivot), squares
+  float i3;
+  auto clear = [&] {
+#pragma unroll
+    for (int k = 0; k < kEdgeCombos; ++k) {
+      m1[k] = m2[k] = make_float2(0.f, 0.f);
+      m3[k] = 0.f;
+    }
+    i1 = i2 = make_float2(0.f, 0.f);
+    i3 = 0.f;
+  };
+  auto flush = [&] {
+#pragma unroll
+    for (int k = 0; k < (COARSE ? kEdgeCombos : 2); ++k) {
+      double* s = sum + k * kEdgeMom;
+      s[0] += m1[k].x;
+      s[1] += m1[k].y;
+      s[2] += m2[k].x;
+      s[3] += m2[k].y;
+      s[4] += m3[k];
+    }
+    if (NCC) {
+      double* s = sum + kEdgeStats;
+      s[0] += i1.x;
+      s[1] += i1.y;
+      s[2] += i2.x;
+      s[3] += i2.y;
+      s[4] += i3;
+    }
+  };
   const int lo = max(jb.rb, e.crop), hi = min(jb.re, e.H - e.crop);  // interior rows of this job
   EdgeMarch<COARSE> march;
   march.init();
   const int t_end = jb.re + (COARSE ? 2 : 1);
   RowReader rows;
   rows.init(e, jb.a, jb.b, jb.rb - 2, c);
-#pragma unroll 2
-  for (int t = jb.rb - 2; t < t_end; ++t) {
+  int t = jb.rb - 2;
+  auto row = [&] {
     float2 x[2];
     rows.next(x);
     if (NCC && t >= jb.rb && t < jb.re) {
@@ -291,27 +316,28 @@ __global__ void __launch_bounds__(32 * kEdgeWarps, 4) edge_moments_kernel(EdgeAr
           add(3, gby[j]);
         }
     }
+    ++t;
+  };
+  while (t < t_end) {  // a row past the end adds nothing
+    clear();
+    row();
+    row();
+    flush();
   }
   double v[32];
 #pragma unroll
   for (int k = 0; k < 32; ++k) v[k] = 0.0;
 #pragma unroll
-  for (int k = 0; k < kEdgeCombos; ++k) {
-    v[k * kEdgeMom] = m1[k].x;
-    v[k * kEdgeMom + 1] = m1[k].y;
-    v[k * kEdgeMom + 2] = m2[k].x;
-    v[k * kEdgeMom + 3] = m2[k].y;
-    v[k * kEdgeMom + 4] = m3[k];
-  }
+  for (int k = 0; k < kEdgeStats; ++k) v[k] = sum[k];
   if (NCC) {
     const double n = static_cast<double>((mine[0] ? 1 : 0) + (mine[1] ? 1 : 0)) * (jb.re - jb.rb);
-    const double pu = pivot.x, pv = pivot.y, su = i1.x, sv = i1.y;
-    double* im = v + kEdgeCombos * kEdgeMom;
+    const double pu = pivot.x, pv = pivot.y, su = sum[kEdgeStats], sv = sum[kEdgeStats + 1];
+    double* im = v + kEdgeStats;
     im[0] = su + n * pu;
     im[1] = sv + n * pv;
-    im[2] = i2.x + pu * (2.0 * su + n * pu);
-    im[3] = i2.y + pv * (2.0 * sv + n * pv);
-    im[4] = i3 + pu * sv + pv * su + n * pu * pv;
+    im[2] = sum[kEdgeStats + 2] + pu * (2.0 * su + n * pu);
+    im[3] = sum[kEdgeStats + 3] + pv * (2.0 * sv + n * pv);
+    im[4] = sum[kEdgeStats + 4] + pu * sv + pv * su + n * pu * pv;
   }
   const double s = warp_sum_each(v);
   if (lane < kEdgeNM) partial[(pair * jobs + job) * kEdgeNM + lane] = s;
@@ -381,21 +407,20 @@ __global__ void edge_mean_kernel(const double* __restrict__ value, int B, float*
 // fields g_k(q) = alpha_k (v_k(q) - mean v_k) + beta_k (u_k(q) - mean u_k) on
 // the interior, transposed Sobel, and for the blurred scale the transposed box
 // filter; the fine and the coarse fields go through the transposed Sobel
-// together as one f32x2 value.  Row t enters, row t - 4 leaves.  Three CTAs an
-// SM (168 registers): 71 us with the coefficients and means in registers, 84 with
-// four CTAs, which spill (72 before the fields were centred).
+// together as one f32x2 value.  Row t enters, row t - 4 leaves.  Sixteen
+// warps an SM, 66 us (twelve warps, without spills: 69; CTAs of four warps: 71
+// with twelve and 84 with sixteen).
 template <bool COARSE, bool NCC>
-__global__ void __launch_bounds__(32 * kEdgeWarps, 3) edge_grad_kernel(EdgeArgs e, int strips, int jobs, int groups,
-                                                                    const double* __restrict__ stats,
-                                                                    const float* __restrict__ g, int64_t g_stride,
-                                                                    double g_scale, int swap) {
+__global__ void __launch_bounds__(32, 16) edge_grad_kernel(EdgeArgs e, int strips, int jobs,
+                                                           const double* __restrict__ stats,
+                                                           const float* __restrict__ g, int64_t g_stride,
+                                                           double g_scale, int swap) {
   // alpha, beta, -mean u, -mean v, and what the means' rounding to float leaves of alpha mean v + beta mean u
   __shared__ float4 coef[kEdgeCombos + 1];
   __shared__ float rest[kEdgeCombos + 1];
-  const int64_t pair = blockIdx.x / groups;
-  const int job = static_cast<int>(blockIdx.x - pair * groups) * kEdgeWarps + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  const EdgeJob jb = edge_job(e, pair, job < jobs ? job : 0, strips);
+  const int64_t pair = blockIdx.x / jobs;
+  const int lane = threadIdx.x;
+  const EdgeJob jb = edge_job(e, pair, static_cast<int>(blockIdx.x - pair * jobs), strips);
   if (threadIdx.x < kEdgeCombos + 1) {
     const int k = threadIdx.x;
     const bool kept = (k + 1) * kEdgeMom <= e.nm;
@@ -417,8 +442,7 @@ __global__ void __launch_bounds__(32 * kEdgeWarps, 3) edge_grad_kernel(EdgeArgs 
     coef[k] = make_float4(static_cast<float>(al), static_cast<float>(be), -fu, -fv);
     rest[k] = static_cast<float>(al * (fv - mv) + be * (fu - mu));
   }
-  __syncthreads();
-  if (job >= jobs) return;
+  __syncwarp();
   const int c = jb.strip * kGradCols - 4 + 2 * lane;
   const bool own = lane >= 2 && lane <= 29;
   bool in_img[2], in_edge[2];
@@ -587,23 +611,21 @@ static int64_t edge_ws_bytes(int64_t views, int64_t B, int64_t C, int64_t H, int
 
 template <typename K>
 static int edge_grid(const EdgeArgs& e, int cols, K launch) {
-  const int64_t jobs = edge_jobs(e.H, e.W, cols), groups = cdiv64(jobs, kEdgeWarps);
-  const int64_t n = static_cast<int64_t>(e.views) * e.B * e.Cch * groups;
+  const int64_t jobs = edge_jobs(e.H, e.W, cols);
+  const int64_t n = static_cast<int64_t>(e.views) * e.B * e.Cch * jobs;
   if (n > 2147483647) return FVR_ERR_ARG;
-  launch(static_cast<unsigned>(n), static_cast<int>(cdiv64(e.W, cols)), static_cast<int>(jobs),
-         static_cast<int>(groups));
+  launch(static_cast<unsigned>(n), static_cast<int>(cdiv64(e.W, cols)), static_cast<int>(jobs));
   FVR_LAUNCH_CHECK();
   return FVR_OK;
 }
 
 static int edge_forward(const EdgeArgs& e, void* workspace, double* stats, float* out, bool mean, cudaStream_t s) {
   double* part = static_cast<double*>(workspace);
-  const int rc = edge_grid(e, kMomCols, [&](unsigned n, int strips, int jobs, int groups) {
-    const dim3 block(32 * kEdgeWarps);
-    if (e.coarse && e.cn != 0.0) edge_moments_kernel<true, true><<<n, block, 0, s>>>(e, strips, jobs, groups, part);
-    else if (e.coarse) edge_moments_kernel<true, false><<<n, block, 0, s>>>(e, strips, jobs, groups, part);
-    else if (e.cn != 0.0) edge_moments_kernel<false, true><<<n, block, 0, s>>>(e, strips, jobs, groups, part);
-    else edge_moments_kernel<false, false><<<n, block, 0, s>>>(e, strips, jobs, groups, part);
+  const int rc = edge_grid(e, kMomCols, [&](unsigned n, int strips, int jobs) {
+    if (e.coarse && e.cn != 0.0) edge_moments_kernel<true, true><<<n, 32, 0, s>>>(e, strips, jobs, part);
+    else if (e.coarse) edge_moments_kernel<true, false><<<n, 32, 0, s>>>(e, strips, jobs, part);
+    else if (e.cn != 0.0) edge_moments_kernel<false, true><<<n, 32, 0, s>>>(e, strips, jobs, part);
+    else edge_moments_kernel<false, false><<<n, 32, 0, s>>>(e, strips, jobs, part);
   });
   if (rc) return rc;
   const int jobs = (int)edge_jobs(e.H, e.W, kMomCols);
@@ -620,16 +642,15 @@ static int edge_forward(const EdgeArgs& e, void* workspace, double* stats, float
 
 static int edge_backward(const EdgeArgs& e, const double* stats, const float* g, int64_t g_stride, double g_scale,
                          int swap, cudaStream_t s) {
-  return edge_grid(e, kGradCols, [&](unsigned n, int strips, int jobs, int groups) {
-    const dim3 block(32 * kEdgeWarps);
+  return edge_grid(e, kGradCols, [&](unsigned n, int strips, int jobs) {
     if (e.coarse && e.cn != 0.0)
-      edge_grad_kernel<true, true><<<n, block, 0, s>>>(e, strips, jobs, groups, stats, g, g_stride, g_scale, swap);
+      edge_grad_kernel<true, true><<<n, 32, 0, s>>>(e, strips, jobs, stats, g, g_stride, g_scale, swap);
     else if (e.coarse)
-      edge_grad_kernel<true, false><<<n, block, 0, s>>>(e, strips, jobs, groups, stats, g, g_stride, g_scale, swap);
+      edge_grad_kernel<true, false><<<n, 32, 0, s>>>(e, strips, jobs, stats, g, g_stride, g_scale, swap);
     else if (e.cn != 0.0)
-      edge_grad_kernel<false, true><<<n, block, 0, s>>>(e, strips, jobs, groups, stats, g, g_stride, g_scale, swap);
+      edge_grad_kernel<false, true><<<n, 32, 0, s>>>(e, strips, jobs, stats, g, g_stride, g_scale, swap);
     else
-      edge_grad_kernel<false, false><<<n, block, 0, s>>>(e, strips, jobs, groups, stats, g, g_stride, g_scale, swap);
+      edge_grad_kernel<false, false><<<n, 32, 0, s>>>(e, strips, jobs, stats, g, g_stride, g_scale, swap);
   });
 }
 

@@ -35,3 +35,28 @@ def test_image_ncc_of_images_with_a_mean(mean, H, W, monkeypatch):
     assert rel_l2(loss.detach().cpu().numpy(), want.detach().cpu().numpy()) < 1e-6
     for p, q in zip(got, want_g):
         assert rel_l2(p.cpu().numpy(), q.cpu().numpy()) < 1e-6
+
+
+def test_moments_add_few_products_in_float32():
+    """A triangle wave whose Sobel response is +-a with a long mantissa: every sum
+    of squares rounds the same way in every lane.  Four products in float32
+    before float64: partial sums of 1/4 .. 1, so at most 2.5 x 2^-24 relative (64
+    in a row would give 9.5e-7)."""
+    import fvr._lib as L
+
+    H, W, crop = 128, 250, 8
+    s = 1.0 + 4031 / 4096
+    dev = torch.device("cuda", 0)
+    x = torch.arange(W, device=dev) % 16
+    img = (s * torch.where(x < 8, x, 16 - x).float())[None, None, None].expand(1, 1, H, W).contiguous()
+    wsb = L.query("fvr_edge_ncc_workspace", 1, 1, H, W, crop)
+    ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
+    stats, out = torch.zeros(40, dtype=torch.float64, device=dev), torch.empty(1, device=dev)
+    L.call("fvr_edge_ncc_forward", L.ptr(img), L.ptr(img), 1, 1, 1, H, W, crop, 0.0, 0, L.ptr(ws), wsb, L.ptr(stats),
+           L.ptr(out), L.stream_ptr(dev))
+    row = img[0, 0, 0].double()
+    g = 4.0 * (row[2:] - row[:-2])[crop - 1:W - crop - 1]  # Sobel x of columns crop .. W - crop - 1
+    want = float((g * g).sum()) * (H - 2 * crop)
+    got = stats.cpu().numpy()
+    for k in (2, 3, 4):  # S_uu, S_vv, S_uv
+        assert abs(got[k] / want - 1.0) < 2.5 * 2.0 ** -24, got[k] / want - 1.0
