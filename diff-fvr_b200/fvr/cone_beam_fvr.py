@@ -159,27 +159,36 @@ _LATTICE_USED = (0, 2, 3, 4, 5, 6, 7)  # src0, u0, v0, n0, rx, ry, ic of the lat
 # exactly, so a pixel's sampling position moves by about the rounding of the
 # position arithmetic itself.
 _SEPARABLE_REL = 2.0 ** -20
+# The separable warp samples every pixel at its column's and row's midpoint, in
+# the forward too.  It takes spreads of one rounding step of the largest ray at
+# most (the lattices of make_pinhole_lattice): a midpoint is then as near to the
+# exact ray as the pixel's own value.  Lattices in between are rendered pixel by
+# pixel; at the wider limit a midpoint is up to 6e-5 image pixels off.
+_ROUNDING_REL = 2.0 ** -23
 
 
 def _separable_tables(rx, ry):
-    """``(sep, monotone)`` of a lattice's rays: sep = (rxc [W], ryr [H]), the
-    midpoints of the per-column rx and per-row ry ranges, or None when the rays
-    do not separate (see _SEPARABLE_REL); monotone says whether both tables run
-    in one direction (the separable warp adjoint marches along them)."""
+    """``(sep, monotone, rounding)`` of a lattice's rays: sep = (rxc [W], ryr
+    [H]), the midpoints of the per-column rx and per-row ry ranges, or None when
+    the rays do not separate (see _SEPARABLE_REL); monotone says whether both
+    tables run in one direction (the separable warp adjoint marches along them),
+    rounding whether the spreads are a rounding step's (see _ROUNDING_REL)."""
     if rx.ndim != 2 or rx.shape != ry.shape:
-        return None, False
+        return None, False, False
     # per column / row: the largest, the smallest and the largest magnitude, in one host transfer
     cols, rows = torch.stack([rx.amax(0), rx.amin(0)]), torch.stack([ry.amax(1), ry.amin(1)])
     host = torch.cat([cols, rows], dim=1).cpu().numpy().astype(np.float64)
-    tables = []
+    tables, rounding = [], True
     for hi, lo in (host[:, :rx.shape[1]], host[:, rx.shape[1]:]):
-        if not (hi - lo).max() <= _SEPARABLE_REL * max(np.abs(hi).max(), np.abs(lo).max(), 1e-30):
-            return None, False
+        spread, largest = (hi - lo).max(), max(np.abs(hi).max(), np.abs(lo).max(), 1e-30)
+        if not spread <= _SEPARABLE_REL * largest:
+            return None, False, False
+        rounding = rounding and bool(spread <= _ROUNDING_REL * largest)
         tables.append((0.5 * (hi + lo)).astype(np.float32))
     steps = [np.diff(t) for t in tables]
     monotone = all(bool((d >= 0).all()) or bool((d <= 0).all()) for d in steps)
     both = torch.from_numpy(np.concatenate(tables)).to(rx.device)
-    return (both[:rx.shape[1]].clone(), both[rx.shape[1]:].clone()), monotone
+    return (both[:rx.shape[1]].clone(), both[rx.shape[1]:].clone()), monotone, rounding
 
 
 def _separable_rays(rx, ry):
@@ -197,8 +206,9 @@ _GRAD_IMAGE_BYTES = 4 << 30
 def _prepared_lattice(lattice, device):
     """Device copies of an 11-tuple lattice's ray tables and its basis
     (src0, u0, v0, n0) as 12 host doubles, its separable ray tables when
-    it has them, whether those are monotone and a place for the native
-    binding's record of them, cached per device and view of storage (address, shape, strides, type:
+    it has them, whether those are monotone, a place for the native binding's
+    record of them and the tables again where the separable warp may sample
+    at them (else None), cached per device and view of storage (address, shape, strides, type:
     a crop or every second pixel starts at the same address): the lattice is a
     per-geometry constant, moved once, and prepared again after a write to it
     (the tensors' versions; inference tensors have none).  The entry holds the
@@ -217,8 +227,8 @@ def _prepared_lattice(lattice, device):
         basis = torch.cat([lattice[i].reshape(3) for i in (0, 2, 3, 4)]).detach().double().cpu()
         base = (_ct.c_double * 12)(*[float(x) for x in basis])
         rays = tuple(t.detach().to(device=device, dtype=torch.float32).contiguous() for t in lattice[5:8])
-        sep, monotone = _separable_tables(rays[0], rays[1])
-        hit = (versions, base, rays, tuple(lattice[:8]), sep, monotone, [None])
+        sep, monotone, rounding = _separable_tables(rays[0], rays[1])
+        hit = (versions, base, rays, tuple(lattice[:8]), sep, monotone, [None], sep if rounding else None)
         _LATTICE_CACHE[key] = hit
     return hit
 
@@ -227,9 +237,9 @@ def _lattice_plan(native, entry):
     """The native binding's record of a prepared separable lattice, made when the
     binding first takes a call on it (the lattice may have been prepared where
     only the Python nodes run)."""
-    _, base, rays, _, sep, _, plan = entry
+    _, base, rays, _, _, _, plan, tables = entry
     if plan[0] is None:
-        plan[0] = native.PouLattice(list(base), sep[0], sep[1], rays[2])
+        plan[0] = native.PouLattice(list(base), tables[0], tables[1], rays[2])
     return plan[0]
 
 
@@ -291,15 +301,15 @@ class _PinholeFn(torch.autograd.Function):
         m = mats.detach().to(device=dev, dtype=torch.float32).contiguous()
         N = int(m.shape[0])
         B, P = model.B, model.P
-        _, base, (rx, ry, ic), _, sep, monotone, _ = lattice
+        _, base, (rx, ry, ic), _, sep, monotone, _, tables = lattice
         geo = torch.empty((N, int(L.query("fvr_pou_geo_stride"))), dtype=torch.float64, device=dev)
         offs = torch.empty((B, N, 3), dtype=torch.float64, device=dev)
         s = L.stream_ptr(dev)
         vscale = float(P) * model.ds_block
         H, W = int(rx.shape[0]), int(rx.shape[1])
         out = torch.empty((N, 1, H, W), dtype=torch.float32, device=dev)
-        ctx.meta = (model, base, mats.dtype, sep, monotone)
-        if sep is not None and not profiling.active() and L.query("fvr_pou_pinhole_supported", P, H, W):
+        ctx.meta = (model, base, mats.dtype, sep, monotone and tables is not None)
+        if tables is not None and not profiling.active() and L.query("fvr_pou_pinhole_supported", P, H, W):
             st = model._stencil
             imgs = torch.empty((B, N, P, P), dtype=torch.float32, device=dev)
             L.call("fvr_pou_pinhole_forward", st.code, L.ptr(st.data), L.ptr(st.scales), B, P, L.ptr(m), N, base,
@@ -311,7 +321,7 @@ class _PinholeFn(torch.autograd.Function):
         with profiling.section("pou_slice"):
             imgs = _block_images(model, geo, N, s)
         with profiling.section("pou_warp"):
-            if sep is not None and L.query("fvr_pou_warp_sep_supported", P, H, W):
+            if tables is not None and L.query("fvr_pou_warp_sep_supported", P, H, W):
                 L.call("fvr_pou_warp_sep", L.ptr(imgs), B, N, P, L.ptr(offs), L.ptr(sep[0]), L.ptr(sep[1]), L.ptr(ic),
                        H, W, 1.0 / model.ds_block, float(P // 2), L.ptr(out), s)
             else:
@@ -599,12 +609,12 @@ class PerspectiveSlabFVR(nn.Module):
             return torch.zeros((0, 1, H, W), dtype=torch.float32, device=home) + 0.0 * pose_mats.sum()
         if len(lattice) >= 11:
             entry = _prepared_lattice(lattice, self._dev)
-            _, _, (rx, _, _), _, sep, monotone, _ = entry
+            _, _, (rx, _, _), _, _, monotone, _, tables = entry
             mats = pose_mats if home == self._dev else pose_mats.to(self._dev)
             H, W = int(rx.shape[0]), int(rx.shape[1])
             native = NA.module()
             grad = mats.requires_grad and torch.is_grad_enabled()
-            if (native is not None and sep is not None and tuple(mats.shape[1:]) == (4, 4)
+            if (native is not None and tables is not None and tuple(mats.shape[1:]) == (4, 4)
                     and L.query("fvr_pou_pinhole_supported", self.P, H, W)
                     and (not grad or _gather_adjoint(self, monotone, int(mats.shape[0]), H, W))):
                 out = NA.call(native.pinhole, 7 if grad else 3, mats, self._native_plan(native),
