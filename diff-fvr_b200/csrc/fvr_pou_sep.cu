@@ -363,17 +363,18 @@ __global__ void __launch_bounds__(256) pou_warp_sep_weigh_kernel(const float* __
 
 // One CTA per (pose, block).  A detector pixel lies in one cell of the block
 // image, [x, x + 1) x [y, y + 1), at fractions (tx, ty); everything the adjoint
-// needs of the pixels is their four moments per cell, sums of g ic times 1, tx,
-// ty, tx ty.  The CTA walks down the image rows that the detector reaches in
+// needs of the pixels is four sums per cell, of g ic times the weights of the
+// cell's four corners (each weight by itself: 1 - tx taken from sums of 1 and tx
+// would cancel on samples next to the far side).  The CTA walks down the image rows that the detector reaches in
 // steps of a few 8-row bands, over as many 32-column groups as its buffer holds
 // the detector columns of:
 //   its warps march down the detector rows of the step's cells, 128 detector
 //   columns at a time, four neighbours per lane in f32x2 pairs: per cell row
-//   and column A0 = sum g ic and A1 = sum ty g ic, to the buffer;
+//   and column A0 = sum (1 - ty) g ic and A1 = sum ty g ic, to the buffer;
 //   then a warp takes a band of a group: lane x sums its cell's columns, S0, S1
-//   = sum A0, A1 and T0, T1 = sum tx A0, tx A1, and with S = S0 - S1 + S1(y - 1)
-//   and T alike, dL/dimg[y][x] = S - T + T(x - 1); the pose-offset sums take
-//   the image's differences over the cell.
+//   = sum (1 - tx) A0, A1 and T0, T1 = sum tx A0, A1, and with S = S0 + S1(y - 1)
+//   and T alike, dL/dimg[y][x] = S + T(x - 1); the pose-offset sums take the
+//   image's differences over the cell.
 // Every element of dL/dimgs is written once (nothing to clear, no atomics).
 // The sums of g rx dv/dpx and g ry dv/dpy come from rx = (x + tx - ox) / scale
 // and ry alike, in f32 relative to the integer next to ox, oy.
@@ -528,10 +529,10 @@ __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(Sep
               for (int j = 0; j < 4; ++j) {
                 if (kr + j < kr1) {
                   while (kr + j >= kend) flush();
-                  const float2 ty = bcast(rty[kr + j]);
+                  const float2 ty = bcast(rty[kr + j]), uy = bcast(1.f - rty[kr + j]);
                   const float2 g0 = make_float2(cur[j].x, cur[j].y), g1 = make_float2(cur[j].z, cur[j].w);
-                  A0[0] = __fadd2_rn(A0[0], g0);
-                  A0[1] = __fadd2_rn(A0[1], g1);
+                  A0[0] = __ffma2_rn(uy, g0, A0[0]);
+                  A0[1] = __ffma2_rn(uy, g1, A0[1]);
                   A1[0] = __ffma2_rn(ty, g0, A1[0]);
                   A1[1] = __ffma2_rn(ty, g1, A1[1]);
                 }
@@ -568,15 +569,16 @@ __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(Sep
             t1 = min(t1, ke);
             for (int k = max(t0, kp); k < t1; ++k) {
               if (!fvr_checked(k - kp, pitch, kSiteWarpFused)) continue;
-              const float2 t = bcast(__int_as_float(cmap[k].y));
+              const float tx = __int_as_float(cmap[k].y);
+              const float2 t = bcast(tx), u = bcast(1.f - tx);
               const float* q = bq + k;
 #pragma unroll
               for (int i = 0; i < kSepPairs; ++i) {
                 const float2 v0 = make_float2(q[4 * i * pitch], q[(4 * i + 2) * pitch]);
                 const float2 v1 = make_float2(q[(4 * i + 1) * pitch], q[(4 * i + 3) * pitch]);
-                S0[i] = __fadd2_rn(S0[i], v0);
+                S0[i] = __ffma2_rn(u, v0, S0[i]);
                 T0[i] = __ffma2_rn(t, v0, T0[i]);
-                S1[i] = __fadd2_rn(S1[i], v1);
+                S1[i] = __ffma2_rn(u, v1, S1[i]);
                 T1[i] = __ffma2_rn(t, v1, T1[i]);
               }
             }
@@ -595,7 +597,7 @@ __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(Sep
             float ux = 0.f, urx = 0.f, uy = 0.f, ury = 0.f;
             // the left cell's S and T of image row y0 + lane - 1 (lane >= 1)
             const float up = __shfl_up_sync(0xffffffffu, L1, 1), upt = __shfl_up_sync(0xffffffffu, LT1, 1);
-            const float LS = (L0 - L1) + up, LT = (LT0 - LT1) + upt;
+            const float LS = L0 + up, LT = LT0 + upt;
             if (xg == 0 && l0 < l1) {  // column -1 is no image column: its sums are taken here, image values 0 there
               const int y = y0 + lane - 1;  // row y of the cell
               const float v = lane <= nr && y >= 0 ? img[y * P] : 0.f;
@@ -605,29 +607,29 @@ __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(Sep
                 drx = fmaf(fmaf(static_cast<float>(-1 - rox), LS, LT), v, drx);
               }
               if (lane < nr || (lane == nr && y0 + nr == P)) {
-                const float D = below - v, p = LT0 * D;
+                const float D = below - v, p = (LT0 + LT1) * D;
                 uy = p;
                 ury = fmaf(static_cast<float>(lane), p, LT1 * D);
               }
             }
             float* gq = gimg + y0 * P + x;
-            float vp = vi[0], dp = ri[0] - vi[0];
+            float vp = vi[0], rp = ri[0];
             auto at = [](const float2(&a)[kSepPairs], int i) { return i & 1 ? a[i / 2].y : a[i / 2].x; };
             auto row = [&](int i) {
-              const float v = vi[i + 1], d = ri[i + 1] - v;
-              const float SG = (at(S0, i + 1) - at(S1, i + 1)) + at(S1, i);
-              const float TG = (at(T0, i + 1) - at(T1, i + 1)) + at(T1, i);
+              const float v = vi[i + 1], r = ri[i + 1], d = r - v;
+              const float SG = at(S0, i + 1) + at(S1, i);
+              const float TG = at(T0, i + 1) + at(T1, i);
               const float tl = __shfl_up_sync(0xffffffffu, TG, 1), t0l = __shfl_sync(0xffffffffu, LT, i + 1);
-              if (in) gq[i * P] = (SG - TG) + (lane == 0 ? t0l : tl);
-              ux = fmaf(SG, d, ux);
+              if (in) gq[i * P] = SG + (lane == 0 ? t0l : tl);
+              ux = fmaf(SG + TG, d, ux);
               urx = fmaf(TG, d, urx);
-              const float Dv = v - vp, Dd = d - dp;  // cell y - 1
-              const float p = fmaf(at(T0, i), Dd, at(S0, i) * Dv);
+              const float Dv = v - vp, Dr = r - rp;  // cell y - 1, at x and x + 1
+              const float p = fmaf(at(T0, i) + at(T1, i), Dr, (at(S0, i) + at(S1, i)) * Dv);
               uy += p;
               ury = fmaf(at(S1, i), Dv, fmaf(static_cast<float>(i), p, ury));
-              ury = fmaf(at(T1, i), Dd, ury);
+              ury = fmaf(at(T1, i), Dr, ury);
               vp = v;
-              dp = d;
+              rp = r;
             };
             if (nr == kSepBand && y0 + nr < P) {
 #pragma unroll
@@ -638,10 +640,10 @@ __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(Sep
                 if (i < nr) {
                   row(i);
                   if (i + 1 == nr && y0 + nr == P) {  // the last cell's lower row lies outside the image
-                    const float p = fmaf(at(T0, i + 1), -dp, at(S0, i + 1) * -vp);
+                    const float p = fmaf(at(T0, i + 1) + at(T1, i + 1), -rp, (at(S0, i + 1) + at(S1, i + 1)) * -vp);
                     uy += p;
                     ury = fmaf(at(S1, i + 1), -vp, fmaf(static_cast<float>(i + 1), p, ury));
-                    ury = fmaf(at(T1, i + 1), -dp, ury);
+                    ury = fmaf(at(T1, i + 1), -rp, ury);
                   }
                 }
             }
