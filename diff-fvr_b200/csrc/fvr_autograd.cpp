@@ -454,6 +454,27 @@ at::Tensor sncc_loss(const at::Tensor& poses, const SnccCall& call) {
 
 }  // namespace
 
+// What tells tensors apart that a preparation may be kept for: addresses, shapes,
+// strides and types; and their versions, which a write in place advances
+// (inference tensors have none).
+std::pair<pybind11::bytes, pybind11::bytes> tensor_keys(const std::vector<at::Tensor>& tensors) {
+  std::vector<int64_t> key, versions;
+  key.reserve(8 * tensors.size());
+  versions.reserve(tensors.size());
+  for (const at::Tensor& t : tensors) {
+    key.push_back(reinterpret_cast<intptr_t>(t.const_data_ptr()));
+    key.push_back(static_cast<int64_t>(t.scalar_type()));
+    key.push_back(t.dim());
+    for (int64_t n : t.sizes()) key.push_back(n);
+    for (int64_t n : t.strides()) key.push_back(n);
+    versions.push_back(t.is_inference() ? 0 : static_cast<int64_t>(t._version()));
+  }
+  auto bytes = [](const std::vector<int64_t>& v) {
+    return pybind11::bytes(reinterpret_cast<const char*>(v.data()), v.size() * sizeof(int64_t));
+  };
+  return {bytes(key), bytes(versions)};
+}
+
 void bind(const std::map<std::string, int64_t>& a, int64_t geo_stride, int64_t reg_stats) {
   auto set = [&](auto& f, const char* name) {
     const auto it = a.find(name);
@@ -525,6 +546,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         k->tw = std::move(tw);
         return k;
       }));
+  m.def("tensor_keys", torch::wrap_pybind_function(tensor_keys), "(identity, versions) of the tensors, as bytes");
   m.def("set_error_type", [](py::object type) { error_type = type.release().ptr(); },
         "the exception raised for a library status");
   // wrapped: torch's own exceptions (out of memory among them) and ours arrive as their Python types

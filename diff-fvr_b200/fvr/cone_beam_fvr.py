@@ -214,12 +214,8 @@ def _prepared_lattice(lattice, device):
     (the tensors' versions; inference tensors have none).  The entry holds the
     lattice's own tensors, so their storage cannot be freed and reused by
     another lattice while the entry exists."""
-    key, versions = [device], []
-    for i in _LATTICE_USED:
-        t = lattice[i]
-        key += (t.data_ptr(), t.shape, t.stride(), t.dtype)
-        versions.append(0 if t.is_inference() else t._version)
-    key = tuple(key)
+    key, versions = NA.tensor_keys([lattice[i] for i in _LATTICE_USED])
+    key = (key, device)
     hit = _LATTICE_CACHE.get(key)
     if hit is None or hit[0] != versions:
         if len(_LATTICE_CACHE) > 64:

@@ -22,10 +22,14 @@ def _view(lattice, f):
 VIEWS = {"coarse": lambda t: t[::2, ::2], "crop": lambda t: t[:5, :7], "rows": lambda t: t[:6]}
 
 
+@pytest.mark.parametrize("native", [True, False])
 @pytest.mark.parametrize("name", VIEWS)
-def test_views_of_a_lattice_are_their_own(name):
+def test_views_of_a_lattice_are_their_own(name, native, monkeypatch):
+    import fvr._native as NA
     from fvr.cone_beam_fvr import _prepared_lattice
 
+    if not native:
+        monkeypatch.setattr(NA, "_MOD", None)
     lat = _lattice(12, 16)
     dev = torch.device("cpu")
     full = _prepared_lattice(lat, dev)
@@ -38,9 +42,13 @@ def test_views_of_a_lattice_are_their_own(name):
     assert _prepared_lattice(lat, dev) is full and _prepared_lattice(sub, dev) is got
 
 
-def test_a_written_lattice_is_prepared_again():
+@pytest.mark.parametrize("native", [True, False])
+def test_a_written_lattice_is_prepared_again(native, monkeypatch):
+    import fvr._native as NA
     from fvr.cone_beam_fvr import _prepared_lattice
 
+    if not native:
+        monkeypatch.setattr(NA, "_MOD", None)
     lat = _lattice(12, 16)
     dev = torch.device("cpu")
     first = _prepared_lattice(lat, dev)
