@@ -47,8 +47,8 @@ namespace {
 struct Api {
   decltype(&fvr_status_string) status = nullptr;
   decltype(&fvr_pou_pinhole_forward) pinhole_forward = nullptr;
-  decltype(&fvr_pou_pinhole_backward) pinhole_backward = nullptr;
-  decltype(&fvr_pou_pinhole_backward_workspace) pinhole_backward_workspace = nullptr;
+  decltype(&fvr_pou_pinhole_backward_chunked) pinhole_backward = nullptr;
+  decltype(&fvr_pou_pinhole_backward_chunked_workspace) pinhole_backward_workspace = nullptr;
   decltype(&fvr_pou_rays_forward) rays_forward = nullptr;
   decltype(&fvr_pou_rays_backward) rays_backward = nullptr;
   decltype(&fvr_pou_rays_backward_workspace) rays_backward_workspace = nullptr;
@@ -131,7 +131,8 @@ using LatticePtr = c10::intrusive_ptr<PouLattice>;
 
 class Pinhole : public torch::autograd::Function<Pinhole> {
  public:
-  static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& mats, ModelPtr m, LatticePtr l) {
+  static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& mats, ModelPtr m, LatticePtr l,
+                            int64_t chunk) {
     const at::Device d = m->device();
     c10::cuda::CUDAGuard guard(d);
     const at::Tensor x = as(mats, d, at::kFloat);
@@ -151,13 +152,14 @@ class Pinhole : public torch::autograd::Function<Pinhole> {
     ctx->save_for_backward({geo, offs, imgs, l->ic.is_inference() ? at::Tensor() : l->ic});
     ctx->saved_data["model"] = keep(m);
     ctx->saved_data["lattice"] = keep(l);
+    ctx->saved_data["chunk"] = chunk;  // poses whose image gradients are held at a time
     ctx->saved_data["type"] = static_cast<int64_t>(mats.scalar_type());
     return out;
   }
 
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
                                                  torch::autograd::variable_list go) {
-    if (!go[0].defined()) return {at::Tensor(), at::Tensor(), at::Tensor()};
+    if (!go[0].defined()) return {at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
     const auto saved = ctx->get_saved_variables();
     const at::Tensor &geo = saved[0], &offs = saved[1], &imgs = saved[2];
     const ModelPtr m = kept<PouModel>(ctx->saved_data["model"]);
@@ -165,17 +167,19 @@ class Pinhole : public torch::autograd::Function<Pinhole> {
     const at::Tensor& ic = saved[3].defined() ? saved[3] : l->ic;
     const at::Device d = m->device();
     c10::cuda::CUDAGuard guard(d);
-    const int64_t N = geo.size(0), ws_bytes = api.pinhole_backward_workspace(m->B, N, l->H, l->W);
+    const int64_t N = geo.size(0), chunk = std::min(N, ctx->saved_data["chunk"].toInt());
+    const int64_t ws_bytes = api.pinhole_backward_workspace(m->B, N, l->H, l->W, chunk);
     const at::Tensor g = as(go[0], d, at::kFloat);
-    at::Tensor ws = at::empty({ws_bytes}, on(d, at::kByte)), gimgs = at::empty_like(imgs);
+    at::Tensor ws = at::empty({ws_bytes}, on(d, at::kByte));
+    at::Tensor gimgs = at::empty({m->B, chunk, m->P, m->P}, on(d, at::kFloat));
     at::Tensor grad = at::empty({N, 4, 4}, on(d, at::kFloat));
     check(api.pinhole_backward(m->dtype, m->stencil.data_ptr(), fptr(m->scales), m->B, m->P, geo.data_ptr<double>(),
                                offs.data_ptr<double>(), N, l->base.data(), m->vscale(), fptr(m->centers),
                                fptr(m->freqs), fptr(imgs), fptr(l->rxc), fptr(l->ryr), fptr(ic), l->H, l->W,
-                               1.0 / m->ds, m->c(), fptr(g), gimgs.data_ptr<float>(), ws.data_ptr(), ws_bytes,
+                               1.0 / m->ds, m->c(), fptr(g), chunk, gimgs.data_ptr<float>(), ws.data_ptr(), ws_bytes,
                                grad.data_ptr<float>(), current_stream(d.index())),
-          "fvr_pou_pinhole_backward");
-    return {to_type(grad, ctx->saved_data["type"].toInt()), at::Tensor(), at::Tensor()};
+          "fvr_pou_pinhole_backward_chunked");
+    return {to_type(grad, ctx->saved_data["type"].toInt()), at::Tensor(), at::Tensor(), at::Tensor()};
   }
 };
 
@@ -483,8 +487,8 @@ void bind(const std::map<std::string, int64_t>& a, int64_t geo_stride, int64_t r
   };
   set(api.status, "fvr_status_string");
   set(api.pinhole_forward, "fvr_pou_pinhole_forward");
-  set(api.pinhole_backward, "fvr_pou_pinhole_backward");
-  set(api.pinhole_backward_workspace, "fvr_pou_pinhole_backward_workspace");
+  set(api.pinhole_backward, "fvr_pou_pinhole_backward_chunked");
+  set(api.pinhole_backward_workspace, "fvr_pou_pinhole_backward_chunked_workspace");
   set(api.rays_forward, "fvr_pou_rays_forward");
   set(api.rays_backward, "fvr_pou_rays_backward");
   set(api.rays_backward_workspace, "fvr_pou_rays_backward_workspace");
@@ -550,8 +554,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("set_error_type", [](py::object type) { error_type = type.release().ptr(); },
         "the exception raised for a library status");
   // wrapped: torch's own exceptions (out of memory among them) and ours arrive as their Python types
-  m.def("pinhole", torch::wrap_pybind_function(
-                       [](const at::Tensor& mats, ModelPtr k, LatticePtr l) { return Pinhole::apply(mats, k, l); }));
+  m.def("pinhole", torch::wrap_pybind_function([](const at::Tensor& mats, ModelPtr k, LatticePtr l, int64_t chunk) {
+          return Pinhole::apply(mats, k, l, chunk);
+        }));
   m.def("lattice_rays", torch::wrap_pybind_function([](const at::Tensor& srcs, const at::Tensor& trg, ModelPtr k) {
           return LatticeRays::apply(srcs, trg, k);
         }));

@@ -322,8 +322,8 @@ __host__ __device__ constexpr int64_t sep_adj_smem(int P, int Hd, int W) {
 
 struct SepGrad {
   const float* gout;  // [N][Hd W]
-  const float4* gic;  // [N][Hd][Wp / 4]: gout ic, rows padded with zeros
-  float* gimgs;       // [B][N][P][P]
+  const float4* gic;  // [poses of this launch][Hd][Wp / 4]: gout ic, rows padded with zeros
+  float* gimgs;       // [B][poses of this launch][P][P]
   double* goffs;      // [3][B][N]: dL/d(d_b, cu, cv)
 };
 
@@ -361,7 +361,8 @@ __global__ void __launch_bounds__(256) pou_warp_sep_weigh_kernel(const float* __
   gic[static_cast<int64_t>(blockIdx.y) * quads + q] = v;
 }
 
-// One CTA per (pose, block).  A detector pixel lies in one cell of the block
+// One CTA per (pose, block) of a range of poses (the pointers are those of its
+// first pose, a.N is the pose count of the whole arrays).  A detector pixel lies in one cell of the block
 // image, [x, x + 1) x [y, y + 1), at fractions (tx, ty); everything the adjoint
 // needs of the pixels is four sums per cell, of g ic times the weights of the
 // cell's four corners (each weight by itself: 1 - tx taken from sums of 1 and tx
@@ -424,7 +425,7 @@ __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(Sep
     c1 = rev_c ? W - f0 : f1;
   };
   const float* img = a.imgs + bn * P * P;
-  float* gimg = w.gimgs + bn * P * P;
+  float* gimg = w.gimgs + (static_cast<int64_t>(b) * gridDim.x + n) * P * P;
   const float* gout = w.gout + static_cast<int64_t>(n) * Hd * W;
   // image rows that any detector row reaches: cells -1 .. P - 1 give rows cell, cell + 1
   int ya = P, yb = P;
@@ -712,14 +713,14 @@ static int sep_args(const float* imgs, int64_t B, int64_t N, int64_t P, const do
 }
 
 template <int THREADS, int MINB>
-static int sep_adjoint(const SepArgs& a, const SepGrad& w, cudaStream_t s) {
+static int sep_adjoint(const SepArgs& a, const SepGrad& w, int64_t poses, cudaStream_t s) {
   const int64_t smem = sep_adj_smem(a.P, a.Hd, a.W);
   // the shared-memory opt-in is a per-device setting: made before every launch
   if (cudaFuncSetAttribute(pou_warp_sep_adjoint_kernel<THREADS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(smem)) != cudaSuccess)
     return FVR_ERR_CUDA;
   pou_warp_sep_adjoint_kernel<THREADS, MINB>
-      <<<dim3(static_cast<unsigned>(a.N), static_cast<unsigned>(a.B)), THREADS, smem, s>>>(a, w);
+      <<<dim3(static_cast<unsigned>(poses), static_cast<unsigned>(a.B)), THREADS, smem, s>>>(a, w);
   FVR_LAUNCH_CHECK();
   return FVR_OK;
 }
@@ -781,27 +782,39 @@ int64_t fvr_pou_warp_sep_adjoint_workspace(int64_t N, int64_t H, int64_t W) {
   return N < 1 || H < 1 || W < 1 ? 0 : 4 * N * H * ((W + 3) / 4 * 4);
 }
 
-int fvr_pou_warp_sep_adjoint(const float* imgs, int64_t B, int64_t N, int64_t P, const double* offs, const float* rxc,
-                             const float* ryr, const float* ic, int64_t H, int64_t W, double inv_ds, double c_idx,
-                             const float* gout, void* workspace, int64_t ws_bytes, float* grad_imgs, double* goffs,
-                             void* stream) {
+int fvr_pou_warp_sep_adjoint_poses(const float* imgs, int64_t B, int64_t N, int64_t P, const double* offs,
+                                   const float* rxc, const float* ryr, const float* ic, int64_t H, int64_t W,
+                                   double inv_ds, double c_idx, const float* gout, int64_t n0, int64_t count,
+                                   void* workspace, int64_t ws_bytes, float* grad_imgs, double* goffs, void* stream) {
   SepArgs a;
   const int rc = sep_args(imgs, B, N, P, offs, rxc, ryr, ic, H, W, inv_ds, c_idx, &a);
   if (rc) return rc;
   if (!gout || !grad_imgs || !goffs || !workspace || (reinterpret_cast<uintptr_t>(workspace) & 15)) return FVR_ERR_ARG;
-  if (ws_bytes < fvr_pou_warp_sep_adjoint_workspace(N, H, W)) return FVR_ERR_WORKSPACE;
+  if (n0 < 0 || count < 1 || count > N - n0) return FVR_ERR_ARG;
+  if (ws_bytes < fvr_pou_warp_sep_adjoint_workspace(count, H, W)) return FVR_ERR_WORKSPACE;
   if (!fvr_pou_warp_sep_adjoint_supported(P, H, W)) return FVR_ERR_UNSUPPORTED;
+  a.imgs += n0 * P * P;
+  a.offs += 3 * n0;
+  gout += n0 * H * W;
   float4* gic = static_cast<float4*>(workspace);
-  const SepGrad w{gout, gic, grad_imgs, goffs};
+  const SepGrad w{gout, gic, grad_imgs, goffs + n0};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int Wp = sep_padded((int)W);
   const bool vec = W % 4 == 0 && ((reinterpret_cast<uintptr_t>(gout) | reinterpret_cast<uintptr_t>(ic)) & 15) == 0;
-  pou_warp_sep_weigh_kernel<<<dim3((unsigned)cdiv64(H * (Wp / 4), 256), (unsigned)N), 256, 0, s>>>(
+  pou_warp_sep_weigh_kernel<<<dim3((unsigned)cdiv64(H * (Wp / 4), 256), (unsigned)count), 256, 0, s>>>(
       gout, ic, (int)H, (int)W, Wp, vec, gic);
   FVR_LAUNCH_CHECK();
   // 256 threads once two CTAs per SM can run, else all 16 warps on one (pose, block)
-  if (B * N >= 296) return sep_adjoint<256, 2>(a, w, s);
-  return sep_adjoint<512, 1>(a, w, s);
+  if (B * count >= 296) return sep_adjoint<256, 2>(a, w, count, s);
+  return sep_adjoint<512, 1>(a, w, count, s);
+}
+
+int fvr_pou_warp_sep_adjoint(const float* imgs, int64_t B, int64_t N, int64_t P, const double* offs, const float* rxc,
+                             const float* ryr, const float* ic, int64_t H, int64_t W, double inv_ds, double c_idx,
+                             const float* gout, void* workspace, int64_t ws_bytes, float* grad_imgs, double* goffs,
+                             void* stream) {
+  return fvr_pou_warp_sep_adjoint_poses(imgs, B, N, P, offs, rxc, ryr, ic, H, W, inv_ds, c_idx, gout, 0, N, workspace,
+                                        ws_bytes, grad_imgs, goffs, stream);
 }
 
 int fvr_pou_pinhole_supported(int64_t P, int64_t H, int64_t W) {
@@ -821,14 +834,51 @@ int fvr_pou_pinhole_forward(int dtype, const void* stencil, const float* scales,
   return rc;
 }
 
-// Workspace of the backward: weighed detector gradient | offset gradients |
-// slice-adjoint records, each on a 256-byte boundary.
+// Workspace of the backward: weighed detector gradient of a chunk | offset
+// gradients | slice-adjoint records, each on a 256-byte boundary.
 static int64_t pinhole_round(int64_t bytes) { return (bytes + 255) / 256 * 256; }
 
-int64_t fvr_pou_pinhole_backward_workspace(int64_t B, int64_t N, int64_t H, int64_t W) {
-  if (B < 1 || N < 1) return 0;
-  return pinhole_round(fvr_pou_warp_sep_adjoint_workspace(N, H, W)) + pinhole_round(24 * B * N) +
+int64_t fvr_pou_pinhole_backward_chunked_workspace(int64_t B, int64_t N, int64_t H, int64_t W, int64_t chunk) {
+  if (B < 1 || N < 1 || chunk < 1) return 0;
+  return pinhole_round(fvr_pou_warp_sep_adjoint_workspace(chunk < N ? chunk : N, H, W)) + pinhole_round(24 * B * N) +
          fvr_pou_slice_image_adjoint_workspace(B, N);
+}
+
+int64_t fvr_pou_pinhole_backward_workspace(int64_t B, int64_t N, int64_t H, int64_t W) {
+  return fvr_pou_pinhole_backward_chunked_workspace(B, N, H, W, N);
+}
+
+// Poses are independent up to the pose gradients at the end: dL/dimgs is formed
+// and reduced for `chunk` of them at a time.
+int fvr_pou_pinhole_backward_chunked(int dtype, const void* stencil, const float* scales, int64_t B, int64_t P,
+                                     const double* geo, const double* offs, int64_t N, const double* base12,
+                                     double vscale, const float* centers, const float* freqs, const float* imgs,
+                                     const float* rxc, const float* ryr, const float* ic, int64_t H, int64_t W,
+                                     double inv_ds, double c_idx, const float* gout, int64_t chunk, float* grad_imgs,
+                                     void* workspace, int64_t ws_bytes, float* gmats, void* stream) {
+  if (!workspace || !grad_imgs || (reinterpret_cast<uintptr_t>(workspace) & 15) || !gmats || !offs || !geo || N < 1 ||
+      chunk < 1)
+    return FVR_ERR_ARG;
+  if (!fvr_pou_pinhole_supported(P, H, W) || !fvr_pou_warp_sep_adjoint_supported(P, H, W)) return FVR_ERR_UNSUPPORTED;
+  if (ws_bytes < fvr_pou_pinhole_backward_chunked_workspace(B, N, H, W, chunk)) return FVR_ERR_WORKSPACE;
+  if (chunk > N) chunk = N;
+  const int64_t gic_bytes = fvr_pou_warp_sep_adjoint_workspace(chunk, H, W);
+  char* w = static_cast<char*>(workspace);
+  double* goffs = reinterpret_cast<double*>(w + pinhole_round(gic_bytes));
+  double* part = reinterpret_cast<double*>(reinterpret_cast<char*>(goffs) + pinhole_round(24 * B * N));
+  int rc = FVR_OK;
+  for (int64_t n0 = 0; n0 < N && !rc; n0 += chunk) {
+    const int64_t count = chunk < N - n0 ? chunk : N - n0;
+    rc = fvr_pou_warp_sep_adjoint_poses(imgs, B, N, P, offs, rxc, ryr, ic, H, W, inv_ds, c_idx, gout, n0, count,
+                                        workspace, gic_bytes, grad_imgs, goffs, stream);
+    if (!rc)  // records [pose][block][6]
+      rc = fvr_pou_slice_image_adjoint(dtype, stencil, scales, B, P, geo + n0 * fvr_pou_geo_stride(), count, freqs,
+                                       grad_imgs, part + 6 * B * n0, fvr_pou_slice_image_adjoint_workspace(B, count),
+                                       stream);
+  }
+  if (!rc)
+    rc = fvr_pou_pose_backward(part, 1, goffs, nullptr, 0, geo, centers, B, N, base12, vscale, gmats, nullptr, stream);
+  return rc;
 }
 
 int fvr_pou_pinhole_backward(int dtype, const void* stencil, const float* scales, int64_t B, int64_t P,
@@ -837,21 +887,9 @@ int fvr_pou_pinhole_backward(int dtype, const void* stencil, const float* scales
                              const float* ryr, const float* ic, int64_t H, int64_t W, double inv_ds, double c_idx,
                              const float* gout, float* grad_imgs, void* workspace, int64_t ws_bytes, float* gmats,
                              void* stream) {
-  if (!workspace || !grad_imgs || (reinterpret_cast<uintptr_t>(workspace) & 15) || !gmats || !offs) return FVR_ERR_ARG;
-  if (!fvr_pou_pinhole_supported(P, H, W) || !fvr_pou_warp_sep_adjoint_supported(P, H, W)) return FVR_ERR_UNSUPPORTED;
-  if (ws_bytes < fvr_pou_pinhole_backward_workspace(B, N, H, W)) return FVR_ERR_WORKSPACE;
-  const int64_t gic_bytes = fvr_pou_warp_sep_adjoint_workspace(N, H, W);
-  const int64_t part_bytes = fvr_pou_slice_image_adjoint_workspace(B, N);
-  char* w = static_cast<char*>(workspace);
-  double* goffs = reinterpret_cast<double*>(w + pinhole_round(gic_bytes));
-  double* part = reinterpret_cast<double*>(reinterpret_cast<char*>(goffs) + pinhole_round(24 * B * N));
-  int rc = fvr_pou_warp_sep_adjoint(imgs, B, N, P, offs, rxc, ryr, ic, H, W, inv_ds, c_idx, gout, workspace, gic_bytes,
-                                    grad_imgs, goffs, stream);
-  if (!rc)
-    rc = fvr_pou_slice_image_adjoint(dtype, stencil, scales, B, P, geo, N, freqs, grad_imgs, part, part_bytes, stream);
-  if (!rc)
-    rc = fvr_pou_pose_backward(part, 1, goffs, nullptr, 0, geo, centers, B, N, base12, vscale, gmats, nullptr, stream);
-  return rc;
+  return fvr_pou_pinhole_backward_chunked(dtype, stencil, scales, B, P, geo, offs, N, base12, vscale, centers, freqs,
+                                          imgs, rxc, ryr, ic, H, W, inv_ds, c_idx, gout, N, grad_imgs, workspace,
+                                          ws_bytes, gmats, stream);
 }
 
 }  // extern "C"

@@ -105,6 +105,8 @@ SIGNATURES = {
     "fvr_pou_warp_sep_adjoint_supported": (I32, [I64, I64, I64]),
     "fvr_pou_warp_sep_adjoint_workspace": (I64, [I64, I64, I64]),
     "fvr_pou_warp_sep_adjoint": (I32, [P, I64, I64, I64, P, P, P, P, I64, I64, F64, F64, P, P, I64, P, P, P]),
+    "fvr_pou_warp_sep_adjoint_poses": (I32, [P, I64, I64, I64, P, P, P, P, I64, I64, F64, F64, P, I64, I64, P, I64, P,
+                                             P, P]),
     "fvr_pou_rays_forward": (I32, [I32, P, P, I64, I64, P, P, I64, I64, I64, F64, P, P, F64, F64, P, P, P, P, P, P]),
     "fvr_pou_rays_backward_workspace": (I64, [I64, I64, I64, I64]),
     "fvr_pou_rays_backward": (I32, [I32, P, P, I64, I64, P, I64, I64, I64, F64, P, P, F64, F64, P, P, P, P, P, P, P,
@@ -115,6 +117,9 @@ SIGNATURES = {
     "fvr_pou_pinhole_backward_workspace": (I64, [I64, I64, I64, I64]),
     "fvr_pou_pinhole_backward": (I32, [I32, P, P, I64, I64, P, P, I64, P, F64, P, P, P, P, P, P, I64, I64, F64, F64, P,
                                        P, P, I64, P, P]),
+    "fvr_pou_pinhole_backward_chunked_workspace": (I64, [I64, I64, I64, I64, I64]),
+    "fvr_pou_pinhole_backward_chunked": (I32, [I32, P, P, I64, I64, P, P, I64, P, F64, P, P, P, P, P, P, I64, I64, F64,
+                                               F64, P, I64, P, P, I64, P, P]),
     "fvr_pou_warp": (I32, [P, I64, I64, I64, P, P, P, I32, I64, P, P, P, I64, I64, F64, F64, P, P]),
     "fvr_pou_warp_bwd_workspace": (I64, [I64, I64, I64]),
     "fvr_pou_warp_bwd": (I32, [P, I64, I64, I64, P, P, P, I32, I64, P, P, P, I64, I64, F64, F64, P, P, P, P, P, I64,
@@ -181,10 +186,12 @@ KERNELS_PER_CALL = {
     "fvr_cncc_image": 2,
     "fvr_pou_warp_bwd": 2,
     "fvr_pou_warp_sep_adjoint": 2,
+    "fvr_pou_warp_sep_adjoint_poses": 2,
     "fvr_pou_pinhole_forward": 3,
     "fvr_pou_rays_forward": 5,
     "fvr_pou_rays_backward": 6,
     "fvr_pou_pinhole_backward": 4,
+    "fvr_pou_pinhole_backward_chunked": 4,  # and three more for each further chunk
     "fvr_np_ncc_moments": 2,
     "fvr_np_pair_moments": 2,
     "fvr_edge_ncc_forward": 2,

@@ -22,8 +22,8 @@ except ImportError:
 if hasattr(_MOD, "set_error_type"):
     _MOD.set_error_type(L.FvrError)
 
-_ENTRIES = ("fvr_status_string", "fvr_pou_pinhole_forward", "fvr_pou_pinhole_backward",
-            "fvr_pou_pinhole_backward_workspace", "fvr_pou_rays_forward", "fvr_pou_rays_backward",
+_ENTRIES = ("fvr_status_string", "fvr_pou_pinhole_forward", "fvr_pou_pinhole_backward_chunked",
+            "fvr_pou_pinhole_backward_chunked_workspace", "fvr_pou_rays_forward", "fvr_pou_rays_backward",
             "fvr_pou_rays_backward_workspace", "fvr_tc_image", "fvr_tc_image_backward", "fvr_cncc_image",
             "fvr_cncc_image_workspace", "fvr_reg_loss_forward", "fvr_reg_loss_backward", "fvr_reg_loss_workspace")
 _bound = None  # the loaded library the binding's addresses belong to

@@ -197,10 +197,9 @@ def _separable_rays(rx, ry):
 
 
 # The separable warp adjoint hands dL/dimgs to the block-image adjoint in a
-# [blocks, poses, P, P] buffer.  Beyond this size the one-launch adjoint runs
-# instead where it can: it keeps that gradient in shared memory (64 blocks x 64
-# poses x 128^2 is 268 MB: 1.23 against 1.42 ms).
-_GRAD_IMAGE_BYTES = 4 << 30
+# [blocks, poses, P, P] buffer of at most this size: more poses go in chunks.
+# 64 blocks x 64 poses x 128^2 just fill it.
+_GRAD_IMAGE_BYTES = 256 << 20
 
 
 def _prepared_lattice(lattice, device):
@@ -281,10 +280,17 @@ def _block_images_adjoint(model, geo, N, grad_imgs, s):
     return ws, (P * P + 255) // 256
 
 
-def _gather_adjoint(model, monotone, N, H, W):
-    """Whether the backward of N poses takes the separable warp adjoint."""
-    return (monotone and model.fused_warp_adjoint and 4 * model.B * N * model.P * model.P <= _GRAD_IMAGE_BYTES
+def _gather_adjoint(model, monotone, H, W):
+    """Whether the backward takes the separable warp adjoint."""
+    return (monotone and model.fused_warp_adjoint
             and bool(L.query("fvr_pou_warp_sep_adjoint_supported", model.P, H, W)))
+
+
+def _pose_chunk(model, N):
+    """Poses of a backward of N whose image gradients are held at a time: as few
+    chunks as _GRAD_IMAGE_BYTES allows, of like size."""
+    most = max(1, _GRAD_IMAGE_BYTES // (4 * model.B * model.P * model.P))
+    return -(-N // -(-N // most))
 
 
 class _PinholeFn(torch.autograd.Function):
@@ -336,29 +342,34 @@ class _PinholeFn(torch.autograd.Function):
         H, W = int(rx.shape[0]), int(rx.shape[1])
         s = L.stream_ptr(dev)
         g = g_out.detach().to(device=dev, dtype=torch.float32).contiguous()
-        gather = _gather_adjoint(model, monotone, N, H, W)
+        gather, chunk = _gather_adjoint(model, monotone, H, W), _pose_chunk(model, N)
         if gather and not profiling.active() and L.query("fvr_pou_image_supported", P):
             st = model._stencil
-            wsb = L.query("fvr_pou_pinhole_backward_workspace", B, N, H, W)
+            wsb = L.query("fvr_pou_pinhole_backward_chunked_workspace", B, N, H, W, chunk)
             ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
-            grad_imgs = torch.empty_like(imgs)  # of the block images' size: the allocator reuses their blocks
+            grad_imgs = torch.empty((B, chunk, P, P), dtype=torch.float32, device=dev)
             gm = torch.empty((N, 4, 4), dtype=torch.float32, device=dev)
-            L.call("fvr_pou_pinhole_backward", st.code, L.ptr(st.data), L.ptr(st.scales), B, P, L.ptr(geo),
+            L.call("fvr_pou_pinhole_backward_chunked", st.code, L.ptr(st.data), L.ptr(st.scales), B, P, L.ptr(geo),
                    L.ptr(offs), N, base, float(P) * model.ds_block, L.ptr(model.centers), L.ptr(model._freqs),
                    L.ptr(imgs), L.ptr(sep[0]), L.ptr(sep[1]), L.ptr(ic), H, W, 1.0 / model.ds_block, float(P // 2),
-                   L.ptr(g), L.ptr(grad_imgs), L.ptr(ws), wsb, L.ptr(gm), s)
+                   L.ptr(g), chunk, L.ptr(grad_imgs), L.ptr(ws), wsb, L.ptr(gm), s)
             return gm.to(mdt), None, None
         goffs = torch.empty((3, B, N), dtype=torch.float64, device=dev)
         if gather:
-            grad_imgs = torch.empty((B, N, P, P), dtype=torch.float32, device=dev)
-            wsb = L.query("fvr_pou_warp_sep_adjoint_workspace", N, H, W)
+            wsb = L.query("fvr_pou_warp_sep_adjoint_workspace", chunk, H, W)
             ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
-            with profiling.section("pou_warp_bwd"):
-                L.call("fvr_pou_warp_sep_adjoint", L.ptr(imgs), B, N, P, L.ptr(offs), L.ptr(sep[0]), L.ptr(sep[1]),
-                       L.ptr(ic), H, W, 1.0 / model.ds_block, float(P // 2), L.ptr(g), L.ptr(ws), wsb,
-                       L.ptr(grad_imgs), L.ptr(goffs), s)
-            ws2, tiles = _block_images_adjoint(model, geo, N, grad_imgs, s)
-            del grad_imgs
+            records = []  # of the poses in order
+            for n0 in range(0, N, chunk):
+                n = min(chunk, N - n0)
+                grad_imgs = torch.empty((B, n, P, P), dtype=torch.float32, device=dev)
+                with profiling.section("pou_warp_bwd"):
+                    L.call("fvr_pou_warp_sep_adjoint_poses", L.ptr(imgs), B, N, P, L.ptr(offs), L.ptr(sep[0]),
+                           L.ptr(sep[1]), L.ptr(ic), H, W, 1.0 / model.ds_block, float(P // 2), L.ptr(g), n0, n,
+                           L.ptr(ws), wsb, L.ptr(grad_imgs), L.ptr(goffs), s)
+                part, tiles = _block_images_adjoint(model, geo[n0:n0 + n], n, grad_imgs, s)
+                records.append(part)
+                del grad_imgs
+            ws2 = records[0] if len(records) == 1 else torch.cat(records)
         elif (sep is not None and model.fused_warp_adjoint and g.data_ptr() % 16 == 0 and ic.data_ptr() % 16 == 0
               and L.query("fvr_pou_warp_image_adjoint_supported", P, H, W)):
             # warp adjoint + block-image adjoint in one launch: dL/dimgs stays in shared memory
@@ -612,9 +623,11 @@ class PerspectiveSlabFVR(nn.Module):
             grad = mats.requires_grad and torch.is_grad_enabled()
             if (native is not None and tables is not None and tuple(mats.shape[1:]) == (4, 4)
                     and L.query("fvr_pou_pinhole_supported", self.P, H, W)
-                    and (not grad or _gather_adjoint(self, monotone, int(mats.shape[0]), H, W))):
-                out = NA.call(native.pinhole, 7 if grad else 3, mats, self._native_plan(native),
-                              _lattice_plan(native, entry))
+                    and (not grad or _gather_adjoint(self, monotone, H, W))):
+                N = int(mats.shape[0])
+                chunk = _pose_chunk(self, N)
+                out = NA.call(native.pinhole, 3 + (1 + 3 * -(-N // chunk) if grad else 0), mats,
+                              self._native_plan(native), _lattice_plan(native, entry), chunk)
             else:
                 out = _PinholeFn.apply(mats, self, entry)
         else:

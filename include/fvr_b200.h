@@ -337,6 +337,13 @@ int fvr_pou_warp_sep_adjoint(const float* imgs, int64_t B, int64_t N, int64_t P,
                              const float* gout, void* workspace, int64_t ws_bytes, float* grad_imgs, double* goffs,
                              void* stream);
 int64_t fvr_pou_warp_sep_adjoint_workspace(int64_t N, int64_t H, int64_t W);
+/* The same for the poses n0 .. n0 + count - 1 alone: imgs, offs, gout and goffs
+ * are the whole arrays, grad_imgs[B][count][P][P] and the workspace (of count
+ * poses) are this range's. */
+int fvr_pou_warp_sep_adjoint_poses(const float* imgs, int64_t B, int64_t N, int64_t P, const double* offs,
+                                   const float* rxc, const float* ryr, const float* ic, int64_t H, int64_t W,
+                                   double inv_ds, double c_idx, const float* gout, int64_t n0, int64_t count,
+                                   void* workspace, int64_t ws_bytes, float* grad_imgs, double* goffs, void* stream);
 /* The explicit-ray step with the detector axes taken from the lattice
  * (cone_beam_fvr.py:423-478, 575-596), one call per direction: srcs[N][3],
  * trg[N][H][W][3] f32 -> out[N][H][W]; geo, offs, rays[3][N][H*W] and
@@ -372,6 +379,14 @@ int fvr_pou_pinhole_backward(int dtype, const void* stencil, const float* scales
                              const float* ryr, const float* ic, int64_t H, int64_t W, double inv_ds, double c_idx,
                              const float* gout, float* grad_imgs, void* workspace, int64_t ws_bytes, float* gmats,
                              void* stream);
+/* The same over at most `chunk` poses at a time: grad_imgs[B][min(chunk, N)][P][P]. */
+int64_t fvr_pou_pinhole_backward_chunked_workspace(int64_t B, int64_t N, int64_t H, int64_t W, int64_t chunk);
+int fvr_pou_pinhole_backward_chunked(int dtype, const void* stencil, const float* scales, int64_t B, int64_t P,
+                                     const double* geo, const double* offs, int64_t N, const double* base12,
+                                     double vscale, const float* centers, const float* freqs, const float* imgs,
+                                     const float* rxc, const float* ryr, const float* ic, int64_t H, int64_t W,
+                                     double inv_ds, double c_idx, const float* gout, int64_t chunk, float* grad_imgs,
+                                     void* workspace, int64_t ws_bytes, float* gmats, void* stream);
 /* Fused warp + block-image adjoint for a separable pinhole lattice (every
  * detector column shares one ray coordinate rxc[c], every row one ryr[r]):
  * from the detector gradient gout[N][H][W] (times ic[H][W]) and the forward
