@@ -362,7 +362,8 @@ __global__ void __launch_bounds__(256) pou_warp_sep_weigh_kernel(const float* __
 }
 
 // One CTA per (pose, block) of a range of poses (the pointers are those of its
-// first pose, a.N is the pose count of the whole arrays).  A detector pixel lies in one cell of the block
+// first pose, a.N is the pose count of the whole arrays; WHOLE: the range is all
+// of them, and one index serves both images, worth 10 us).  A detector pixel lies in one cell of the block
 // image, [x, x + 1) x [y, y + 1), at fractions (tx, ty); everything the adjoint
 // needs of the pixels is four sums per cell, of g ic times the weights of the
 // cell's four corners (each weight by itself: 1 - tx taken from sums of 1 and tx
@@ -384,7 +385,7 @@ __global__ void __launch_bounds__(256) pou_warp_sep_weigh_kernel(const float* __
 // interpolated at every detector column (two loads and nine operations per
 // image row and detector column); 8 blocks x 64 poses x 512^2 pixels: 138
 // against 265.
-template <int THREADS, int MINB>
+template <int THREADS, int MINB, bool WHOLE>
 __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(SepArgs a, SepGrad w) {
   constexpr int NW = THREADS / 32;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -425,7 +426,7 @@ __global__ void __launch_bounds__(THREADS, MINB) pou_warp_sep_adjoint_kernel(Sep
     c1 = rev_c ? W - f0 : f1;
   };
   const float* img = a.imgs + bn * P * P;
-  float* gimg = w.gimgs + (static_cast<int64_t>(b) * gridDim.x + n) * P * P;
+  float* gimg = w.gimgs + (WHOLE ? bn : static_cast<int64_t>(b) * gridDim.x + n) * P * P;
   const float* gout = w.gout + static_cast<int64_t>(n) * Hd * W;
   // image rows that any detector row reaches: cells -1 .. P - 1 give rows cell, cell + 1
   int ya = P, yb = P;
@@ -712,14 +713,14 @@ static int sep_args(const float* imgs, int64_t B, int64_t N, int64_t P, const do
   return FVR_OK;
 }
 
-template <int THREADS, int MINB>
+template <int THREADS, int MINB, bool WHOLE>
 static int sep_adjoint(const SepArgs& a, const SepGrad& w, int64_t poses, cudaStream_t s) {
   const int64_t smem = sep_adj_smem(a.P, a.Hd, a.W);
   // the shared-memory opt-in is a per-device setting: made before every launch
-  if (cudaFuncSetAttribute(pou_warp_sep_adjoint_kernel<THREADS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if (cudaFuncSetAttribute(pou_warp_sep_adjoint_kernel<THREADS, MINB, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(smem)) != cudaSuccess)
     return FVR_ERR_CUDA;
-  pou_warp_sep_adjoint_kernel<THREADS, MINB>
+  pou_warp_sep_adjoint_kernel<THREADS, MINB, WHOLE>
       <<<dim3(static_cast<unsigned>(poses), static_cast<unsigned>(a.B)), THREADS, smem, s>>>(a, w);
   FVR_LAUNCH_CHECK();
   return FVR_OK;
@@ -805,8 +806,9 @@ int fvr_pou_warp_sep_adjoint_poses(const float* imgs, int64_t B, int64_t N, int6
       gout, ic, (int)H, (int)W, Wp, vec, gic);
   FVR_LAUNCH_CHECK();
   // 256 threads once two CTAs per SM can run, else all 16 warps on one (pose, block)
-  if (B * count >= 296) return sep_adjoint<256, 2>(a, w, count, s);
-  return sep_adjoint<512, 1>(a, w, count, s);
+  if (B * count >= 296)
+    return count == N ? sep_adjoint<256, 2, true>(a, w, count, s) : sep_adjoint<256, 2, false>(a, w, count, s);
+  return count == N ? sep_adjoint<512, 1, true>(a, w, count, s) : sep_adjoint<512, 1, false>(a, w, count, s);
 }
 
 int fvr_pou_warp_sep_adjoint(const float* imgs, int64_t B, int64_t N, int64_t P, const double* offs, const float* rxc,
