@@ -24,6 +24,7 @@ __global__ void __launch_bounds__(256) copy_bytes_kernel(unsigned char* __restri
 #ifdef FVR_CHECK
 namespace fvr {
 int check_word_tc(unsigned long long* out, int clear);
+int check_word_image(unsigned long long* out, int clear);
 int check_word_pou(unsigned long long* out, int clear);
 int check_word_pou_sep(unsigned long long* out, int clear);
 int check_word_slice3d(unsigned long long* out, int clear);
@@ -41,8 +42,10 @@ int fvr_check_words(unsigned long long* out, int n, int clear) {
   if (!out || n < kUnits) return FVR_ERR_ARG;
   for (int i = 0; i < kUnits; ++i)
     if (readers[i](out + i, clear)) return FVR_ERR_CUDA;
-  unsigned long long sep = 0;  // the separable warp's word reports with the PoU family's
-  if (fvr::check_word_pou_sep(&sep, clear)) return FVR_ERR_CUDA;
+  // the whole-image kernels' word reports with the parallel-beam family's, the separable warp's with the PoU family's
+  unsigned long long image = 0, sep = 0;
+  if (fvr::check_word_image(&image, clear) || fvr::check_word_pou_sep(&sep, clear)) return FVR_ERR_CUDA;
+  if (out[0] == 0) out[0] = image;
   if (out[1] == 0) out[1] = sep;
   return FVR_OK;
 #else

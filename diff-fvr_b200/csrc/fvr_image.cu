@@ -698,3 +698,5 @@ int fvr_cncc_image(const float* pred, const float* target, int64_t B, int64_t Bt
 }
 
 }  // extern "C"
+
+FVR_CHECK_ACCESSOR(check_word_image)
