@@ -346,6 +346,12 @@ __global__ void pou_rays_axes_bwd_kernel(const float* __restrict__ trg, const do
   axis_backward(e, gu, ge[0]);
   for (int k = 0; k < 3; ++k) e[k] = static_cast<double>(trg[ov + k]) - static_cast<double>(trg[o0 + k]);
   axis_backward(e, gv, ge[1]);
+  // a lattice of one column or row: the axis' two points are one, and its shares (1e12 and more, the axis being a zero
+  // vector) cancel
+  for (int k = 0; k < 3; ++k) {
+    if (W == 1) ge[0][k] = 0.0;
+    if (H == 1) ge[1][k] = 0.0;
+  }
   for (int k = 0; k < 3; ++k) {
     gtrg[ou + k] = static_cast<float>(gtrg[ou + k] + ge[0][k]);
     gtrg[ov + k] = static_cast<float>(gtrg[ov + k] + ge[1][k]);

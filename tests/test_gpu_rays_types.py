@@ -46,3 +46,31 @@ def test_whole_number_points_stay_refused():
     src, trg = _points(3, 4, torch.float32)
     with pytest.raises(RuntimeError):
         m.project_rays_batched(src, trg.round().to(torch.int64))
+
+
+@pytest.mark.parametrize("H,W", [(1, 1), (1, 6), (5, 1)])
+def test_lattices_of_one_row_or_column(H, W):
+    """An axis without extent is a zero vector and gets no gradient; the other
+    axis and the rays keep theirs."""
+    from fvr.cone_beam_rays import project_rays_batched
+
+    m = _model()
+    src, trg = _points(H, W, torch.float32)
+    res = []
+    for given in (False, True):
+        s, t = src.clone().requires_grad_(True), trg.clone().requires_grad_(True)
+        if given:
+            u, v, n = (torch.zeros_like(s) for _ in range(3))
+            if W > 1:
+                u = t[:, 0, -1] - t[:, 0, 0]
+                u = u / (u.norm(dim=-1, keepdim=True) + 1e-12)
+            if H > 1:
+                v = t[:, -1, 0] - t[:, 0, 0]
+                v = v / (v.norm(dim=-1, keepdim=True) + 1e-12)
+            out = project_rays_batched(m, s, t, u, v, n.detach())
+        else:
+            out = m.project_rays_batched(s, t)
+        up = torch.linspace(0.5, 1.5, out.numel(), device="cuda").view(out.shape)
+        res.append((out.detach(), *torch.autograd.grad(out, (s, t), up)))
+    for a, b in zip(*res):
+        assert torch.allclose(a, b, rtol=1e-3, atol=1e-4 * float(b.abs().max()) + 1e-6)
