@@ -25,6 +25,7 @@ from __future__ import annotations
 from typing import Optional, Tuple, Union
 
 import ctypes
+import functools
 
 import numpy as np
 import torch
@@ -38,6 +39,13 @@ from . import autotune, profiling
 _NATIVE = NA._MOD  # native autograd binding (csrc/fvr_autograd.cpp, built next to the CUDA library), or None
 
 VIEW_AP, VIEW_LATERAL = 0, 1
+
+
+@functools.lru_cache(maxsize=256)
+def _whole_images(n0, n1):
+    """Whether images of this size are transformed whole in shared memory (asked up to four times a step)."""
+    return bool(L.query("fvr_image_supported", n0, n1))
+
 
 
 def _view_code(view: str) -> int:
@@ -330,7 +338,7 @@ class _ImageFn(torch.autograd.Function):
         s = L.stream_ptr(dev)
         kap = RT.kappa(R, eng.spacing[0])
         img = torch.empty((C, 1, R, R), dtype=torch.float32, device=dev)
-        whole = bool(L.query("fvr_image_supported", R, R))
+        whole = _whole_images(R, R)
         ctx.meta = (eng, view, R, kap, poses.dtype, whole)
         if whole:
             L.call("fvr_tc_image", *st.args(), L.ptr(p), C, view, L.ptr(RT.linspace(R, dev)), R, kap,
@@ -382,7 +390,7 @@ class _ImageSpectralNCCFn(torch.autograd.Function):
         x = pred.detach().float().contiguous()
         t = target.detach().to(device=dev, dtype=torch.float32).contiguous()
         loss = torch.empty((), dtype=torch.float32, device=dev)
-        whole = tuple(target.shape[-2:]) == (H, W) and bool(L.query("fvr_image_supported", H, W))
+        whole = tuple(target.shape[-2:]) == (H, W) and _whole_images(H, W)
         ctx.meta = (hp, B, Bt, H, W, pred.shape, pred.dtype, whole)
         if whole:
             grad = torch.empty(pred.shape, dtype=torch.float32, device=dev) if ctx.needs_input_grad[0] else None
@@ -533,7 +541,7 @@ class TorchDiffFVREngine(nn.Module):
             return torch.zeros((0, 1, R, R), dtype=torch.float32, device=self._dev) + 0.0 * p.sum()
         R = int(out_res)
         native = NA.module()
-        if native is not None and p.dim() == 2 and p.shape[1] == 6 and L.query("fvr_image_supported", R, R):
+        if native is not None and p.dim() == 2 and p.shape[1] == 6 and _whole_images(R, R):
             grad = p.requires_grad and torch.is_grad_enabled()
             return NA.call(native.image, 2 if grad else 1, p, self._image_plan(native, R), _view_code(view))
         return _ImageFn.apply(p, self, _view_code(view), R)
@@ -616,7 +624,7 @@ class TorchDiffFVREngine(nn.Module):
         hp = RT.hp_filter(H, W, cutoff_sigma, pred.device) if high_pass else None
         native = NA.module()
         if (native is not None and pred.numel() > 0 and tuple(target_drr.shape[-2:]) == (H, W)
-                and not pred.is_complex() and not target_drr.is_complex() and L.query("fvr_image_supported", H, W)):
+                and not pred.is_complex() and not target_drr.is_complex() and _whole_images(H, W)):
             return NA.call(native.image_ncc, 2, pred, target_drr, hp, RT.twiddles(H, L.F32_, pred.device),
                            RT.twiddles(W, L.F32_, pred.device))
         return _ImageSpectralNCCFn.apply(pred, target_drr, hp)
