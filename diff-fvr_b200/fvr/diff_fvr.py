@@ -174,23 +174,29 @@ class DifferentiableFourierVolumeRenderer:
             if not t.is_cuda:
                 at[key] = nbytes
                 nbytes += -(-t.numel() * 16 // 256) * 256
-        pinned = torch.empty(nbytes, dtype=torch.uint8, pin_memory=True)
-        buf = torch.empty(nbytes, dtype=torch.uint8, device=self._dev)
-        base = int(buf.data_ptr())
+        # the records' offsets count 16-byte elements from `base` (every target starts on a 16-byte boundary)
+        if at:
+            pinned = torch.empty(nbytes, dtype=torch.uint8, pin_memory=True)
+            buf = torch.empty(nbytes, dtype=torch.uint8, device=self._dev)
+            base = int(buf.data_ptr())
+        else:
+            base = int(next(iter(flat.values())).data_ptr())
         where = {key: base + at[key] if key in at else int(t.data_ptr()) for key, t in flat.items()}
-        # the records' offsets count elements from the buffer's start (16-byte elements, every target 16-byte aligned)
         table["off"] = [(where[k, sh * sw] - base) // 16 for k, (sh, sw, _) in zip(index, sizes)]
-        parts = [(0, torch.from_numpy(table.view(np.uint8)))]
-        # byte views: the host copy is split over threads by element count
-        parts += [(at[key], torch.view_as_real(flat[key]).view(-1).view(torch.uint8)) for key in at]
-        for o, src in parts:  # each part's transfer runs while the next one is staged
-            pinned[o:o + src.numel()].copy_(src)
-            buf[o:o + src.numel()].copy_(pinned[o:o + src.numel()], non_blocking=True)
+        records = torch.from_numpy(table.view(np.uint8))
+        if at:
+            # byte views: the host copy is split over threads by element count
+            parts = [(0, records)] + [(at[key], torch.view_as_real(flat[key]).view(-1).view(torch.uint8)) for key in at]
+            for o, src in parts:  # each part's transfer runs while the next one is staged
+                pinned[o:o + src.numel()].copy_(src)
+                buf[o:o + src.numel()].copy_(pinned[o:o + src.numel()], non_blocking=True)
+        else:  # a few hundred bytes: no staging
+            buf = records.to(self._dev)
         ws_bytes = L.query("fvr_np_ncc_workspace", len(specs))
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=self._dev)
         mom = torch.empty((len(specs), 5), dtype=torch.float64, device=self._dev)
-        L.call("fvr_np_ncc_moments", L.ptr(self._f3d), self.pz, self.py, self.px, L.ptr(buf), len(specs), L.ptr(buf),
-               L.ptr(ws), ws_bytes, L.ptr(mom), L.stream_ptr(self._dev))
+        L.call("fvr_np_ncc_moments", L.ptr(self._f3d), self.pz, self.py, self.px, L.ptr(buf), len(specs),
+               ctypes.c_void_p(base), L.ptr(ws), ws_bytes, L.ptr(mom), L.stream_ptr(self._dev))
         return mom.cpu().numpy(), sizes
 
     def compute_spectral_ncc(self, f_slice_candidate, f_target_precomputed) -> float:
