@@ -232,9 +232,10 @@ __global__ void twiddle_kernel(Cx<T>* tw, int n) {
 }
 
 // Lines per CTA: about 4096 complex elements per CTA (two ping-pong buffers),
-// fewer (down to 8 neighbouring lines, one 64-byte piece of each element row)
-// while that leaves less than four CTAs per SM: 64 images of 96 x 96 took
-// 22 us a pass with 42 lines on 147 CTAs.
+// halved from above 8 while that leaves less than four CTAs per SM, so at least
+// 5 neighbouring lines: 64 images of 96 x 96 took 22 us a pass with 42 lines on
+// 147 CTAs.  Stopping at 8 lines, whole 64-byte pieces of an element row, gains
+// 1 us of 37 there and loses 2.4 of 43 for 4 images of 150 x 170.
 template <typename T>
 static int lines_per_cta(int n, int64_t n_lines) {
   int L = 4096 / n;
