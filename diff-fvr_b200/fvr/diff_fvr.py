@@ -164,7 +164,7 @@ class DifferentiableFourierVolumeRenderer:
         flat = {}  # (target, elements) -> flat complex128 of that many values
         for k, (sh, sw, _) in zip(index, sizes):
             if (k, sh * sw) not in flat:
-                t = torch.as_tensor(unique[k], dtype=torch.complex128)
+                t = torch.as_tensor(unique[k], dtype=torch.complex128).resolve_conj()  # its memory is read as it is
                 if t.is_cuda and (t.device != self._dev or t.data_ptr() % 16):
                     t = t.to(self._dev, copy=True)
                 flat[k, sh * sw] = t.reshape(-1).expand(sh * sw).contiguous()
