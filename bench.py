@@ -701,6 +701,13 @@ def _sncc_step_roofline(storage, C, R, ms):
             "fallback 6.65 TB/s", "timing": "whole step (graph replay)"}
 
 
+_REFERENCE_ROOT = REPO / "baseline" / "_ref" / "fvr"
+
+
+def _reference_installed():
+    return (_REFERENCE_ROOT / "torch_engine.py").exists()
+
+
 def _reference_modules():
     """The unmodified reference package installed in baseline/_ref, imported
     under the package name ``fvr_reference`` (its modules import one another
@@ -710,9 +717,9 @@ def _reference_modules():
     import importlib
     import types
 
-    root = REPO / "baseline" / "_ref" / "fvr"
-    if not (root / "torch_engine.py").exists():
+    if not _reference_installed():
         return None
+    root = _REFERENCE_ROOT
     if "fvr_reference" not in sys.modules:
         pkg = types.ModuleType("fvr_reference")
         pkg.__path__ = [str(root)]
@@ -1009,12 +1016,15 @@ def _cpu_baseline_leg(vol, poses_np, f_ap, f_lat, results):
 
 
 def run_reference(args):
-    """The reference's CPU path for this workload: the float64 C/OpenMP oracle
-    restatement of TorchDiffFVREngine.forward_spectral_ncc + backward (the
-    reference is Python/PyTorch and does not travel), timed on all host cores."""
+    """The reference's CPU path for this workload, where the reference is
+    installed: the float64 C/OpenMP oracle restatement of
+    TorchDiffFVREngine.forward_spectral_ncc + backward and, beside it, the
+    reference's own PyTorch-CPU implementation, timed on all host cores."""
     ws, rank, _ = _dist()
     if rank != 0:
         return None
+    if not _reference_installed():  # a port alone is no reference arm
+        return {"impl": "reference", "unavailable": "the reference is not installed in baseline/_ref"}
     from fvr import synthetic
     from oracle import c_oracle
     from oracle import torch_convention as tc
