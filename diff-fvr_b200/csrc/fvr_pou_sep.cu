@@ -8,8 +8,8 @@
 // the two transposed ones in the other order.  The kernels march down the
 // detector rows: forward, the position arithmetic (fp64), a column's two image
 // loads and its x interpolation are paid once per image row instead of once per
-// pixel; the adjoint reduces the pixels to four moments per image cell, which is
-// all that the image gradient and the pose offsets need of them.
+// pixel; the adjoint reduces the pixels to four weighted sums per image cell,
+// which is all that the image gradient and the pose offsets need of them.
 #include <type_traits>
 
 #include "fvr_common.cuh"
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(256) pou_warp_sep_weigh_kernel(const float* __
 // Every element of dL/dimgs is written once (nothing to clear, no atomics).
 // The sums of g rx dv/dpx and g ry dv/dpy come from rx = (x + tx - ox) / scale
 // and ry alike, in f32 relative to the integer next to ox, oy.
-// Bound by issue.  64 blocks x 64 poses x 256^2 pixels: 437 us, against 495
+// Bound by issue.  64 blocks x 64 poses x 256^2 pixels: 444 us, against 495
 // with bands marched by one warp each and the image's values and differences
 // interpolated at every detector column (two loads and nine operations per
 // image row and detector column); 8 blocks x 64 poses x 512^2 pixels: 138

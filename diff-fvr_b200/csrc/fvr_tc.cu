@@ -428,8 +428,8 @@ __global__ void __launch_bounds__(kSnccThreads, MINB) tc_sncc_moments_kernel(Snc
 // Value-and-gradient epilogue, launched right after the moments kernel as its
 // programmatic dependent (CTAs of 512 threads).  The work goes in chunks
 // of candidates whose (view, candidate) items fit in shared memory, one CTA per
-// chunk (256 candidates x 2 views, 512^3 spectrum: the step takes 219 us, and
-// 227 us with one CTA serial over the chunks).
+// chunk (256 candidates x 2 views, 512^3 spectrum: the step takes 216 us, and
+// 226 us with one CTA serial over the chunks).
 // A single chunk also reduces the losses; several leave that to a small
 // dependent kernel that reads every candidate's ncc:
 //  0. the slice-axes Jacobians of the chunk's items, formed while the moments

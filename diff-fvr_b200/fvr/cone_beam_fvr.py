@@ -87,7 +87,7 @@ def sample_isocenter_parity_offsets(vox_spacing) -> torch.Tensor:
 
 
 class _EdgeNCCFn(torch.autograd.Function):
-    """Edge-dominant gradient NCC on ``libfvr_b200.so``: one tiled Sobel +
+    """Edge-dominant gradient NCC on ``libfvr_b200.so``: one marching Sobel +
     moment pass and a finalize forward; backward applies the transposed Sobel
     and box filters to the closed-form NCC gradient fields."""
 
