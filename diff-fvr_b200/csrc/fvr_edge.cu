@@ -13,7 +13,7 @@
 // applies the transposed Sobel and box filters to closed-form fields.
 //
 // Both passes march: a warp owns a strip of 64 columns (two per lane, the
-// outer lanes are halo) and walks down kEdgeRows rows, keeping the last rows'
+// outer lanes are halo) and walks down 8 to 32 rows, keeping the last rows'
 // horizontal sums in registers; horizontal neighbours come from the lane's
 // other column or one shuffle.  The pair (a, b) goes through the filters as
 // one packed f32x2 value.  No shared memory and no barriers.  Measured on 64
@@ -29,7 +29,6 @@
 
 namespace fvr {
 
-constexpr int kEdgeRows = 32;     // rows a CTA (one warp) produces
 constexpr int kEdgeMom = 5;       // S_u, S_v, S_uu, S_vv, S_uv
 constexpr int kEdgeCombos = 4;    // fine x, fine y, coarse x, coarse y
 constexpr int kEdgeStats = kEdgeCombos * kEdgeMom;     // moments kept for the backward of the edge NCC
@@ -46,6 +45,7 @@ struct EdgeArgs {
   int views, B, Cch, H, W, crop;
   int coarse;        // 1: blurred scale enabled
   int nm;            // moments per pair in stats: kEdgeStats or kEdgeNM
+  int rows;          // rows a CTA (one warp) produces
   int vec;           // 1: every row starts on an 8-byte boundary
   double base, ce, cn;  // out = base + sum over views (ce edge + cn ncc)
   float w;           // weight of the blurred scale
@@ -70,8 +70,8 @@ __device__ __forceinline__ EdgeJob edge_job(const EdgeArgs& e, int64_t pair, int
   j.b = e.b[j.view] + (static_cast<int64_t>(e.Bt[j.view] == 1 ? 0 : j.bi) * e.Cch + j.ch) * plane;
   const int chunk = job / strips;
   j.strip = job - chunk * strips;
-  j.rb = chunk * kEdgeRows;
-  j.re = min(e.H, j.rb + kEdgeRows);
+  j.rb = chunk * e.rows;
+  j.re = min(e.H, j.rb + e.rows);
   return j;
 }
 
@@ -350,13 +350,15 @@ __device__ __forceinline__ double edge_ncc(const double* m, double n) {
   return suv / sqrt(fmax(suu * svv, 1e-12));
 }
 
-// One CTA per batch item: strip sums -> stats[pair][nm] in job order,
+// One CTA of NW warps per batch item: strip sums -> stats[pair][nm] in a fixed order,
 // then out = base + sum over views (ce edge + cn ncc), edge = the channel mean
 // of (1 - w) fine + w coarse.
-__global__ void __launch_bounds__(128) edge_finalize_kernel(EdgeArgs e, int jobs, const double* __restrict__ partial,
-                                                            double* __restrict__ stats, float* __restrict__ out,
-                                                            double* __restrict__ value) {
-  __shared__ double part[4][kEdgeNM];
+template <int NW>
+__global__ void __launch_bounds__(32 * NW) edge_finalize_kernel(EdgeArgs e, int jobs,
+                                                               const double* __restrict__ partial,
+                                                               double* __restrict__ stats, float* __restrict__ out,
+                                                               double* __restrict__ value) {
+  __shared__ double part[NW][kEdgeNM];
   const int bi = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const double n = static_cast<double>(e.H - 2 * e.crop) * static_cast<double>(e.W - 2 * e.crop);
   const double n_img = static_cast<double>(e.H) * static_cast<double>(e.W);
@@ -367,12 +369,15 @@ __global__ void __launch_bounds__(128) edge_finalize_kernel(EdgeArgs e, int jobs
       const int64_t pair = (static_cast<int64_t>(v) * e.B + bi) * e.Cch + ch;
       if (lane < kEdgeNM) {
         double s = 0.0;
-        for (int t = wid; t < jobs; t += 4) s += partial[(pair * jobs + t) * kEdgeNM + lane];
+#pragma unroll 8
+        for (int t = wid; t < jobs; t += NW) s += partial[(pair * jobs + t) * kEdgeNM + lane];
         part[wid][lane] = s;
       }
       __syncthreads();
       if (threadIdx.x < kEdgeNM) {
-        const double s = ((part[0][lane] + part[1][lane]) + part[2][lane]) + part[3][lane];
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < NW; ++k) s += part[k][lane];
         part[0][lane] = s;
         if (lane < e.nm) stats[pair * e.nm + lane] = s;
       }
@@ -602,25 +607,60 @@ static int edge_view(EdgeArgs* e, int v, const float* a, const float* b, int64_t
   return FVR_OK;
 }
 
-static int64_t edge_jobs(int64_t H, int64_t W, int cols) { return cdiv64(H, kEdgeRows) * cdiv64(W, cols); }
+static int64_t edge_jobs(int64_t H, int64_t W, int rows, int cols) { return cdiv64(H, rows) * cdiv64(W, cols); }
+
+// Rows per warp.  A warp's time is its rows and about six more (halo, prologue,
+// sums) whether it is alone on an SM or one of the twelve that fit, so the
+// moments take the rows with the shortest waves x (rows + 6), a smaller count
+// only for a tenth less of it.  8 / 12 / 16 / 24 / 32 rows, us: one 256^2 image
+// 5.8 / 7.1 / 8.4 / 11.0 / 13.7, 16 images 12.8 / 9.5 / 11.2 / 13.1 / 16.1, 64
+// images 36 / 33 / 30 / 29 / 33, 64 x two views with the image NCC 77 / 68 / 63 /
+// 59 / 57.
+constexpr int kMomSlots = 148 * 12, kGradSlots = 148 * 16;
+static int edge_mom_rows(int64_t pairs, int64_t H, int64_t W) {
+  int best = 32;
+  int64_t cost = 0;
+  for (int rows : {32, 24, 16, 12, 8}) {
+    const int64_t c = cdiv64(pairs * edge_jobs(H, W, rows, kMomCols), kMomSlots) * (rows + 6);
+    if (cost == 0 || 10 * c < 9 * cost) {
+      best = rows;
+      cost = c;
+    }
+  }
+  return best;
+}
+
+// The adjoint has eight halo rows and sixteen warps an SM: the fewest rows whose
+// warps are on the GPU together, else 32, which issue least.  One 256^2 image
+// 9.8 / 11.4 / 12.3 / 15.2 / 18.0, 16 images 21 / 15 / 17 / 18 / 21, 64 images
+// 58 / 47 / 44 / 41 / 42, 64 x two views with the image NCC 100 / 85 / 76 / 67 / 67.
+static int edge_grad_rows(int64_t pairs, int64_t H, int64_t W) {
+  for (int rows : {8, 12, 16, 24})
+    if (pairs * edge_jobs(H, W, rows, kGradCols) <= kGradSlots) return rows;
+  return 32;
+}
 
 // Strip records, then one fp64 value per item (for the batch mean).
 static int64_t edge_ws_bytes(int64_t views, int64_t B, int64_t C, int64_t H, int64_t W) {
-  return (views * B * C * edge_jobs(H, W, kMomCols) * kEdgeNM + B) * (int64_t)sizeof(double);
+  const int64_t pairs = views * B * C;
+  return (pairs * edge_jobs(H, W, edge_mom_rows(pairs, H, W), kMomCols) * kEdgeNM + B) * (int64_t)sizeof(double);
 }
+
+static int64_t edge_pairs(const EdgeArgs& e) { return static_cast<int64_t>(e.views) * e.B * e.Cch; }
 
 template <typename K>
 static int edge_grid(const EdgeArgs& e, int cols, K launch) {
-  const int64_t jobs = edge_jobs(e.H, e.W, cols);
-  const int64_t n = static_cast<int64_t>(e.views) * e.B * e.Cch * jobs;
+  const int64_t jobs = edge_jobs(e.H, e.W, e.rows, cols);
+  const int64_t n = edge_pairs(e) * jobs;
   if (n > 2147483647) return FVR_ERR_ARG;
   launch(static_cast<unsigned>(n), static_cast<int>(cdiv64(e.W, cols)), static_cast<int>(jobs));
   FVR_LAUNCH_CHECK();
   return FVR_OK;
 }
 
-static int edge_forward(const EdgeArgs& e, void* workspace, double* stats, float* out, bool mean, cudaStream_t s) {
+static int edge_forward(EdgeArgs e, void* workspace, double* stats, float* out, bool mean, cudaStream_t s) {
   double* part = static_cast<double*>(workspace);
+  e.rows = edge_mom_rows(edge_pairs(e), e.H, e.W);
   const int rc = edge_grid(e, kMomCols, [&](unsigned n, int strips, int jobs) {
     if (e.coarse && e.cn != 0.0) edge_moments_kernel<true, true><<<n, 32, 0, s>>>(e, strips, jobs, part);
     else if (e.coarse) edge_moments_kernel<true, false><<<n, 32, 0, s>>>(e, strips, jobs, part);
@@ -628,10 +668,12 @@ static int edge_forward(const EdgeArgs& e, void* workspace, double* stats, float
     else edge_moments_kernel<false, false><<<n, 32, 0, s>>>(e, strips, jobs, part);
   });
   if (rc) return rc;
-  const int jobs = (int)edge_jobs(e.H, e.W, kMomCols);
-  double* value = part + static_cast<int64_t>(e.views) * e.B * e.Cch * jobs * kEdgeNM;
-  edge_finalize_kernel<<<static_cast<unsigned>(e.B), 128, 0, s>>>(e, jobs, part, stats, mean ? nullptr : out,
-                                                                  mean ? value : nullptr);
+  const int jobs = (int)edge_jobs(e.H, e.W, e.rows, kMomCols);
+  double* value = part + edge_pairs(e) * jobs * kEdgeNM;
+  if (e.B == 1) mean = false;  // of one item
+  const auto finalize = jobs > 32 ? edge_finalize_kernel<16> : edge_finalize_kernel<4>;
+  finalize<<<static_cast<unsigned>(e.B), jobs > 32 ? 512 : 128, 0, s>>>(e, jobs, part, stats, mean ? nullptr : out,
+                                                                        mean ? value : nullptr);
   FVR_LAUNCH_CHECK();
   if (mean) {
     edge_mean_kernel<<<1, 32, 0, s>>>(value, e.B, out);
@@ -640,8 +682,9 @@ static int edge_forward(const EdgeArgs& e, void* workspace, double* stats, float
   return FVR_OK;
 }
 
-static int edge_backward(const EdgeArgs& e, const double* stats, const float* g, int64_t g_stride, double g_scale,
-                         int swap, cudaStream_t s) {
+static int edge_backward(EdgeArgs e, const double* stats, const float* g, int64_t g_stride, double g_scale, int swap,
+                         cudaStream_t s) {
+  e.rows = edge_grad_rows(edge_pairs(e), e.H, e.W);
   return edge_grid(e, kGradCols, [&](unsigned n, int strips, int jobs) {
     if (e.coarse && e.cn != 0.0)
       edge_grad_kernel<true, true><<<n, 32, 0, s>>>(e, strips, jobs, stats, g, g_stride, g_scale, swap);
