@@ -231,24 +231,32 @@ __global__ void twiddle_kernel(Cx<T>* tw, int n) {
   tw[m] = Cx<T>{static_cast<T>(c), static_cast<T>(-s)};
 }
 
+template <typename T>
+static size_t smem_bytes(int n, int L) {
+  return 2 * static_cast<size_t>(L) * (n + 1) * sizeof(Cx<T>);
+}
+
 // Lines per CTA: about 4096 complex elements per CTA (two ping-pong buffers),
-// halved from above 8 while that leaves less than four CTAs per SM, so at least
-// 5 neighbouring lines: 64 images of 96 x 96 took 22 us a pass with 42 lines on
-// 147 CTAs.  Stopping at 8 lines, whole 64-byte pieces of an element row, gains
-// 1 us of 37 there and loses 2.4 of 43 for 4 images of 150 x 170.
+// halved from above 8 (so at least 5 neighbouring lines) while that leaves less
+// than 2.25 CTAs per SM, or a second wave that is mostly empty.  Both passes of
+// a batch, us, unhalved / halved while under four CTAs per SM / by this rule: 64
+// images of 96 x 96 45 / 38 / 33, 128 of 128 x 128 (512 CTAs on 444 slots) 101 /
+// 78 / 78, but 512 of 50 x 50 (400 CTAs on 592) 49 / 53 / 49 and 32 of 150 x 170
+// 93 / 102 / 73.  Stopping at 8 lines, whole 64-byte pieces of an element row,
+// gains 1 us of 37 for the first and loses 2.4 of 43 for 4 images of 150 x 170.
 template <typename T>
 static int lines_per_cta(int n, int64_t n_lines) {
   int L = 4096 / n;
   if (L < 1) L = 1;
   if (L > 64) L = 64;
-  while (L > 8 && cdiv64(n_lines, L) < 592) L = (L + 1) / 2;
+  while (L > 8) {
+    const int64_t ctas = cdiv64(n_lines, L), fit = 227 * 1024 / static_cast<int64_t>(smem_bytes<T>(n, L) + 1024);
+    const int64_t slots = 148 * (fit < 8 ? fit : 8);
+    if (ctas >= 333 && (ctas <= slots || ctas >= 592)) break;
+    L = (L + 1) / 2;
+  }
   if (L > n_lines) L = static_cast<int>(n_lines);
   return L;
-}
-
-template <typename T>
-static size_t smem_bytes(int n, int L) {
-  return 2 * static_cast<size_t>(L) * (n + 1) * sizeof(Cx<T>);
 }
 
 template <typename T, class LD, class ST>
