@@ -435,9 +435,10 @@ __global__ void __launch_bounds__(kSnccThreads, MINB) tc_sncc_moments_kernel(Snc
 //  0. the slice-axes Jacobians of the chunk's items, formed while the moments
 //     kernel still runs (its CTAs release this launch once whatever wrote the
 //     poses has completed; read at L2, where that is visible);
-//  1. after griddepcontrol.wait, one thread per (item, moment): the item's
-//     records summed in record order, every load of a thread issued in one
-//     round, kept in shared memory;
+//  1. after griddepcontrol.wait, one thread per (item, moment), or several where
+//     items are few: the item's records summed in a fixed order, every load of a
+//     thread issued in one round, kept in shared memory (one thread to the 64
+//     records of one item: 16.1 us for a 128^2 step, 7.4 shared);
 //  2. one thread per item: its ncc and its per-view part of the pose gradient
 //     (per axis gc (a A + 2 b B) through the Jacobian, translations from the
 //     phase moments);
@@ -447,6 +448,8 @@ constexpr int kFinalThreads = 512;
 constexpr int kFinalChunkItems = 128;  // 128 items x 44 doubles = 44 KB of shared memory
 constexpr int kFinalPairs = (kFinalChunkItems * M_NGRAD + kFinalThreads - 1) / kFinalThreads;  // per thread
 constexpr int kFinalRecords = 4;  // records per (item, moment) per load round
+constexpr int kFinalShares = 16;  // threads that share an (item, moment)'s records, while items are few
+static_assert(kFinalThreads <= kFinalChunkItems * 6, "the shares' sums lie where the items' gradients come");
 
 // loss[v] = 1 - mean_c ncc from per-thread ncc sums (fixed order: per thread,
 // per warp, across warps), loss[nv] their sum.
@@ -500,41 +503,67 @@ __global__ void __launch_bounds__(kFinalThreads) tc_sncc_final_kernel(SnccArgs a
     }
     if (gridDim.x > 1) pdl_launch_dependents();  // the loss kernel
     pdl_wait();  // the moments kernel has completed and its records are visible
-    // record sums: the thread's pairs p = t + k * 512, all their loads in one round
-    const double* src[kFinalPairs];
+    const int np = ni * M_NGRAD, shares = min(min(kFinalThreads / np, tiles), kFinalShares);
+    // the moment record of pair p = (item, moment): consecutive threads, consecutive doubles
+    auto keep = [&](int p, double x) {
+      const int li = p / M_NGRAD, m = p - li * M_NGRAD, v = li / cn;
+      s_mom[li][m] = x;
+      a.mom[(static_cast<int64_t>(v) * C + c0 + (li - v * cn)) * kMomStride + m] = x;
+    };
+    auto records = [&](int p) {
+      const int li = p / M_NGRAD, m = p - li * M_NGRAD, v = li / cn;
+      return a.partial + (static_cast<int64_t>(v) * C + c0 + (li - v * cn)) * tiles * M_NGRAD + m;
+    };
+    if (shares > 1) {  // few items of many records: several threads to a pair, their sums added in order
+      double* part = &s_part[0][0];
+      const int sh = t / np, p = t - sh * np;
+      if (sh < shares) {
+        const double* src = records(p);
+        double x[kFinalRecords], sum = 0.0;
+        for (int r0 = sh; r0 < tiles; r0 += kFinalRecords * shares) {
 #pragma unroll
-    for (int k = 0; k < kFinalPairs; ++k) {
-      const int p = t + k * kFinalThreads;
-      src[k] = nullptr;
-      if (p < ni * M_NGRAD) {
-        const int li = p / M_NGRAD, m = p - li * M_NGRAD, v = li / cn;
-        const int64_t it = static_cast<int64_t>(v) * C + c0 + (li - v * cn);
-        src[k] = a.partial + it * tiles * M_NGRAD + m;
+          for (int k = 0; k < kFinalRecords; ++k) {
+            const int r = r0 + k * shares;
+            x[k] = r < tiles ? __ldcg(src + static_cast<int64_t>(r) * M_NGRAD) : 0.0;
+          }
+#pragma unroll
+          for (int k = 0; k < kFinalRecords; ++k) sum += x[k];
+        }
+        part[t] = sum;
       }
-    }
-    double sum[kFinalPairs];
+      __syncthreads();
+      if (t < np) {
+        double sum = 0.0;
+        for (int k = 0; k < shares; ++k) sum += part[k * np + t];
+        keep(t, sum);
+      }
+    } else {
+      // the thread's pairs p = t + k * 512, all their loads in one round
+      const double* src[kFinalPairs];
 #pragma unroll
-    for (int k = 0; k < kFinalPairs; ++k) sum[k] = 0.0;
-    for (int r0 = 0; r0 < tiles; r0 += kFinalRecords) {
-      double x[kFinalPairs][kFinalRecords];
+      for (int k = 0; k < kFinalPairs; ++k) {
+        const int p = t + k * kFinalThreads;
+        src[k] = p < np ? records(p) : nullptr;
+      }
+      double sum[kFinalPairs];
 #pragma unroll
-      for (int k = 0; k < kFinalPairs; ++k)
+      for (int k = 0; k < kFinalPairs; ++k) sum[k] = 0.0;
+      for (int r0 = 0; r0 < tiles; r0 += kFinalRecords) {
+        double x[kFinalPairs][kFinalRecords];
 #pragma unroll
-        for (int r = 0; r < kFinalRecords; ++r)
-          x[k][r] = src[k] && r0 + r < tiles ? __ldcg(src[k] + static_cast<int64_t>(r0 + r) * M_NGRAD) : 0.0;
+        for (int k = 0; k < kFinalPairs; ++k)
 #pragma unroll
-      for (int k = 0; k < kFinalPairs; ++k)
+          for (int r = 0; r < kFinalRecords; ++r)
+            x[k][r] = src[k] && r0 + r < tiles ? __ldcg(src[k] + static_cast<int64_t>(r0 + r) * M_NGRAD) : 0.0;
 #pragma unroll
-        for (int r = 0; r < kFinalRecords; ++r) sum[k] += x[k][r];
-    }
+        for (int k = 0; k < kFinalPairs; ++k)
 #pragma unroll
-    for (int k = 0; k < kFinalPairs; ++k) {
-      const int p = t + k * kFinalThreads;
-      if (p < ni * M_NGRAD) {
-        const int li = p / M_NGRAD, m = p - li * M_NGRAD, v = li / cn;
-        s_mom[li][m] = sum[k];
-        // the moment record (consecutive threads, consecutive doubles)
-        a.mom[(static_cast<int64_t>(v) * C + c0 + (li - v * cn)) * kMomStride + m] = sum[k];
+          for (int r = 0; r < kFinalRecords; ++r) sum[k] += x[k][r];
+      }
+#pragma unroll
+      for (int k = 0; k < kFinalPairs; ++k) {
+        const int p = t + k * kFinalThreads;
+        if (p < np) keep(p, sum[k]);
       }
     }
     __syncthreads();
