@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(kFinalThreads) tc_sncc_final_kernel(SnccArgs a
     }
     if (gridDim.x > 1) pdl_launch_dependents();  // the loss kernel
     pdl_wait();  // the moments kernel has completed and its records are visible
-    const int np = ni * M_NGRAD, shares = min(min(kFinalThreads / np, tiles), kFinalShares);
+    const int np = ni * M_NGRAD, shares = max(1, min(min(kFinalThreads / np, tiles), kFinalShares));
     // the moment record of pair p = (item, moment): consecutive threads, consecutive doubles
     auto keep = [&](int p, double x) {
       const int li = p / M_NGRAD, m = p - li * M_NGRAD, v = li / cn;
@@ -514,20 +514,21 @@ __global__ void __launch_bounds__(kFinalThreads) tc_sncc_final_kernel(SnccArgs a
       const int li = p / M_NGRAD, m = p - li * M_NGRAD, v = li / cn;
       return a.partial + (static_cast<int64_t>(v) * C + c0 + (li - v * cn)) * tiles * M_NGRAD + m;
     };
-    if (shares > 1) {  // few items of many records: several threads to a pair, their sums added in order
+    if (np <= kFinalThreads) {  // few items of many records: several threads to a pair, their sums added in order
       double* part = &s_part[0][0];
       const int sh = t / np, p = t - sh * np;
       if (sh < shares) {
         const double* src = records(p);
-        double x[kFinalRecords], sum = 0.0;
-        for (int r0 = sh; r0 < tiles; r0 += kFinalRecords * shares) {
+        constexpr int kRound = 2 * kFinalRecords;  // one pair a thread: twice the records in flight
+        double x[kRound], sum = 0.0;
+        for (int r0 = sh; r0 < tiles; r0 += kRound * shares) {
 #pragma unroll
-          for (int k = 0; k < kFinalRecords; ++k) {
+          for (int k = 0; k < kRound; ++k) {
             const int r = r0 + k * shares;
             x[k] = r < tiles ? __ldcg(src + static_cast<int64_t>(r) * M_NGRAD) : 0.0;
           }
 #pragma unroll
-          for (int k = 0; k < kFinalRecords; ++k) sum += x[k];
+          for (int k = 0; k < kRound; ++k) sum += x[k];
         }
         part[t] = sum;
       }
@@ -659,7 +660,11 @@ static void launch_sncc_final(cudaStream_t s, const SnccArgs& a) {
 }
 
 // Record sums (fp64, fixed order) -> mom[v][c][0..NM), ncc in mom[v][c][17];
-// loss[v] = 1 - mean_c ncc, loss[nv] = sum_v loss[v].  One CTA, warp per (v, c).
+// loss[v] = 1 - mean_c ncc, loss[nv] = sum_v loss[v].  One CTA, warp per (v, c);
+// from 24 records on as many lanes to a moment as the warp has (three moments
+// without the gradient: ten lanes each; one pose at 128^2 has 64 records: 10.6 us
+// with the moments kernel by one lane, 7.6 by ten; the ten's exchange costs 8 of
+// 41 us at 512 candidates of 2 records).
 __global__ void __launch_bounds__(1024) tc_sncc_finalize_kernel(const double* __restrict__ partial, int C, int nv,
                                                                 int tiles, int NM, double* __restrict__ mom,
                                                                 float* __restrict__ loss,
@@ -667,12 +672,21 @@ __global__ void __launch_bounds__(1024) tc_sncc_finalize_kernel(const double* __
   __shared__ double red[32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   pdl_wait();  // launched as a programmatic dependent of the moments kernel
+  const int shares = 32 / NM, share = lane / NM;
   for (int item = w; item < nv * C; item += nw) {
+    const double* rec = partial + static_cast<int64_t>(item) * tiles * NM;
     double s = 0.0;
-    if (lane < NM) {
-      for (int t = 0; t < tiles; ++t) s += partial[(static_cast<int64_t>(item) * tiles + t) * NM + lane];
-      mom[static_cast<int64_t>(item) * kMomStride + lane] = s;
+    if (tiles < 24) {
+      if (lane < NM)
+        for (int t = 0; t < tiles; ++t) s += rec[t * NM + lane];
+    } else {
+      double part = 0.0;
+      if (share < shares)
+#pragma unroll 4
+        for (int t = share; t < tiles; t += shares) part += rec[t * NM + (lane - share * NM)];
+      for (int k = 0; k < shares; ++k) s += __shfl_sync(0xffffffffu, part, (k * NM + lane) & 31);
     }
+    if (lane < NM) mom[static_cast<int64_t>(item) * kMomStride + lane] = s;
     const double cross = __shfl_sync(0xffffffffu, s, 0), ep = __shfl_sync(0xffffffffu, s, 1),
                  et = __shfl_sync(0xffffffffu, s, 2);
     if (lane == 0) {
